@@ -171,6 +171,33 @@ void fill_common(PrepArgs& args, const hc_attn_params* p) {
     args.table_positions = p->rope ? p->rope->positions : 0;
 }
 
+// The tcgen05 decode kernel norms, rotates and rounds queries (and a token's own k and v) itself, with 8- and
+// 16-byte loads: buffers off a 16-byte boundary go through the general prologue kernel instead.
+bool decode_takes_raw(const hc_attn_params* p, const void* q, const void* k, const void* v) {
+    uintptr_t bits = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v);
+    if (p->norm_q == 1) bits |= reinterpret_cast<uintptr_t>(p->q_norm_weight);
+    if (k && p->norm_k == 1) bits |= reinterpret_cast<uintptr_t>(p->k_norm_weight);
+    return (bits & 15) == 0;
+}
+DecodeSource raw_source(const hc_attn_params* p, const void* q, const void* k, const void* v) {
+    DecodeSource src{};
+    src.q = q;
+    src.k = k;
+    src.v = v;
+    src.dtype = p->io_dtype;
+    src.q_head_stride = p->head_dim * (p->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1);
+    src.norm_q = p->norm_q;
+    src.norm_k = p->norm_k;
+    src.norm_v = p->norm_v;
+    src.q_weight = static_cast<const uint16_t*>(p->q_norm_weight);
+    src.k_weight = static_cast<const uint16_t*>(p->k_norm_weight);
+    src.eps = p->norm_eps;
+    src.cos = p->rope ? p->rope->cos : nullptr;
+    src.sin = p->rope ? p->rope->sin : nullptr;
+    src.table_positions = p->rope ? p->rope->positions : 0;
+    return src;
+}
+
 const unsigned char* offset_rows(const void* base, size_t rows, size_t row_elems, int dtype) {
     return static_cast<const unsigned char*>(base) + rows * row_elems * dtype_bytes(dtype);
 }
@@ -366,19 +393,28 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
         }
         const unsigned char* q_rows = offset_rows(q, size_t(start), size_t(p->q_heads) * d * mult, p->io_dtype);
         const uint16_t* q_bf16 = reinterpret_cast<const uint16_t*>(q_rows);
-        if (prep || k_fused) {
+        const size_t kv_row = size_t(p->kv_heads) * d;
+        const void* k_rows = k_fused ? offset_rows(k_fused, size_t(start), kv_row, p->io_dtype) : nullptr;
+        const void* v_rows = k_fused ? offset_rows(v_fused, size_t(start), kv_row, p->io_dtype) : nullptr;
+        if (k_fused) {
+            for (int b = 0; b < count; ++b) {
+                st = ensure_pages(cache, L, meta.seq[b], meta.pos[b], 1, stream);
+                if (st != HC_OK) return st;
+            }
+        }
+        DecodeSource src{};
+        src.dtype = HC_BF16;
+        src.q_head_stride = d;
+        const bool in_kernel = tensor && decode_takes_raw(p, q_rows, k_rows, v_rows);
+        if (in_kernel) {
+            src = raw_source(p, q_rows, k_rows, v_rows);
+        } else if (prep || k_fused) {
             PrepArgs args{};
             fill_common(args, p);
             int jobs = 0;
             if (prep) fill_q_job(args.job[jobs++], p, q_rows, cache->ws.qprep);
             if (k_fused) {
-                for (int b = 0; b < count; ++b) {
-                    st = ensure_pages(cache, L, meta.seq[b], meta.pos[b], 1, stream);
-                    if (st != HC_OK) return st;
-                }
-                const size_t kv_row = size_t(p->kv_heads) * d;
-                fill_kv_jobs(args, jobs, p, offset_rows(k_fused, size_t(start), kv_row, p->io_dtype),
-                             offset_rows(v_fused, size_t(start), kv_row, p->io_dtype));
+                fill_kv_jobs(args, jobs, p, k_rows, v_rows);
                 jobs += 2;
             }
             args.n_jobs = jobs;
@@ -404,7 +440,8 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
         } else if (ep.gate_layout == HC_GATE_INTERLEAVED) {
             ep.gate = q_rows;
         }
-        if (tensor) st = tc_decode(ctx, shape, L, view, meta, count, q_bf16, cache->ws, ep, stream);
+        if (!in_kernel) src.q = q_bf16;
+        if (tensor) st = tc_decode(ctx, shape, L, view, meta, count, src, cache->ws, ep, stream);
         else st = simt_decode(ctx, shape, view, meta, count, q_bf16, cache->ws, ep, stream);
         if (st != HC_OK) return st;
     }
@@ -494,7 +531,8 @@ hc_status hc_context_create(int device, hc_context** out) {
     // The fixed scratch of hc_attention_decode_static: its address is looked up here, once, with this
     // device current, which also makes the runtime load that module (and reserve the array) now
     // rather than inside the first call that must not allocate.
-    const hc_status scratch = static_scratch_prepare(device, &ctx->static_scratch);
+    hc_status scratch = static_scratch_prepare(device, &ctx->static_scratch);
+    if (scratch == HC_OK) scratch = decode_cluster_slots(ctx);
     if (scratch != HC_OK) {
         const std::string message = g_last_error;
         hc_context_destroy(ctx);
@@ -652,6 +690,7 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
     cache->layers.resize(size_t(n_layers));
 
     size_t max_q_elems = 0, max_kv_elems = 0, part_o_floats = 0, part_ml_floats = 0, prefill_o_floats = 0, prefill_ml_floats = 0;
+    size_t n_tickets = 0;
     hc_status st = HC_OK;
     if (total_pages > 0) {
         cache->total_pages = total_pages;
@@ -741,7 +780,8 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         const size_t decode_slots = size_t(((decode_reach + kTileKeys - 1) / kTileKeys + world - 1) / world + 1);
         const size_t decode_rows = size_t(std::min(max_seqs, kMaxBatch)) * L.desc.q_heads;
         part_o_floats = std::max(part_o_floats, decode_rows * decode_slots * d);
-        part_ml_floats = std::max(part_ml_floats, decode_rows * decode_slots * 2);
+        part_ml_floats = std::max(part_ml_floats, decode_rows * decode_slots * 2 + 4);
+        n_tickets = std::max(n_tickets, size_t(std::min(max_seqs, kMaxBatch)) * L.desc.kv_heads * 16);
         if (few_rows) {
             const size_t prefill_slots = size_t((((reach + kTileKeys - 1) / kTileKeys) >> kLogSegmentSmall) + 2);
             const size_t prefill_rows = size_t(prefill_chunk) * L.desc.q_heads;
@@ -769,6 +809,9 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         err = cudaMalloc(&ws.qprep, 2 * ws.qprep_slot_elems * 2);
         if (err == cudaSuccess) err = cudaMalloc(&ws.part_o, part_o_floats * sizeof(float));
         if (err == cudaSuccess) err = cudaMalloc(&ws.part_ml, part_ml_floats * sizeof(float));
+        ws.n_tickets = n_tickets;
+        if (err == cudaSuccess) err = cudaMalloc(&ws.tickets, n_tickets * sizeof(unsigned));
+        if (err == cudaSuccess) err = cudaMemset(ws.tickets, 0, n_tickets * sizeof(unsigned));
         // Staging for the host-buffer entry points, two slots: q (twice as wide when the gate is
         // interleaved), gate, out, k, v.
         cache->stage_bytes = (size_t(ws.qprep_tokens) * (4 * max_q_elems + 2 * max_kv_elems) * 4 + 1023) & ~size_t(1023);
@@ -806,6 +849,7 @@ void hc_kv_cache_destroy(hc_kv_cache* cache) {
     if (cache->ws.qprep) cudaFree(cache->ws.qprep);
     if (cache->ws.part_o) cudaFree(cache->ws.part_o);
     if (cache->ws.part_ml) cudaFree(cache->ws.part_ml);
+    if (cache->ws.tickets) cudaFree(cache->ws.tickets);
     if (cache->stage_dev) cudaFree(cache->stage_dev);
     if (cache->pages_dev) cudaFree(cache->pages_dev);
     if (cache->pages_host) cudaFreeHost(cache->pages_host);

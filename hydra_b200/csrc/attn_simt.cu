@@ -815,7 +815,9 @@ hc_status launch_combine(hc_context* ctx, const float* gathered, int world, int 
 // hc_kv_cache_create would size.  Every GPU that loads the library holds these 8 MiB until the
 // process exits.
 constexpr size_t kStaticScratchFloats = size_t(2) << 20;               // 8 MiB
-static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats];
+// Behind the partials: the decode kernel's tickets.
+constexpr size_t kStaticTickets = size_t(64) << 10;
+static __device__ __align__(256) float g_static_scratch[kStaticScratchFloats + kStaticTickets];
 
 // `g_static_scratch` in host code is only a handle, not a device address: a kernel given it would
 // fault or, where the GPU can reach host memory, quietly use the wrong memory.  The device address
@@ -861,31 +863,43 @@ hc_status hc_attention_decode_static(hc_context* ctx, hc_kv_cache* cache, int la
                                         &view, &meta, &ep, &store, &tensor);
     if (st != HC_OK) return st;
     if (!ctx->static_scratch) return fail(HC_CUDA_ERROR, "this context has no static scratch address");
-    // The cut the default path would make (given this much room), and its partials: [rows][slots][2]
-    // first, then [rows][slots][d].  A whole-row cut leaves no partials; the tensor-core kernels then
-    // keep their second-fold state, if any, where the partials would be.
-    const DecodePlan plan = tensor ? tc_plan_decode(ctx, shape, view.map, meta, n_seq, kStaticScratchFloats)
-                                   : simt_plan_decode(ctx, shape, view.map, meta, n_seq);
+    // What a call may be is stated in terms of the general cut of its rows' keys into tiles and segments (as the header
+    // puts it), whichever kernels run: a caller's program is not refused by one build and served by the next.
     const size_t rows = size_t(n_seq) * shape.q_heads;
-    const size_t ml_floats = plan.finish ? 0 : (rows * plan.slots * 2 + 3) & ~size_t(3);
-    const size_t need = plan.finish ? 0 : ml_floats + rows * plan.slots * shape.head_dim;
-    if (need > kStaticScratchFloats) {
-        return fail(HC_KV_OVERFLOW, "hc_attention_decode_static: this call needs " + std::to_string(need * 4) +
+    const int target = tensor ? (shape.head_dim == 256 ? 1 : 6) * std::max(ctx->sm_count, 1) : 0;
+    const DecodePlan plan = tensor ? plan_decode(shape, view.map, meta, n_seq, target, true, 64)
+                                   : simt_plan_decode(ctx, shape, view.map, meta, n_seq);
+    size_t ml_floats = plan.finish ? 0 : (rows * plan.slots * 2 + 3) & ~size_t(3);
+    size_t o_floats = plan.finish ? 0 : rows * plan.slots * shape.head_dim;
+    TcDecodePlan tc{};
+    if (tensor) {
+        // The tensor-core kernel's own cut leaves fewer partials, if any.
+        tc = tc_plan_decode(ctx, shape, view.map, meta, n_seq);
+        ml_floats = std::max(ml_floats, tc.part_ml_floats);
+        o_floats = std::max(o_floats, tc.part_o_floats);
+    }
+    if (ml_floats + o_floats > kStaticScratchFloats || tc.tickets > kStaticTickets) {
+        return fail(HC_KV_OVERFLOW, "hc_attention_decode_static: this call needs " + std::to_string((ml_floats + o_floats) * 4) +
                                         " bytes of partials, the fixed scratch holds " +
                                         std::to_string(kStaticScratchFloats * 4));
     }
-    // Every partial the merge reads is written by this call's split kernel first, so nothing in the
-    // array has to start at zero.
+    // Every partial the merge reads is written by this call first, so nothing in the array has to start
+    // at zero but the tickets behind it, which every launch leaves at zero.
     Workspace ws;
     ws.part_ml = ctx->static_scratch;
     ws.part_ml_floats = ml_floats;
     ws.part_o = ctx->static_scratch + ml_floats;
     ws.part_o_floats = kStaticScratchFloats - ml_floats;
+    ws.tickets = reinterpret_cast<unsigned*>(ctx->static_scratch + kStaticScratchFloats);
+    ws.n_tickets = kStaticTickets;
     // The same kernels, in the same order, as hc_attention_decode: only the partials live elsewhere,
     // so the two entry points return the same bits.
     if (tensor) {
-        return tc_decode(ctx, shape, *store, view, meta, n_seq, static_cast<const uint16_t*>(q), ws, ep,
-                         static_cast<cudaStream_t>(stream));
+        DecodeSource src{};
+        src.q = q;
+        src.dtype = HC_BF16;
+        src.q_head_stride = shape.head_dim;
+        return tc_decode(ctx, shape, *store, view, meta, n_seq, src, ws, ep, static_cast<cudaStream_t>(stream));
     }
     return simt_decode(ctx, shape, view, meta, n_seq, static_cast<const uint16_t*>(q), ws, ep,
                        static_cast<cudaStream_t>(stream));

@@ -1117,67 +1117,4 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
     return launch_merge_prefill(ctx, shape, cache.map, tokens, first_position, ws, slots, ep, stream);
 }
 
-DecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const RowMap& map, const BatchMeta& meta, int n_seq,
-                          size_t part_o_floats) {
-    // About six items per thread block, so that the static round-robin balances (measured best of
-    // 3 .. 12 on uniform and ragged batches); the head_dim 256 kernel does not look ahead across
-    // items: about one per thread block.
-    const int target = (shape.head_dim == 256 ? 1 : 6) * std::max(ctx->sm_count, 1);
-    DecodePlan plan = plan_decode(shape, map, meta, n_seq, target, true, 64);
-    if (plan.finish && row_state_floats(ctx, shape) > part_o_floats) {
-        // A whole row that spans two segments needs the second fold's state, for which there is no room.
-        bool spans = false;
-        for (int b = 0; b < n_seq; ++b) spans = spans || visible_groups(meta.pos[b], meta.pos[b], shape.window, map.log_segment) > 1;
-        if (spans) plan = plan_decode(shape, map, meta, n_seq, target, false, 64);
-    }
-    return plan;
-}
-
-hc_status tc_decode(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
-                    const BatchMeta& meta, int n_seq, const uint16_t* q, const Workspace& ws,
-                    const EpilogueArgs& ep, cudaStream_t stream) {
-    if (!layer.tmap_k || !layer.tmap_v) return fail(HC_UNSUPPORTED, "this layer has no tensor maps");
-    if (n_seq <= 0) return HC_OK;
-    TcArgs args{};
-    fill_common_args(args, ctx, shape, cache, q, ws, ep);
-    args.tokens = n_seq;
-    args.decode = 1;
-    args.meta = meta;
-    const DecodePlan plan = tc_plan_decode(ctx, shape, cache.map, meta, n_seq, ws.part_o_floats);
-    args.finish = plan.finish;
-    args.log_run = plan.log_run;
-    args.tile_partials = plan.tile_partials;
-    args.slots = plan.slots;
-    // One item per (sequence, kv head, run of the sequence's visible key tiles).
-    int next = 0;
-    for (int b = 0; b < n_seq; ++b) {
-        int n = 1;
-        if (plan.tile_partials) {
-            n = visible_groups(meta.pos[b], meta.pos[b], shape.window, plan.log_run);
-        } else if (!plan.finish) {
-            // The sequence's segments in runs of one size, about plan.run_segments each.
-            const int segments = visible_groups(meta.pos[b], meta.pos[b], shape.window, cache.map.log_segment);
-            const int want = (segments + plan.run_segments - 1) / plan.run_segments;
-            const int run = (segments + want - 1) / want;
-            n = (segments + run - 1) / run;
-            args.seq_run[b] = static_cast<unsigned short>(run);
-        }
-        args.item_start[b] = next;
-        args.seq_slots[b] = static_cast<unsigned short>(n);
-        args.seq_magic[b] = division_magic(uint32_t(n), uint32_t(n) * uint32_t(shape.kv_heads));
-        next += n * shape.kv_heads;
-    }
-    for (int b = n_seq; b <= kMaxBatch; ++b) args.item_start[b] = next;
-    args.n_items = next;
-    if (!args.finish) {
-        const size_t rows = size_t(n_seq) * shape.q_heads;
-        if (rows * plan.slots * shape.head_dim > ws.part_o_floats || rows * plan.slots * 2 > ws.part_ml_floats) {
-            return fail(HC_KV_OVERFLOW, "decode: the split-attention workspace is too small for this call");
-        }
-    }
-    const hc_status st = launch_any(ctx, shape, args, layer, stream);
-    if (st != HC_OK || args.finish) return st;
-    return launch_merge_decode(ctx, shape, cache.map, meta, n_seq, ws, plan, ep, stream);
-}
-
 }  // namespace hc

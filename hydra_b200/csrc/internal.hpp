@@ -109,6 +109,27 @@ struct Workspace {
     // working in the upper halves [prefill_o_floats, 2 prefill_o_floats) and likewise for part_ml.
     size_t prefill_o_floats = 0;
     size_t prefill_ml_floats = 0;
+    // Counters by which the last thread block of a decode row (or of a row's segment) to finish knows that it
+    // is the last; zero between launches.
+    unsigned* tickets = nullptr;
+    size_t n_tickets = 0;
+};
+
+// What the tcgen05 decode kernel prepares itself: the queries as the caller has them and, when k is set, the
+// tokens' own key and value rows on their way into the cache.
+struct DecodeSource {
+    const void* q;
+    const void* k;
+    const void* v;
+    int dtype;               // hc_dtype of the three
+    int q_head_stride;       // elements between heads of q (2 d for an interleaved gate)
+    int norm_q, norm_k, norm_v;
+    const uint16_t* q_weight;
+    const uint16_t* k_weight;
+    float eps;
+    const float* cos;        // null: no rotation
+    const float* sin;
+    int table_positions;
 };
 
 }  // namespace hc
@@ -119,6 +140,7 @@ struct hc_context {
     uint64_t launches = 0;
     int* status_dev = nullptr;    // one word the kernels may set on a bounded-wait timeout
     int* status_host = nullptr;   // pinned mirror
+    int cluster_slots[4] = {};    // thread blocks resident at once in clusters of 2, 4, 8, 16 (see attn_decode.cu)
     float* static_scratch = nullptr;   // device address of the fixed scratch of hc_attention_decode_static
 };
 
@@ -207,10 +229,8 @@ struct DecodePlan {
 // The coarsest cut that gives at least target_items items, runs of max_run_segments segments at most.
 DecodePlan plan_decode(const AttnShape& shape, const RowMap& map, const BatchMeta& meta, int n_seq, int target_items,
                        bool allow_whole, int max_run_segments);
-// The cuts simt_decode and tc_decode make (the latter given the room for partials or row state).
+// The cut simt_decode makes.
 DecodePlan simt_plan_decode(const hc_context* ctx, const AttnShape& shape, const RowMap& map, const BatchMeta& meta, int n_seq);
-DecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const RowMap& map, const BatchMeta& meta, int n_seq,
-                          size_t part_o_floats);
 // Both folds (tile partials) or the second fold (segment partials) over the partials in `ws`, then the
 // epilogue: for the rows of a decode batch, or for the query tokens of a prefill chunk.
 hc_status launch_merge_decode(hc_context* ctx, const AttnShape& shape, const RowMap& map, const BatchMeta& meta,
@@ -232,8 +252,19 @@ bool tc_supported(const AttnShape& shape);
 hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer,
                      const CacheView& cache, int seq, const uint16_t* q, int tokens,
                      int first_position, const Workspace& ws, const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends = nullptr);
+// attn_decode.cu
+// How a tcgen05 decode launch cuts its rows' keys, and the workspace that takes.
+struct TcDecodePlan {
+    int finish;              // whole rows per item
+    int cluster;             // otherwise: thread blocks that share a run of segments (1: none) ..
+    int run_segments;        // .. and about how many segments a run has
+    int slots;               // partial slots per row: segments
+    size_t part_o_floats, part_ml_floats, tickets;
+};
+hc_status decode_cluster_slots(hc_context* ctx);
+TcDecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const RowMap& map, const BatchMeta& meta, int n_seq);
 hc_status tc_decode(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer,
-                    const CacheView& cache, const BatchMeta& meta, int n_seq, const uint16_t* q,
+                    const CacheView& cache, const BatchMeta& meta, int n_seq, const DecodeSource& src,
                     const Workspace& ws, const EpilogueArgs& ep, cudaStream_t stream);
 // linear_tc.cu
 // n_jobs (1 to 4) projections of the same x in one launch; bias / residual may be null, or hold nulls.

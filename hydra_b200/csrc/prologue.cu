@@ -15,6 +15,7 @@
 #include <algorithm>
 
 #include "internal.hpp"
+#include "prologue.cuh"
 
 namespace hc {
 namespace {
@@ -22,25 +23,6 @@ namespace {
 constexpr int kPrepWarps = 8;
 constexpr int kMaxHeadDim = 512;
 
-// Four consecutive elements of an activation row as fp32 (8-byte load for bf16, 16-byte for fp32).
-__device__ __forceinline__ void load_io4(const void* base, size_t index, int dtype, float (&out)[4]) {
-    if (dtype == 0) {
-        const float4 v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + index);
-        out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
-    } else {
-        const uint2 v = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(base) + index);
-        out[0] = bf16_bits_to_float(uint16_t(v.x & 0xffffu));
-        out[1] = bf16_bits_to_float(uint16_t(v.x >> 16));
-        out[2] = bf16_bits_to_float(uint16_t(v.y & 0xffffu));
-        out[3] = bf16_bits_to_float(uint16_t(v.y >> 16));
-    }
-}
-__device__ __forceinline__ uint2 pack_bf16x4(const float (&v)[4]) {
-    uint2 r;
-    r.x = uint32_t(float_to_bf16_bits(v[0])) | (uint32_t(float_to_bf16_bits(v[1])) << 16);
-    r.y = uint32_t(float_to_bf16_bits(v[2])) | (uint32_t(float_to_bf16_bits(v[3])) << 16);
-    return r;
-}
 __device__ __forceinline__ void store_io4(void* base, size_t index, int dtype, const float (&v)[4]) {
     if (dtype == 0) {
         *reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + index) = make_float4(v[0], v[1], v[2], v[3]);
@@ -49,28 +31,26 @@ __device__ __forceinline__ void store_io4(void* base, size_t index, int dtype, c
     }
 }
 
-// The kernel for head_dim 64, 128 and 256 (LPV = head_dim / 8 lanes per head vector, so a warp holds
-// 4, 2 or 1 vectors at a time).  Lane m of a vector owns elements 4m..4m+3 of each half, which keeps
-// both members of every rotation pair (i, i + d/2) in one lane and makes every access an 8- or 16-byte
-// one.  The launcher checks the alignment this needs and otherwise uses the general kernel below.
-template <int LPV>
+// The kernel for head_dim 64, 128, 256 and 512 (see HeadLanes: a warp holds 4, 2 or 1 vectors at a time and
+// every access is an 8- or 16-byte one).  The launcher checks the alignment this needs and otherwise
+// uses the general kernel below.
+template <int D>
 __global__ void __launch_bounds__(kPrepWarps * 32)
 prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
-    constexpr int d = 8 * LPV;
-    constexpr int half = 4 * LPV;
-    constexpr int kPerWarp = 32 / LPV;
+    using HL = HeadLanes<D>;
     pdl_launch_dependents();
     pdl_wait();
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int sub = lane / LPV;
-    const int m = lane % LPV;
+    const int sub = lane / HL::kLanes;
+    const int m = lane % HL::kLanes;
+    const bool any_norm = (args.job[0].norm | (args.n_jobs > 1 ? args.job[1].norm : 0) | (args.n_jobs > 2 ? args.job[2].norm : 0)) != 0;
     // 32-bit indices: a launch covers at most 32768 tokens x a few hundred heads.
     const unsigned vectors = unsigned(args.tokens) * unsigned(total_heads);
-    const unsigned groups = (vectors + kPerWarp - 1) / kPerWarp;
+    const unsigned groups = (vectors + HL::kPerWarp - 1) / HL::kPerWarp;
     const unsigned stride = gridDim.x * kPrepWarps;
     for (unsigned grp = blockIdx.x * kPrepWarps + warp; grp < groups; grp += stride) {
-        unsigned vec = grp * kPerWarp + sub;
+        unsigned vec = grp * HL::kPerWarp + sub;
         bool active = vec < vectors;
         if (!active) vec = vectors - 1;              // keeps the lane's loads legal; nothing is stored
         const int token = int(vec / unsigned(total_heads));
@@ -87,70 +67,34 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
         if (to_cache && !row_is_local(args.cache.map, position)) active = false;   // another rank's tile
 
         const size_t src_base = size_t(token) * size_t(job.token_stride) + size_t(head) * job.head_stride;
-        float x[8];
-        {
-            float lo[4], hi[4];
-            load_io4(job.src, src_base + 4 * m, job.src_dtype, lo);
-            load_io4(job.src, src_base + half + 4 * m, job.src_dtype, hi);
-            #pragma unroll
-            for (int j = 0; j < 4; ++j) { x[j] = lo[j]; x[4 + j] = hi[j]; }
-        }
-        float4 cosv = make_float4(1.0f, 1.0f, 1.0f, 1.0f), sinv = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float lo[HL::kElems], hi[HL::kElems], c[HL::kElems], s[HL::kElems];
+        load_head<D>(job.src, src_base, job.src_dtype, m, lo, hi);
         if (job.rope != 0) {
             const int table_row = position < args.table_positions ? position : args.table_positions - 1;
-            cosv = *reinterpret_cast<const float4*>(args.cos + size_t(table_row) * half + 4 * m);
-            sinv = *reinterpret_cast<const float4*>(args.sin + size_t(table_row) * half + 4 * m);
+            load_rotation<D>(args.cos + size_t(table_row) * (D / 2), args.sin + size_t(table_row) * (D / 2), m, c, s);
         }
-        if (job.norm != 0) {
-            float sum = 0.0f;
-            #pragma unroll
-            for (int j = 0; j < 8; ++j) sum = __fmaf_rn(x[j], x[j], sum);
-            #pragma unroll
-            for (int offset = LPV / 2; offset > 0; offset >>= 1) {
-                sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, offset));
-            }
-            const float inverse = __frsqrt_rn(__fadd_rn(__fdiv_rn(sum, float(d)), args.eps));
-            #pragma unroll
-            for (int j = 0; j < 8; ++j) x[j] = __fmul_rn(x[j], inverse);
-            if (job.norm == 1) {
-                float wl[4], wh[4];
-                load_io4(job.weight, size_t(4 * m), 1, wl);
-                load_io4(job.weight, size_t(half + 4 * m), 1, wh);
-                #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    x[j] = __fmul_rn(x[j], wl[j]);
-                    x[4 + j] = __fmul_rn(x[4 + j], wh[j]);
-                }
-            }
-        }
-        float lo[4], hi[4];
-        if (job.rope != 0) {
-            const float c[4] = {cosv.x, cosv.y, cosv.z, cosv.w};
-            const float s[4] = {sinv.x, sinv.y, sinv.z, sinv.w};
-            #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                lo[j] = __fmaf_rn(x[j], c[j], -__fmul_rn(x[4 + j], s[j]));
-                hi[j] = __fmaf_rn(x[4 + j], c[j], __fmul_rn(x[j], s[j]));
-            }
-        } else {
-            #pragma unroll
-            for (int j = 0; j < 4; ++j) { lo[j] = x[j]; hi[j] = x[4 + j]; }
-        }
+        prepare_head<D>(lo, hi, job.norm, job.weight, args.eps, job.rope != 0, c, s, m, any_norm);
         if (!active) continue;
-        if (job.kind == 3) {
-            store_io4(job.dst, src_base + 4 * m, job.src_dtype, lo);
-            store_io4(job.dst, src_base + half + 4 * m, job.src_dtype, hi);
-        } else {
-            uint16_t* dst16;
-            if (job.kind == 0) {
-                dst16 = reinterpret_cast<uint16_t*>(job.dst) + (size_t(token) * job.heads + head) * d;
+        #pragma unroll
+        for (int u = 0; u < HL::kVecs; ++u) {
+            const float a[4] = {lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]};
+            const float b[4] = {hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]};
+            const int at = 4 * (m + u * HL::kLanes);
+            if (job.kind == 3) {
+                store_io4(job.dst, src_base + at, job.src_dtype, a);
+                store_io4(job.dst, src_base + D / 2 + at, job.src_dtype, b);
             } else {
-                const int row = cache_row(args.cache.map, seq, position);
-                uint16_t* base = job.kind == 1 ? args.cache.k : args.cache.v;
-                dst16 = base + (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity + row) * d;
+                uint16_t* dst16;
+                if (job.kind == 0) {
+                    dst16 = reinterpret_cast<uint16_t*>(job.dst) + (size_t(token) * job.heads + head) * D;
+                } else {
+                    const int row = cache_row(args.cache.map, seq, position);
+                    uint16_t* base = job.kind == 1 ? args.cache.k : args.cache.v;
+                    dst16 = base + (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity + row) * D;
+                }
+                *reinterpret_cast<uint2*>(dst16 + at) = pack_bf16x4(a);
+                *reinterpret_cast<uint2*>(dst16 + D / 2 + at) = pack_bf16x4(b);
             }
-            *reinterpret_cast<uint2*>(dst16 + 4 * m) = pack_bf16x4(lo);
-            *reinterpret_cast<uint2*>(dst16 + half + 4 * m) = pack_bf16x4(hi);
         }
     }
 }
@@ -254,7 +198,7 @@ prepare_heads_kernel(const PrepArgs args) {
 // after the other (12 us for one 2880-wide row).  The sum's order is fixed by the width alone.
 constexpr int kNormVecs = 4;      // float4 per thread held in registers: 256 threads x 16 values
 
-__device__ __forceinline__ float4 load_io4(const void* p, size_t index, int dtype) {
+__device__ __forceinline__ float4 load_vec4(const void* p, size_t index, int dtype) {
     if (dtype == HC_F32) return *reinterpret_cast<const float4*>(static_cast<const float*>(p) + index);
     const uint2 bits = *reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(p) + index);
     return make_float4(__uint_as_float(bits.x << 16), __uint_as_float(bits.x & 0xffff0000u),
@@ -273,7 +217,7 @@ rms_norm_rows_kernel(const void* __restrict__ x, const uint16_t* __restrict__ sc
         #pragma unroll
         for (int u = 0; u < kNormVecs; ++u) {
             const int i = (threadIdx.x + u * 256) * 4;
-            held[u] = i < width ? load_io4(x, base + i, x_dtype) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            held[u] = i < width ? load_vec4(x, base + i, x_dtype) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
         #pragma unroll
         for (int u = 0; u < kNormVecs; ++u) {
@@ -362,7 +306,7 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
     const int d = args.head_dim;
     const long long cap = (long long)std::max(ctx->sm_count, 1) * 16;
     // The vector kernel needs 16-byte aligned rows everywhere it touches.
-    bool vector_ok = d == 64 || d == 128 || d == 256;
+    bool vector_ok = d == 64 || d == 128 || d == 256 || d == 512;
     for (int j = 0; j < args.n_jobs && vector_ok; ++j) {
         const PrepJob& job = args.job[j];
         if (job.heads == 0) continue;
@@ -371,12 +315,12 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
                     ((job.kind != 0 && job.kind != 3) || aligned16(job.dst));
     }
     if (vector_ok) {
-        const int per_warp = 256 / d;
+        const int per_warp = d >= 256 ? 1 : 256 / d;
         const long long groups = (vectors + per_warp - 1) / per_warp;
         const int grid = int(std::min<long long>((groups + kPrepWarps - 1) / kPrepWarps, cap));
-        if (d == 64) launch_pdl(prepare_heads_vec_kernel<8>, grid, kPrepWarps * 32, 0, stream, args, total_heads);
-        else if (d == 128) launch_pdl(prepare_heads_vec_kernel<16>, grid, kPrepWarps * 32, 0, stream, args, total_heads);
-        else launch_pdl(prepare_heads_vec_kernel<32>, grid, kPrepWarps * 32, 0, stream, args, total_heads);
+        auto kernel = d == 64 ? prepare_heads_vec_kernel<64> : d == 128 ? prepare_heads_vec_kernel<128>
+                    : d == 256 ? prepare_heads_vec_kernel<256> : prepare_heads_vec_kernel<512>;
+        launch_pdl(kernel, grid, kPrepWarps * 32, 0, stream, args, total_heads);
     } else {
         const long long wanted = (vectors + kPrepWarps - 1) / kPrepWarps;
         const int grid = int(std::min<long long>(wanted, cap));

@@ -38,7 +38,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return done != 0;
 }
-// The same with a suspend-time hint: the hardware may park the warp for up to `ns` nanoseconds
+// Returns at once, for a thread that has other things to look after (try_wait may suspend it).
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
+}
+// try_wait with a suspend-time hint: the hardware may park the warp for up to `ns` nanoseconds
 // instead of returning at once, so a waiting warp does not compete for issue slots.
 __device__ __forceinline__ bool mbar_try_wait_parked(uint64_t* bar, uint32_t parity, uint32_t ns) {
     uint32_t done;
