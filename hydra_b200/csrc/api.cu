@@ -382,7 +382,9 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
     const int mult = p->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
     const bool prep = needs_q_prepare(p);
     // A launch takes as many sequences as the prepared-query buffer has rows for.
-    const int per_launch = prep ? std::min(kMaxBatch, cache->ws.qprep_tokens) : kMaxBatch;
+    // (The tcgen05 decode kernel lists its rows, 512 of them at most, in shared memory.)
+    int per_launch = prep ? std::min(kMaxBatch, cache->ws.qprep_tokens) : kMaxBatch;
+    if (tensor) per_launch = std::max(1, std::min(per_launch, 512 / p->kv_heads));
 
     for (int start = 0; start < n_seq; start += per_launch) {
         const int count = std::min(per_launch, n_seq - start);
@@ -763,15 +765,18 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         //   prefill: when even a full chunk gives too few (row tile, kv head) pairs to occupy the SMs
         //            (half of them; a quarter for head_dim 256, whose kernel pays more per item) and a
         //            row can span more than two short segments;
-        //   decode:  a cache for batches of sequences, whose split kernel then leaves one partial per
-        //            1024 keys instead of one per 128.
+        //   decode:  a cache for batches of sequences, whose rows are cut at segment boundaries, and wide
+        //            heads, whose spans of segments have to fit the shared memory of a cluster (one
+        //            sequence of 32768 keys, head_dim 256: 4096-key segments made two waves of clusters
+        //            of what is one with 1024).
         const int tokens_per_tile = kTileKeys / (L.desc.q_heads / L.desc.kv_heads);
         const int chunk_row_tiles = (prefill_chunk + tokens_per_tile - 1) / tokens_per_tile;
         const int reach = windowed ? std::min(L.desc.window + prefill_chunk, context_length) : context_length;
         const bool few_rows = (d == 256 ? 4 : 2) * chunk_row_tiles * L.desc.kv_heads <= std::max(ctx->sm_count, 1) &&
                               reach > (2 * kTileKeys << kLogSegmentSmall);
         const bool batched = max_seqs >= 8;
-        L.log_segment = few_rows || batched ? kLogSegmentSmall : kLogSegmentLarge;
+        L.log_segment_general = few_rows || batched ? kLogSegmentSmall : kLogSegmentLarge;
+        L.log_segment = d >= 256 ? kLogSegmentSmall : L.log_segment_general;
         // Workspace for the partials of split launches.  Decode, at its finest cut: one per (batch
         // entry, query head, key tile of this rank).  Prefill, layers with short segments only: one
         // per (query token, query head, segment).

@@ -26,15 +26,18 @@
 //   warps 12-15  fold, thread = head_dim column: the tile partials of an item into its segment, partials
 //                out, and the merge
 //
-// Three ways to cut a launch (tc_plan_decode):
-//   rows       an item is a whole row; its thread block finishes it.
+// Two ways to cut a launch (tc_plan_decode):
+//   a line     the rows (sequence, kv head) with their key tiles lie one behind the other, and every thread block takes
+//              an equal stretch of the line, cut at segment boundaries.  A row that lies inside one stretch
+//              is finished there; the others leave one partial per segment in global memory.  (Dealing
+//              out runs of segments round robin left the last thread block of 64 ragged sequences 25 % behind
+//              the average; equal stretches leave half a segment.)
 //   clusters   few long rows: the 2 to 16 thread blocks of a cluster share a row, or a span of its segments, and
 //              every tile's partial is pushed, value by value, into the shared memory of the block
 //              that folds that slice of the columns: no partial touches global memory, no
 //              thread block folds more than its slice, and a row that fits a cluster needs no ticket.
-//   segments   many rows: an item is a run of whole segments, whose partials go to global memory.
-// Spans and segments end in tickets: the thread block that draws a row's (or slice's) last one folds what the others
-// left.  Nobody waits for anybody.  The last one also puts the ticket back to zero.
+// Cut rows end in tickets that count tiles: the thread block whose tiles complete a row (or a slice of it) folds what
+// the others left.  Nobody waits for anybody.  It also puts the ticket back to zero.
 //
 // Every wait on an mbarrier is bounded (see tc_ptx.cuh).
 
@@ -103,20 +106,18 @@ struct DecArgs {
     int count_sink;
     EpilogueArgs ep;
     int* status;
-    // The cut (see TcDecodePlan): whole rows (finish), clusters of `cluster` blocks per span of seq_run[b] segments,
-    // or items of seq_run[b] segments.
+    // The cut (see TcDecodePlan): a line of n_tiles tiles over the thread blocks, or clusters of `cluster` blocks per
+    // span of seq_run[b] segments.
     int n_seq;
-    int n_items;                     // rows, spans or runs
-    int finish;
-    int cluster;                     // 1: not in clusters
+    int cluster;                     // 1: a line
     int slots;                       // partial slots per row: segments
     float* part_o;                   // fp32 [rows][slots][d]
     float* part_ml;                  // fp32 [rows][slots][2]
-    unsigned* tickets;               // [n_seq * kv_heads][cluster]
-    int item_start[kMaxBatch + 1];
-    unsigned short seq_slots[kMaxBatch];
+    unsigned* tickets;               // [n_seq * kv_heads][cluster]: tiles whose partials are there
+    int n_tiles;
+    int start[kMaxBatch + 1];        // line: tiles (of all kv heads) before sequence b; clusters: spans before it
     unsigned short seq_run[kMaxBatch];
-    uint32_t seq_magic[kMaxBatch];
+    unsigned short seq_spans[kMaxBatch];
     BatchMeta meta;
 };
 
@@ -124,45 +125,47 @@ struct DecItem {
     int b, kv_head;
     int tile_first, n_tiles;         // key tiles, `world` apart
     bool last;                       // holds the row's last key tile: the one the token's own key lies in
-    int span_first, span_tiles;      // what the blocks of its cluster share (not kept in the list)
+    bool whole;                      // line: all of the row, finished by this block
 };
 
-__device__ __forceinline__ DecItem dec_item(const DecArgs& args, int index) {
-    DecItem w;
-    int lo = 0, hi = args.n_seq;                     // item_start[lo] <= index < item_start[hi]
+// b with start[b] <= index < start[b + 1]
+__device__ __forceinline__ int dec_search(const DecArgs& args, int index) {
+    int lo = 0, hi = args.n_seq;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (index >= args.item_start[mid]) lo = mid; else hi = mid;
+        if (index >= args.start[mid]) lo = mid; else hi = mid;
     }
-    const int local = index - args.item_start[lo];
-    const int runs = args.seq_slots[lo];
-    const int pos = args.meta.pos[lo];
-    w.b = lo;
-    w.kv_head = fast_div(local, runs, args.seq_magic[lo]);
-    const int ordinal = local - w.kv_head * runs;
-    TileRange tiles;
-    if (args.finish) {
-        tiles = row_tiles(args.cache.map, pos, pos, args.window);
-    } else {
-        const int run = args.seq_run[lo];
-        tiles = segment_run_tiles(args.cache.map, pos, pos, args.window, ordinal * run, run);
-    }
+    return lo;
+}
+
+// Where thread block c's stretch of the line begins: a row and a tile of it, the equal share's end moved to the nearest
+// segment boundary.
+struct DecPlace {
+    int row, t;
+};
+__device__ __forceinline__ DecPlace dec_place(const DecArgs& args, int c) {
+    DecPlace p;
+    p.row = args.n_seq * args.cache.kv_heads;
+    p.t = 0;
+    if (c >= int(gridDim.x)) return p;
+    const int at = int((long long)c * args.n_tiles / int(gridDim.x));
+    const int b = dec_search(args, at);
     const int world = args.cache.map.world > 1 ? args.cache.map.world : 1;
-    w.span_first = tiles.first;
-    w.span_tiles = max(tiles.count, 0);
-    w.last = tiles.count > 0 && tiles.first + (tiles.count - 1) * world == pos / kTileKeys;
-    if (args.cluster > 1) {
-        // This block's share of the cluster's span.
-        const int rank = int(blockIdx.x) & (args.cluster - 1);
-        const int share = (w.span_tiles + args.cluster - 1) / args.cluster;
-        const int count = min(share, w.span_tiles - rank * share);
-        w.last = w.last && count > 0 && rank * share + count == w.span_tiles;
-        tiles.first += rank * share * world;
-        tiles.count = count;
+    const int log_segment = args.cache.map.log_segment;
+    const TileRange row = row_tiles(args.cache.map, args.meta.pos[b], args.meta.pos[b], args.window);
+    if (row.count <= 0) return p;                        // (an empty launch)
+    const int head = (at - args.start[b]) / row.count;
+    const int t = at - args.start[b] - head * row.count;
+    const int segment_tile = ((row.first + t * world) >> log_segment) << log_segment;
+    const int before = segment_tile <= row.first ? 0 : (segment_tile - row.first + world - 1) / world;
+    const int after = min(row.count, (segment_tile + (1 << log_segment) - row.first + world - 1) / world);
+    p.row = b * args.cache.kv_heads + head;
+    p.t = t - before <= after - t ? before : after;
+    if (p.t == row.count) {
+        p.t = 0;
+        ++p.row;
     }
-    w.tile_first = tiles.first;
-    w.n_tiles = max(tiles.count, 0);
-    return w;
+    return p;
 }
 
 // A thread block's items, worked out once by all its threads side by side (finding an item takes a search and
@@ -172,37 +175,67 @@ constexpr int kDecItems = 512;       // of one thread block, at most
 struct DecList {
     uint2 packed[kDecItems];
     int pos[kMaxBatch], seq[kMaxBatch];
+    int count;
     int span_first, span_tiles;      // of the cluster
 };
-__device__ __forceinline__ int dec_item_count(const DecArgs& args) {
-    if (args.cluster > 1) return 1;
-    return (args.n_items - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);
-}
-__device__ __forceinline__ void dec_list_build(const DecArgs& args, DecList* list) {
-    const int count = dec_item_count(args);
-    for (int i = threadIdx.x; i < count; i += kTcThreads) {
-        const DecItem w = dec_item(args, args.cluster > 1 ? int(blockIdx.x) / args.cluster : int(blockIdx.x) + i * int(gridDim.x));
-        list->packed[i] = make_uint2(uint32_t(w.b) | (uint32_t(w.kv_head) << 8) | (w.last ? 0x80000000u : 0u),
-                                     uint32_t(w.tile_first) | (uint32_t(w.n_tiles) << 16));
-        if (args.cluster > 1) {
-            list->span_first = w.span_first;
-            list->span_tiles = w.span_tiles;
-        }
-    }
-    for (int i = threadIdx.x; i < args.n_seq; i += kTcThreads) {
-        list->pos[i] = args.meta.pos[i];
-        list->seq[i] = args.meta.seq[i];
-    }
+__device__ __forceinline__ uint2 dec_pack(const DecItem& w) {
+    return make_uint2(uint32_t(w.b) | (uint32_t(w.kv_head) << 8) | (w.whole ? 0x40000000u : 0u) | (w.last ? 0x80000000u : 0u),
+                      uint32_t(w.tile_first) | (uint32_t(w.n_tiles) << 16));
 }
 __device__ __forceinline__ DecItem dec_unpack(const uint2& p) {
     DecItem w;
     w.b = int(p.x & 0xffu);
-    w.kv_head = int((p.x >> 8) & 0x7fffffu);
+    w.kv_head = int((p.x >> 8) & 0x3fffffu);
+    w.whole = (p.x & 0x40000000u) != 0;
     w.last = (p.x >> 31) != 0;
     w.tile_first = int(p.y & 0xffffu);
     w.n_tiles = int(p.y >> 16);
-    w.span_first = w.span_tiles = 0;
     return w;
+}
+__device__ __forceinline__ void dec_list_build(const DecArgs& args, DecList* list) {
+    const int world = args.cache.map.world > 1 ? args.cache.map.world : 1;
+    for (int i = threadIdx.x; i < args.n_seq; i += kTcThreads) {
+        list->pos[i] = args.meta.pos[i];
+        list->seq[i] = args.meta.seq[i];
+    }
+    if (args.cluster > 1) {
+        if (threadIdx.x != 0) return;
+        // This block's share of the cluster's span.
+        const int span = int(blockIdx.x) / args.cluster, rank = int(blockIdx.x) & (args.cluster - 1);
+        DecItem w;
+        w.b = dec_search(args, span);
+        const int spans = args.seq_spans[w.b], run = args.seq_run[w.b], pos = args.meta.pos[w.b];
+        w.kv_head = (span - args.start[w.b]) / spans;
+        const int ordinal = span - args.start[w.b] - w.kv_head * spans;
+        const TileRange tiles = segment_run_tiles(args.cache.map, pos, pos, args.window, ordinal * run, run);
+        const int share = (max(tiles.count, 0) + args.cluster - 1) / args.cluster;
+        w.n_tiles = max(min(share, tiles.count - rank * share), 0);
+        w.tile_first = tiles.first + rank * share * world;
+        w.last = w.n_tiles > 0 && w.tile_first + (w.n_tiles - 1) * world == pos / kTileKeys;
+        w.whole = false;
+        list->packed[0] = dec_pack(w);
+        list->count = 1;
+        list->span_first = tiles.first;
+        list->span_tiles = max(tiles.count, 0);
+        return;
+    }
+    const DecPlace from = dec_place(args, int(blockIdx.x)), to = dec_place(args, int(blockIdx.x) + 1);
+    const int count = min(to.row - from.row + (to.t > 0 ? 1 : 0), kDecItems);
+    if (threadIdx.x == 0) list->count = count;
+    for (int i = threadIdx.x; i < count; i += kTcThreads) {
+        DecItem w;
+        const int r = from.row + i;
+        w.b = r / args.cache.kv_heads;
+        w.kv_head = r - w.b * args.cache.kv_heads;
+        const int pos = args.meta.pos[w.b];
+        const TileRange row = row_tiles(args.cache.map, pos, pos, args.window);
+        const int t0 = i == 0 ? from.t : 0, t1 = r == to.row ? to.t : max(row.count, 0);
+        w.tile_first = row.first + t0 * world;
+        w.n_tiles = t1 - t0;
+        w.last = w.n_tiles > 0 && t1 == row.count && row.first + (row.count - 1) * world == pos / kTileKeys;
+        w.whole = t0 == 0 && t1 == row.count;
+        list->packed[i] = dec_pack(w);
+    }
 }
 
 // The walk over the list; items without tiles (sequence shards) are passed over.
@@ -217,10 +250,10 @@ __device__ __forceinline__ void dec_seek(const DecList* list, DecIter& it) {
         if (it.w.n_tiles > 0) return;
     }
 }
-__device__ __forceinline__ DecIter dec_begin(const DecArgs& args, const DecList* list) {
+__device__ __forceinline__ DecIter dec_begin(const DecList* list) {
     DecIter it;
     it.i = 0;
-    it.count = dec_item_count(args);
+    it.count = list->count;
     it.w = DecItem{};
     dec_seek(list, it);
     return it;
@@ -239,7 +272,8 @@ struct DecBarriers {
     uint64_t merge_full[2];
     uint32_t tmem_base;
     int abort_flag;
-    int n_work;                             // items whose tickets were the last ones
+    int n_work;                             // rows that this block completes
+    int cut;                                // line: some item is not a whole row
     uint32_t staged;                        // items whose queries and appended rows are written
     __align__(16) float red[2][2][4][kQRows];           // per softmax group, alternate tiles: the warps' maxima
     __align__(16) float mm[4][kQRows];                  // scaled maxima of a tile, softmax -> fold (ring of 4 tiles)
@@ -460,33 +494,27 @@ __device__ __forceinline__ void dec_fold(const DecArgs& args, const DecItem& w, 
     __syncthreads();
 }
 
-__device__ __forceinline__ bool dec_last_ticket(unsigned* ticket, int of) {
-    if (atomicAdd(ticket, 1u) + 1u != unsigned(of)) return false;
+// Counts tiles on a ticket; true for whoever completes the row.
+__device__ __forceinline__ bool dec_last_ticket(unsigned* ticket, int tiles, int of) {
+    if (atomicAdd(ticket, unsigned(tiles)) + unsigned(tiles) != unsigned(of)) return false;
     atomicExch(ticket, 0u);
     return true;
 }
-// Items (or spans) with tiles that a row was cut into.
-__device__ __forceinline__ int dec_row_parts(const DecArgs& args, int b, int pos) {
-    if (args.cache.map.world <= 1) return args.seq_slots[b];
-    int parts = 0;
-    for (int k = 0; k < args.seq_slots[b]; ++k) {
-        parts += segment_run_tiles(args.cache.map, pos, pos, args.window, k * args.seq_run[b], args.seq_run[b]).count > 0 ? 1 : 0;
-    }
-    return parts;
-}
 
-// Segments: a block that has written all its items' partials takes the tickets of its items (all at once, a thread
-// each), and folds the rows these were the last ones of.
+// A line's block that has written its partials counts them on its rows' tickets (all at once, a thread each), and folds
+// the rows that this completes.
 template <int D, int NG>
-__device__ __forceinline__ void dec_close(const DecArgs& args, const DecList* list, int count, float* ring, DecMerge* sm, int* work, int* n_work,
+__device__ __forceinline__ void dec_close(const DecArgs& args, const DecList* list, float* ring, DecMerge* sm, int* work, int* n_work,
                                           uint64_t* bars, volatile int* abort_flag) {
     uint32_t loads = 0;
     __threadfence();                                    // the partials, before the tickets
     __syncthreads();
-    for (int i = threadIdx.x; i < count; i += kTcThreads) {
+    for (int i = threadIdx.x; i < list->count; i += kTcThreads) {
         const DecItem w = dec_unpack(list->packed[i]);
-        if (w.n_tiles == 0) continue;
-        if (dec_last_ticket(args.tickets + w.b * args.cache.kv_heads + w.kv_head, dec_row_parts(args, w.b, list->pos[w.b]))) {
+        if (w.n_tiles == 0 || w.whole) continue;
+        const int pos = list->pos[w.b];
+        if (dec_last_ticket(args.tickets + w.b * args.cache.kv_heads + w.kv_head, w.n_tiles,
+                            row_tiles(args.cache.map, pos, pos, args.window).count)) {
             work[atomicAdd(n_work, 1)] = i;
         }
     }
@@ -503,17 +531,9 @@ __device__ __forceinline__ void dec_close(const DecArgs& args, const DecList* li
 // ---- clusters ----------------------------------------------------------------------------------------------
 // The G x D values of a row group are cut into as many slices as the cluster has blocks, G D / cluster consecutive
 // values each: part of one row, or several whole rows.
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-    return r;
-}
 __device__ __forceinline__ void cluster_store(uint32_t addr, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 // This block's slice: both folds over the span's pushed tile partials when the span is the whole row, otherwise the
 // first fold of every segment, and the second by the slice's last span.
 template <int D>
@@ -532,7 +552,7 @@ __device__ __forceinline__ void dec_fold_slice(const DecArgs& args, const DecLis
     const int first_row = rank * width / D;
     const int first_segment = first_visible_tile(pos, args.window) >> log_segment;
     const int base_segment = (tile0 >> log_segment) - first_segment;         // ordinal of the span's first segment
-    const bool whole = args.seq_slots[w.b] == 1;
+    const bool whole = args.seq_spans[w.b] == 1;
     const size_t row0 = size_t(w.b) * args.q_heads + size_t(w.kv_head) * G;
     const size_t slot0 = (row0 + first_row) * args.slots;                    // partial slot 0 of the slice's first row
     const int segments = tiles > 0 ? ((tile0 + (tiles - 1) * world) >> log_segment) - (tile0 >> log_segment) + 1 : 0;
@@ -606,49 +626,61 @@ __device__ __forceinline__ void dec_fold_slice(const DecArgs& args, const DecLis
     __threadfence();
     __syncthreads();
     if (tid == 0) {
-        *n_last = tiles > 0 && dec_last_ticket(args.tickets + (w.b * args.cache.kv_heads + w.kv_head) * args.cluster + rank,
-                                               dec_row_parts(args, w.b, pos)) ? 1u : 0u;
+        *n_last = tiles > 0 && dec_last_ticket(args.tickets + (w.b * args.cache.kv_heads + w.kv_head) * args.cluster + rank, tiles,
+                                               row_tiles(args.cache.map, pos, pos, args.window).count) ? 1u : 0u;
         __threadfence();
     }
     __syncthreads();
     if (*n_last == 0) return;
+    // The second fold over the slice's segments, up to 32 at a time: the values' loads go out before the coefficients,
+    // which a warp per row works out, are there.
     const int count = visible_groups(pos, pos, args.window, log_segment);
+    float M = kEmptyMax, L = args.count_sink ? 1.0f : 0.0f;                  // of row `warp`, in its warp
+    if (args.count_sink && warp < rows) M = dec_sink(args, w.kv_head * G + first_row + warp);
     #pragma unroll 1
-    for (int i = tid; i < width + rows; i += kTcThreads) {
-        const bool is_sum = i >= width;
-        const int row = is_sum ? i - width : (width > D ? i / D : 0);
-        const int col = (rank * width + i) % D;
-        const float* ml = args.part_ml + (slot0 + size_t(row) * args.slots) * 2;
-        const float* src = is_sum ? ml + 1 : args.part_o + (slot0 + size_t(row) * args.slots) * D + col;
-        const int stride = is_sum ? 2 : D;
-        float M = args.count_sink ? dec_sink(args, w.kv_head * G + first_row + row) : kEmptyMax;
-        float A = is_sum && args.count_sink ? 1.0f : 0.0f;
-        #pragma unroll 1
-        for (int s0 = 0; s0 < count; s0 += 8) {
-            float m[8], v[8];
+    for (int s0 = 0; s0 < count; s0 += 32) {
+        const int n = min(32, count - s0);
+        float2 ml = make_float2(0.0f, 0.0f);
+        if (warp < rows && lane < n) ml = __ldcg(reinterpret_cast<const float2*>(args.part_ml + (slot0 + size_t(warp) * args.slots + s0 + lane) * 2));
+        float v[16];
+        auto load = [&](int i, int u0) {
+            const int row = width > D ? i / D : 0;
+            const float* src = args.part_o + (slot0 + size_t(row) * args.slots + s0 + u0) * D + (rank * width + i) % D;
             #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int s = min(s0 + u, count - 1);
-                m[u] = __ldcg(ml + 2 * s);
-                v[u] = __ldcg(src + size_t(s) * stride);
-            }
-            #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (s0 + u >= count || !dec_segment_present(args, pos, s0 + u)) continue;
-                float Mn, a, b;
-                fold_coefficients(M, m[u], Mn, a, b);
-                M = Mn;
-                A = fold_value(A, a, v[u], b);
+            for (int u = 0; u < 16; ++u) v[u] = u0 + u < n ? __ldcg(src + size_t(u) * D) : 0.0f;
+        };
+        if (tid < width) load(tid, 0);
+        if (warp < rows) {
+            const bool there = lane < n && dec_segment_present(args, pos, s0 + lane);
+            const float2 c = warp_fold_coefficients(there ? ml.x : __int_as_float(0xff800000), M);
+            sm->slice.coef[warp * 32 + lane] = c;
+            const float lb = there ? __fmul_rn(ml.y, c.y) : 0.0f;
+            #pragma unroll 1
+            for (int u = 0; u < n; ++u) L = __fmaf_rn(L, __shfl_sync(0xffffffffu, c.x, u), __shfl_sync(0xffffffffu, lb, u));
+            if (lane == 0) {
+                sm->M[warp] = M;
+                sm->L[warp] = L;
             }
         }
-        if (is_sum) {
-            sm->L[row] = A;
-            sm->M[row] = M;
-        } else {
+        __syncthreads();
+        #pragma unroll 1
+        for (int i = tid; i < width; i += kTcThreads) {
+            const float2* coef = sm->slice.coef + (width > D ? i / D : 0) * 32;
+            float A = s0 == 0 ? 0.0f : pushed[i];
+            #pragma unroll 1
+            for (int u0 = 0; u0 < n; u0 += 16) {
+                if (i != tid || u0 != 0) load(i, u0);
+                #pragma unroll
+                for (int u = 0; u < 16; ++u) {
+                    if (u0 + u >= n || !dec_segment_present(args, pos, s0 + u0 + u)) continue;
+                    const float2 c = coef[u0 + u];
+                    A = fold_value(A, c.x, v[u], c.y);
+                }
+            }
             const_cast<float*>(pushed)[i] = A;
         }
+        __syncthreads();
     }
-    __syncthreads();
     #pragma unroll 1
     for (int i = tid; i < width; i += kTcThreads) {
         const int row = width > D ? i / D : 0;
@@ -761,6 +793,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
             bars->abort_flag = 0;
             bars->staged = 0;
             bars->n_work = 0;
+            bars->cut = 0;
             mbar_init(&bars->merge_full[0], 1);
             mbar_init(&bars->merge_full[1], 1);
         }
@@ -781,7 +814,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
-    const DecIter start = dec_begin(args, list);
+    const DecIter start = dec_begin(list);
     if (args.cluster > 1) cluster_wait();
     pdl_wait();        // from here on the kernel reads what earlier kernels of the stream wrote
 
@@ -1100,7 +1133,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                 #pragma unroll
                 for (int q = 0; q < NG; ++q) A[mb][q] = 0.0f;
             }
-            if (args.finish) {
+            if (w.whole) {
                 // The second fold's seed.
                 if (args.count_sink) {
                     const uint16_t bits = args.sinks && q_self < G ? args.sinks[w.kv_head * G + q_self] : kNoSinkBits;
@@ -1114,6 +1147,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                     for (int q = 0; q < NG; ++q) state[(mb * NG + q) * 128 + tid] = seed;
                 }
             }
+            if (tid == 0 && !w.whole) bars->cut = 1;
             for (int j = 0; j < w.n_tiles; ++j, ++t) {
                 const int ob = int(t & 1);
                 const int tile = w.tile_first + j * world;
@@ -1182,7 +1216,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                 const int segment = tile >> log_segment;
                 if (j + 1 < w.n_tiles && ((tile + world) >> log_segment) == segment) continue;
                 // The segment's last tile here: its partial is complete.
-                if (args.finish) {
+                if (w.whole) {
                     fold_coefficients(M2, M, Mn, a, b);
                     L2 = __fmaf_rn(L2, a, __fmul_rn(L, b));
                     M2 = Mn;
@@ -1222,7 +1256,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                 M = kEmptyMax;
                 L = 0.0f;
             }
-            if (args.finish) {
+            if (w.whole) {
                 // The row's denominators to all threads, then the epilogue.
                 float* denom = bars->denom[it & 1];
                 if (DL::kSumOnTensor) {
@@ -1272,8 +1306,8 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         cluster_arrive();
         cluster_wait();                // every partial of the span has been pushed
         dec_fold_slice<D>(args, list, state, bars->push_m, bars->push_l, reinterpret_cast<DecMerge*>(p_smem), &bars->n_last);
-    } else if (!args.finish) {
-        dec_close<D, NG>(args, list, start.count, reinterpret_cast<float*>(k_ring), reinterpret_cast<DecMerge*>(p_smem),
+    } else if (bars->cut) {
+        dec_close<D, NG>(args, list, reinterpret_cast<float*>(k_ring), reinterpret_cast<DecMerge*>(p_smem),
                          reinterpret_cast<int*>(state), &bars->n_work, bars->merge_full, abort_flag);
     }
     if (world > 1) dec_seed_rows<D, NG>(args);
@@ -1297,11 +1331,11 @@ hc_status configure_decode_kernel(hc_context* ctx) {
 }
 
 template <int D, int NG>
-hc_status launch_decode_kernel(hc_context* ctx, const DecArgs& args, const hc_layer_store& layer, cudaStream_t stream) {
+hc_status launch_decode_kernel(hc_context* ctx, const DecArgs& args, int grid, const hc_layer_store& layer, cudaStream_t stream) {
     const hc_status st = configure_decode_kernel<D, NG>(ctx);
     if (st != HC_OK) return st;
     cudaLaunchConfig_t config = {};
-    config.gridDim = args.cluster > 1 ? args.n_items * args.cluster : std::max(1, std::min(args.n_items, std::max(ctx->sm_count, 1)));
+    config.gridDim = grid;
     config.blockDim = kTcThreads;
     config.dynamicSmemBytes = decode_smem<D, NG>();
     config.stream = stream;
@@ -1321,8 +1355,9 @@ hc_status launch_decode_kernel(hc_context* ctx, const DecArgs& args, const hc_la
 }
 
 template <int D>
-hc_status launch_decode_dim(hc_context* ctx, const DecArgs& args, const hc_layer_store& layer, cudaStream_t stream) {
-    return args.log_group <= 3 ? launch_decode_kernel<D, 8>(ctx, args, layer, stream) : launch_decode_kernel<D, 16>(ctx, args, layer, stream);
+hc_status launch_decode_dim(hc_context* ctx, const DecArgs& args, int grid, const hc_layer_store& layer, cudaStream_t stream) {
+    return args.log_group <= 3 ? launch_decode_kernel<D, 8>(ctx, args, grid, layer, stream)
+                               : launch_decode_kernel<D, 16>(ctx, args, grid, layer, stream);
 }
 
 }  // namespace
@@ -1356,8 +1391,7 @@ hc_status decode_cluster_slots(hc_context* ctx) {
 
 // How a launch cuts its rows, by the time of its busiest thread block in units of one key tile (about 0.75 us of
 // HBM at head_dim 64, proportional to it).  A launch's (or a wave of clusters') ramp is about 1.3 us, the merge
-// 1 us inside a cluster, 2.5 us when it goes over global memory and tickets, whatever the head_dim; an item costs about
-// half a tile.
+// 1.5 us inside a cluster, 3.5 us when it goes over global memory and tickets, whatever the head_dim.
 TcDecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const RowMap& map, const BatchMeta& meta, int n_seq) {
     const int sms = std::max(ctx->sm_count, 1);
     TcDecodePlan plan{};
@@ -1366,40 +1400,30 @@ TcDecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const
     for (int b = 0; b < n_seq; ++b) {
         const int n = row_tiles(map, meta.pos[b], meta.pos[b], shape.window).count;
         most_tiles = std::max(most_tiles, n);
-        tiles += n;
+        tiles += std::max(n, 0);
         const int g = visible_groups(meta.pos[b], meta.pos[b], shape.window, map.log_segment);
         most_segments = std::max(most_segments, g);
         segments += g;
     }
     const int d = shape.head_dim;
-    const long long rows = (long long)n_seq * shape.kv_heads;
-    const double even = double(tiles) * shape.kv_heads / sms;
+    const int segment_tiles = 1 << map.log_segment;
     const double us = 85.0 / d;                     // tiles per microsecond
-    plan.finish = 1;
+    // A line over all SMs, or over as many thread blocks as there are segments.
+    const long long all_segments = segments * shape.kv_heads;
     plan.cluster = 1;
-    plan.slots = 1;
+    plan.blocks = int(std::max(1LL, std::min<long long>(sms, all_segments)));
     plan.run_segments = 1;
-    double best = rows <= sms ? most_tiles : even + 0.7 * most_tiles;
+    plan.slots = most_segments;
+    const bool rows_cut = (long long)n_seq * shape.kv_heads < plan.blocks || most_segments > 1;
+    const double even = double(tiles) * shape.kv_heads / plan.blocks;
+    double best = std::max(even + (all_segments > plan.blocks ? 0.5 * std::min(most_tiles, segment_tiles) : 0.0),
+                           double(std::min(most_tiles, segment_tiles))) + (rows_cut ? 3.5 * us : 0.0) + 1.3 * us;
     if (most_tiles > 2) {
-        const int segment_tiles = 1 << map.log_segment;
-        const double size = std::min(most_tiles, segment_tiles);
-        const long long items = segments * shape.kv_heads;
-        const double per_item = size + 0.5;
-        const double filled = double(tiles) / std::max(1.0, segments * size);
-        double t = items <= 4LL * sms ? double((items + sms - 1) / sms) * per_item : double(items) / sms * per_item + 0.5 * size;
-        t = std::max(t * filled, even) + 2.5 * us;
-        if (t < best) {
-            best = t;
-            plan.finish = 0;
-            // About six items per thread block, so that the static round robin evens out.
-            plan.run_segments = int(std::max(1LL, std::min(64LL, items / (6LL * sms))));
-            plan.slots = most_segments;
-        }
         for (int i = 0; i < 4; ++i) {
             const int cluster = 2 << i;
-            const int slots = ctx->cluster_slots[i];
+            const int resident = ctx->cluster_slots[i] / cluster;
             const int width = shape.group * d / cluster;
-            if (slots < cluster || width < 4) continue;
+            if (resident < 1 || width < 4) continue;
             const int slice_rows = std::max(1, width / d);
             const int most_span = std::min(kPushBytes / 4 / width, kPushTiles / slice_rows);
             // A whole row per cluster, or spans of as many segments as fit, evened out.
@@ -1417,23 +1441,22 @@ TcDecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const
             }
             clusters *= shape.kv_heads;
             const int span_tiles = std::min(most_tiles, run * segment_tiles);
-            const long long waves = (clusters * cluster + slots - 1) / slots;
-            const double tc = double(waves) * ((span_tiles + cluster - 1) / cluster + 1.3 * us) + (run < most_segments ? 2.5 : 1.0) * us;
-            if (tc < best) {
-                best = tc;
-                plan.finish = 0;
+            const long long waves = (clusters + resident - 1) / resident;
+            // The slice's last span folds width x segments values that others left, 512 at a time.
+            const double merge = run == most_segments ? 1.5 : 3.5 + (width * most_segments >> 9) * 0.04;
+            const double t = double(waves) * ((span_tiles + cluster - 1) / cluster + 1.3 * us) + merge * us;
+            if (t < best) {
+                best = t;
                 plan.cluster = cluster;
+                plan.blocks = int(std::min<long long>(clusters * cluster, 1 << 30));
                 plan.run_segments = run;
-                plan.slots = most_segments;
             }
         }
     }
-    if (!plan.finish) {
-        const size_t q_rows = size_t(n_seq) * shape.q_heads;
-        plan.part_o_floats = q_rows * plan.slots * d;
-        plan.part_ml_floats = (q_rows * plan.slots * 2 + 3) & ~size_t(3);
-        plan.tickets = size_t(rows) * plan.cluster;
-    }
+    const size_t q_rows = size_t(n_seq) * shape.q_heads;
+    plan.part_o_floats = q_rows * plan.slots * d;
+    plan.part_ml_floats = (q_rows * plan.slots * 2 + 3) & ~size_t(3);
+    plan.tickets = size_t(n_seq) * shape.kv_heads * plan.cluster;
     return plan;
 }
 
@@ -1471,40 +1494,41 @@ hc_status tc_decode(hc_context* ctx, const AttnShape& shape, const hc_layer_stor
     args.ep = ep;
     args.status = ctx->status_dev;
     args.n_seq = n_seq;
-    args.finish = plan.finish;
     args.cluster = plan.cluster;
     args.slots = plan.slots;
     args.part_o = ws.part_o;
     args.part_ml = ws.part_ml;
     args.tickets = ws.tickets;
     args.meta = meta;
-    // One item per (sequence, kv head, run of the sequence's visible segments).
-    int next = 0;
+    long long next = 0;
     for (int b = 0; b < n_seq; ++b) {
-        int n = 1;
-        if (!plan.finish) {
-            // Runs of one size, plan.run_segments each at most.
+        args.start[b] = int(next);
+        if (plan.cluster == 1) {
+            next += (long long)std::max(row_tiles(cache.map, meta.pos[b], meta.pos[b], shape.window).count, 0) * shape.kv_heads;
+        } else {
+            // Spans of one size, plan.run_segments each at most.
             const int segments = visible_groups(meta.pos[b], meta.pos[b], shape.window, cache.map.log_segment);
             const int want = (segments + plan.run_segments - 1) / plan.run_segments;
             const int run = (segments + want - 1) / want;
-            n = (segments + run - 1) / run;
             args.seq_run[b] = static_cast<unsigned short>(run);
+            args.seq_spans[b] = static_cast<unsigned short>((segments + run - 1) / run);
+            next += (long long)args.seq_spans[b] * shape.kv_heads;
         }
-        args.item_start[b] = next;
-        args.seq_slots[b] = static_cast<unsigned short>(n);
-        args.seq_magic[b] = division_magic(uint32_t(n), uint32_t(n) * uint32_t(shape.kv_heads));
-        next += n * shape.kv_heads;
     }
-    for (int b = n_seq; b <= kMaxBatch; ++b) args.item_start[b] = next;
-    args.n_items = next;
-    if (plan.cluster == 1 && next > kDecItems * std::max(ctx->sm_count, 1)) {
-        return fail(HC_UNSUPPORTED, "decode: too many (sequence, kv head) rows for one launch");
+    for (int b = n_seq; b <= kMaxBatch; ++b) args.start[b] = int(next);
+    args.n_tiles = int(next);
+    const int grid = plan.blocks;
+    // A thread block's stretch of the line touches no more rows than it has tiles, nor more than there are.
+    const long long rows = (long long)n_seq * shape.kv_heads;
+    const long long stretch = next / grid + 2 * (1 << cache.map.log_segment) + 2;
+    if (next > 0x7fffffffLL || (plan.cluster == 1 && std::min(rows, stretch) > kDecItems)) {
+        return fail(HC_UNSUPPORTED, "decode: too many key tiles or rows for one launch");
     }
     switch (shape.head_dim) {
-        case 64: return launch_decode_dim<64>(ctx, args, layer, stream);
-        case 128: return launch_decode_dim<128>(ctx, args, layer, stream);
-        case 256: return launch_decode_dim<256>(ctx, args, layer, stream);
-        default: return launch_decode_dim<512>(ctx, args, layer, stream);
+        case 64: return launch_decode_dim<64>(ctx, args, grid, layer, stream);
+        case 128: return launch_decode_dim<128>(ctx, args, grid, layer, stream);
+        case 256: return launch_decode_dim<256>(ctx, args, grid, layer, stream);
+        default: return launch_decode_dim<512>(ctx, args, grid, layer, stream);
     }
 }
 

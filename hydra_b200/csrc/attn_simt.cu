@@ -867,7 +867,9 @@ hc_status hc_attention_decode_static(hc_context* ctx, hc_kv_cache* cache, int la
     // puts it), whichever kernels run: a caller's program is not refused by one build and served by the next.
     const size_t rows = size_t(n_seq) * shape.q_heads;
     const int target = tensor ? (shape.head_dim == 256 ? 1 : 6) * std::max(ctx->sm_count, 1) : 0;
-    const DecodePlan plan = tensor ? plan_decode(shape, view.map, meta, n_seq, target, true, 64)
+    RowMap general = view.map;
+    general.log_segment = store->log_segment_general;
+    const DecodePlan plan = tensor ? plan_decode(shape, general, meta, n_seq, target, true, 64)
                                    : simt_plan_decode(ctx, shape, view.map, meta, n_seq);
     size_t ml_floats = plan.finish ? 0 : (rows * plan.slots * 2 + 3) & ~size_t(3);
     size_t o_floats = plan.finish ? 0 : rows * plan.slots * shape.head_dim;

@@ -161,6 +161,7 @@ struct hc_layer_store {
                                   // append at once and how far a rewind may reach
     int capacity = 0;
     int log_segment = 0;          // key tiles per segment, as a power of two (see common.cuh)
+    int log_segment_general = 0;  // the same by the head counts alone: what hc_attention_decode_static's limit goes by
     bool keeps_history = false;
     void* tmap_k = nullptr;       // tensor maps of the tcgen05 path (host copies), or null
     void* tmap_v = nullptr;
@@ -255,9 +256,9 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
 // attn_decode.cu
 // How a tcgen05 decode launch cuts its rows' keys, and the workspace that takes.
 struct TcDecodePlan {
-    int finish;              // whole rows per item
-    int cluster;             // otherwise: thread blocks that share a run of segments (1: none) ..
-    int run_segments;        // .. and about how many segments a run has
+    int cluster;             // thread blocks that share a span of run_segments segments; 1: equal stretches of all rows
+    int blocks;              // thread blocks
+    int run_segments;
     int slots;               // partial slots per row: segments
     size_t part_o_floats, part_ml_floats, tickets;
 };
