@@ -10,12 +10,14 @@
 // of the weight once per token, this kernel computes a 128 x 256 tile of y per step, so a weight
 // tile fetched by TMA serves 128 tokens.
 //
-// One persistent CTA per SM walks the output tiles (all row tiles of one 256-wide column tile are
-// adjacent in the walk, so the CTAs running at one time share a weight tile in L2):
-//   warp 0      TMA producer: x tile (128 x 64) and w tile (256 x 64) per K step into a 4-stage ring
+// Two kernels.  A call of up to 128 tokens reads the weights once and little else: linear_few_kernel, one CTA
+// per SM, 128 x 32 output tiles with nine stages in flight.  Prompts are bound by the tensor pipe:
+// linear_pair_kernel, where two SMs share a 256-row output tile (cta_group::2: each loads its own 128
+// rows of x and half of the weight tile, so a K step brings 24 to 32 KB into each SM for 256 x BN outputs where a
+// CTA of its own needed 48 KB for 128 x 256), six to eight stages, two accumulators in tensor memory.
+//   warp 0      TMA producer: x tile and w tile per K step of 64 into the ring
 //               (a launch may carry up to four projections of the same x: one list of tiles)
-//   warp 1      MMA issuer: four tcgen05.mma (M 128, N 256, K 16) per K step into one of two
-//               accumulators in tensor memory (2 x 256 columns)
+//   warp 1      MMA issuer (of the leading CTA): four tcgen05.mma per K step into one of two accumulators
 //   warps 4-7   epilogue: the finished accumulator from tensor memory, + bias (+ residual), to y (fp32 or bf16),
 //               thread = row, while the next tile's MMAs fill the other accumulator
 // Every mbarrier wait is bounded and reports through the context's status word.
@@ -32,27 +34,34 @@ constexpr int kLinM = 128;
 constexpr int kLinK = 64;                       // one 128-byte swizzled row of bf16
 constexpr int kLinABytes = kLinM * kLinK * 2;   // 16 KB
 constexpr int kLinThreads = 256;
-constexpr int kLinMaxStages = 9;
 
-// Two shapes of the same kernel.  Wide: 128 x 256 output tiles, 4 stages: tensor-bound, for prompts.
-// Narrow: 128 x 32 tiles, 9 stages: when there are at most 128 tokens (decode) the work is reading
-// the weight once, and narrow column tiles spread its rows over all SMs with enough of them in
-// flight (9 x 4 KB per SM).  An output element is the same sum in the same order in both, so a token
-// projected alone and inside a prompt gets the same bits.
+// Few tokens: 128 x 32 tiles, nine stages: narrow column tiles spread the weight's rows over all SMs with
+// enough of them in flight (9 x 4 KB per SM).
+constexpr int kFewN = 32;
+constexpr int kFewStages = 9;
+constexpr int kFewBBytes = kFewN * kLinK * 2;
+constexpr int kFewTmemCols = 64;                // two accumulators
+constexpr int kFewSmemBytes = 1024 + kFewStages * (kLinABytes + kFewBBytes);
+
+// Pairs: 256 x BN tiles, each CTA holding 128 rows of x and BN / 2 rows of w per stage.  An output element is the same
+// sum in the same order in every shape, so a token projected alone and inside a prompt gets the same bits.
 template <int BN>
-struct LinShape {
-    static constexpr int kStages = BN == 256 ? 4 : kLinMaxStages;
-    static constexpr int kBBytes = BN * kLinK * 2;
-    static constexpr int kTmemCols = BN == 256 ? 512 : 64;      // two accumulators
+struct PairShape {
+    static constexpr int kStages = BN >= 224 ? 6 : BN >= 160 ? 7 : 8;
+    static constexpr int kBBytes = BN / 2 * kLinK * 2;
+    static constexpr int kTmemCols = 2 * BN <= 256 ? 256 : 512;
     static constexpr int kSmemBytes = 1024 + kStages * (kLinABytes + kBBytes);
 };
 
+constexpr int kLinMaxStages = 9;
 struct LinBarriers {
     uint64_t full[kLinMaxStages], empty[kLinMaxStages];
     uint64_t acc_full[2], acc_empty[2];
     uint32_t tmem_base;
     int abort_flag;
+    int pad[2];
 };
+static_assert(sizeof(LinBarriers) % 16 == 0, "the staging behind it is 16-byte aligned");
 
 constexpr int kLinJobs = 4;
 
@@ -71,7 +80,7 @@ struct LinArgs {
     int n_jobs;
     int y_dtype;              // HC_F32 or HC_BF16
     int tokens;
-    int tiles_m, n_tiles, k_steps;
+    int tiles_m, n_tiles, k_steps;   // tiles of 128 rows (few tokens) or 256 (pairs)
     int a_bytes;              // of one x box: 128 rows x 128 bytes, fewer rows for a call of few tokens
     int* status;
 };
@@ -99,20 +108,86 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
         : "memory");
 }
 
-template <int BN>
+// 32 accumulator columns of a warp's 32 rows (lane = row in `v`): + bias (+ residual), to y.  The block goes through
+// 4 KB of shared memory so that a store instruction writes four rows' whole 128-byte lines (64 for bf16)
+// instead of 16 bytes of 32 rows, and the residual is read the same way, a block ahead: it may be y itself, so the
+// compiler may not move a load across a store, and a block's eight loads one after the other cost more
+// than its MMAs (o_proj of 4096 tokens: 141 us).
+constexpr int kLinStageBytes = 32 * 128;
+__device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob& job, int row0, int col0, float4 (&z)[8]) {
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) z[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (job.residual == nullptr) return;
+    const int lane = threadIdx.x & 31;
+    const int col = col0 + (lane & 7) * 4;
+    if (col + 4 > job.out_features || (job.out_features & 3) != 0) return;      // read element by element when it is added
+    const bool aligned = (reinterpret_cast<uintptr_t>(job.residual) & 15) == 0;
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int row = row0 + k * 4 + (lane >> 3);
+        if (row >= args.tokens) continue;
+        const float* src = job.residual + size_t(row) * job.out_features + col;
+        if (aligned) z[k] = *reinterpret_cast<const float4*>(src);
+        else z[k] = make_float4(src[0], src[1], src[2], src[3]);
+    }
+}
+__device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4 (&z)[8], int row0,
+                                            int col0, unsigned char* stage) {
+    if (col0 >= job.out_features || row0 >= args.tokens) return;          // warp-uniform
+    const int lane = threadIdx.x & 31;
+    #pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        *reinterpret_cast<uint4*>(stage + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    }
+    __syncwarp();
+    const int chunk = lane & 7, col = col0 + chunk * 4;
+    const bool vectors = col + 4 <= job.out_features && (job.out_features & 3) == 0;
+    float b[4];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = job.bias != nullptr && col + i < job.out_features ? bf16_bits_to_float(__ldg(job.bias + col + i)) : 0.0f;
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int r = k * 4 + (lane >> 3);
+        if (row0 + r >= args.tokens) continue;
+        const float4 x = *reinterpret_cast<const float4*>(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
+        float y[4] = {__fadd_rn(x.x, b[0]), __fadd_rn(x.y, b[1]), __fadd_rn(x.z, b[2]), __fadd_rn(x.w, b[3])};
+        const size_t at = size_t(row0 + r) * job.out_features + col;
+        if (vectors) {
+            if (job.residual != nullptr) {
+                y[0] = __fadd_rn(y[0], z[k].x); y[1] = __fadd_rn(y[1], z[k].y); y[2] = __fadd_rn(y[2], z[k].z); y[3] = __fadd_rn(y[3], z[k].w);
+            }
+            if (args.y_dtype == HC_F32) {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(job.y) + at) = make_float4(y[0], y[1], y[2], y[3]);
+            } else {
+                uint2 packed;
+                packed.x = uint32_t(float_to_bf16_bits(y[0])) | (uint32_t(float_to_bf16_bits(y[1])) << 16);
+                packed.y = uint32_t(float_to_bf16_bits(y[2])) | (uint32_t(float_to_bf16_bits(y[3])) << 16);
+                *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(job.y) + at) = packed;
+            }
+        } else {
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (col + i >= job.out_features) continue;
+                if (job.residual != nullptr) y[i] = __fadd_rn(y[i], job.residual[at + i]);
+                store_io(job.y, at + i, args.y_dtype, y[i]);
+            }
+        }
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(kLinThreads, 1)
-linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
+linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
                  const __grid_constant__ CUtensorMap tmap_w1, const __grid_constant__ CUtensorMap tmap_w2,
                  const __grid_constant__ CUtensorMap tmap_w3, const LinArgs args) {
-    using LS = LinShape<BN>;
-    constexpr int kLinN = BN;
-    constexpr int kLinStages = LS::kStages;
-    constexpr int kLinBBytes = LS::kBBytes;
+    constexpr int kLinN = kFewN;
+    constexpr int kLinStages = kFewStages;
+    constexpr int kLinBBytes = kFewBBytes;
     extern __shared__ unsigned char raw_smem[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
     unsigned char* a_smem = base;                                   // [stages][128 x 64]
     unsigned char* b_smem = a_smem + kLinStages * kLinABytes;       // [stages][256 x 64]
-    LinBarriers* bars = reinterpret_cast<LinBarriers*>(b_smem + kLinStages * kLinBBytes);
+    LinBarriers* bars = reinterpret_cast<LinBarriers*>(b_smem + kLinStages * kLinBBytes);        // and the epilogue's staging
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &bars->abort_flag;
@@ -130,7 +205,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         bars->abort_flag = 0;
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(&bars->tmem_base, LS::kTmemCols);
+    if (warp == 1) tmem_alloc(&bars->tmem_base, kFewTmemCols);
     if (warp == 0 && lane == 0) {
         prefetch_tensormap(&tmap_x);
         prefetch_tensormap(&tmap_w0);
@@ -194,7 +269,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     } else if (warp >= 4) {
         // ===== epilogue: thread = row of the tile =====
         const int quad = warp & 3;
-        const int row_in_tile = quad * 32 + lane;
+        unsigned char* stage = reinterpret_cast<unsigned char*>(bars + 1) + quad * kLinStageBytes;
         const uint32_t lane_base = uint32_t(quad * 32) << 16;
         uint32_t count = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++count) {
@@ -202,57 +277,16 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             const int tn = where.tn, tm = where.tm;
             const LinJob& job = args.job[where.job];
             const int acc = int(count & 1);
+            float4 z[8];
+            load_residual(args, job, tm * kLinM + quad * 32, tn * kLinN, z);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
-            const int row = tm * kLinM + row_in_tile;
-            const bool row_ok = row < args.tokens;
-            #pragma unroll 1
+            static_assert(kLinN == 32, "one block per tile");
             for (int chunk = 0; chunk < kLinN / 32; ++chunk) {
                 uint32_t v[32];
                 HC_TMEM_LD32(tmem + lane_base + acc * kLinN + chunk * 32, v);
                 tc_wait_ld();
-                const int col0 = tn * kLinN + chunk * 32;
-                if (row_ok && col0 < job.out_features) {
-                float r[32];
-                #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int col = col0 + i;
-                    const float b = (job.bias != nullptr && col < job.out_features) ? bf16_bits_to_float(__ldg(job.bias + col)) : 0.0f;
-                    r[i] = __fadd_rn(__uint_as_float(v[i]), b);
-                }
-                const size_t offset = size_t(row) * job.out_features + col0;
-                if (job.residual != nullptr) {
-                    #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        if (col0 + i < job.out_features) r[i] = __fadd_rn(r[i], __ldg(job.residual + offset + i));
-                    }
-                }
-                const bool whole = col0 + 32 <= job.out_features && (job.out_features & 7) == 0;
-                if (args.y_dtype == HC_F32) {
-                    float* dst = reinterpret_cast<float*>(job.y) + offset;
-                    if (whole) {
-                        #pragma unroll
-                        for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(r[i], r[i + 1], r[i + 2], r[i + 3]);
-                    } else {
-                        for (int i = 0; i < 32 && col0 + i < job.out_features; ++i) dst[i] = r[i];
-                    }
-                } else {
-                    uint16_t* dst = reinterpret_cast<uint16_t*>(job.y) + offset;
-                    if (whole) {
-                        #pragma unroll
-                        for (int i = 0; i < 32; i += 8) {
-                            uint4 packed;
-                            packed.x = uint32_t(float_to_bf16_bits(r[i])) | (uint32_t(float_to_bf16_bits(r[i + 1])) << 16);
-                            packed.y = uint32_t(float_to_bf16_bits(r[i + 2])) | (uint32_t(float_to_bf16_bits(r[i + 3])) << 16);
-                            packed.z = uint32_t(float_to_bf16_bits(r[i + 4])) | (uint32_t(float_to_bf16_bits(r[i + 5])) << 16);
-                            packed.w = uint32_t(float_to_bf16_bits(r[i + 6])) | (uint32_t(float_to_bf16_bits(r[i + 7])) << 16);
-                            *reinterpret_cast<uint4*>(dst + i) = packed;
-                        }
-                    } else {
-                        for (int i = 0; i < 32 && col0 + i < job.out_features; ++i) dst[i] = float_to_bf16_bits(r[i]);
-                    }
-                }
-                }
+                store_block(args, job, v, z, tm * kLinM + quad * 32, tn * kLinN + chunk * 32, stage);
                 __syncwarp();          // the next tcgen05.ld is warp-wide
             }
             tc_fence_before();
@@ -267,7 +301,146 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, LS::kTmemCols);
+    if (warp == 1) tmem_dealloc(tmem, kFewTmemCols);
+}
+
+// Two SMs per 256 x BN tile; see the head of the file.  The leading CTA's barriers count both CTAs' loads.
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLinThreads, 1)
+linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
+                   const __grid_constant__ CUtensorMap tmap_w1, const __grid_constant__ CUtensorMap tmap_w2,
+                   const __grid_constant__ CUtensorMap tmap_w3, const LinArgs args) {
+    using PS = PairShape<BN>;
+    extern __shared__ unsigned char raw_smem[];
+    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
+    unsigned char* a_smem = base;                                   // [stages][128 x 64]
+    unsigned char* b_smem = a_smem + PS::kStages * kLinABytes;      // [stages][BN / 2 x 64]
+    LinBarriers* bars = reinterpret_cast<LinBarriers*>(b_smem + PS::kStages * PS::kBBytes);      // and the epilogue's staging
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int rank = int(cluster_rank());
+    const int pair = int(blockIdx.x) >> 1, pairs = int(gridDim.x) >> 1;
+    volatile int* abort_flag = &bars->abort_flag;
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < PS::kStages; ++i) {
+            mbar_init(&bars->full[i], 1);
+            mbar_init(&bars->empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->acc_full[i], 1);
+            mbar_init(&bars->acc_empty[i], 8);                      // the epilogue warps of both CTAs
+        }
+        bars->abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc_pair(&bars->tmem_base, PS::kTmemCols);
+    if (warp == 0 && lane == 0) {
+        prefetch_tensormap(&tmap_x);
+        prefetch_tensormap(&tmap_w0);
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();                 // the peer's barriers are there
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    pdl_wait();
+
+    const int n_tiles = args.n_tiles;
+    if (warp == 0) {
+        // ===== producer: this CTA's rows of x and its half of the weight tile, counted by the leader =====
+        if (lane == 0) {
+            uint32_t step = 0;
+            bool ok = true;
+            for (int tile = pair; ok && tile < n_tiles; tile += pairs) {
+                const LinTile where = decode_tile(args, tile);
+                const int tn = where.tn, tm = where.tm;
+                const CUtensorMap* tmap_w = where.job == 0 ? &tmap_w0 : where.job == 1 ? &tmap_w1 : where.job == 2 ? &tmap_w2 : &tmap_w3;
+                for (int k = 0; k < args.k_steps; ++k, ++step) {
+                    const int slot = int(step % PS::kStages);
+                    const uint32_t round = step / PS::kStages;
+                    if (round > 0 && !mbar_wait(&bars->empty[slot], (round - 1) & 1, abort_flag, args.status, 21)) { ok = false; break; }
+                    const uint32_t full = cluster_addr(&bars->full[slot], 0);
+                    if (rank == 0) mbar_expect_tx(&bars->full[slot], 2 * (kLinABytes + PS::kBBytes));
+                    tma_load_2d_pair(a_smem + slot * kLinABytes, &tmap_x, full, k * kLinK, tm * (2 * kLinM) + rank * kLinM);
+                    tma_load_2d_pair(b_smem + slot * PS::kBBytes, tmap_w, full, k * kLinK, tn * BN + rank * (BN / 2));
+                }
+            }
+        }
+    } else if (warp == 1 && rank == 0) {
+        // ===== MMA issuer (the warp walks the loop converged; one elected lane issues) =====
+        constexpr uint32_t idesc = instr_desc_pair(BN, false);
+        const uint64_t a_desc0 = smem_desc(smem_u32(a_smem), 16);
+        const uint64_t b_desc0 = smem_desc(smem_u32(b_smem), 16);
+        uint32_t step = 0, count = 0;
+        bool ok = true;
+        for (int tile = pair; ok && tile < n_tiles; tile += pairs, ++count) {
+            const int acc = int(count & 1);
+            // The epilogues must have taken this accumulator's previous tile out.
+            if (count >= 2 && !mbar_wait(&bars->acc_empty[acc], ((count >> 1) - 1) & 1, abort_flag, args.status, 22)) break;
+            tc_fence_after();
+            for (int k = 0; k < args.k_steps; ++k, ++step) {
+                const int slot = int(step % PS::kStages);
+                if (!mbar_wait(&bars->full[slot], (step / PS::kStages) & 1, abort_flag, args.status, 23)) { ok = false; break; }
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint64_t a_desc = a_desc0 + uint64_t((slot * kLinABytes) >> 4);
+                    const uint64_t b_desc = b_desc0 + uint64_t((slot * PS::kBBytes) >> 4);
+                    #pragma unroll
+                    for (int ks = 0; ks < kLinK / 16; ++ks) {
+                        mma_ss_pair(tmem + acc * BN, a_desc + uint64_t((ks * 32) >> 4), b_desc + uint64_t((ks * 32) >> 4), idesc,
+                                    (k | ks) != 0 ? 1u : 0u);
+                    }
+                    tc_commit_pair(&bars->empty[slot]);
+                    if (k + 1 == args.k_steps) tc_commit_pair(&bars->acc_full[acc]);
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp >= 4) {
+        // ===== epilogue: thread = row of this CTA's half of the tile =====
+        const int quad = warp & 3;
+        unsigned char* stage = reinterpret_cast<unsigned char*>(bars + 1) + quad * kLinStageBytes;
+        const uint32_t lane_base = uint32_t(quad * 32) << 16;
+        uint32_t count = 0;
+        for (int tile = pair; tile < n_tiles; tile += pairs, ++count) {
+            const LinTile where = decode_tile(args, tile);
+            const LinJob& job = args.job[where.job];
+            const int row0 = where.tm * (2 * kLinM) + rank * kLinM + quad * 32;
+            const int acc = int(count & 1);
+            float4 z[8], z_next[8];
+            load_residual(args, job, row0, where.tn * BN, z);
+            if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
+            tc_fence_after();
+            #pragma unroll 1
+            for (int chunk = 0; chunk < BN / 32; ++chunk) {
+                uint32_t v[32];
+                HC_TMEM_LD32(tmem + lane_base + acc * BN + chunk * 32, v);
+                if (chunk + 1 < BN / 32) load_residual(args, job, row0, where.tn * BN + (chunk + 1) * 32, z_next);
+                tc_wait_ld();
+                store_block(args, job, v, z, row0, where.tn * BN + chunk * 32, stage);
+                #pragma unroll
+                for (int k = 0; k < 8; ++k) z[k] = z_next[k];
+                __syncwarp();          // the next tcgen05.ld is warp-wide
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(&bars->acc_empty[acc], 0));
+        }
+    }
+
+    // Teardown.  On the abort path the producer first lets its copies in flight land (bounded).
+    if (warp == 0 && lane == 0 && *abort_flag != 0) {
+        const long long start = clock64();
+        while (static_cast<unsigned long long>(clock64() - start) < 200000000ull) { }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();                 // neither CTA leaves while the other's MMAs or arrivals may still name it
+    if (warp == 1) tmem_dealloc_pair(tmem, PS::kTmemCols);
 }
 
 }  // namespace
@@ -308,43 +481,68 @@ static hc_status cached_map(CUtensorMap* out, const void* base, uint64_t rows, u
     return HC_OK;
 }
 
-template <int BN>
-static hc_status launch_linear(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features,
-                               cudaStream_t stream) {
-    using LS = LinShape<BN>;
-    CUtensorMap tmap_x, tmap_w[kLinJobs];
+// Tensor maps and the tile list of a launch with column tiles of `bn` and row tiles of `bm` over boxes of x_rows and
+// w_rows rows.
+struct LinMaps {
+    CUtensorMap x, w[kLinJobs];
+};
+static hc_status prepare_linear(LinMaps& maps, const void* x, const void* const* w, LinArgs& args, int in_features, int bm, int bn,
+                                int x_rows, int w_rows) {
+    hc_status st = cached_map(&maps.x, x, uint64_t(args.tokens), uint64_t(in_features), uint32_t(x_rows));
+    args.tiles_m = (args.tokens + bm - 1) / bm;
+    int tiles = 0;
+    for (int j = 0; j < kLinJobs && st == HC_OK; ++j) {
+        const int source = j < args.n_jobs ? j : 0;            // unused maps repeat the first
+        st = cached_map(&maps.w[j], w[source], uint64_t(args.job[source].out_features), uint64_t(in_features), uint32_t(w_rows));
+        if (j < args.n_jobs) {
+            args.job[j].first_tile = tiles;
+            tiles += args.tiles_m * ((args.job[j].out_features + bn - 1) / bn);
+        }
+    }
+    args.n_tiles = tiles;
+    return st;
+}
+
+template <typename Kernel>
+static hc_status launch_linear_kernel(hc_context* ctx, Kernel kernel, bool (&configured)[64], int grid, int smem, const LinMaps& maps,
+                                      const LinArgs& args, cudaStream_t stream) {
+    if (!configured[ctx->device & 63]) {
+        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (err != cudaSuccess) return check_cuda(err, "linear kernel shared memory");
+        configured[ctx->device & 63] = true;
+    }
+    const cudaError_t launched = launch_pdl(kernel, grid, kLinThreads, size_t(smem), stream, maps.x, maps.w[0], maps.w[1], maps.w[2],
+                                            maps.w[3], args);
+    ctx->launches += 1;
+    return check_cuda(launched, "linear kernel launch");
+}
+
+static hc_status launch_few(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features, cudaStream_t stream) {
+    LinMaps maps;
     // A box that reaches past the last token is filled with zeros, and that fill measured slower than
     // reading real rows (one token: 21 us against 13 us for 128): a call of few tokens loads only the
     // rows it has.  The rows of the 128-row operand tile it leaves unwritten feed accumulator rows that
     // are never stored (a row of the result depends on its own row of x alone).
     const int x_rows = std::min(kLinM, (args.tokens + 7) & ~7);
     args.a_bytes = x_rows * kLinK * 2;
-    hc_status st = cached_map(&tmap_x, x, uint64_t(args.tokens), uint64_t(in_features), uint32_t(x_rows));
-    args.tiles_m = (args.tokens + kLinM - 1) / kLinM;
-    int tiles = 0;
-    for (int j = 0; j < kLinJobs && st == HC_OK; ++j) {
-        const int source = j < args.n_jobs ? j : 0;            // unused maps repeat the first
-        st = cached_map(&tmap_w[j], w[source], uint64_t(args.job[source].out_features), uint64_t(in_features), BN);
-        if (j < args.n_jobs) {
-            args.job[j].first_tile = tiles;
-            tiles += args.tiles_m * ((args.job[j].out_features + BN - 1) / BN);
-        }
-    }
+    const hc_status st = prepare_linear(maps, x, w, args, in_features, kLinM, kFewN, x_rows, kFewN);
     if (st != HC_OK) return st;
-    args.n_tiles = tiles;
-    const int smem = LS::kSmemBytes + int(sizeof(LinBarriers));
     static bool configured[64] = {};
-    if (!configured[ctx->device & 63]) {
-        cudaError_t err = cudaFuncSetAttribute(linear_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (err != cudaSuccess) return check_cuda(err, "linear_tc_kernel shared memory");
-        configured[ctx->device & 63] = true;
-    }
-    const int grid = std::max(1, std::min(tiles, std::max(ctx->sm_count, 1)));
-    const cudaError_t launched = launch_pdl(linear_tc_kernel<BN>, grid, kLinThreads, size_t(smem), stream, tmap_x, tmap_w[0],
-                                            tmap_w[1], tmap_w[2], tmap_w[3], args);
-    ctx->launches += 1;
-    if (launched != cudaSuccess) return check_cuda(launched, "linear_tc_kernel launch");
-    return check_cuda(cudaGetLastError(), "linear_tc_kernel launch");
+    const int grid = std::max(1, std::min(args.n_tiles, std::max(ctx->sm_count, 1)));
+    return launch_linear_kernel(ctx, linear_few_kernel, configured, grid, kFewSmemBytes + int(sizeof(LinBarriers)) + 4 * kLinStageBytes, maps,
+                                args, stream);
+}
+
+template <int BN>
+static hc_status launch_pair(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features, cudaStream_t stream) {
+    LinMaps maps;
+    const hc_status st = prepare_linear(maps, x, w, args, in_features, 2 * kLinM, BN, kLinM, BN / 2);
+    if (st != HC_OK) return st;
+    static bool configured[64] = {};
+    constexpr int smem = PairShape<BN>::kSmemBytes + int(sizeof(LinBarriers)) + 4 * kLinStageBytes;
+    static_assert(smem <= 227 * 1024, "shared memory of one CTA");
+    const int grid = 2 * std::max(1, std::min(args.n_tiles, std::max(ctx->sm_count / 2, 1)));
+    return launch_linear_kernel(ctx, linear_pair_kernel<BN>, configured, grid, smem, maps, args, stream);
 }
 
 hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* const* w, const void* const* bias,
@@ -362,8 +560,31 @@ hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* cons
     args.tokens = tokens;
     args.k_steps = in_features / kLinK;
     args.status = ctx->status_dev;
-    if (tokens <= kLinM) return launch_linear<32>(ctx, x, w, args, in_features, stream);
-    return launch_linear<256>(ctx, x, w, args, in_features, stream);
+    if (tokens <= kLinM) return launch_few(ctx, x, w, args, in_features, stream);
+    // The column tile whose rounds of pairs take least.  A K step costs an SM the larger of its MMAs (2 clocks a column)
+    // and of (128 + BN / 2) x 128 bytes out of L2, of which about 60 arrive per clock and SM with all of them
+    // loading: 546 clocks for 256 columns, 478, 443, 410.  Measured on 4096, 1024, 600 and 300 tokens of the three
+    // geometries: the choice is the fastest of the four or within a few percent of it.
+    const int pairs = std::max(ctx->sm_count / 2, 1);
+    const int widths[4] = {256, 192, 160, 128};
+    const double step[4] = {546.0, 478.0, 443.0, 410.0};
+    int best = 0;
+    double least = 0.0;
+    for (int i = 0; i < 4; ++i) {
+        long long tiles = 0;
+        for (int j = 0; j < n_jobs; ++j) tiles += (long long)((tokens + 2 * kLinM - 1) / (2 * kLinM)) * ((out_features[j] + widths[i] - 1) / widths[i]);
+        const double t = double((tiles + pairs - 1) / pairs) * step[i];
+        if (i == 0 || t < least) {
+            least = t;
+            best = i;
+        }
+    }
+    switch (widths[best]) {
+        case 256: return launch_pair<256>(ctx, x, w, args, in_features, stream);
+        case 192: return launch_pair<192>(ctx, x, w, args, in_features, stream);
+        case 160: return launch_pair<160>(ctx, x, w, args, in_features, stream);
+        default: return launch_pair<128>(ctx, x, w, args, in_features, stream);
+    }
 }
 
 }  // namespace hc

@@ -210,6 +210,8 @@ rms_norm_rows_kernel(const void* __restrict__ x, const uint16_t* __restrict__ sc
                      float eps, int x_dtype, int out_dtype, int vectors) {
     __shared__ float warp_sum[8];
     __shared__ float inverse;
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t base = size_t(blockIdx.x) * width;
     float partial = 0.0f;
     float4 held[kNormVecs];
@@ -337,7 +339,8 @@ hc_status launch_rms_norm_rows(hc_context* ctx, const void* x, const uint16_t* s
     const bool vectors = width % 4 == 0 && width <= 256 * 4 * 4 && aligned16(x) && aligned16(out) &&
                          (scale == nullptr || (reinterpret_cast<uintptr_t>(scale) & 7u) == 0) &&
                          (width % 8 == 0 || (x_dtype == HC_F32 && out_dtype == HC_F32));
-    rms_norm_rows_kernel<<<unsigned(tokens), 256, 0, stream>>>(x, scale, out, width, eps, x_dtype, out_dtype, vectors ? 1 : 0);
+    launch_pdl(rms_norm_rows_kernel, dim3(unsigned(tokens)), dim3(256), 0, stream, x, scale, out, width, eps, x_dtype, out_dtype,
+               vectors ? 1 : 0);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "rms_norm_rows_kernel launch");
 }
