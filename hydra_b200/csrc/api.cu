@@ -208,7 +208,7 @@ bool use_tensor_path(const hc_attn_params* p, const AttnShape& shape, hc_status*
     if (p->kernel_path == HC_PATH_SIMT || (p->kernel_path == HC_PATH_AUTO && env && env[0] == '1')) return false;
     const bool ok = tc_supported(shape);
     if (p->kernel_path == HC_PATH_TENSOR && !ok) {
-        *status = fail(HC_UNSUPPORTED, "the tcgen05 path serves head_dim 64, 128 and 256 only");
+        *status = fail(HC_UNSUPPORTED, "the tcgen05 path serves head_dim 64, 128, 256 and 512 only");
         return false;
     }
     return ok;
@@ -762,21 +762,21 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         max_kv_elems = std::max(max_kv_elems, size_t(L.desc.kv_heads) * d);
         // How the layer groups its key tiles (see common.cuh): short segments where launches gain from
         // cutting their rows' keys at little cost in partials, long ones elsewhere.
-        //   prefill: when even a full chunk gives too few (row tile, kv head) pairs to occupy the SMs
-        //            (half of them; a quarter for head_dim 256, whose kernel pays more per item) and a
-        //            row can span more than two short segments;
+        //   prefill: when even a full chunk gives too few (row tile, kv head) items to occupy half of the SMs
+        //            and a row can span more than two short segments;
         //   decode:  a cache for batches of sequences, whose rows are cut at segment boundaries, and wide
         //            heads, whose spans of segments have to fit the shared memory of a cluster (one
         //            sequence of 32768 keys, head_dim 256: 4096-key segments made two waves of clusters
-        //            of what is one with 1024).
-        const int tokens_per_tile = kTileKeys / (L.desc.q_heads / L.desc.kv_heads);
+        //            of what is one with 2048).
+        const bool pairs = d == 256 || d == 512;               // row tiles of 256 rows on pairs of SMs
+        const int tokens_per_tile = (pairs ? 2 : 1) * kTileKeys / (L.desc.q_heads / L.desc.kv_heads);
         const int chunk_row_tiles = (prefill_chunk + tokens_per_tile - 1) / tokens_per_tile;
         const int reach = windowed ? std::min(L.desc.window + prefill_chunk, context_length) : context_length;
-        const bool few_rows = (d == 256 ? 4 : 2) * chunk_row_tiles * L.desc.kv_heads <= std::max(ctx->sm_count, 1) &&
+        const bool few_rows = 2 * chunk_row_tiles * L.desc.kv_heads * (pairs ? d / 256 : 1) <= std::max(ctx->sm_count, 1) / (pairs ? 2 : 1) &&
                               reach > (2 * kTileKeys << kLogSegmentSmall);
         const bool batched = max_seqs >= 8;
         L.log_segment_general = few_rows || batched ? kLogSegmentSmall : kLogSegmentLarge;
-        L.log_segment = d >= 256 ? kLogSegmentSmall : L.log_segment_general;
+        L.log_segment = L.log_segment_general == kLogSegmentLarge && d >= 256 ? kLogSegmentWide : L.log_segment_general;
         // Workspace for the partials of split launches.  Decode, at its finest cut: one per (batch
         // entry, query head, key tile of this rank).  Prefill, layers with short segments only: one
         // per (query token, query head, segment).
@@ -787,15 +787,20 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         part_o_floats = std::max(part_o_floats, decode_rows * decode_slots * d);
         part_ml_floats = std::max(part_ml_floats, decode_rows * decode_slots * 2 + 4);
         n_tickets = std::max(n_tickets, size_t(std::min(max_seqs, kMaxBatch)) * L.desc.kv_heads * 16);
-        if (few_rows) {
+        if (few_rows || pairs) {
             const size_t prefill_slots = size_t((((reach + kTileKeys - 1) / kTileKeys) >> kLogSegmentSmall) + 2);
             const size_t prefill_rows = size_t(prefill_chunk) * L.desc.q_heads;
-            prefill_o_floats = std::max(prefill_o_floats, prefill_rows * prefill_slots * d);
-            prefill_ml_floats = std::max(prefill_ml_floats, prefill_rows * prefill_slots * 2);
+            // Wide heads take what a short call's split needs, 128 MB at most: a long one has row tiles enough.
+            const size_t most = few_rows ? ~size_t(0) : (size_t(32) << 20) / d;
+            const size_t parts = std::min(prefill_rows * prefill_slots, most);
+            prefill_o_floats = std::max(prefill_o_floats, parts * d);
+            prefill_ml_floats = std::max(prefill_ml_floats, parts * 2);
         }
         // The tensor-core kernels keep a whole-row launch's second-fold state in the same buffer:
-        // head_dim x 128 floats per thread block.
-        if (d == 64 || d == 128 || d == 256) prefill_o_floats = std::max(prefill_o_floats, size_t(std::max(ctx->sm_count, 1)) * d * 128);
+        // head_dim (256 of it at most) x 128 floats per thread block.
+        if (d == 64 || d == 128 || d == 256 || d == 512) {
+            prefill_o_floats = std::max(prefill_o_floats, size_t(std::max(ctx->sm_count, 1)) * std::min(d, 256) * 128);
+        }
         st = tc_make_tensor_maps(cache, L);
     }
     if (st == HC_OK && max_q_elems == 0) st = fail(HC_UNSUPPORTED, "no layer keeps a key/value history");

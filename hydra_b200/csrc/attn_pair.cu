@@ -1,0 +1,665 @@
+// attn_pair.cu — prefill attention for head_dim 256 and 512 (Gemma- and Qwen-shaped layers) on pairs of SMs.
+//
+// Same arithmetic as attn_tc.cu; what changes is how a wide row tile fits the machine.  Two CTAs form a cluster and
+// share every MMA (cta_group::2): 256 query rows, 128 in each CTA, against key and value tiles of which each
+// CTA loads half.  A 128-key tile then costs an SM 64 KB of loads and 2048 clocks of tensor pipe at head_dim
+// 256, 32 bytes a clock; one CTA per 128 rows needed twice that, more than L2 gives 148 SMs at once,
+// and with single 64 KB K and V stages each tile's load was exposed too (measured 0.21 of the bf16
+// peak on an 8192-token prompt through six layers).
+//
+// Tensor memory holds two S buffers (2 x 128 columns) and ONE O buffer of 256 columns: all 512.  Head_dim 512 has
+// twice as many columns of O, so there a work item is a row tile's 256-column half, and the logits are
+// computed once for each half (a third more MMA work than a layout that kept 512 columns would need).
+// Shared memory holds one Q tile (64 or 128 KB) and a ring of 16 KB stages through which K and V tiles
+// pass in the order the MMAs take them: K0 K1 V0 K2 V1 .., across item boundaries.
+//
+//   warpgroup 0    warp 0 loads K and V, warp 1 of the leading CTA issues the MMAs, warp 2 loads Q (all TMA)
+//   warpgroups 1-2 softmax, thread = row; each group takes 64 of a tile's 128 columns.  With two S buffers the loop
+//                  S -> softmax -> P V -> next S of the buffer sets the pace, so what counts is the softmax's
+//                  latency (whole tiles in turn: 3100 clocks of it, 3250 a tile)
+//   warpgroups 3-4 fold: a row of O is 256 floats, too many for one thread, so each folds a 128-column half
+//
+// The code of a tile is kept short (rolled loops over 32 columns): every launch fetches it cold, and straight-line
+// code for 128 columns took 11000 clocks on its first pass.
+// Registers per thread after setmaxnreg: 32 / 64 / 64 / 160 / 160.  Every mbarrier wait is bounded.
+
+#include <algorithm>
+
+#include "internal.hpp"
+#include "tc_common.cuh"
+#include "tc_ptx.cuh"
+
+namespace hc {
+namespace {
+
+constexpr int kPairThreads = 640;                    // five warpgroups
+constexpr int kPairRows = 2 * kRows;                 // query rows of a pair
+constexpr int kPairO = 256;                          // O columns of an item
+constexpr int kPairOCol = 2 * kTileKeys;             // their place in tensor memory
+constexpr int kPairStageBytes = 16 * 1024;           // K: 64 keys x 128 of head_dim; V: 128 keys x 64 columns; per CTA
+constexpr int kPairBoxBytes = 64 * 128;              // a box of 64 rows x 64 elements
+
+template <int D>
+struct PairLayout {
+    static constexpr int kHalves = D / kPairO;               // items per row tile
+    static constexpr int kQBytes = kRows * D * 2;
+    static constexpr int kStages = D == 256 ? 9 : 5;
+    static constexpr int kKChunks = D / 128;                 // stages of a K tile
+    static constexpr int kSmemBytes = 1024 + kQBytes + kStages * kPairStageBytes;
+};
+
+struct PairBarriers {
+    uint64_t q_full, q_empty;
+    uint64_t full[9], empty[9];
+    uint64_t s_full[2], p_full[2], m_full[4], o_full[2], o_free[2];
+    uint32_t tmem_base;
+    int abort_flag;
+    float red[2][2][kRows];             // alternate tiles: the two halves' row maxima
+    float mm[4][kRows];                 // scaled maxima, softmax -> fold (ring of 4 tiles, like m_full and l)
+    float l[4][3][kRows];               // row sums: columns 0-63, 64-95, 96-127
+    float m2[2][kRows], l2[2][kRows];   // the rows' second fold between segments, per half
+};
+
+struct PairItem {
+    int kv_head;
+    int half;          // 256-column half of O (head_dim 512)
+    int row0;          // first token of the row tile in the call
+    int valid_tokens;
+    int first_pos;
+    int tile_first, n_tiles;
+    int slot;          // ordinal of the item's segment among those the rows see (segment partials)
+};
+template <int D>
+__device__ __forceinline__ PairItem pair_item(const TcArgs& args, int index) {
+    PairItem w;
+    const int tokens_per_tile = kPairRows >> args.log_group;
+    // Longest key ranges first: descending row tile; a row tile's halves, segments and kv heads adjacent.
+    w.half = PairLayout<D>::kHalves > 1 ? index % PairLayout<D>::kHalves : 0;
+    const int rest = index / PairLayout<D>::kHalves;
+    const int rows = rest / args.slots;
+    w.slot = rest - rows * args.slots;
+    const int tile_index = rows / args.kv_heads;
+    w.kv_head = rows - tile_index * args.kv_heads;
+    const int mtile = args.mtiles - 1 - tile_index;
+    w.row0 = mtile * tokens_per_tile;
+    w.valid_tokens = min(tokens_per_tile, args.tokens - w.row0);
+    w.first_pos = args.first_position + w.row0;
+    const int last_pos = args.block_ends != nullptr ? args.appended - 1 : w.first_pos + w.valid_tokens - 1;
+    const TileRange tiles = args.finish ? row_tiles(args.map, w.first_pos, last_pos, args.window)
+                                        : group_tiles(args.map, w.first_pos, last_pos, args.window, w.slot, args.map.log_segment);
+    w.tile_first = tiles.first;
+    w.n_tiles = tiles.count;
+    return w;
+}
+struct PairIter {
+    int item;
+    PairItem w;
+};
+template <int D>
+__device__ __forceinline__ void pair_seek(const TcArgs& args, PairIter& it) {
+    for (; it.item < args.n_items; it.item += int(gridDim.x) >> 1) {
+        it.w = pair_item<D>(args, it.item);
+        if (it.w.n_tiles > 0) return;
+    }
+    it.item = args.n_items;
+}
+template <int D>
+__device__ __forceinline__ PairIter pair_begin(const TcArgs& args) {
+    PairIter it;
+    it.item = int(blockIdx.x) >> 1;
+    it.w = PairItem{};
+    pair_seek<D>(args, it);
+    return it;
+}
+template <int D>
+__device__ __forceinline__ void pair_next(const TcArgs& args, PairIter& it) {
+    it.item += int(gridDim.x) >> 1;
+    pair_seek<D>(args, it);
+}
+
+// The walk tile by tile.
+template <int D>
+struct PairCursor {
+    PairIter walk;
+    int j;
+    __device__ __forceinline__ explicit PairCursor(const TcArgs& args) : walk(pair_begin<D>(args)), j(0) {}
+    __device__ __forceinline__ bool more(const TcArgs& args) const { return walk.item < args.n_items; }
+    __device__ __forceinline__ void next(const TcArgs& args) {
+        if (++j == walk.w.n_tiles) {
+            j = 0;
+            pair_next<D>(args, walk);
+        }
+    }
+};
+
+// (x0 + y0, x1 + y1) of two bf16 pairs, as one packed addition.
+__device__ __forceinline__ uint64_t unpack_pair(uint32_t w) { return uint64_t(w << 16) | (uint64_t(w & 0xffff0000u) << 32); }
+__device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+    return r;
+}
+
+// FINISH: the kernel finishes an item's rows; otherwise it leaves segment partials (a template argument, so that a
+// launch carries only its own code).
+template <int D, bool FINISH>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                      const __grid_constant__ CUtensorMap tmap_q, const TcArgs args) {
+    using PL = PairLayout<D>;
+    extern __shared__ unsigned char raw_smem[];
+    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
+    unsigned char* q_smem = base;
+    unsigned char* ring = q_smem + PL::kQBytes;
+    PairBarriers* bars = reinterpret_cast<PairBarriers*>(ring + PL::kStages * kPairStageBytes);
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const int wg = warp >> 2;
+    const int G = 1 << args.log_group;
+    const int world = max(args.map.world, 1);
+    const int rank = int(cluster_rank());
+    const int token0 = rank * (kRows >> args.log_group);     // the first token of this CTA's half of a row tile
+    volatile int* abort_flag = &bars->abort_flag;
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        mbar_init(&bars->q_full, 1);
+        mbar_init(&bars->q_empty, 1);
+        for (int i = 0; i < PL::kStages; ++i) {
+            mbar_init(&bars->full[i], 1);
+            mbar_init(&bars->empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->s_full[i], 1);
+            mbar_init(&bars->p_full[i], 16);                 // the softmax warps of both CTAs
+            mbar_init(&bars->o_full[i], 1);
+            mbar_init(&bars->o_free[i], 8);                  // a half's fold warps of both CTAs
+        }
+        for (int i = 0; i < 4; ++i) mbar_init(&bars->m_full[i], 8);      // those of this one
+        bars->abort_flag = 0;
+        fence_barrier_init();
+    }
+    if (warp == 1) tmem_alloc_pair(&bars->tmem_base, 512);
+    if (warp == 0 && lane == 0) {
+        prefetch_tensormap(&tmap_k);
+        prefetch_tensormap(&tmap_v);
+        prefetch_tensormap(&tmap_q);
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();        // the peer's barriers are there
+    tc_fence_after();
+    const uint32_t tmem = bars->tmem_base;
+    pdl_wait();            // set-up done; from here on the kernel reads what earlier kernels wrote
+
+    if (wg == 0) {
+    reg_dealloc<32>();
+    if (warp == 0) {
+        // ===== producer: this CTA's halves of the tiles, in the order of the MMAs; the leader's barriers count
+        // both CTAs' loads. =====
+        if (lane == 0) {
+            uint32_t n = 0;
+            bool ok = true;
+            auto load = [&](const CUtensorMap* map, int col0, int row, int plane, bool two_boxes) {
+                const int slot = int(n % PL::kStages);
+                const uint32_t round = n / PL::kStages;
+                ++n;
+                if (round > 0 && !mbar_wait(&bars->empty[slot], (round - 1) & 1, abort_flag, args.status, 1)) { ok = false; return; }
+                if (rank == 0) mbar_expect_tx(&bars->full[slot], 2 * kPairStageBytes);
+                const uint32_t full = cluster_addr(&bars->full[slot], 0);
+                unsigned char* dst = ring + slot * kPairStageBytes;
+                tma_load_3d_pair(dst, map, full, col0, row, plane);
+                if (two_boxes) tma_load_3d_pair(dst + kPairBoxBytes, map, full, col0 + 64, row, plane);
+            };
+            // K one tile ahead of V.
+            PairCursor<D> keys(args), values(args);
+            auto load_keys = [&]() {                         // this CTA's 64 keys of the tile
+                const PairItem& w = keys.walk.w;
+                const int plane = cache_plane(args.map, args.seq, args.kv_heads, w.kv_head);
+                const int row = cache_row(args.map, args.seq, (w.tile_first + keys.j * world) * kTileKeys) + rank * 64;
+                for (int c = 0; ok && c < PL::kKChunks; ++c) load(&tmap_k, c * 128, row, plane, true);
+                keys.next(args);
+            };
+            if (keys.more(args)) load_keys();
+            while (ok && values.more(args)) {
+                if (keys.more(args)) load_keys();
+                const PairItem& w = values.walk.w;           // this CTA's 64 columns of each half of O
+                const int plane = cache_plane(args.map, args.seq, args.kv_heads, w.kv_head);
+                const int row = cache_row(args.map, args.seq, (w.tile_first + values.j * world) * kTileKeys);
+                for (int h = 0; ok && h < 2; ++h) load(&tmap_v, w.half * kPairO + h * 128 + rank * 64, row, plane, false);
+                values.next(args);
+            }
+        }
+    } else if (warp == 1) {
+        // ===== MMA issuer of the pair: S of the next tile (of the next item, at an item's end) is issued before P of
+        // this one is awaited.  The whole warp walks the loop and waits, so control flow stays
+        // warp-uniform; one elected lane issues the tcgen05 instructions. =====
+        if (rank == 0) {
+            constexpr uint32_t idesc_qk = instr_desc_pair(kTileKeys, false);
+            constexpr uint32_t idesc_pv = instr_desc_pair(kPairO / 2, true);
+            const uint64_t q_desc0 = smem_desc(smem_u32(q_smem), 16);
+            const uint64_t k_desc0 = smem_desc(smem_u32(ring), 16);
+            const uint64_t v_desc0 = smem_desc(smem_u32(ring), 16);
+            uint32_t n = 0;
+            PairCursor<D> ahead(args);
+            uint32_t ta = 0, it = 0;                         // tile and item of S
+            auto issue_qk = [&]() -> bool {
+                const uint32_t t = ta;
+                const bool last = ahead.j + 1 == ahead.walk.w.n_tiles;
+                if (ahead.j == 0 && !mbar_wait(&bars->q_full, it & 1, abort_flag, args.status, 4)) return false;
+                const uint32_t s_tmem = tmem + (t & 1) * kTileKeys;
+                #pragma unroll 1
+                for (int c = 0; c < PL::kKChunks; ++c, ++n) {
+                    const int slot = int(n % PL::kStages);
+                    if (!mbar_wait(&bars->full[slot], (n / PL::kStages) & 1, abort_flag, args.status, 3)) return false;
+                    tc_fence_after();
+                    if (elect_one()) {
+                        #pragma unroll
+                        for (int b = 0; b < 2; ++b) {
+                            #pragma unroll
+                            for (int ks = 0; ks < 4; ++ks) {
+                                mma_ss_pair(s_tmem, q_desc0 + uint64_t(((2 * c + b) * (kRows * 128) + ks * 32) >> 4),
+                                            k_desc0 + uint64_t((slot * kPairStageBytes + b * kPairBoxBytes + ks * 32) >> 4), idesc_qk,
+                                            (c | b | ks) != 0 ? 1u : 0u);
+                            }
+                        }
+                        tc_commit_pair(&bars->empty[slot]);
+                        if (c == PL::kKChunks - 1) {
+                            tc_commit_pair(&bars->s_full[t & 1]);
+                            if (last) tc_commit_pair(&bars->q_empty);
+                        }
+                    }
+                    __syncwarp();
+                }
+                ++ta;
+                if (last) ++it;
+                ahead.next(args);
+                return true;
+            };
+            bool ok = !ahead.more(args) || issue_qk();
+            for (uint32_t t = 0; ok && t < ta; ++t) {
+                if (ahead.more(args) && !issue_qk()) break;
+                if (!mbar_wait(&bars->p_full[t & 1], (t >> 1) & 1, abort_flag, args.status, 5)) break;
+                const uint32_t p_tmem = tmem + (t & 1) * kTileKeys;
+                // The two halves of O one after the other: one is folded while the other is computed.
+                #pragma unroll 1
+                for (int h = 0; h < 2; ++h, ++n) {
+                    const int slot = int(n % PL::kStages);
+                    if (t > 0 && !mbar_wait(&bars->o_free[h], (t - 1) & 1, abort_flag, args.status, 7)) { ok = false; break; }
+                    if (!mbar_wait(&bars->full[slot], (n / PL::kStages) & 1, abort_flag, args.status, 6)) { ok = false; break; }
+                    tc_fence_after();
+                    if (elect_one()) {
+                        #pragma unroll
+                        for (int ks = 0; ks < kTileKeys / 16; ++ks) {
+                            mma_ts_pair(tmem + kPairOCol + h * 128, p_tmem + (ks & 3) * 8 + (ks >> 2) * 64,
+                                        v_desc0 + uint64_t((slot * kPairStageBytes + ks * 2048) >> 4), idesc_pv, ks != 0 ? 1u : 0u);
+                        }
+                        tc_commit_pair(&bars->empty[slot]);
+                        tc_commit_pair(&bars->o_full[h]);
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else if (warp == 2) {
+        // ===== Q loader: this CTA's 128 rows (128 / G tokens x G heads) of the prepared queries =====
+        if (lane == 0) {
+            uint32_t it = 0;
+            const uint32_t q_full = cluster_addr(&bars->q_full, 0);
+            for (PairIter walk = pair_begin<D>(args); walk.item < args.n_items; pair_next<D>(args, walk), ++it) {
+                const PairItem& w = walk.w;
+                if (it > 0 && !mbar_wait(&bars->q_empty, (it - 1) & 1, abort_flag, args.status, 10)) break;
+                if (rank == 0) mbar_expect_tx(&bars->q_full, 2 * PL::kQBytes);
+                for (int b = 0; b < D / 64; ++b) {
+                    tma_load_3d_pair(q_smem + b * (kRows * 128), &tmap_q, q_full, b * 64, w.kv_head * G, w.row0 + token0);
+                }
+            }
+        }
+    }
+    } else if (wg <= 2) {
+        // ===== softmax: thread = row, 64 columns.  The two warps of a row meet at a named barrier, so none leaves early: a
+        // wait that gives up is not acted on, and the walk goes on over whatever is in the buffers, in bounds. =====
+        reg_dealloc<64>();
+        const int cols = wg - 1;                             // columns 64 cols .. 64 cols + 63
+        const int quad = warp & 3;
+        const int row = quad * 32 + lane;
+        const int t_local = token0 + (row >> args.log_group);
+        const uint32_t s_base = tmem + (uint32_t(quad * 32) << 16) + cols * 64;
+        const uint32_t p_full[2] = {cluster_addr(&bars->p_full[0], 0), cluster_addr(&bars->p_full[1], 0)};
+        const float neg_inf = __int_as_float(0xff800000);
+        uint32_t t = 0;
+        for (PairIter walk = pair_begin<D>(args); walk.item < args.n_items; pair_next<D>(args, walk)) {
+            const PairItem& w = walk.w;
+            const bool valid = t_local < w.valid_tokens;
+            const bool warp_has_rows = quad * 32 < ((w.valid_tokens - token0) << args.log_group);
+            int pos = valid ? w.first_pos + t_local : -1;
+            const int lo = args.window > 0 ? max(0, pos - args.window + 1) : 0;
+            // From here on the last key the row sees: its own, or the end of its bidirectional block.
+            if (args.block_ends != nullptr && valid) {
+                pos = max(pos, min(__ldg(args.block_ends + (w.first_pos - args.first_position) + t_local), args.appended) - 1);
+            }
+            for (int j = 0; j < w.n_tiles; ++j, ++t) {
+                const int sb = int(t & 1);
+                mbar_wait(&bars->s_full[sb], (t >> 1) & 1, abort_flag, args.status, 8);
+                tc_fence_after();
+                if (warp_has_rows) {
+                    const uint32_t s_tmem = s_base + sb * kTileKeys;
+                    const int key0 = (w.tile_first + j * world) * kTileKeys + cols * 64;
+                    const int c_lo = lo - key0;
+                    const int c_hi = pos - key0;
+                    const bool full = c_lo <= 0 && c_hi >= 63;
+                    auto mask = [&](uint32_t (&s)[32], int base_col) {
+                        const int a = c_lo - base_col, b = c_hi - base_col;
+                        #pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            if (i < a || i > b) s[i] = __float_as_uint(neg_inf);
+                        }
+                    };
+                    // Pass 1: the row maximum (exact under any association).
+                    float m = neg_inf;
+                    #pragma unroll 1
+                    for (int g = 0; g < 2; ++g) {
+                        uint32_t s[32];
+                        HC_TMEM_LD32(s_tmem + g * 32, s);
+                        tc_wait_ld();
+                        if (!full) mask(s, g * 32);
+                        float mx[4];
+                        #pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            mx[u] = fmax3(__uint_as_float(s[u]), __uint_as_float(s[u + 4]), __uint_as_float(s[u + 8]));
+                            mx[u] = fmax3(mx[u], __uint_as_float(s[u + 12]), __uint_as_float(s[u + 16]));
+                            mx[u] = fmax3(mx[u], __uint_as_float(s[u + 20]), __uint_as_float(s[u + 24]));
+                            mx[u] = fmaxf(mx[u], __uint_as_float(s[u + 28]));
+                        }
+                        m = fmax3(m, fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                    }
+                    bars->red[sb][cols][row] = m;
+                    named_barrier(1 + quad, 64);
+                    m = fmaxf(m, bars->red[sb][cols ^ 1][row]);
+                    const float neg_mc = -__fmul_rn((m == neg_inf) ? 0.0f : m, args.c);
+                    // Pass 2: weights; P overwrites the S columns already consumed.  The row sum has a
+                    // fixed shape: groups of 32 columns by the butterfly tree (i with i + 16, then + 8, + 4, + 2,
+                    // + 1; two columns an addition), the four groups in order (the last two are added by the fold).
+                    #pragma unroll 1
+                    for (int g = 0; g < 2; ++g) {
+                        uint32_t s[32];
+                        HC_TMEM_LD32(s_tmem + g * 32, s);
+                        tc_wait_ld();
+                        if (!full) mask(s, g * 32);
+                        #pragma unroll
+                        for (int i = 0; i < 16; ++i) fma2_inplace(s[2 * i], s[2 * i + 1], args.c, neg_mc);
+                        uint32_t packed[16];
+                        #pragma unroll
+                        for (int i = 0; i < 16; ++i) packed[i] = pack_bf16x2(ex2(__uint_as_float(s[2 * i])), ex2(__uint_as_float(s[2 * i + 1])));
+                        HC_TMEM_ST16(s_tmem + g * 16, packed);
+                        uint64_t a[8];
+                        #pragma unroll
+                        for (int i = 0; i < 8; ++i) a[i] = add2(unpack_pair(packed[i]), unpack_pair(packed[i + 8]));
+                        #pragma unroll
+                        for (int i = 0; i < 4; ++i) a[i] = add2(a[i], a[i + 4]);
+                        a[0] = add2(add2(a[0], a[2]), add2(a[1], a[3]));
+                        float group = __fadd_rn(__uint_as_float(uint32_t(a[0])), __uint_as_float(uint32_t(a[0] >> 32)));
+                        if (cols == 0 && g == 1) group = __fadd_rn(bars->l[t & 3][0][row], group);
+                        bars->l[t & 3][cols == 0 ? 0 : 1 + g][row] = group;
+                    }
+                    if (cols == 0) bars->mm[t & 3][row] = __fmul_rn(m, args.c);
+                    tc_wait_st();
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(&bars->m_full[t & 3]);       // the maxima and sums, to this CTA's fold
+                    mbar_arrive_cluster_relaxed(p_full[sb]); // (P itself is ordered by the fences around tensor memory)
+                }
+            }
+        }
+    } else {
+        // ===== fold + epilogue: two threads per row, one per 128-column half of O =====
+        reg_alloc<160>();
+        const int half = wg - 3;
+        const int quad = warp & 3;
+        const int row = quad * 32 + lane;
+        const int t_local = token0 + (row >> args.log_group);
+        const int g = row & (G - 1);
+        const uint32_t o_tmem = tmem + (uint32_t(quad * 32) << 16) + kPairOCol + half * 128;
+        const uint32_t o_free = cluster_addr(&bars->o_free[half], 0);
+        // This thread's values between segments: 32 groups of four, a row's group beside the next row's.
+        float4* const state = reinterpret_cast<float4*>(args.row_state + size_t(blockIdx.x) * (kPairO * kRows)) + half * 32 * kRows + row;
+        // (M, L) the second fold stands at: what the last segment end left, or the seed.
+        auto second_fold_state = [&](bool state_holds, int head, float& M2, float& L2) {
+            if (state_holds) {
+                M2 = bars->m2[half][row];
+                L2 = bars->l2[half][row];
+            } else if (args.count_sink) {
+                M2 = __fmul_rn(bf16_bits_to_float(args.sinks != nullptr ? __ldg(args.sinks + head) : kNoSinkBits), kLog2e);
+                L2 = 1.0f;
+            } else {
+                M2 = kEmptyMax;
+                L2 = 0.0f;
+            }
+        };
+        uint32_t t = 0;
+        bool ok = true;
+        for (PairIter walk = pair_begin<D>(args); ok && walk.item < args.n_items; pair_next<D>(args, walk)) {
+            const PairItem& w = walk.w;
+            const int head = w.kv_head * G + g;
+            const bool valid = t_local < w.valid_tokens;
+            const bool warp_has_rows = quad * 32 < ((w.valid_tokens - token0) << args.log_group);
+            const size_t vec = size_t(w.row0 + t_local) * args.q_heads + head;
+            // The running segment's partial: a fold over its tiles from the empty state (both halves of
+            // the row carry M and L, the same chain, the same bits).
+            float M = kEmptyMax, L = 0.0f;
+            float A[128];
+            #pragma unroll
+            for (int i = 0; i < 128; ++i) A[i] = 0.0f;
+            bool state_holds = false;
+            for (int j = 0; j < w.n_tiles; ++j, ++t) {
+                // The coefficients while O is on its way.
+                if (!mbar_wait(&bars->m_full[t & 3], (t >> 2) & 1, abort_flag, args.status, 11)) { ok = false; break; }
+                float Mn, a, b;
+                fold_coefficients(M, bars->mm[t & 3][row], Mn, a, b);
+                L = __fmaf_rn(L, a, __fmul_rn(__fadd_rn(__fadd_rn(bars->l[t & 3][0][row], bars->l[t & 3][1][row]), bars->l[t & 3][2][row]), b));
+                M = Mn;
+                if (!mbar_wait(&bars->o_full[half], t & 1, abort_flag, args.status, 9)) { ok = false; break; }
+                tc_fence_after();
+                if (warp_has_rows) {
+                    #pragma unroll
+                    for (int chunk = 0; chunk < 8; ++chunk) {
+                        uint32_t o[16];
+                        HC_TMEM_LD16(o_tmem + chunk * 16, o);
+                        tc_wait_ld();
+                        if (chunk == 7) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive_cluster_relaxed(o_free);      // nothing but tensor memory was read
+                        }
+                        #pragma unroll
+                        for (int i = 0; i < 16; i += 2) fold_value2(A[chunk * 16 + i], A[chunk * 16 + i + 1], a, o[i], o[i + 1], b);
+                    }
+                } else {
+                    if (lane == 0) mbar_arrive_cluster_relaxed(o_free);
+                }
+                const int tile = w.tile_first + j * world;
+                if (!FINISH || j + 1 == w.n_tiles || (tile >> args.map.log_segment) == ((tile + world) >> args.map.log_segment)) continue;
+                // A segment is complete and another follows: fold it into the row's state, which is kept out of the
+                // registers ((M2, L2) in shared memory, the values in global memory), and start over.
+                if (!warp_has_rows) continue;
+                float M2, L2;
+                second_fold_state(state_holds, head, M2, L2);
+                float Mn2, a2, b2;
+                fold_coefficients(M2, M, Mn2, a2, b2);
+                bars->m2[half][row] = Mn2;
+                bars->l2[half][row] = __fmaf_rn(L2, a2, __fmul_rn(L, b2));
+                #pragma unroll
+                for (int i0 = 0; i0 < 128; i0 += 16) {
+                    float4 before[4];
+                    #pragma unroll
+                    for (int i = 0; i < 4; ++i) before[i] = state_holds ? state[(i0 / 4 + i) * kRows] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    #pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float* v = &A[i0 + 4 * i];
+                        state[(i0 / 4 + i) * kRows] = make_float4(fold_value(before[i].x, a2, v[0], b2), fold_value(before[i].y, a2, v[1], b2),
+                                                                 fold_value(before[i].z, a2, v[2], b2), fold_value(before[i].w, a2, v[3], b2));
+                        v[0] = v[1] = v[2] = v[3] = 0.0f;
+                    }
+                    asm volatile("" ::: "memory");      // sixteen values in flight, not all of them
+                }
+                M = kEmptyMax;
+                L = 0.0f;
+                state_holds = true;
+            }
+            if (!ok) break;
+            const int col0 = w.half * kPairO + half * 128;
+            if constexpr (!FINISH) {
+                // The segment's partial goes to the workspace (a merge kernel runs the second fold).
+                if (valid) {
+                    const size_t prow = vec * args.slots + w.slot;
+                    float* dst = args.part_o + prow * D + col0;
+                    #pragma unroll
+                    for (int i = 0; i < 128; i += 4) {
+                        *reinterpret_cast<float4*>(dst + i) = make_float4(A[i], A[i + 1], A[i + 2], A[i + 3]);
+                    }
+                    if (half == 0 && w.half == 0) *reinterpret_cast<float2*>(args.part_ml + prow * 2) = make_float2(M, L);
+                }
+                continue;
+            }
+            // The row's last segment: the last step of the second fold, which started from the sink (or
+            // from the empty state).
+            {
+                float M2, L2;
+                second_fold_state(state_holds, valid ? head : 0, M2, L2);
+                float Mn, a, b;
+                fold_coefficients(M2, M, Mn, a, b);
+                L = __fmaf_rn(L2, a, __fmul_rn(L, b));
+                M = Mn;
+                if (state_holds) {
+                    #pragma unroll
+                    for (int i0 = 0; i0 < 128; i0 += 16) {
+                        float4 before[4];
+                        #pragma unroll
+                        for (int i = 0; i < 4; ++i) before[i] = state[(i0 / 4 + i) * kRows];
+                        #pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            float* v = &A[i0 + 4 * i];
+                            v[0] = fold_value(before[i].x, a, v[0], b);
+                            v[1] = fold_value(before[i].y, a, v[1], b);
+                            v[2] = fold_value(before[i].z, a, v[2], b);
+                            v[3] = fold_value(before[i].w, a, v[3], b);
+                        }
+                        asm volatile("" ::: "memory");
+                    }
+                } else {
+                    // fold_value(0, a, A, b) = 0 * a + A * b = A * b exactly: one multiply.
+                    #pragma unroll
+                    for (int i = 0; i < 128; ++i) A[i] = __fmul_rn(A[i], b);
+                }
+            }
+            if (!valid) continue;
+            if (args.ep.write_partial) {
+                float* dst = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2) + col0;
+                #pragma unroll
+                for (int i = 0; i < 128; i += 2) *reinterpret_cast<float2*>(dst + i) = make_float2(A[i], A[i + 1]);
+                if (half == 0 && w.half == 0) {
+                    float* tail = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2) + D;
+                    tail[0] = M;
+                    tail[1] = L;
+                }
+                continue;
+            }
+            const float inverse = __frcp_rn(L);
+            if (args.ep.gate_layout != HC_GATE_NONE) {
+                // Gated: by way of the state's place, so that the gate's code is there once and not 128 times.
+                #pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    state[i * kRows] = make_float4(__fmul_rn(A[4 * i], inverse), __fmul_rn(A[4 * i + 1], inverse),
+                                                  __fmul_rn(A[4 * i + 2], inverse), __fmul_rn(A[4 * i + 3], inverse));
+                }
+                const size_t gate_base = (args.ep.gate_layout == HC_GATE_INTERLEAVED ? vec * size_t(2 * D) + D : vec * size_t(D)) + col0;
+                #pragma unroll 2
+                for (int i = 0; i < 32; ++i) {
+                    const float4 v = state[i * kRows];
+                    float r[4] = {v.x, v.y, v.z, v.w};
+                    #pragma unroll
+                    for (int u = 0; u < 4; ++u) r[u] = __fmul_rn(r[u], sigmoid_gate(load_io(args.ep.gate, gate_base + 4 * i + u, args.ep.io_dtype)));
+                    if (args.ep.io_dtype == HC_F32) {
+                        *reinterpret_cast<float4*>(reinterpret_cast<float*>(args.ep.out) + vec * D + col0 + 4 * i) = make_float4(r[0], r[1], r[2], r[3]);
+                    } else {
+                        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(args.ep.out) + vec * D + col0 + 4 * i) =
+                            make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
+                    }
+                }
+            } else if (args.ep.io_dtype == HC_F32) {
+                float* dst = reinterpret_cast<float*>(args.ep.out) + vec * D + col0;
+                #pragma unroll
+                for (int i = 0; i < 128; i += 4) {
+                    *reinterpret_cast<float4*>(dst + i) = make_float4(__fmul_rn(A[i], inverse), __fmul_rn(A[i + 1], inverse),
+                                                                      __fmul_rn(A[i + 2], inverse), __fmul_rn(A[i + 3], inverse));
+                }
+            } else {
+                uint16_t* dst = reinterpret_cast<uint16_t*>(args.ep.out) + vec * D + col0;
+                #pragma unroll
+                for (int i = 0; i < 128; i += 8) {
+                    uint4 packed;
+                    packed.x = pack_bf16x2(__fmul_rn(A[i], inverse), __fmul_rn(A[i + 1], inverse));
+                    packed.y = pack_bf16x2(__fmul_rn(A[i + 2], inverse), __fmul_rn(A[i + 3], inverse));
+                    packed.z = pack_bf16x2(__fmul_rn(A[i + 4], inverse), __fmul_rn(A[i + 5], inverse));
+                    packed.w = pack_bf16x2(__fmul_rn(A[i + 6], inverse), __fmul_rn(A[i + 7], inverse));
+                    *reinterpret_cast<uint4*>(dst + i) = packed;
+                }
+            }
+        }
+    }
+
+    // Teardown.  On the abort path the producer first lets its copies in flight land (bounded).
+    if (warp == 0 && lane == 0 && *abort_flag != 0) {
+        const long long start = clock64();
+        while (static_cast<unsigned long long>(clock64() - start) < 200000000ull) { }
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();        // neither CTA leaves while the other's MMAs or arrivals may still name it
+    if (warp == 1) tmem_dealloc_pair(tmem, 512);
+}
+
+template <int D, bool FINISH>
+hc_status launch_pair_kernel(hc_context* ctx, const hc_layer_store& layer, const CUtensorMap& tmap_q, const TcArgs& args, cudaStream_t stream) {
+    constexpr int smem = PairLayout<D>::kSmemBytes + int(sizeof(PairBarriers));
+    static_assert(smem <= 227 * 1024, "shared memory of one CTA");
+    static bool configured[64] = {};
+    if (!configured[ctx->device & 63]) {
+        const cudaError_t err = cudaFuncSetAttribute(attention_pair_kernel<D, FINISH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (err != cudaSuccess) return check_cuda(err, "attention_pair_kernel shared memory");
+        configured[ctx->device & 63] = true;
+    }
+    const int grid = 2 * std::max(1, std::min(args.n_items, std::max(ctx->sm_count / 2, 1)));
+    const cudaError_t launched = launch_pdl(attention_pair_kernel<D, FINISH>, grid, kPairThreads, size_t(smem), stream,
+                                            *static_cast<const CUtensorMap*>(layer.tmap_k64),
+                                            *static_cast<const CUtensorMap*>(layer.tmap_v), tmap_q, args);
+    ctx->launches += 1;
+    return check_cuda(launched, "attention_pair_kernel launch");
+}
+
+}  // namespace
+
+int pair_items_per_row_tile(int head_dim) { return head_dim / kPairO; }
+
+hc_status launch_attention_pair(hc_context* ctx, const hc_layer_store& layer, const void* args_ptr, int head_dim, cudaStream_t stream) {
+    const TcArgs& args = *static_cast<const TcArgs*>(args_ptr);
+    // A CTA's Q tile is a box of 64 columns x G heads x 128 / G tokens; rows beyond the last token are zeros.
+    CUtensorMap tmap_q;
+    const int group = 1 << args.log_group;
+    const hc_status st = tc_encode_3d(&tmap_q, args.q, uint64_t(head_dim), uint64_t(args.q_heads), uint64_t(args.tokens), uint32_t(group),
+                                      uint32_t(kRows / group));
+    if (st != HC_OK) return st;
+    if (head_dim == 256) {
+        return args.finish ? launch_pair_kernel<256, true>(ctx, layer, tmap_q, args, stream)
+                           : launch_pair_kernel<256, false>(ctx, layer, tmap_q, args, stream);
+    }
+    return args.finish ? launch_pair_kernel<512, true>(ctx, layer, tmap_q, args, stream)
+                       : launch_pair_kernel<512, false>(ctx, layer, tmap_q, args, stream);
+}
+
+}  // namespace hc

@@ -453,7 +453,7 @@ struct MergeRows {
     int decode;              // 1: rows are batch entries at meta.pos[]
     int first_position;      // prefill
     int tokens;              // query tokens, or batch entries
-    int tokens_per_tile;     // prefill: 128 / group
+    int tokens_per_tile;     // prefill: tokens of a row tile, which share their slots
     BatchMeta meta;
 };
 
@@ -789,11 +789,11 @@ hc_status launch_merge_decode(hc_context* ctx, const AttnShape& shape, const Row
 }
 
 hc_status launch_merge_prefill(hc_context* ctx, const AttnShape& shape, const RowMap& map, int tokens, int first_position,
-                               const Workspace& ws, int slots, const EpilogueArgs& ep, cudaStream_t stream) {
+                               int tokens_per_tile, const Workspace& ws, int slots, const EpilogueArgs& ep, cudaStream_t stream) {
     MergeRows rows{};
     rows.first_position = first_position;
     rows.tokens = tokens;
-    rows.tokens_per_tile = kTileKeys / shape.group;        // a row tile is 128 rows: 128 / group tokens
+    rows.tokens_per_tile = tokens_per_tile;
     return launch_merge_rows(ctx, shape, map, rows, ws, slots, ep, stream);
 }
 

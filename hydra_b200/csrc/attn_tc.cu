@@ -950,7 +950,7 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-bool dim_ok(int d) { return d == 64 || d == 128 || d == 256; }
+bool dim_ok(int d) { return d == 64 || d == 128 || d == 256 || d == 512; }
 
 }  // namespace
 
@@ -968,6 +968,20 @@ hc_status tc_encode_2d(void* map, const void* base, uint64_t rows, uint64_t cols
     return HC_OK;
 }
 
+hc_status tc_encode_3d(void* map, const void* base, uint64_t cols, uint64_t rows, uint64_t planes, uint32_t box_rows, uint32_t box_planes) {
+    EncodeTiledFn encode = encode_tiled();
+    if (!encode) return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from this driver");
+    const cuuint64_t dims[3] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(planes)};
+    const cuuint64_t strides[2] = {cuuint64_t(cols) * 2, cuuint64_t(cols) * rows * 2};
+    const cuuint32_t box[3] = {64, cuuint32_t(box_rows), cuuint32_t(box_planes)};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    const CUresult rc = encode(static_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+                               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
+    return HC_OK;
+}
+
 bool tc_supported(const AttnShape& shape) { return dim_ok(shape.head_dim) && shape.group <= 16; }
 
 hc_status tc_make_tensor_maps(hc_kv_cache* cache, hc_layer_store& layer) {
@@ -975,30 +989,32 @@ hc_status tc_make_tensor_maps(hc_kv_cache* cache, hc_layer_store& layer) {
     EncodeTiledFn encode = encode_tiled();
     if (!encode) return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from this driver");
     const int d = layer.desc.head_dim;
-    for (int which = 0; which < 2; ++which) {
+    void** maps[3] = {&layer.tmap_k, &layer.tmap_v, &layer.tmap_k64};
+    for (int which = 0; which < (d >= 256 ? 3 : 2); ++which) {
         CUtensorMap* map = new CUtensorMap;
         const bool paged = cache->pages_dev != nullptr && layer.ring == 0;       // one plane per head, shared
         const cuuint64_t dims[3] = {cuuint64_t(d), cuuint64_t(layer.capacity),
                                     cuuint64_t(paged ? 1 : cache->max_seqs) * layer.desc.kv_heads};
         const cuuint64_t strides[2] = {cuuint64_t(d) * 2, cuuint64_t(layer.capacity) * d * 2};
-        const cuuint32_t box[3] = {64, cuuint32_t(kTileKeys), 1};
+        const cuuint32_t box[3] = {64, cuuint32_t(which < 2 ? kTileKeys : 64), 1};
         const cuuint32_t elem[3] = {1, 1, 1};
-        const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, which == 0 ? layer.k : layer.v, dims,
+        const CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (which & 1) == 0 ? layer.k : layer.v, dims,
                                    strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (rc != CUDA_SUCCESS) {
             delete map;
             return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
         }
-        (which == 0 ? layer.tmap_k : layer.tmap_v) = map;
+        *maps[which] = map;
     }
     return HC_OK;
 }
 
 void tc_free_tensor_maps(hc_layer_store& layer) {
-    delete static_cast<CUtensorMap*>(layer.tmap_k);
-    delete static_cast<CUtensorMap*>(layer.tmap_v);
-    layer.tmap_k = layer.tmap_v = nullptr;
+    for (void** map : {&layer.tmap_k, &layer.tmap_v, &layer.tmap_k64}) {
+        delete static_cast<CUtensorMap*>(*map);
+        *map = nullptr;
+    }
 }
 
 template <int D, int MODE>
@@ -1051,14 +1067,14 @@ static void fill_common_args(TcArgs& args, hc_context* ctx, const AttnShape& sha
 
 // Floats of row state a whole-row launch needs.
 static size_t row_state_floats(const hc_context* ctx, const AttnShape& shape) {
-    return size_t(std::max(ctx->sm_count, 1)) * shape.head_dim * kRows;
+    return size_t(std::max(ctx->sm_count, 1)) * std::min(shape.head_dim, 256) * kRows;
 }
 
 static hc_status launch_any(hc_context* ctx, const AttnShape& shape, const TcArgs& args, const hc_layer_store& layer,
                             cudaStream_t stream) {
     if (shape.head_dim == 64) return launch_tc<64>(ctx, args, layer, stream);
     if (shape.head_dim == 128) return launch_tc<128>(ctx, args, layer, stream);
-    return launch_tc256(ctx, layer.tmap_k, layer.tmap_v, &args, args.n_items, stream);
+    return launch_attention_pair(ctx, layer, &args, shape.head_dim, stream);
 }
 
 hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
@@ -1072,7 +1088,9 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
     args.first_position = first_position;
     args.seq = seq;
     args.log_run = cache.map.log_segment;
-    const int tokens_per_tile = kRows / shape.group;
+    // Head_dim 256 and 512: row tiles of 256 rows on pairs of SMs.
+    const bool pairs = shape.head_dim >= 256;
+    const int tokens_per_tile = (pairs ? 2 : 1) * kRows / shape.group;
     args.mtiles = (tokens + tokens_per_tile - 1) / tokens_per_tile;
     // Segments and key tiles a row tile spans, at most.
     int slots = 1, most_tiles = 1;
@@ -1083,19 +1101,18 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
         most_tiles = std::max(most_tiles, row_tiles(cache.map, first, last, shape.window).count);
     }
     // Whole rows per item, or one item per (row tile, kv head, segment) merged afterwards: whichever
-    // the longest thread block finishes first, in units of one key tile's time.  An item costs its
-    // tiles plus a start and an end (about four tiles' worth; eight for head_dim 256, whose kernel
-    // does not look ahead across items), the merge and its launch about ten.  Measured on one
-    // GPT-OSS chunk of 512 tokens with 1, 2 and 4 kv heads: the model picks the faster of the two
-    // in all but ties.
-    const int whole_items = args.mtiles * shape.kv_heads;
+    // the longest thread block (or pair) finishes first, in units of one key tile's time.  An item costs its
+    // tiles plus a start and an end (about four tiles' worth at head_dim 64, two of a pair's longer ones), the merge
+    // and its launch about ten of the former, five of the latter.
+    const int whole_items = args.mtiles * shape.kv_heads * (pairs ? pair_items_per_row_tile(shape.head_dim) : 1);
     const size_t rows = size_t(tokens) * shape.q_heads;
     const bool can_split = slots > 1 && rows * slots * shape.head_dim <= ws.part_o_floats && rows * slots * 2 <= ws.part_ml_floats;
     const bool can_finish = slots == 1 || row_state_floats(ctx, shape) <= ws.part_o_floats;
-    const int sms = std::max(ctx->sm_count, 1);
-    const int item_cost = shape.head_dim == 256 ? 8 : 4;
-    const int whole_time = ((whole_items + sms - 1) / sms) * (most_tiles + item_cost);
-    const int split_time = ((whole_items * slots + sms - 1) / sms) * (std::min(most_tiles, 1 << cache.map.log_segment) + item_cost) + 10;
+    const int workers = std::max(pairs ? ctx->sm_count / 2 : ctx->sm_count, 1);
+    const int item_cost = pairs ? 2 : 4;
+    const int whole_time = ((whole_items + workers - 1) / workers) * (most_tiles + item_cost);
+    const int split_time = ((whole_items * slots + workers - 1) / workers) * (std::min(most_tiles, 1 << cache.map.log_segment) + item_cost) +
+                           (pairs ? 5 : 10);
     // With bidirectional blocks a row's last key is known on the device only: whole rows per item, no
     // merge over per-row segment lists (or the general kernel, if the row state does not fit).
     if (block_ends && !can_finish) return simt_prefill(ctx, shape, cache, seq, q, tokens, first_position, ep, stream, block_ends);
@@ -1114,7 +1131,7 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
     args.magic_kv_heads = division_magic(uint32_t(shape.kv_heads), uint32_t(args.n_items));
     const hc_status st = launch_any(ctx, shape, args, layer, stream);
     if (st != HC_OK || args.finish) return st;
-    return launch_merge_prefill(ctx, shape, cache.map, tokens, first_position, ws, slots, ep, stream);
+    return launch_merge_prefill(ctx, shape, cache.map, tokens, first_position, tokens_per_tile, ws, slots, ep, stream);
 }
 
 }  // namespace hc

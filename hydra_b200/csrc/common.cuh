@@ -15,7 +15,7 @@
 //       l    = sum_k p_k ,  O = sum_k p_k V_k                              (fp32)
 //       mm   = m * c
 //   tiles are grouped into segments of 2^log_segment consecutive tiles, absolute like the tiles
-//   (1024 or 4096 keys; a property of the layer, fixed when its cache is created).  A segment's
+//   (1024, 2048 or 4096 keys; a property of the layer, fixed when its cache is created).  A segment's
 //   partial is a left fold over its tiles that hold a visible key, in ascending order, from the
 //   empty state:
 //       (M, L, A) = (-1e30, 0, 0)
@@ -123,7 +123,7 @@ __device__ __forceinline__ void store_io(void* base, size_t index, int dtype, fl
 //   world > 1 (sequence): tile j = pos / 128 belongs to rank j % world and is that rank's local
 //                         tile j / world
 //   log_segment         : a segment is 2^log_segment consecutive tiles, absolute like the tiles
-//                         (3 or 5: 1024 or 4096 keys; fixed per layer when the cache is created)
+//                         (3, 4 or 5: 1024, 2048 or 4096 keys; fixed per layer when the cache is created)
 //   pages != null       : paged storage: the cache is a pool of 128-row pages shared by all sequences,
 //                         and key tile j of sequence s lives in page pages[s * pages_per_seq + j]
 struct RowMap {
@@ -135,6 +135,7 @@ struct RowMap {
     int pages_per_seq;
 };
 constexpr int kLogSegmentSmall = 3;        // layers whose prefill launches need their rows' keys split
+constexpr int kLogSegmentWide = 4;         // others of head_dim 256 and 512
 constexpr int kLogSegmentLarge = 5;        // all others
 __host__ __device__ __forceinline__ bool row_is_local(const RowMap& map, int pos) {
     return map.world <= 1 || ((pos / kTileKeys) % map.world) == map.rank;

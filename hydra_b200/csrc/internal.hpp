@@ -165,6 +165,7 @@ struct hc_layer_store {
     bool keeps_history = false;
     void* tmap_k = nullptr;       // tensor maps of the tcgen05 path (host copies), or null
     void* tmap_v = nullptr;
+    void* tmap_k64 = nullptr;     // keys in boxes of 64 rows: what a CTA of a pair loads (head_dim 256, 512)
 };
 
 struct hc_kv_cache {
@@ -238,8 +239,8 @@ hc_status launch_merge_decode(hc_context* ctx, const AttnShape& shape, const Row
                               int n_seq, const Workspace& ws, const DecodePlan& plan, const EpilogueArgs& ep,
                               cudaStream_t stream);
 hc_status launch_merge_prefill(hc_context* ctx, const AttnShape& shape, const RowMap& map, int tokens,
-                               int first_position, const Workspace& ws, int slots, const EpilogueArgs& ep,
-                               cudaStream_t stream);
+                               int first_position, int tokens_per_tile, const Workspace& ws, int slots,
+                               const EpilogueArgs& ep, cudaStream_t stream);
 hc_status launch_combine(hc_context* ctx, const float* gathered, int world, int rows, int q_heads,
                          int d, const EpilogueArgs& ep, cudaStream_t stream);
 // Device address of the fixed scratch array on `device` (which must be current).
@@ -249,6 +250,8 @@ hc_status static_scratch_prepare(int device, float** address);
 // A tensor map (CUtensorMap behind `map`) over a row-major bf16 matrix: boxes of 64 columns x box_rows
 // rows, 128-byte swizzle, zeros beyond the edges.
 hc_status tc_encode_2d(void* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+// The same over [planes][rows][cols]: boxes of 64 columns x box_rows x box_planes.
+hc_status tc_encode_3d(void* map, const void* base, uint64_t cols, uint64_t rows, uint64_t planes, uint32_t box_rows, uint32_t box_planes);
 bool tc_supported(const AttnShape& shape);
 hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer,
                      const CacheView& cache, int seq, const uint16_t* q, int tokens,
@@ -272,9 +275,9 @@ hc_status tc_decode(hc_context* ctx, const AttnShape& shape, const hc_layer_stor
 hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* const* w, const void* const* bias,
                     const float* const* residual, void* const* y, const int* out_features, int tokens, int in_features,
                     int y_dtype, cudaStream_t stream);
-// attn_tc256.cu (args_ptr: the TcArgs of tc_common.cuh)
-hc_status launch_tc256(hc_context* ctx, const void* tmap_k, const void* tmap_v, const void* args_ptr,
-                       int n_items, cudaStream_t stream);
+// attn_pair.cu (args_ptr: the TcArgs of tc_common.cuh)
+int pair_items_per_row_tile(int head_dim);
+hc_status launch_attention_pair(hc_context* ctx, const hc_layer_store& layer, const void* args_ptr, int head_dim, cudaStream_t stream);
 hc_status tc_make_tensor_maps(hc_kv_cache* cache, hc_layer_store& layer);
 void tc_free_tensor_maps(hc_layer_store& layer);
 

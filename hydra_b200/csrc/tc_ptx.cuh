@@ -161,6 +161,10 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// Without waiting for the thread's earlier stores to be visible to the cluster.
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -235,6 +239,15 @@ __device__ __forceinline__ uint32_t tmem_ld1(uint32_t taddr) {
           "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]),       \
           "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]),       \
           "=r"(v[29]), "=r"(v[30]), "=r"(v[31])                                                             \
+        : "r"(taddr) : "memory")
+
+#define HC_TMEM_LD16(taddr, v)                                                                              \
+    asm volatile(                                                                                           \
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "                                                           \
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"                    \
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),  \
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),         \
+          "=r"(v[15])                                                                                       \
         : "r"(taddr) : "memory")
 
 // 16 lanes x 256 bits, eight times along the columns: 16 rows x 64 columns.  Thread i of the warp
