@@ -110,13 +110,13 @@ bool needs_q_prepare(const hc_attn_params* p) {
 
 // Rows a position range needs; checks capacity the way KVCache.advance does (KVCache.swift:202-213).
 hc_status check_positions(const hc_kv_cache* cache, const hc_layer_store& L, int first, int tokens,
-                          const hc_attn_params* p) {
+                          const hc_attn_params* p, int most_in_ring = -1) {
     if (tokens < 0 || first < 0) return fail(HC_INVALID_ARGUMENT, "negative token count or position");
     if (L.ring == 0 && first + tokens > cache->context_length) {
         return fail(HC_KV_OVERFLOW, "position " + std::to_string(first + tokens - 1) + " beyond capacity " +
                                         std::to_string(cache->context_length));
     }
-    if (L.ring > 0 && tokens > L.ring_margin) {
+    if (L.ring > 0 && tokens > (most_in_ring < 0 ? L.ring_margin : most_in_ring)) {
         return fail(HC_KV_OVERFLOW, "a chunk of " + std::to_string(tokens) + " tokens overruns the ring's margin of " +
                                         std::to_string(L.ring_margin));
     }
@@ -254,25 +254,17 @@ void release_pages(hc_kv_cache* cache, int seq, int first_tile) {
     }
 }
 
-// When `ahead` is given (hc_prefill_chunks), the prologue launch goes to ahead->stream into the
-// ahead->slot-th prepared-query buffer, and `stream` waits for ahead->done, recorded behind it: the
-// prologue of a chunk can then run while the previous chunk's attention is still finishing.
-struct PrologueAhead {
-    cudaStream_t stream;
-    cudaEvent_t done;
-    int slot;
-};
-
+// `most_in_ring`: how many tokens a ring layer may take at once (its margin by default).
 hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, const void* q,
                        void* out, int tokens, int first_position, const hc_attn_params* p,
                        bool partial_mode, cudaStream_t stream, const void* k_fused = nullptr,
-                       const void* v_fused = nullptr, const PrologueAhead* ahead = nullptr) {
+                       const void* v_fused = nullptr, int most_in_ring = -1) {
     if (!ctx || !q || !out) return fail(HC_INVALID_ARGUMENT, "null context or buffer");
     hc_status st = validate_params(cache, layer, p);
     if (st != HC_OK) return st;
     if (seq < 0 || seq >= cache->max_seqs) return fail(HC_INVALID_ARGUMENT, "sequence index out of range");
     hc_layer_store& L = cache->layers[size_t(layer)];
-    st = check_positions(cache, L, first_position, tokens, p);
+    st = check_positions(cache, L, first_position, tokens, p, most_in_ring);
     if (st != HC_OK) return st;
     if (tokens == 0) return HC_OK;
 
@@ -285,7 +277,7 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
     const int d = p->head_dim;
     const int mult = p->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
     const bool prep = needs_q_prepare(p);
-    int step = prep ? cache->ws.qprep_tokens : tokens;
+    int step = prep ? cache->ws.qprep_capacity : tokens;
     // Bidirectional blocks: chunk by chunk (a block ends with its token's chunk).
     const int* blocks = p->block_ends;
     if (blocks) step = std::min(step, cache->prefill_chunk);
@@ -299,10 +291,10 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
             fill_common(args, p);
             int jobs = 0;
             if (k_fused) {
-                st = ensure_pages(cache, L, seq, first_position + start, count, ahead ? ahead->stream : stream);
+                st = ensure_pages(cache, L, seq, first_position + start, count, stream);
                 if (st != HC_OK) return st;
             }
-            uint16_t* prepared = cache->ws.qprep + (ahead ? size_t(ahead->slot) * cache->ws.qprep_slot_elems : 0);
+            uint16_t* prepared = cache->ws.qprep;
             if (prep) fill_q_job(args.job[jobs++], p, q_rows, prepared);
             if (k_fused) {
                 fill_kv_jobs(args, jobs, p, k_fused, v_fused);
@@ -314,13 +306,8 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
             args.batched = 0;
             args.seq = seq;
             args.cache = view;
-            st = launch_prepare(ctx, args, ahead ? ahead->stream : stream);
+            st = launch_prepare(ctx, args, stream);
             if (st != HC_OK) return st;
-            if (ahead) {
-                cudaError_t err = cudaEventRecord(ahead->done, ahead->stream);
-                if (err == cudaSuccess) err = cudaStreamWaitEvent(stream, ahead->done, 0);
-                if (err != cudaSuccess) return check_cuda(err, "prefill: prologue event");
-            }
             if (prep) q_bf16 = prepared;
         }
         EpilogueArgs ep{};
@@ -338,15 +325,7 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
             ep.gate = q_rows;
         }
         if (tensor) {
-            // A chunk attended to on the second stream works in the upper halves of the workspace.
-            Workspace ws = cache->ws;
-            if (ahead) {
-                ws.part_o += size_t(ahead->slot) * ws.prefill_o_floats;
-                ws.part_ml += size_t(ahead->slot) * ws.prefill_ml_floats;
-                ws.part_o_floats = ws.prefill_o_floats;
-                ws.part_ml_floats = ws.prefill_ml_floats;
-            }
-            st = tc_prefill(ctx, shape, L, view, seq, q_bf16, count, first_position + start, ws, ep, stream,
+            st = tc_prefill(ctx, shape, L, view, seq, q_bf16, count, first_position + start, cache->ws, ep, stream,
                             blocks ? blocks + start : nullptr);
         } else {
             st = simt_prefill(ctx, shape, view, seq, q_bf16, count, first_position + start, ep, stream,
@@ -809,14 +788,13 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         ws.qprep_tokens = std::max(std::max(prefill_chunk, std::min(max_seqs, kMaxBatch)), 1);
         prefill_o_floats = (prefill_o_floats + 63) & ~size_t(63);
         prefill_ml_floats = (prefill_ml_floats + 63) & ~size_t(63);
-        part_o_floats = std::max(part_o_floats, 2 * prefill_o_floats);
-        part_ml_floats = std::max(part_ml_floats, 2 * prefill_ml_floats);
+        part_o_floats = std::max(part_o_floats, prefill_o_floats);
+        part_ml_floats = std::max(part_ml_floats, prefill_ml_floats);
         ws.part_o_floats = part_o_floats;
         ws.part_ml_floats = part_ml_floats;
-        ws.prefill_o_floats = prefill_o_floats;
-        ws.prefill_ml_floats = prefill_ml_floats;
-        ws.qprep_slot_elems = size_t(ws.qprep_tokens) * max_q_elems;
-        err = cudaMalloc(&ws.qprep, 2 * ws.qprep_slot_elems * 2);
+        // Prepared queries: a call's, up to 64 MB of them, so that a prompt is one prologue and one attention launch.
+        ws.qprep_capacity = std::max(ws.qprep_tokens, int(std::min<size_t>((size_t(32) << 20) / max_q_elems, size_t(context_length))));
+        err = cudaMalloc(&ws.qprep, size_t(ws.qprep_capacity) * max_q_elems * 2);
         if (err == cudaSuccess) err = cudaMalloc(&ws.part_o, part_o_floats * sizeof(float));
         if (err == cudaSuccess) err = cudaMalloc(&ws.part_ml, part_ml_floats * sizeof(float));
         ws.n_tickets = n_tickets;
@@ -1301,7 +1279,7 @@ hc_status hc_layer_step(hc_context* ctx, hc_kv_cache* cache, int layer, int seq,
     hc_status st = validate_params(cache, layer, params);
     if (st != HC_OK) return st;
     if (tokens <= 0) return fail(HC_INVALID_ARGUMENT, "tokens must be positive");
-    if (tokens > 1 && tokens <= cache->ws.qprep_tokens) {
+    if (tokens > 1 && tokens <= cache->ws.qprep_capacity) {
         // One prologue launch for k, v and q, then the attention kernel.
         return prefill_impl(ctx, cache, layer, seq, q, out, tokens, first_position, params, false,
                             static_cast<cudaStream_t>(stream), k, v);
@@ -1326,30 +1304,24 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
     if (tokens <= 0 || chunk <= 0) return fail(HC_INVALID_ARGUMENT, "tokens and chunk must be positive");
     const int d = params->head_dim;
     const int mult = params->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
-    // A chunk's prologue (K/V append, query norm and rotation) touches nothing the previous chunk's
-    // attention reads, apart from the prepared-query buffer, which has two slots: it runs on a stream
-    // of its own, one chunk ahead, in the SMs the attention kernel leaves idle while its last thread
-    // blocks finish.  (A ring is stored one margin longer than the reference's, so the rows of chunk
-    // i + 1 land on positions older than any key chunk i attends to.)
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // What a chunk is makes no difference to a bit of the results (but for blocks, which end with their token's chunk),
+    // so the library takes as many tokens at a time as it can: all of the keys are appended, then all of the
+    // queries attend, in one launch each, whose row tiles fill the SMs evenly.  (Chunk by chunk, even with two
+    // chunks in flight, every launch had its own ramp and ragged last wave.)  A ring takes what fits beside
+    // the window of its first token.
     const hc_layer_store& L = cache->layers[size_t(layer)];
-    const bool ahead_ok = chunk > 1 && chunk <= cache->ws.qprep_tokens && tokens > chunk && cache->copy_in != nullptr &&
-                          (L.ring == 0 || L.ring >= L.desc.window + 2 * chunk);
-    // Nor does a chunk's attention read anything the previous chunk's attention writes (the workspace
-    // for segment partials and second-fold state exists twice): the chunks alternate between the
-    // caller's stream and a second one, and a chunk's thread blocks take over the SMs as the previous
-    // chunk's thread blocks leave them, instead of waiting for the last one.
-    const bool alternate = ahead_ok && cache->copy_out != nullptr;
-    if (ahead_ok) {
-        cudaError_t err = cudaEventRecord(cache->entry, s);
-        if (err == cudaSuccess) err = cudaStreamWaitEvent(cache->copy_in, cache->entry, 0);
-        if (err == cudaSuccess && alternate) err = cudaStreamWaitEvent(cache->copy_out, cache->entry, 0);
-        if (err != cudaSuccess) return check_cuda(err, "prefill chunks: entry event");
+    if (L.ring > 0 && std::min(chunk, tokens) > L.ring_margin) {
+        return check_positions(cache, L, first_position, std::min(chunk, tokens), params);
     }
-    bool other_used = false;
-    int index = 0;
-    for (int start = 0; start < tokens; start += chunk, ++index) {
-        const int count = std::min(chunk, tokens - start);
+    int step = chunk;
+    if (!params->block_ends) {
+        int most = L.ring > 0 ? L.ring - L.desc.window : tokens;
+        most = std::max(std::min(most, cache->ws.qprep_capacity), std::min(chunk, tokens));
+        const int parts = (tokens + most - 1) / most;
+        step = std::min(most, ((tokens + parts - 1) / parts + kTileKeys - 1) / kTileKeys * kTileKeys);
+    }
+    for (int start = 0; start < tokens; start += step) {
+        const int count = std::min(step, tokens - start);
         hc_attn_params local = *params;
         if (params->block_ends) local.block_ends = params->block_ends + start;
         if (params->gate_layout == HC_GATE_SEPARATE) {
@@ -1359,35 +1331,13 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
         const void* k_rows = offset_rows(k, size_t(start), size_t(params->kv_heads) * d, params->io_dtype);
         const void* v_rows = offset_rows(v, size_t(start), size_t(params->kv_heads) * d, params->io_dtype);
         void* out_rows = const_cast<unsigned char*>(offset_rows(out, size_t(start), size_t(params->q_heads) * d, params->io_dtype));
-        if (ahead_ok && count > 1) {
-            const int slot = index & 1;
-            // The slot's prepared queries were last read by the attention of chunk index - 2.
-            if (index >= 2) {
-                const cudaError_t err = cudaStreamWaitEvent(cache->copy_in, cache->step_done[slot], 0);
-                if (err != cudaSuccess) return check_cuda(err, "prefill chunks: slot event");
-            }
-            const PrologueAhead ahead{cache->copy_in, cache->in_done[slot], slot};
-            const cudaStream_t attend_on = (alternate && slot == 1) ? cache->copy_out : s;
-            other_used = other_used || attend_on != s;
+        if (count > 1 && count <= cache->ws.qprep_capacity) {
             st = prefill_impl(ctx, cache, layer, seq, q_rows, out_rows, count, first_position + start, &local, false,
-                              attend_on, k_rows, v_rows, &ahead);
-            if (st != HC_OK) return st;
-            const cudaError_t err = cudaEventRecord(cache->step_done[slot], attend_on);
-            if (err != cudaSuccess) return check_cuda(err, "prefill chunks: step event");
+                              static_cast<cudaStream_t>(stream), k_rows, v_rows, step);
         } else {
-            if (other_used) {
-                // A chunk outside the pipeline (a last chunk of one token) follows everything before it.
-                const cudaError_t err = cudaStreamWaitEvent(s, cache->step_done[1], 0);
-                if (err != cudaSuccess) return check_cuda(err, "prefill chunks: join event");
-            }
             st = hc_layer_step(ctx, cache, layer, seq, q_rows, k_rows, v_rows, out_rows, count, first_position + start, &local, stream);
-            if (st != HC_OK) return st;
         }
-    }
-    if (other_used) {
-        // The caller's stream ends behind the chunks that ran on the other one.
-        const cudaError_t err = cudaStreamWaitEvent(s, cache->step_done[1], 0);
-        if (err != cudaSuccess) return check_cuda(err, "prefill chunks: join event");
+        if (st != HC_OK) return st;
     }
     return HC_OK;
 }

@@ -96,19 +96,13 @@ struct EpilogueArgs {
 };
 
 struct Workspace {
-    uint16_t* qprep = nullptr;   // bf16 [2][qprep_tokens][q_heads][d]: two slots, so that a chunk's prologue can
-                                 // run while the previous chunk's attention still reads its queries
-    size_t qprep_slot_elems = 0; // elements of one slot
-    int qprep_tokens = 0;
+    uint16_t* qprep = nullptr;   // bf16 [qprep_capacity][q_heads][d]
+    int qprep_capacity = 0;
+    int qprep_tokens = 0;        // what the host-buffer calls take at once: max(prefill_chunk, max_seqs)
     float* part_o = nullptr;     // fp32 [rows][slots][d]: segment partials, rows and slots those of the call
     float* part_ml = nullptr;    // fp32 [rows][slots][2]
     size_t part_o_floats = 0;    // capacities
     size_t part_ml_floats = 0;
-    // What a prefill launch can need of the two (segment partials or second-fold state): the buffers
-    // hold it twice, so that two chunks' attention launches may be in flight at once, the second one
-    // working in the upper halves [prefill_o_floats, 2 prefill_o_floats) and likewise for part_ml.
-    size_t prefill_o_floats = 0;
-    size_t prefill_ml_floats = 0;
     // Counters by which the last thread block of a decode row (or of a row's segment) to finish knows that it
     // is the last; zero between launches.
     unsigned* tickets = nullptr;

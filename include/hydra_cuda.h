@@ -65,7 +65,7 @@ typedef enum hc_storage {
 typedef enum hc_kernel_path {
     HC_PATH_AUTO = 0,
     HC_PATH_SIMT = 1,      /* CUDA-core kernels: any head_dim <= 512                                */
-    HC_PATH_TENSOR = 2     /* tcgen05 / TMEM / TMA kernels: head_dim 64, 128 or 256                 */
+    HC_PATH_TENSOR = 2     /* tcgen05 / TMEM / TMA kernels: head_dim 64, 128, 256 or 512            */
 } hc_kernel_path;
 
 typedef enum hc_gate_layout {
@@ -141,7 +141,7 @@ typedef struct hc_attn_params {
      * The call is worked in chunks of at most the cache's prefill_chunk tokens and a block reaches no
      * further than the end of its token's chunk, the last key appended by then (the reference reads
      * on, into rows not yet written, when a chunk boundary cuts an image).  The tensor-core kernels
-     * take the buffer (head_dim 64, 128, 256: whole rows per item, every item reaching to the chunk's
+     * take the buffer (head_dim 64, 128, 256, 512: whole rows per item, every item reaching to the chunk's
      * last key tile), the general kernel the rest.  Rows outside the blocks keep, bit for bit, the
      * results of the call without the buffer, and so still equal their decode steps. */
     const int* block_ends;
@@ -231,7 +231,7 @@ HC_API hc_status hc_rms_norm(hc_context* ctx, const void* x, const void* scale_b
  * one head's history is contiguous), zero-filled, plus the split-attention workspace.
  * `prefill_chunk` is KVCache.prefillChunk (512 in the reference): a ring reports, and bounds chunks
  * and rewinds by, window + prefill_chunk rows rounded up to a multiple of 128; it is stored one such
- * margin longer (hc_layer_info.capacity), which lets hc_prefill_chunks overlap consecutive chunks.
+ * margin longer (hc_layer_info.capacity), which lets hc_prefill_chunks take several chunks at once.
  * `shard` may be NULL.
  *
  * The call also fixes how each layer groups its 128-key tiles into segments (1024 or 4096 keys),
@@ -481,12 +481,10 @@ HC_API hc_status hc_layer_step(hc_context* ctx, hc_kv_cache* cache, int layer, i
 
 /* hc_layer_step for a whole prompt: `tokens` tokens in chunks of `chunk` (the reference's
  * PrefillRunner loop, Sources/HydraMetal/PrefillRunner.swift:128-184, one call per prompt instead of
- * one per chunk).  Each chunk is one hc_layer_step and the results are bit for bit those of the
- * chunk-by-chunk calls.  The work starts behind whatever `stream` holds at the call and `stream` ends
- * behind all of it, like any other call; in between, on layers with linear storage, the library
- * runs a chunk's prologue one chunk ahead and alternate chunks' attention on two streams of its
- * own (ordered by events), so that a chunk's kernels start while the previous chunk's are still
- * finishing. */
+ * one per chunk).  The results are bit for bit those of the chunk-by-chunk calls.  Chunks do not
+ * matter to the results, except that a bidirectional block ends with its token's chunk, so without
+ * block_ends the library takes as many tokens at a time as its workspace holds (64 MB of prepared
+ * queries), or on a ring as fit beside the window: usually one prologue and one attention launch. */
 HC_API hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int seq,
                                    const void* q, const void* k, const void* v, void* out,
                                    int tokens, int first_position, int chunk,
