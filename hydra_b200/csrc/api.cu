@@ -755,7 +755,8 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
                               reach > (2 * kTileKeys << kLogSegmentSmall);
         const bool batched = max_seqs >= 8;
         L.log_segment_general = few_rows || batched ? kLogSegmentSmall : kLogSegmentLarge;
-        L.log_segment = L.log_segment_general == kLogSegmentLarge && d >= 256 ? kLogSegmentWide : L.log_segment_general;
+        // (A whole row of 256 columns pays 6000 clocks, two key tiles, for every segment it spans.)
+        L.log_segment = pairs && !batched ? kLogSegmentWide : L.log_segment_general;
         // Workspace for the partials of split launches.  Decode, at its finest cut: one per (batch
         // entry, query head, key tile of this rank).  Prefill, layers with short segments only: one
         // per (query token, query head, segment).

@@ -38,14 +38,16 @@ constexpr int kPairO = 256;                          // O columns of an item
 constexpr int kPairOCol = 2 * kTileKeys;             // their place in tensor memory
 constexpr int kPairStageBytes = 16 * 1024;           // K: 64 keys x 128 of head_dim; V: 128 keys x 64 columns; per CTA
 constexpr int kPairBoxBytes = 64 * 128;              // a box of 64 rows x 64 elements
+constexpr int kPairStoreBytes = 32 * 64;
 
 template <int D>
 struct PairLayout {
     static constexpr int kHalves = D / kPairO;               // items per row tile
     static constexpr int kQBytes = kRows * D * 2;
-    static constexpr int kStages = D == 256 ? 9 : 5;
+    static constexpr int kStages = D == 256 ? 8 : 4;
     static constexpr int kKChunks = D / 128;                 // stages of a K tile
-    static constexpr int kSmemBytes = 1024 + kQBytes + kStages * kPairStageBytes;
+    // The epilogue's stores go through 2 KB per fold warp: 32 rows x 64 bytes.
+    static constexpr int kSmemBytes = 1024 + kQBytes + kStages * kPairStageBytes + 8 * kPairStoreBytes;
 };
 
 struct PairBarriers {
@@ -151,7 +153,8 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
     unsigned char* q_smem = base;
     unsigned char* ring = q_smem + PL::kQBytes;
-    PairBarriers* bars = reinterpret_cast<PairBarriers*>(ring + PL::kStages * kPairStageBytes);
+    unsigned char* store_smem = ring + PL::kStages * kPairStageBytes;
+    PairBarriers* bars = reinterpret_cast<PairBarriers*>(store_smem + 8 * kPairStoreBytes);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -556,8 +559,8 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     for (int i = 0; i < 128; ++i) A[i] = __fmul_rn(A[i], b);
                 }
             }
-            if (!valid) continue;
             if (args.ep.write_partial) {
+                if (!valid) continue;
                 float* dst = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2) + col0;
                 #pragma unroll
                 for (int i = 0; i < 128; i += 2) *reinterpret_cast<float2*>(dst + i) = make_float2(A[i], A[i + 1]);
@@ -568,45 +571,73 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                 }
                 continue;
             }
+            // Rows leave through shared memory, 64 bytes of each at a time, so that a store instruction touches 8
+            // lines and not 32 (a thread storing its own row took 4300 clocks an item).  Lane l moves piece l % 4 of
+            // rows l / 4, l / 4 + 8, ..
+            if (!warp_has_rows) continue;
             const float inverse = __frcp_rn(L);
-            if (args.ep.gate_layout != HC_GATE_NONE) {
-                // Gated: by way of the state's place, so that the gate's code is there once and not 128 times.
+            unsigned char* stage = store_smem + (warp - 12) * kPairStoreBytes;
+            auto piece = [&](int r, int c) -> uint4* { return reinterpret_cast<uint4*>(stage + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); };
+            const int c = lane & 3;
+            auto row_of = [&](int k, size_t& out_row) -> bool {
+                const int r = quad * 32 + k * 8 + (lane >> 2);
+                const int token = token0 + (r >> args.log_group);
+                out_row = size_t(w.row0 + token) * args.q_heads + size_t(w.kv_head) * G + (r & (G - 1));
+                return token < w.valid_tokens;
+            };
+            if (args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32) {
+                uint16_t* out = reinterpret_cast<uint16_t*>(args.ep.out) + col0 + c * 8;
                 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    state[i * kRows] = make_float4(__fmul_rn(A[4 * i], inverse), __fmul_rn(A[4 * i + 1], inverse),
-                                                  __fmul_rn(A[4 * i + 2], inverse), __fmul_rn(A[4 * i + 3], inverse));
-                }
-                const size_t gate_base = (args.ep.gate_layout == HC_GATE_INTERLEAVED ? vec * size_t(2 * D) + D : vec * size_t(D)) + col0;
-                #pragma unroll 2
-                for (int i = 0; i < 32; ++i) {
-                    const float4 v = state[i * kRows];
-                    float r[4] = {v.x, v.y, v.z, v.w};
+                for (int i = 0; i < 128; i += 32) {
                     #pragma unroll
-                    for (int u = 0; u < 4; ++u) r[u] = __fmul_rn(r[u], sigmoid_gate(load_io(args.ep.gate, gate_base + 4 * i + u, args.ep.io_dtype)));
-                    if (args.ep.io_dtype == HC_F32) {
-                        *reinterpret_cast<float4*>(reinterpret_cast<float*>(args.ep.out) + vec * D + col0 + 4 * i) = make_float4(r[0], r[1], r[2], r[3]);
-                    } else {
-                        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(args.ep.out) + vec * D + col0 + 4 * i) =
-                            make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
+                    for (int u = 0; u < 4; ++u) {
+                        const float* v = &A[i + u * 8];
+                        *piece(lane, u) = make_uint4(pack_bf16x2(__fmul_rn(v[0], inverse), __fmul_rn(v[1], inverse)),
+                                                     pack_bf16x2(__fmul_rn(v[2], inverse), __fmul_rn(v[3], inverse)),
+                                                     pack_bf16x2(__fmul_rn(v[4], inverse), __fmul_rn(v[5], inverse)),
+                                                     pack_bf16x2(__fmul_rn(v[6], inverse), __fmul_rn(v[7], inverse)));
                     }
-                }
-            } else if (args.ep.io_dtype == HC_F32) {
-                float* dst = reinterpret_cast<float*>(args.ep.out) + vec * D + col0;
-                #pragma unroll
-                for (int i = 0; i < 128; i += 4) {
-                    *reinterpret_cast<float4*>(dst + i) = make_float4(__fmul_rn(A[i], inverse), __fmul_rn(A[i + 1], inverse),
-                                                                      __fmul_rn(A[i + 2], inverse), __fmul_rn(A[i + 3], inverse));
+                    __syncwarp();
+                    #pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        size_t out_row;
+                        if (row_of(k, out_row)) *reinterpret_cast<uint4*>(out + out_row * D + i) = *piece(k * 8 + (lane >> 2), c);
+                    }
+                    __syncwarp();
                 }
             } else {
-                uint16_t* dst = reinterpret_cast<uint16_t*>(args.ep.out) + vec * D + col0;
+                const int gate_layout = args.ep.gate_layout;
+                const size_t gate_stride = gate_layout == HC_GATE_INTERLEAVED ? size_t(2 * D) : size_t(D);
+                const size_t gate_first = (gate_layout == HC_GATE_INTERLEAVED ? D : 0) + col0 + c * 4;
                 #pragma unroll
-                for (int i = 0; i < 128; i += 8) {
-                    uint4 packed;
-                    packed.x = pack_bf16x2(__fmul_rn(A[i], inverse), __fmul_rn(A[i + 1], inverse));
-                    packed.y = pack_bf16x2(__fmul_rn(A[i + 2], inverse), __fmul_rn(A[i + 3], inverse));
-                    packed.z = pack_bf16x2(__fmul_rn(A[i + 4], inverse), __fmul_rn(A[i + 5], inverse));
-                    packed.w = pack_bf16x2(__fmul_rn(A[i + 6], inverse), __fmul_rn(A[i + 7], inverse));
-                    *reinterpret_cast<uint4*>(dst + i) = packed;
+                for (int i = 0; i < 128; i += 16) {
+                    #pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const float* v = &A[i + u * 4];
+                        *piece(lane, u) = make_uint4(__float_as_uint(__fmul_rn(v[0], inverse)), __float_as_uint(__fmul_rn(v[1], inverse)),
+                                                     __float_as_uint(__fmul_rn(v[2], inverse)), __float_as_uint(__fmul_rn(v[3], inverse)));
+                    }
+                    __syncwarp();
+                    #pragma unroll 1
+                    for (int k = 0; k < 4; ++k) {
+                        size_t out_row;
+                        if (!row_of(k, out_row)) continue;
+                        const uint4 x = *piece(k * 8 + (lane >> 2), c);
+                        float r[4] = {__uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z), __uint_as_float(x.w)};
+                        if (gate_layout != HC_GATE_NONE) {
+                            const size_t at = out_row * gate_stride + gate_first + i;
+                            #pragma unroll
+                            for (int u = 0; u < 4; ++u) r[u] = __fmul_rn(r[u], sigmoid_gate(load_io(args.ep.gate, at + u, args.ep.io_dtype)));
+                        }
+                        const size_t at = out_row * D + col0 + i + c * 4;
+                        if (args.ep.io_dtype == HC_F32) {
+                            *reinterpret_cast<float4*>(reinterpret_cast<float*>(args.ep.out) + at) = make_float4(r[0], r[1], r[2], r[3]);
+                        } else {
+                            *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(args.ep.out) + at) =
+                                make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
+                        }
+                    }
+                    __syncwarp();
                 }
             }
         }
