@@ -319,8 +319,9 @@ __device__ __forceinline__ void dec_stage(const DecArgs& args, const DecList* li
             if (p0 + u * stride >= passes) break;                 // warp-uniform
             const int vec = (p0 + u * stride) * HL::kPerWarp + sub;
             const int norm = vec < G ? args.norm_q : vec == G ? args.norm_k : args.norm_v;
-            prepare_head<D>(lo[u], hi[u], norm, vec < G ? args.q_weight : args.k_weight, args.eps, rotate && vec <= G, c, s, m,
-                            any_norm);
+            float wl[HL::kElems], wh[HL::kElems];
+            if (norm == 1) load_head<D>(vec < G ? args.q_weight : args.k_weight, 0, 1, m, wl, wh);
+            prepare_head<D>(lo[u], hi[u], norm, wl, wh, args.eps, rotate && vec <= G, c, s, any_norm);
             if (vec >= total) continue;
             #pragma unroll
             for (int x = 0; x < HL::kVecs; ++x) {

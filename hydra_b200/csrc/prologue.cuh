@@ -24,8 +24,8 @@ __device__ __forceinline__ void load_io4(const void* base, size_t index, int dty
 }
 __device__ __forceinline__ uint2 pack_bf16x4(const float (&v)[4]) {
     uint2 r;
-    r.x = uint32_t(float_to_bf16_bits(v[0])) | (uint32_t(float_to_bf16_bits(v[1])) << 16);
-    r.y = uint32_t(float_to_bf16_bits(v[2])) | (uint32_t(float_to_bf16_bits(v[3])) << 16);
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.x) : "f"(v[1]), "f"(v[0]));
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.y) : "f"(v[3]), "f"(v[2]));
     return r;
 }
 
@@ -66,11 +66,13 @@ __device__ __forceinline__ void load_rotation(const float* cos_row, const float*
 
 // In place: the norm (0 none, 1 with `weight`, 2 weightless), then the rotation when `rope`.  The lanes of
 // a warp may hold vectors with different settings: the shuffles are executed by all of them.
+// wl, wh: the weight's elements of this lane (norm 1).
 template <int D>
 __device__ __forceinline__ void prepare_head(float (&lo)[HeadLanes<D>::kElems], float (&hi)[HeadLanes<D>::kElems], int norm,
-                                             const uint16_t* weight, float eps, bool rope,
+                                             const float (&wl)[HeadLanes<D>::kElems], const float (&wh)[HeadLanes<D>::kElems],
+                                             float eps, bool rope,
                                              const float (&c)[HeadLanes<D>::kElems], const float (&s)[HeadLanes<D>::kElems],
-                                             int m, bool any_norm) {
+                                             bool any_norm) {
     constexpr int kElems = HeadLanes<D>::kElems, kLanes = HeadLanes<D>::kLanes;
     if (any_norm) {                                  // warp-uniform
         float sum = 0.0f;
@@ -87,8 +89,6 @@ __device__ __forceinline__ void prepare_head(float (&lo)[HeadLanes<D>::kElems], 
             #pragma unroll
             for (int j = 0; j < kElems; ++j) { lo[j] = __fmul_rn(lo[j], inverse); hi[j] = __fmul_rn(hi[j], inverse); }
             if (norm == 1) {
-                float wl[kElems], wh[kElems];
-                load_head<D>(weight, 0, 1, m, wl, wh);
                 #pragma unroll
                 for (int j = 0; j < kElems; ++j) { lo[j] = __fmul_rn(lo[j], wl[j]); hi[j] = __fmul_rn(hi[j], wh[j]); }
             }
