@@ -932,12 +932,14 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                     const int slot = int(n % DL::kKStages);
                     if (!mbar_wait(&bars->k_full[slot], (n / DL::kKStages) & 1, abort_flag, args.status, 45)) { ok = false; break; }
                     tc_fence_after();
+                    const uint64_t k_desc = warp_uniform(k_desc0 + uint64_t((slot * kBoxBytes) >> 4));
+                    const uint64_t q_desc = warp_uniform(q_desc0 + uint64_t(((it & 1) * DL::kQBytes + block * DL::kQBlock) >> 4));
+                    const uint32_t d_tmem = warp_uniform(tmem + sb * kQRows);
                     if (elect_one()) {
                         #pragma unroll
                         for (int ks = 0; ks < 4; ++ks) {
-                            mma_ss(tmem + sb * kQRows, k_desc0 + uint64_t((slot * kBoxBytes + ks * 32) >> 4),
-                                   q_desc0 + uint64_t(((it & 1) * DL::kQBytes + block * DL::kQBlock + ks * 32) >> 4), idesc,
-                                   (block | ks) != 0 ? 1u : 0u);
+                            mma_ss(d_tmem, k_desc + uint64_t((ks * 32) >> 4), q_desc + uint64_t((ks * 32) >> 4), idesc,
+                                   ks != 0 ? 1u : uint32_t(block != 0));
                         }
                         tc_commit(&bars->k_empty[slot]);
                         if (block == DL::kBlocks - 1) {
@@ -968,15 +970,15 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                     const int slot = int(n % DL::kVStages);
                     if (!mbar_wait(&bars->v_full[slot], (n / DL::kVStages) & 1, abort_flag, args.status, 48)) { ok = false; break; }
                     tc_fence_after();
+                    const uint32_t v_addr = ring_addr + slot * DL::kVStageBytes;
+                    const uint64_t v_desc = warp_uniform(smem_desc(v_addr, DL::kSumOnTensor ? ones_addr - v_addr : uint32_t(kBoxBytes)));
+                    const uint64_t p_desc = warp_uniform(p_desc0 + uint64_t((ob * kPBytes) >> 4));
+                    const uint32_t o_tmem = warp_uniform(tmem + DL::kOCol + ob * DL::kOCols + part * kQRows);
                     if (elect_one()) {
-                        const uint32_t v_addr = ring_addr + slot * DL::kVStageBytes;
-                        const uint64_t v_desc = smem_desc(v_addr, DL::kSumOnTensor ? ones_addr - v_addr : uint32_t(kBoxBytes));
-                        const uint32_t o_tmem = tmem + DL::kOCol + ob * DL::kOCols + part * kQRows;
                         #pragma unroll
                         for (int ks = 0; ks < kTileKeys / 16; ++ks) {
-                            mma_ss(o_tmem, v_desc + uint64_t((ks * 2048) >> 4),
-                                   p_desc0 + uint64_t((ob * kPBytes + (ks >> 2) * (kQRows * 128) + (ks & 3) * 32) >> 4), idesc,
-                                   ks != 0 ? 1u : 0u);
+                            mma_ss(o_tmem, v_desc + uint64_t((ks * 2048) >> 4), p_desc + uint64_t(((ks >> 2) * (kQRows * 128) + (ks & 3) * 32) >> 4),
+                                   idesc, ks != 0 ? 1u : 0u);
                         }
                         tc_commit(&bars->v_empty[slot]);
                         if (part == DL::kVTileStages - 1) {

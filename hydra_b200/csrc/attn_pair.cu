@@ -258,14 +258,17 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     const int slot = int(n % PL::kStages);
                     if (!mbar_wait(&bars->full[slot], (n / PL::kStages) & 1, abort_flag, args.status, 3)) return false;
                     tc_fence_after();
+                    const uint64_t q_desc = warp_uniform(q_desc0 + uint64_t((2 * c * (kRows * 128)) >> 4));
+                    const uint64_t k_desc = warp_uniform(k_desc0 + uint64_t((slot * kPairStageBytes) >> 4));
+                    const uint32_t d_tmem = warp_uniform(s_tmem);
                     if (elect_one()) {
                         #pragma unroll
                         for (int b = 0; b < 2; ++b) {
                             #pragma unroll
                             for (int ks = 0; ks < 4; ++ks) {
-                                mma_ss_pair(s_tmem, q_desc0 + uint64_t(((2 * c + b) * (kRows * 128) + ks * 32) >> 4),
-                                            k_desc0 + uint64_t((slot * kPairStageBytes + b * kPairBoxBytes + ks * 32) >> 4), idesc_qk,
-                                            (c | b | ks) != 0 ? 1u : 0u);
+                                mma_ss_pair(d_tmem, q_desc + uint64_t((b * (kRows * 128) + ks * 32) >> 4),
+                                            k_desc + uint64_t((b * kPairBoxBytes + ks * 32) >> 4), idesc_qk,
+                                            (b | ks) != 0 ? 1u : uint32_t(c != 0));
                             }
                         }
                         tc_commit_pair(&bars->empty[slot]);
@@ -293,11 +296,13 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     if (t > 0 && !mbar_wait(&bars->o_free[h], (t - 1) & 1, abort_flag, args.status, 7)) { ok = false; break; }
                     if (!mbar_wait(&bars->full[slot], (n / PL::kStages) & 1, abort_flag, args.status, 6)) { ok = false; break; }
                     tc_fence_after();
+                    const uint64_t v_desc = warp_uniform(v_desc0 + uint64_t((slot * kPairStageBytes) >> 4));
+                    const uint32_t d_tmem = warp_uniform(tmem + kPairOCol + h * 128), a_tmem = warp_uniform(p_tmem);
                     if (elect_one()) {
                         #pragma unroll
                         for (int ks = 0; ks < kTileKeys / 16; ++ks) {
-                            mma_ts_pair(tmem + kPairOCol + h * 128, p_tmem + (ks & 3) * 8 + (ks >> 2) * 64,
-                                        v_desc0 + uint64_t((slot * kPairStageBytes + ks * 2048) >> 4), idesc_pv, ks != 0 ? 1u : 0u);
+                            mma_ts_pair(d_tmem, a_tmem + (ks & 3) * 8 + (ks >> 2) * 64, v_desc + uint64_t((ks * 2048) >> 4), idesc_pv,
+                                        ks != 0 ? 1u : 0u);
                         }
                         tc_commit_pair(&bars->empty[slot]);
                         tc_commit_pair(&bars->o_full[h]);

@@ -11,7 +11,7 @@
 // tile fetched by TMA serves 128 tokens.
 //
 // Two kernels.  A call of up to 128 tokens reads the weights once and little else: linear_few_kernel, one CTA
-// per SM, 128 x 32 output tiles with nine stages in flight.  Prompts are bound by the tensor pipe:
+// per SM, narrow output tiles, up to nine 16 to 40 KB stages in flight.  Prompts are bound by the tensor pipe:
 // linear_pair_kernel, where two SMs share a 256-row output tile (cta_group::2: each loads its own 128
 // rows of x and half of the weight tile, so a K step brings 24 to 32 KB into each SM for 256 x BN outputs where a
 // CTA of its own needed 48 KB for 128 x 256), six to eight stages, two accumulators in tensor memory.
@@ -35,13 +35,13 @@ constexpr int kLinK = 64;                       // one 128-byte swizzled row of 
 constexpr int kLinABytes = kLinM * kLinK * 2;   // 16 KB
 constexpr int kLinThreads = 256;
 
-// Few tokens: 128 x 32 tiles, nine stages: narrow column tiles spread the weight's rows over all SMs with
-// enough of them in flight (9 x 4 KB per SM).
-constexpr int kFewN = 32;
-constexpr int kFewStages = 9;
-constexpr int kFewBBytes = kFewN * kLinK * 2;
-constexpr int kFewTmemCols = 64;                // two accumulators
-constexpr int kFewSmemBytes = 1024 + kFewStages * (kLinABytes + kFewBBytes);
+// Few tokens: the work is reading the weight once.  Column tiles of BN weight rows, as narrow as gives every SM one tile
+// and none two (a second tile doubles the call's time; columns cost little), and stages of `subs` K steps of
+// 64 each: with one K step a stage the waits and the issue around its four MMAs took longer than they did
+// (137 clocks an MMA against the 41 it takes), with four they do not.
+constexpr int kFewMaxStages = 9;
+constexpr int kFewSmemBytes = 208 * 1024;       // ring and the x tile's overhang (see launch_few)
+constexpr int kFewTmemCols = 128;               // two accumulators of up to 64 columns
 
 // Pairs: 256 x BN tiles, each CTA holding 128 rows of x and BN / 2 rows of w per stage.  An output element is the same
 // sum in the same order in every shape, so a token projected alone and inside a prompt gets the same bits.
@@ -81,7 +81,8 @@ struct LinArgs {
     int y_dtype;              // HC_F32 or HC_BF16
     int tokens;
     int tiles_m, n_tiles, k_steps;   // tiles of 128 rows (few tokens) or 256 (pairs)
-    int a_bytes;              // of one x box: 128 rows x 128 bytes, fewer rows for a call of few tokens
+    int a_bytes;              // few tokens: of one x box, as many rows of 128 bytes as there are tokens (rounded up to 8)
+    int stages;               // few tokens
     int* status;
 };
 
@@ -132,7 +133,7 @@ __device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob&
     }
 }
 __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4 (&z)[8], int row0,
-                                            int col0, unsigned char* stage) {
+                                            int col0, unsigned char* stage, int width = 32) {
     if (col0 >= job.out_features || row0 >= args.tokens) return;          // warp-uniform
     const int lane = threadIdx.x & 31;
     #pragma unroll
@@ -141,6 +142,7 @@ __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& j
     }
     __syncwarp();
     const int chunk = lane & 7, col = col0 + chunk * 4;
+    const bool mine = chunk * 4 < width;
     const bool vectors = col + 4 <= job.out_features && (job.out_features & 3) == 0;
     float b[4];
     #pragma unroll
@@ -148,7 +150,7 @@ __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& j
     #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const int r = k * 4 + (lane >> 3);
-        if (row0 + r >= args.tokens) continue;
+        if (row0 + r >= args.tokens || !mine) continue;
         const float4 x = *reinterpret_cast<const float4*>(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
         float y[4] = {__fadd_rn(x.x, b[0]), __fadd_rn(x.y, b[1]), __fadd_rn(x.z, b[2]), __fadd_rn(x.w, b[3])};
         const size_t at = size_t(row0 + r) * job.out_features + col;
@@ -176,121 +178,150 @@ __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& j
     __syncwarp();
 }
 
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1) : "memory");
+}
+
+template <int BN, int SUBS>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
-                 const __grid_constant__ CUtensorMap tmap_w1, const __grid_constant__ CUtensorMap tmap_w2,
-                 const __grid_constant__ CUtensorMap tmap_w3, const LinArgs args) {
-    constexpr int kLinN = kFewN;
-    constexpr int kLinStages = kFewStages;
-    constexpr int kLinBBytes = kFewBBytes;
+                  const __grid_constant__ CUtensorMap tmap_w1, const __grid_constant__ CUtensorMap tmap_w2,
+                  const __grid_constant__ CUtensorMap tmap_w3, const LinArgs args) {
+    constexpr int kWBytes = BN * kLinK * 2;                         // weight rows of a K step
     extern __shared__ unsigned char raw_smem[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
-    unsigned char* a_smem = base;                                   // [stages][128 x 64]
-    unsigned char* b_smem = a_smem + kLinStages * kLinABytes;       // [stages][256 x 64]
-    LinBarriers* bars = reinterpret_cast<LinBarriers*>(b_smem + kLinStages * kLinBBytes);        // and the epilogue's staging
+    const int a_stage = SUBS * args.a_bytes, w_stage = SUBS * kWBytes;
+    unsigned char* a_smem = base;                                   // [stages][subs][x rows x 64]
+    unsigned char* w_smem = a_smem + args.stages * a_stage;         // [stages][subs][BN x 64]
+    LinBarriers* bars = reinterpret_cast<LinBarriers*>(base + kFewSmemBytes);        // and the epilogue's staging
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     volatile int* abort_flag = &bars->abort_flag;
+    const int n_tiles = args.n_tiles, k_steps = args.k_steps;
+    auto weight_map = [&](int job) { return job == 0 ? &tmap_w0 : job == 1 ? &tmap_w1 : job == 2 ? &tmap_w2 : &tmap_w3; };
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kLinStages; ++i) {
+        for (int i = 0; i < kFewMaxStages; ++i) {
             mbar_init(&bars->full[i], 1);
             mbar_init(&bars->empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bars->acc_full[i], 1);
-            mbar_init(&bars->acc_empty[i], 128);
+            mbar_init(&bars->acc_empty[i], 4);
         }
         bars->abort_flag = 0;
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc(&bars->tmem_base, kFewTmemCols);
-    if (warp == 0 && lane == 0) {
-        prefetch_tensormap(&tmap_x);
-        prefetch_tensormap(&tmap_w0);
+    if (warp == 2 && int(blockIdx.x) < n_tiles) {
+        // While the kernel before this one finishes, the weights come into L2 (where it may still change them: nothing
+        // is read into this CTA before the wait below).
+        const LinTile where = decode_tile(args, blockIdx.x);
+        for (int k = lane; k < k_steps; k += 32) tma_prefetch_2d(weight_map(where.job), k * kLinK, where.tn * BN);
     }
+    if (warp == 0 && lane == 0) prefetch_tensormap(&tmap_x);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = bars->tmem_base;
     pdl_wait();
 
-    const int n_tiles = args.n_tiles;
     if (warp == 0) {
         // ===== producer =====
         if (lane == 0) {
-            uint32_t step = 0;
+            int slot = 0;
+            uint32_t round = 0;
             bool ok = true;
             for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x) {
                 const LinTile where = decode_tile(args, tile);
-                const int tn = where.tn, tm = where.tm;
-                const CUtensorMap* tmap_w = where.job == 0 ? &tmap_w0 : where.job == 1 ? &tmap_w1 : where.job == 2 ? &tmap_w2 : &tmap_w3;
-                for (int k = 0; k < args.k_steps; ++k, ++step) {
-                    const int slot = int(step % kLinStages);
-                    const uint32_t round = step / kLinStages;
+                const CUtensorMap* tmap_w = weight_map(where.job);
+                for (int k = 0; k < k_steps; k += SUBS) {
+                    const int count = min(SUBS, k_steps - k);
                     if (round > 0 && !mbar_wait(&bars->empty[slot], (round - 1) & 1, abort_flag, args.status, 21)) { ok = false; break; }
-                    mbar_expect_tx(&bars->full[slot], uint32_t(args.a_bytes) + kLinBBytes);
-                    tma_load_2d(a_smem + slot * kLinABytes, &tmap_x, &bars->full[slot], k * kLinK, tm * kLinM);
-                    tma_load_2d(b_smem + slot * kLinBBytes, tmap_w, &bars->full[slot], k * kLinK, tn * kLinN);
+                    mbar_expect_tx(&bars->full[slot], uint32_t(count * (args.a_bytes + kWBytes)));
+                    for (int u = 0; u < count; ++u) {
+                        tma_load_2d(w_smem + slot * w_stage + u * kWBytes, tmap_w, &bars->full[slot], (k + u) * kLinK, where.tn * BN);
+                    }
+                    for (int u = 0; u < count; ++u) {
+                        tma_load_2d(a_smem + slot * a_stage + u * args.a_bytes, &tmap_x, &bars->full[slot], (k + u) * kLinK, 0);
+                    }
+                    if (++slot == args.stages) {
+                        slot = 0;
+                        ++round;
+                    }
                 }
             }
         }
     } else if (warp == 1) {
         // ===== MMA issuer (the warp walks the loop converged; one elected lane issues) =====
-        constexpr uint32_t idesc = instr_desc(kLinN, false);
+        constexpr uint32_t idesc = instr_desc(BN, false);
         const uint64_t a_desc0 = smem_desc(smem_u32(a_smem), 16);
-        const uint64_t b_desc0 = smem_desc(smem_u32(b_smem), 16);
-        uint32_t step = 0, count = 0;
+        const uint64_t w_desc0 = smem_desc(smem_u32(w_smem), 16);
+        int slot = 0;
+        uint32_t round = 0, count = 0;
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x, ++count) {
             const int acc = int(count & 1);
             // The epilogue must have taken this accumulator's previous tile out.
             if (count >= 2 && !mbar_wait(&bars->acc_empty[acc], ((count >> 1) - 1) & 1, abort_flag, args.status, 22)) break;
             tc_fence_after();
-            for (int k = 0; k < args.k_steps; ++k, ++step) {
-                const int slot = int(step % kLinStages);
-                if (!mbar_wait(&bars->full[slot], (step / kLinStages) & 1, abort_flag, args.status, 23)) { ok = false; break; }
+            for (int k = 0; k < k_steps; k += SUBS) {
+                if (!mbar_wait(&bars->full[slot], round & 1, abort_flag, args.status, 23)) { ok = false; break; }
                 tc_fence_after();
+                const uint64_t a_desc = warp_uniform(a_desc0 + uint64_t((slot * a_stage) >> 4));
+                const uint64_t w_desc = warp_uniform(w_desc0 + uint64_t((slot * w_stage) >> 4));
+                const uint32_t x_step = warp_uniform(uint32_t(args.a_bytes >> 4)), d_tmem = warp_uniform(tmem + acc * 64);
+                const int n = min(SUBS, k_steps - k);
                 if (elect_one()) {
-                    const uint64_t a_desc = a_desc0 + uint64_t((slot * kLinABytes) >> 4);
-                    const uint64_t b_desc = b_desc0 + uint64_t((slot * kLinBBytes) >> 4);
                     #pragma unroll
-                    for (int ks = 0; ks < kLinK / 16; ++ks) {
-                        mma_ss(tmem + acc * kLinN, a_desc + uint64_t((ks * 32) >> 4), b_desc + uint64_t((ks * 32) >> 4), idesc,
-                               (k | ks) != 0 ? 1u : 0u);
+                    for (int u = 0; u < SUBS; ++u) {
+                        if (u < n) {
+                            #pragma unroll
+                            for (int ks = 0; ks < kLinK / 16; ++ks) {
+                                mma_ss(d_tmem, a_desc + uint64_t(u * x_step + ((ks * 32) >> 4)), w_desc + uint64_t((u * kWBytes + ks * 32) >> 4), idesc,
+                                       (u | ks) != 0 ? 1u : uint32_t(k != 0));
+                            }
+                        }
                     }
                     tc_commit(&bars->empty[slot]);
-                    if (k + 1 == args.k_steps) tc_commit(&bars->acc_full[acc]);
+                    if (k + n == k_steps) tc_commit(&bars->acc_full[acc]);
                 }
                 __syncwarp();
+                if (++slot == args.stages) {
+                    slot = 0;
+                    ++round;
+                }
             }
         }
     } else if (warp >= 4) {
-        // ===== epilogue: thread = row of the tile =====
+        // ===== epilogue: thread = token =====
         const int quad = warp & 3;
         unsigned char* stage = reinterpret_cast<unsigned char*>(bars + 1) + quad * kLinStageBytes;
         const uint32_t lane_base = uint32_t(quad * 32) << 16;
         uint32_t count = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++count) {
             const LinTile where = decode_tile(args, tile);
-            const int tn = where.tn, tm = where.tm;
             const LinJob& job = args.job[where.job];
             const int acc = int(count & 1);
+            const bool rows = quad * 32 < args.tokens;              // warp-uniform
             float4 z[8];
-            load_residual(args, job, tm * kLinM + quad * 32, tn * kLinN, z);
+            if (rows) load_residual(args, job, quad * 32, where.tn * BN, z);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
-            static_assert(kLinN == 32, "one block per tile");
-            for (int chunk = 0; chunk < kLinN / 32; ++chunk) {
+            #pragma unroll 1
+            for (int col = 0; rows && col < BN; col += 32) {
                 uint32_t v[32];
-                HC_TMEM_LD32(tmem + lane_base + acc * kLinN + chunk * 32, v);
+                HC_TMEM_LD32(tmem + lane_base + acc * 64 + col, v);
                 tc_wait_ld();
-                store_block(args, job, v, z, tm * kLinM + quad * 32, tn * kLinN + chunk * 32, stage);
+                if (col > 0) load_residual(args, job, quad * 32, where.tn * BN + col, z);
+                store_block(args, job, v, z, quad * 32, where.tn * BN + col, stage, BN - col);
                 __syncwarp();          // the next tcgen05.ld is warp-wide
             }
             tc_fence_before();
-            mbar_arrive(&bars->acc_empty[acc]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->acc_empty[acc]);
         }
     }
 
@@ -385,9 +416,9 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 const int slot = int(step % PS::kStages);
                 if (!mbar_wait(&bars->full[slot], (step / PS::kStages) & 1, abort_flag, args.status, 23)) { ok = false; break; }
                 tc_fence_after();
+                const uint64_t a_desc = warp_uniform(a_desc0 + uint64_t((slot * kLinABytes) >> 4));
+                const uint64_t b_desc = warp_uniform(b_desc0 + uint64_t((slot * PS::kBBytes) >> 4));
                 if (elect_one()) {
-                    const uint64_t a_desc = a_desc0 + uint64_t((slot * kLinABytes) >> 4);
-                    const uint64_t b_desc = b_desc0 + uint64_t((slot * PS::kBBytes) >> 4);
                     #pragma unroll
                     for (int ks = 0; ks < kLinK / 16; ++ks) {
                         mma_ss_pair(tmem + acc * BN, a_desc + uint64_t((ks * 32) >> 4), b_desc + uint64_t((ks * 32) >> 4), idesc,
@@ -517,20 +548,29 @@ static hc_status launch_linear_kernel(hc_context* ctx, Kernel kernel, bool (&con
     return check_cuda(launched, "linear kernel launch");
 }
 
+template <int BN>
 static hc_status launch_few(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features, cudaStream_t stream) {
     LinMaps maps;
     // A box that reaches past the last token is filled with zeros, and that fill measured slower than
     // reading real rows (one token: 21 us against 13 us for 128): a call of few tokens loads only the
-    // rows it has.  The rows of the 128-row operand tile it leaves unwritten feed accumulator rows that
-    // are never stored (a row of the result depends on its own row of x alone).
+    // rows it has.  The rows of the 128-row operand tile it leaves unwritten are whatever lies behind it in shared memory
+    // and feed accumulator rows that are never stored (a row of the result depends on its own row of x alone).
     const int x_rows = std::min(kLinM, (args.tokens + 7) & ~7);
     args.a_bytes = x_rows * kLinK * 2;
-    const hc_status st = prepare_linear(maps, x, w, args, in_features, kLinM, kFewN, x_rows, kFewN);
+    // Stages of four K steps while there is room for four of them, of two beyond; the last x tile's overhang
+    // stays inside the ring (there are at least 16 KB of weights behind the x tiles, or room).
+    const int step_bytes = args.a_bytes + BN * kLinK * 2;
+    const int room = kFewSmemBytes - kLinABytes;
+    const int subs = 16 * step_bytes <= room ? 4 : 2;
+    args.stages = std::max(1, std::min(kFewMaxStages, room / (subs * step_bytes)));
+    const hc_status st = prepare_linear(maps, x, w, args, in_features, kLinM, BN, x_rows, BN);
     if (st != HC_OK) return st;
-    static bool configured[64] = {};
+    static bool configured4[64] = {}, configured2[64] = {};
     const int grid = std::max(1, std::min(args.n_tiles, std::max(ctx->sm_count, 1)));
-    return launch_linear_kernel(ctx, linear_few_kernel, configured, grid, kFewSmemBytes + int(sizeof(LinBarriers)) + 4 * kLinStageBytes, maps,
-                                args, stream);
+    constexpr int smem = 1024 + kFewSmemBytes + int(sizeof(LinBarriers)) + 4 * kLinStageBytes;
+    static_assert(smem <= 227 * 1024, "shared memory of one CTA");
+    return subs == 4 ? launch_linear_kernel(ctx, linear_few_kernel<BN, 4>, configured4, grid, smem, maps, args, stream)
+                     : launch_linear_kernel(ctx, linear_few_kernel<BN, 2>, configured2, grid, smem, maps, args, stream);
 }
 
 template <int BN>
@@ -560,7 +600,18 @@ hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* cons
     args.tokens = tokens;
     args.k_steps = in_features / kLinK;
     args.status = ctx->status_dev;
-    if (tokens <= kLinM) return launch_few(ctx, x, w, args, in_features, stream);
+    if (tokens <= kLinM) {
+        const int sms = std::max(ctx->sm_count, 1);
+        auto tiles = [&](int bn) {
+            int n = 0;
+            for (int j = 0; j < n_jobs; ++j) n += (out_features[j] + bn - 1) / bn;
+            return n;
+        };
+        if (tiles(16) <= sms) return launch_few<16>(ctx, x, w, args, in_features, stream);
+        if (tiles(32) <= sms) return launch_few<32>(ctx, x, w, args, in_features, stream);
+        if (tiles(48) <= sms) return launch_few<48>(ctx, x, w, args, in_features, stream);
+        return launch_few<64>(ctx, x, w, args, in_features, stream);
+    }
     // The column tile whose rounds of pairs take least.  A K step costs an SM the larger of its MMAs (2 clocks a column)
     // and of (128 + BN / 2) x 128 bytes out of L2, of which about 60 arrive per clock and SM with all of them
     // loading: 546 clocks for 256 columns, 478, 443, 410.  Measured on 4096, 1024, 600 and 300 tokens of the three

@@ -123,6 +123,15 @@ __device__ __forceinline__ bool elect_one() {
         : "=r"(chosen));
     return chosen != 0;
 }
+// The same value in every lane, in a way the compiler sees: descriptors then live in uniform registers, and the adds
+// between two MMAs cost the issuing thread next to nothing.  (Moved there one by one, 96 clocks an MMA of N = 32
+// that takes 41.)  For converged warps.
+__device__ __forceinline__ uint64_t warp_uniform(uint64_t v) {
+    const uint32_t lo = __shfl_sync(0xffffffffu, uint32_t(v), 0), hi = __shfl_sync(0xffffffffu, uint32_t(v >> 32), 0);
+    return uint64_t(lo) | (uint64_t(hi) << 32);
+}
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // D[tmem] (+)= A[smem] * B[smem]
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                        uint32_t accumulate) {
