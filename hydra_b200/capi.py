@@ -42,6 +42,11 @@ class AttnParamsStruct(ctypes.Structure):
     ]
 
 
+class BlockWeightsStruct(ctypes.Structure):
+    _fields_ = [(name, c_void_p) for name in ("input_norm", "wq", "bq", "wk", "bk", "wv", "bv", "wo", "bo")] \
+        + [("params", AttnParamsStruct)]
+
+
 class LayerInfo(ctypes.Structure):
     _fields_ = [("keys", c_void_p), ("values", c_void_p), ("ring_size", c_int), ("capacity", c_int),
                 ("entry_bytes", c_int), ("windowed", c_int), ("keeps_history", c_int)]
@@ -115,6 +120,9 @@ _PROTOTYPES = {
                               POINTER(AttnParamsStruct), _P]),
     "hc_prefill_chunks": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, _P, c_int, c_int, c_int,
                                   POINTER(AttnParamsStruct), _P]),
+    "hc_attention_stack_bytes": (c_size_t, [POINTER(BlockWeightsStruct), c_int, c_int, c_int]),
+    "hc_attention_stack_host": (c_int, [_P, _P, POINTER(BlockWeightsStruct), c_int, c_int, _P, _P, c_int, c_int, c_int,
+                                        c_float, _P, _P]),
     "hc_prefill_host": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, _P, c_int, c_int, c_int,
                                 POINTER(AttnParamsStruct), _P]),
     "hc_layer_step_host": (c_int, [_P, _P, c_int, c_int, _P, _P, _P, _P, c_int, c_int,

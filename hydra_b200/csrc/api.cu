@@ -501,9 +501,8 @@ hc_status hc_context_create(int device, hc_context** out) {
     if (!ctx) return fail(HC_ALLOC_FAILED, "out of host memory");
     ctx->device = device;
     ctx->sm_count = prop.multiProcessorCount;
-    err = cudaMalloc(&ctx->status_dev, sizeof(int));
-    if (err == cudaSuccess) err = cudaMemset(ctx->status_dev, 0, sizeof(int));
-    if (err == cudaSuccess) err = cudaMallocHost(&ctx->status_host, sizeof(int));
+    err = cudaHostAlloc(&ctx->status_host, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (err == cudaSuccess) err = cudaHostGetDevicePointer(&ctx->status_dev, ctx->status_host, 0);
     if (err != cudaSuccess) {
         hc_context_destroy(ctx);
         return fail(HC_ALLOC_FAILED, std::string("context status word: ") + cudaGetErrorString(err));
@@ -526,7 +525,6 @@ hc_status hc_context_create(int device, hc_context** out) {
 
 void hc_context_destroy(hc_context* ctx) {
     if (!ctx) return;
-    if (ctx->status_dev) cudaFree(ctx->status_dev);
     if (ctx->status_host) cudaFreeHost(ctx->status_host);
     delete ctx;
 }
@@ -534,13 +532,12 @@ void hc_context_destroy(hc_context* ctx) {
 hc_status hc_context_check(hc_context* ctx, void* stream) {
     if (!ctx) return fail(HC_INVALID_ARGUMENT, "null context");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    cudaError_t err = cudaMemcpyAsync(ctx->status_host, ctx->status_dev, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(s);
+    const cudaError_t err = cudaStreamSynchronize(s);
     if (err != cudaSuccess) return check_cuda(err, "stream synchronise");
-    const int word = *ctx->status_host;
+    volatile int* status = ctx->status_host;
+    const int word = *status;
     if (word != 0) {
-        cudaMemsetAsync(ctx->status_dev, 0, sizeof(int), s);
-        cudaStreamSynchronize(s);
+        *status = 0;
         return fail(HC_TIMEOUT, "a kernel gave up a bounded wait (status word " + std::to_string(word) + ")");
     }
     return HC_OK;
@@ -1341,6 +1338,70 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
         if (st != HC_OK) return st;
     }
     return HC_OK;
+}
+
+// The workspace of a stack: hidden (fp32), then normed, q, k, v and attended (bf16), each on a 256-byte boundary.
+struct StackSpace {
+    size_t normed, q, k, v, attended, bytes;
+};
+static StackSpace stack_space(const hc_block_weights* layers, int n_layers, int tokens, int width) {
+    size_t q_row = 0, o_row = 0, kv_row = 0;
+    for (int i = 0; i < n_layers; ++i) {
+        const hc_attn_params& p = layers[i].params;
+        const size_t o = size_t(p.q_heads) * p.head_dim;
+        q_row = std::max(q_row, o * (p.gate_layout == HC_GATE_INTERLEAVED ? 2 : 1));
+        o_row = std::max(o_row, o);
+        kv_row = std::max(kv_row, size_t(p.kv_heads) * p.head_dim);
+    }
+    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
+    const size_t n = size_t(tokens);
+    StackSpace s;
+    s.normed = align(n * width * 4);
+    s.q = s.normed + align(n * width * 2);
+    s.k = s.q + align(n * q_row * 2);
+    s.v = s.k + align(n * kv_row * 2);
+    s.attended = s.v + align(n * kv_row * 2);
+    s.bytes = s.attended + align(n * o_row * 2);
+    return s;
+}
+
+size_t hc_attention_stack_bytes(const hc_block_weights* layers, int n_layers, int tokens, int width) {
+    if (!layers || n_layers <= 0 || tokens <= 0 || width <= 0) return 0;
+    return stack_space(layers, n_layers, tokens, width).bytes;
+}
+
+hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_block_weights* layers, int n_layers, int seq,
+                                  const float* hidden_in, float* hidden_out, int tokens, int width, int first_position, float eps,
+                                  void* workspace, void* stream) {
+    if (!ctx || !cache || !layers || !hidden_in || !hidden_out || !workspace) return fail(HC_INVALID_ARGUMENT, "null context or buffer");
+    if (n_layers <= 0 || n_layers > int(cache->layers.size()) || tokens <= 0 || width <= 0) return fail(HC_INVALID_ARGUMENT, "bad sizes");
+    for (int i = 0; i < n_layers; ++i) {
+        const hc_status st = validate_params(cache, i, &layers[i].params);
+        if (st != HC_OK) return st;
+        if (layers[i].params.io_dtype != HC_BF16) return fail(HC_INVALID_ARGUMENT, "hc_attention_stack_host: io_dtype must be HC_BF16");
+    }
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const StackSpace space = stack_space(layers, n_layers, tokens, width);
+    unsigned char* base = static_cast<unsigned char*>(workspace);
+    float* hidden = reinterpret_cast<float*>(base);
+    const size_t bytes = size_t(tokens) * width * sizeof(float);
+    hc_status st = check_cuda(cudaMemcpyAsync(hidden, hidden_in, bytes, cudaMemcpyHostToDevice, s), "hidden states in");
+    for (int i = 0; i < n_layers && st == HC_OK; ++i) {
+        const hc_block_weights& w = layers[i];
+        const hc_attn_params& p = w.params;
+        const int o_width = p.q_heads * p.head_dim, kv_width = p.kv_heads * p.head_dim;
+        const void* weights[3] = {w.wq, w.wk, w.wv};
+        const void* biases[3] = {w.bq, w.bk, w.bv};
+        void* qkv[3] = {base + space.q, base + space.k, base + space.v};
+        const int widths[3] = {o_width * (p.gate_layout == HC_GATE_INTERLEAVED ? 2 : 1), kv_width, kv_width};
+        st = hc_rms_norm(ctx, hidden, w.input_norm, base + space.normed, tokens, width, eps, HC_F32, HC_BF16, stream);
+        if (st == HC_OK) st = hc_linear_group(ctx, base + space.normed, 3, weights, biases, qkv, widths, tokens, width, HC_BF16, stream);
+        if (st == HC_OK) st = hc_layer_step(ctx, cache, i, seq, qkv[0], qkv[1], qkv[2], base + space.attended, tokens, first_position, &p, stream);
+        if (st == HC_OK) st = hc_linear(ctx, base + space.attended, w.wo, w.bo, hidden, hidden, tokens, o_width, width, HC_F32, stream);
+    }
+    if (st == HC_OK) st = check_cuda(cudaMemcpyAsync(hidden_out, hidden, bytes, cudaMemcpyDeviceToHost, s), "hidden states out");
+    if (st != HC_OK) return st;
+    return hc_context_check(ctx, stream);
 }
 
 // The body of the host-buffer entry points.  Chunk i's inputs are copied in on one stream while chunk

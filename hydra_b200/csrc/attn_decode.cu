@@ -907,7 +907,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
                 if (idle_since == 0) idle_since = now;
                 if (static_cast<unsigned long long>(now - idle_since) > kWaitCycles) {
                     *abort_flag = 1;
-                    atomicCAS(args.status, 0, 0x100 + 42);
+                    report_status(args.status, 0x100 + 42);
                     break;
                 }
                 __nanosleep(20);

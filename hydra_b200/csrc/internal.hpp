@@ -132,8 +132,8 @@ struct hc_context {
     int device = 0;
     int sm_count = 0;
     uint64_t launches = 0;
-    int* status_dev = nullptr;    // one word the kernels may set on a bounded-wait timeout
-    int* status_host = nullptr;   // pinned mirror
+    int* status_host = nullptr;   // one word the kernels may set on a bounded-wait timeout, in pinned host memory:
+    int* status_dev = nullptr;    // a check is a synchronisation and a read; its address on the device
     int cluster_slots[4] = {};    // thread blocks resident at once in clusters of 2, 4, 8, 16 (see attn_decode.cu)
     float* static_scratch = nullptr;   // device address of the fixed scratch of hc_attention_decode_static
 };

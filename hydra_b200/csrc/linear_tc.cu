@@ -115,6 +115,13 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 // compiler may not move a load across a store, and a block's eight loads one after the other cost more
 // than its MMAs (o_proj of 4096 tokens: 141 us).
 constexpr int kLinStageBytes = 32 * 128;
+__device__ __forceinline__ float4 load_bias(const LinJob& job, int col0) {
+    const int col = col0 + (threadIdx.x & 7) * 4;
+    float b[4];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = job.bias != nullptr && col + i < job.out_features ? bf16_bits_to_float(__ldg(job.bias + col + i)) : 0.0f;
+    return make_float4(b[0], b[1], b[2], b[3]);
+}
 __device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob& job, int row0, int col0, float4 (&z)[8]) {
     #pragma unroll
     for (int k = 0; k < 8; ++k) z[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -132,7 +139,7 @@ __device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob&
         else z[k] = make_float4(src[0], src[1], src[2], src[3]);
     }
 }
-__device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4 (&z)[8], int row0,
+__device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4& bias, const float4 (&z)[8], int row0,
                                             int col0, unsigned char* stage, int width = 32) {
     if (col0 >= job.out_features || row0 >= args.tokens) return;          // warp-uniform
     const int lane = threadIdx.x & 31;
@@ -144,15 +151,12 @@ __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& j
     const int chunk = lane & 7, col = col0 + chunk * 4;
     const bool mine = chunk * 4 < width;
     const bool vectors = col + 4 <= job.out_features && (job.out_features & 3) == 0;
-    float b[4];
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) b[i] = job.bias != nullptr && col + i < job.out_features ? bf16_bits_to_float(__ldg(job.bias + col + i)) : 0.0f;
     #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const int r = k * 4 + (lane >> 3);
         if (row0 + r >= args.tokens || !mine) continue;
         const float4 x = *reinterpret_cast<const float4*>(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
-        float y[4] = {__fadd_rn(x.x, b[0]), __fadd_rn(x.y, b[1]), __fadd_rn(x.z, b[2]), __fadd_rn(x.w, b[3])};
+        float y[4] = {__fadd_rn(x.x, bias.x), __fadd_rn(x.y, bias.y), __fadd_rn(x.z, bias.z), __fadd_rn(x.w, bias.w)};
         const size_t at = size_t(row0 + r) * job.out_features + col;
         if (vectors) {
             if (job.residual != nullptr) {
@@ -308,6 +312,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             const bool rows = quad * 32 < args.tokens;              // warp-uniform
             float4 z[8];
             if (rows) load_residual(args, job, quad * 32, where.tn * BN, z);
+            float4 bias = load_bias(job, where.tn * BN);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
             #pragma unroll 1
@@ -315,8 +320,11 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 uint32_t v[32];
                 HC_TMEM_LD32(tmem + lane_base + acc * 64 + col, v);
                 tc_wait_ld();
-                if (col > 0) load_residual(args, job, quad * 32, where.tn * BN + col, z);
-                store_block(args, job, v, z, quad * 32, where.tn * BN + col, stage, BN - col);
+                if (col > 0) {
+                    load_residual(args, job, quad * 32, where.tn * BN + col, z);
+                    bias = load_bias(job, where.tn * BN + col);
+                }
+                store_block(args, job, v, bias, z, quad * 32, where.tn * BN + col, stage, BN - col);
                 __syncwarp();          // the next tcgen05.ld is warp-wide
             }
             tc_fence_before();
@@ -451,7 +459,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 HC_TMEM_LD32(tmem + lane_base + acc * BN + chunk * 32, v);
                 if (chunk + 1 < BN / 32) load_residual(args, job, row0, where.tn * BN + (chunk + 1) * 32, z_next);
                 tc_wait_ld();
-                store_block(args, job, v, z, row0, where.tn * BN + chunk * 32, stage);
+                store_block(args, job, v, load_bias(job, where.tn * BN + chunk * 32), z, row0, where.tn * BN + chunk * 32, stage);
                 #pragma unroll
                 for (int k = 0; k < 8; ++k) z[k] = z_next[k];
                 __syncwarp();          // the next tcgen05.ld is warp-wide

@@ -59,6 +59,10 @@ __device__ __forceinline__ bool mbar_try_wait_parked(uint64_t* bar, uint32_t par
         : "=r"(done) : "r"(smem_u32(bar)), "r"(parity), "r"(ns) : "memory");
     return done != 0;
 }
+// The status word lies in the host's memory: a plain store, the first to come stays.
+__device__ __forceinline__ void report_status(volatile int* word, int value) {
+    if (*word == 0) *word = value;
+}
 // Bounded wait.  Returns false if the CTA is aborting (this wait or another one ran out of time).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status_word, int where) {
@@ -70,7 +74,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         if (*abort_flag != 0) return false;
         if (static_cast<unsigned long long>(clock64() - start) > kWaitCycles) {
             *abort_flag = 1;
-            atomicCAS(status_word, 0, 0x100 + where);
+            report_status(status_word, 0x100 + where);
             return false;
         }
     }

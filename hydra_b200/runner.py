@@ -4,7 +4,9 @@
 The reference's runners embed tokens, run every layer (attention half and mixture-of-experts half)
 and project to logits.  Only the attention half is in this library, so the runner here takes and
 returns HIDDEN STATES instead of tokens and logits and runs, per layer, the attention block of
-ReferenceLayer.decode (Sources/HydraReference/ReferenceLayer.swift:126-187):
+ReferenceLayer.decode (Sources/HydraReference/ReferenceLayer.swift:126-187), all layers in one call
+of the library (hc_attention_stack_host), because a token's kernels take less time than calling them
+one by one from here does:
 
     normed = rms_norm(hidden, input_norm)                      hc_rms_norm
     q, k, v = normed W_q^T + b_q, ...                           hc_linear_group (one launch)
@@ -15,7 +17,7 @@ with the protocol's bookkeeping around it: `position`, `prefill` in chunks of `p
 (the reference's loop: every chunk through every layer before the next chunk), `forward` for one
 token, `verify` (a draft's tokens in one pass, one output per position: the prefill kernels
 already return every position), `can_rewind` / `rewind` / `reset` on the KV cache.  Device memory
-and streams come from torch; nothing here computes.
+comes from torch; nothing here computes.
 """
 from __future__ import annotations
 
@@ -25,7 +27,7 @@ from typing import List, Optional, Sequence
 import numpy as np
 
 from . import capi
-from .backend import AttentionBackend, AttnParams, Context, KVCache, RopeTable
+from .backend import AttentionBackend, AttnParams, Context, KVCache, RopeTable, _check
 
 
 @dataclass
@@ -79,6 +81,20 @@ class AttentionStackRunner:
                                           sm_scale=1.0 / np.sqrt(head_dim), io_dtype=capi.HC_BF16, sinks=t["sinks"],
                                           rope=table))
 
+        # What a call needs besides the hidden states, laid out once: the layers' pointers and parameters, the
+        # device workspace, and pinned host buffers (a copy from or to pageable memory is two).
+        self._blocks = (capi.BlockWeightsStruct * len(layers))()
+        for block, t, params in zip(self._blocks, self.weights, self.params):
+            for name in ("input_norm", "wq", "bq", "wk", "bk", "wv", "bv", "wo", "bo"):
+                setattr(block, name, t[name].data_ptr())
+            block.params = params.struct()
+        self._lib = capi.load()
+        chunk = self.prefill_chunk_tokens
+        need = self._lib.hc_attention_stack_bytes(self._blocks, len(layers), chunk, hidden)
+        self._workspace = torch.empty(need, dtype=torch.uint8, device="cuda")
+        self._pinned = [torch.empty((chunk, hidden), dtype=torch.float32, pin_memory=True) for _ in range(2)]
+        self._host = [p.numpy() for p in self._pinned]
+
     # -- TextModelRunner's bookkeeping ------------------------------------------------------------
     @property
     def position(self) -> int:
@@ -94,24 +110,11 @@ class AttentionStackRunner:
         self.kv_cache.reset()
 
     # -- the passes -------------------------------------------------------------------------------
-    def _layers(self, hidden, first_position: int):
-        """`hidden` (device, fp32 [n][hidden], updated in place) through every layer's attention block."""
-        torch, be = self.torch, self.backend
-        n = hidden.shape[0]
-        bf = torch.bfloat16
-        q_dim, kv_dim = self.q_heads * self.d, self.kv_heads * self.d
-        normed = torch.empty((n, self.hidden), device="cuda", dtype=bf)
-        q = torch.empty((n, q_dim), device="cuda", dtype=bf)
-        k = torch.empty((n, kv_dim), device="cuda", dtype=bf)
-        v = torch.empty((n, kv_dim), device="cuda", dtype=bf)
-        attended = torch.empty((n, q_dim), device="cuda", dtype=bf)
-        for layer, (w, params) in enumerate(zip(self.weights, self.params)):
-            be.rms_norm(hidden, w["input_norm"], normed, n, self.hidden, self.eps)
-            be.linear_group(normed, [w["wq"], w["wk"], w["wv"]], [w["bq"], w["bk"], w["bv"]], [q, k, v], n, self.hidden,
-                            y_dtype=capi.HC_BF16)
-            be.layer_step(self.kv_cache, layer, q, k, v, attended, n, first_position, params)
-            be.linear(attended, w["wo"], w["bo"], hidden, n, q_dim, self.hidden, y_dtype=capi.HC_F32, residual=hidden)
-        return hidden
+    def _layers(self, tokens: int, first_position: int) -> None:
+        """`tokens` hidden states from the first pinned buffer through every layer's attention block to the second."""
+        _check(self._lib.hc_attention_stack_host(
+            self.ctx.handle, self.kv_cache.handle, self._blocks, len(self._blocks), 0, self._host[0].ctypes.data,
+            self._host[1].ctypes.data, tokens, self.hidden, first_position, self.eps, self._workspace.data_ptr(), None))
 
     def prefill(self, hidden_states: np.ndarray) -> np.ndarray:
         """A prompt's hidden states [tokens][hidden] in chunks, each chunk through every layer before
@@ -127,16 +130,15 @@ class AttentionStackRunner:
     def verify(self, hidden_states: np.ndarray) -> np.ndarray:
         """Several tokens in one pass, one output per position (TextModelRunner.verify): the caller
         keeps the accepted prefix by rewinding to it."""
-        torch = self.torch
         states = np.asarray(hidden_states, np.float32).reshape(-1, self.hidden)
         outputs = np.empty_like(states)
-        for start in range(0, states.shape[0], self.prefill_chunk_tokens):
-            chunk = states[start:start + self.prefill_chunk_tokens]
-            hidden = torch.from_numpy(np.ascontiguousarray(chunk)).cuda()
-            self._layers(hidden, self.position)
-            self.ctx.check()
-            outputs[start:start + chunk.shape[0]] = hidden.cpu().numpy()
-            self.kv_cache.advance(chunk.shape[0])
+        total, chunk = states.shape[0], self._host[0].shape[0]
+        for start in range(0, total, chunk):
+            n = min(chunk, total - start)
+            self._host[0][:n] = states[start:start + n]
+            self._layers(n, self.position)
+            outputs[start:start + n] = self._host[1][:n]
+            self.kv_cache.advance(n)
         return outputs
 
     def close(self) -> None:

@@ -490,6 +490,36 @@ HC_API hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int laye
                                    int tokens, int first_position, int chunk,
                                    const hc_attn_params* params, void* stream);
 
+/* ---- a stack of attention blocks ---------------------------------------------------------------- */
+
+/* One layer's weights as the reference stores them (bf16, device, projections row-major [out][in], biases may
+ * be NULL) and its attention parameters (io_dtype HC_BF16; layer i of the cache). */
+typedef struct hc_block_weights {
+    const void* input_norm;  /* [width] */
+    const void* wq;          /* [q_heads * head_dim][width] (twice as tall for an interleaved gate) */
+    const void* bq;
+    const void* wk;          /* [kv_heads * head_dim][width] */
+    const void* bk;
+    const void* wv;
+    const void* bv;
+    const void* wo;          /* [width][q_heads * head_dim] */
+    const void* bo;
+    hc_attn_params params;
+} hc_block_weights;
+
+/* The attention half of every layer for `tokens` tokens of one sequence, hidden states in HOST memory in and out
+ * (fp32 [tokens][width]), in one call: per layer hc_rms_norm, hc_linear_group, hc_layer_step and hc_linear with the
+ * residual, in that order and with their results bit for bit (ReferenceLayer.decode's attention block,
+ * Sources/HydraReference/ReferenceLayer.swift:126-187; a TextModelRunner's loop over its layers).  Returns when
+ * hidden_out is written (it may be hidden_in), having checked the context's status word; it does not move the
+ * sequence length.  `workspace` is device memory of hc_attention_stack_bytes(.., tokens, width) bytes, 256-byte
+ * aligned.  width must be a multiple of 64. */
+HC_API size_t hc_attention_stack_bytes(const hc_block_weights* layers, int n_layers, int tokens, int width);
+HC_API hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_block_weights* layers,
+                                         int n_layers, int seq, const float* hidden_in, float* hidden_out,
+                                         int tokens, int width, int first_position, float eps,
+                                         void* workspace, void* stream);
+
 /* ---- host-buffer convenience (what a runner without device buffers of its own calls) --------- */
 
 /* One whole step of the path with HOST buffers: copies q, k, v (and gate) to the device, appends,
