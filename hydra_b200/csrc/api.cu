@@ -1404,10 +1404,26 @@ hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_
     return hc_context_check(ctx, stream);
 }
 
-// The body of the host-buffer entry points.  Chunk i's inputs are copied in on one stream while chunk
-// i - 1 runs on the caller's stream and chunk i - 2's output is copied back on a third; two staging
-// slots, ordered by events.  One cudaMemcpyAsync per buffer.
-static hc_status host_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, const void* q, const void* k,
+// Where a call's next piece ends.  Each copy from the host costs some 15 us beside the traffic the other way, so
+// pieces are large; the first is short because nothing runs until it is there, and the last ones are, because their
+// kernel and their way back have nothing left to hide behind: 1, 2, 4, 4, 3 and 2 sixteenths of the call, in
+// steps of `quantum` tokens (about 2 MB of queries).  (4096 GPT-OSS tokens as eight pieces of 512 with a copy each
+// for q, k and v: 1410 us, now 1222; the two directions' bytes at the rate of both together take 810.)
+static int host_piece_end(int start, int tokens, int quantum, int most) {
+    static const int kEnds[6] = {1, 3, 7, 11, 14, 16};
+    int end = tokens;
+    for (int i = 5; i >= 0; --i) {
+        const long long at = ((long long)tokens * kEnds[i] / 16 + quantum - 1) / quantum * quantum;
+        if (at > start) end = int(std::min<long long>(at, tokens));
+    }
+    return std::min(end, start + most);
+}
+
+// The body of the host-buffer entry points.  A piece's inputs are copied in on one stream while the pieces before it
+// run on the caller's stream and their outputs are copied back on a third; queries and outputs in two slots,
+// ordered by events, K and V (where they fit beside the slots) in one copy each ahead of everything.  What a piece is
+// makes no difference to the results, but for blocks, which end with their token's chunk.
+static hc_status host_pieces(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, const void* q, const void* k,
                              const void* v, void* out, int tokens, int first_position, int chunk,
                              const hc_attn_params* params, cudaStream_t s) {
     const size_t eb = dtype_bytes(params->io_dtype);
@@ -1417,55 +1433,94 @@ static hc_status host_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int
     const size_t q_row = size_t(params->q_heads) * d * mult * eb;
     const size_t kv_row = size_t(params->kv_heads) * d * eb;
     const size_t o_row = size_t(params->q_heads) * d * eb;
+    const size_t g_row = sep_gate ? o_row : 0;
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t off_k = align(q_row * chunk);
-    const size_t off_v = off_k + align(kv_row * chunk);
-    const size_t off_g = off_v + align(kv_row * chunk);
-    const size_t off_o = off_g + (sep_gate ? align(o_row * chunk) : 0);
-    if (off_o + o_row * chunk > cache->stage_bytes) return fail(HC_KV_OVERFLOW, "staging buffer too small for this chunk");
-    // The copies may start once the work already in the caller's stream has been reached.
-    cudaError_t err = cudaEventRecord(cache->entry, s);
-    if (err == cudaSuccess) err = cudaStreamWaitEvent(cache->copy_in, cache->entry, 0);
-    if (err != cudaSuccess) return check_cuda(err, "host step: entry event");
+    const size_t kv_all = align(kv_row * tokens);
+    const size_t least = 5 * 256 + (q_row + g_row + o_row) * std::min(chunk, tokens);
+    const bool kv_ahead = kv_all <= cache->stage_bytes / 2 && cache->stage_bytes - kv_all >= least + 256;
+    const size_t slots_at = kv_ahead ? 2 * kv_all : 0;
+    const size_t slot_bytes = (cache->stage_bytes - slots_at / 2) & ~size_t(255);
+    const size_t piece_row = q_row + g_row + o_row + (kv_ahead ? 0 : 2 * kv_row);
+    if (slot_bytes < 5 * 256 + piece_row * std::min(chunk, tokens)) return fail(HC_KV_OVERFLOW, "staging buffer too small for this chunk");
+    const hc_layer_store& L = cache->layers[size_t(layer)];
+    if (L.ring > 0 && std::min(chunk, tokens) > L.ring_margin) {
+        return check_positions(cache, L, first_position, std::min(chunk, tokens), params);
+    }
+    int most = int(std::min<size_t>((slot_bytes - 5 * 256) / piece_row, size_t(tokens)));
+    if (L.ring > 0) most = std::min(most, std::max(L.ring - L.desc.window, std::min(chunk, tokens)));
+    if (params->block_ends) most = chunk;
+    const int quantum = int(((size_t(2) << 20) / q_row / kTileKeys + 1) * kTileKeys);
+    auto end_of = [&](int start) {
+        return params->block_ends ? std::min(start + chunk, tokens) : host_piece_end(start, tokens, quantum, most);
+    };
+    // One piece has nothing to overlap with: everything in the caller's stream, no events.
+    const bool one = end_of(0) == tokens;
+    cudaStream_t in = one ? s : cache->copy_in, back = one ? s : cache->copy_out;
+    unsigned char* stage = static_cast<unsigned char*>(cache->stage_dev);
     const unsigned char* hq = static_cast<const unsigned char*>(q);
     const unsigned char* hk = static_cast<const unsigned char*>(k);
     const unsigned char* hv = static_cast<const unsigned char*>(v);
     const unsigned char* hg = static_cast<const unsigned char*>(params->gate);
     unsigned char* ho = static_cast<unsigned char*>(out);
+    cudaError_t err = cudaSuccess;
+    auto record = [&](cudaEvent_t event, cudaStream_t stream) { if (!one && err == cudaSuccess) err = cudaEventRecord(event, stream); };
+    auto wait = [&](cudaStream_t stream, cudaEvent_t event) { if (!one && err == cudaSuccess) err = cudaStreamWaitEvent(stream, event, 0); };
+    auto copy = [&](void* dst, const void* src, size_t bytes, cudaMemcpyKind kind, cudaStream_t stream) {
+        if (err == cudaSuccess) err = cudaMemcpyAsync(dst, src, bytes, kind, stream);
+    };
+    hc_status st = HC_OK;
+    // The copies may start once the work already in the caller's stream has been reached.
+    record(cache->entry, s);
+    wait(in, cache->entry);
+    if (kv_ahead) {
+        copy(stage, hk, kv_row * tokens, cudaMemcpyHostToDevice, in);
+        copy(stage + kv_all, hv, kv_row * tokens, cudaMemcpyHostToDevice, in);
+    }
     int index = 0;
-    for (int start = 0; start < tokens; start += chunk, ++index) {
-        const int count = std::min(chunk, tokens - start);
-        const int slot = index & 1;
-        unsigned char* base = static_cast<unsigned char*>(cache->stage_dev) + size_t(slot) * cache->stage_bytes;
-        // The slot's previous occupant (chunk index - 2) must have run and its output left.
-        if (index >= 2) {
-            err = cudaStreamWaitEvent(cache->copy_in, cache->out_done[slot], 0);
-            if (err != cudaSuccess) return check_cuda(err, "host step: slot reuse");
+    for (int start = 0, end = 0; start < tokens && st == HC_OK && err == cudaSuccess; start = end, ++index) {
+        end = end_of(start);
+        const int count = end - start, slot = index & 1;
+        unsigned char* base = stage + slots_at + size_t(slot) * slot_bytes;
+        unsigned char* dev_g = base + align(q_row * count);
+        unsigned char* dev_o = dev_g + align(g_row * count);
+        unsigned char* dev_k = kv_ahead ? stage + kv_row * start : dev_o + align(o_row * count);
+        unsigned char* dev_v = kv_ahead ? stage + kv_all + kv_row * start : dev_k + align(kv_row * count);
+        // The slot's previous occupant (piece index - 2) must have run, and its output left.
+        if (index >= 2) wait(in, cache->out_done[slot]);
+        copy(base, hq + size_t(start) * q_row, q_row * count, cudaMemcpyHostToDevice, in);
+        if (!kv_ahead) {
+            copy(dev_k, hk + size_t(start) * kv_row, kv_row * count, cudaMemcpyHostToDevice, in);
+            copy(dev_v, hv + size_t(start) * kv_row, kv_row * count, cudaMemcpyHostToDevice, in);
         }
-        err = cudaMemcpyAsync(base, hq + size_t(start) * q_row, q_row * count, cudaMemcpyHostToDevice, cache->copy_in);
-        if (err == cudaSuccess) err = cudaMemcpyAsync(base + off_k, hk + size_t(start) * kv_row, kv_row * count, cudaMemcpyHostToDevice, cache->copy_in);
-        if (err == cudaSuccess) err = cudaMemcpyAsync(base + off_v, hv + size_t(start) * kv_row, kv_row * count, cudaMemcpyHostToDevice, cache->copy_in);
-        if (err == cudaSuccess && sep_gate) err = cudaMemcpyAsync(base + off_g, hg + size_t(start) * o_row, o_row * count, cudaMemcpyHostToDevice, cache->copy_in);
-        if (err == cudaSuccess) err = cudaEventRecord(cache->in_done[slot], cache->copy_in);
-        if (err == cudaSuccess) err = cudaStreamWaitEvent(s, cache->in_done[slot], 0);
-        if (err != cudaSuccess) return check_cuda(err, "host to device copy");
+        if (sep_gate) copy(dev_g, hg + size_t(start) * o_row, o_row * count, cudaMemcpyHostToDevice, in);
+        record(cache->in_done[slot], in);
+        wait(s, cache->in_done[slot]);
+        if (err != cudaSuccess) break;
         hc_attn_params local = *params;
         if (params->block_ends) local.block_ends = params->block_ends + start;    // device memory, like the sinks
-        if (sep_gate) local.gate = base + off_g;
-        const hc_status st = hc_layer_step(ctx, cache, layer, seq, base, base + off_k, base + off_v, base + off_o, count,
-                                           first_position + start, &local, s);
-        if (st != HC_OK) return st;
-        err = cudaEventRecord(cache->step_done[slot], s);
-        if (err == cudaSuccess) err = cudaStreamWaitEvent(cache->copy_out, cache->step_done[slot], 0);
-        if (err == cudaSuccess) err = cudaMemcpyAsync(ho + size_t(start) * o_row, base + off_o, o_row * count, cudaMemcpyDeviceToHost, cache->copy_out);
-        if (err == cudaSuccess) err = cudaEventRecord(cache->out_done[slot], cache->copy_out);
-        if (err != cudaSuccess) return check_cuda(err, "device to host copy");
+        if (sep_gate) local.gate = dev_g;
+        if (count > 1 && count <= cache->ws.qprep_capacity) {
+            st = prefill_impl(ctx, cache, layer, seq, base, dev_o, count, first_position + start, &local, false, s, dev_k, dev_v, most);
+        } else {
+            st = hc_layer_step(ctx, cache, layer, seq, base, dev_k, dev_v, dev_o, count, first_position + start, &local, s);
+        }
+        if (st != HC_OK) break;
+        record(cache->step_done[slot], s);
+        wait(back, cache->step_done[slot]);
+        copy(ho + size_t(start) * o_row, dev_o, o_row * count, cudaMemcpyDeviceToHost, back);
+        record(cache->out_done[slot], back);
     }
-    // The call returns when the results are on the host.
-    err = cudaStreamSynchronize(cache->copy_out);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(s);
-    if (err != cudaSuccess) return check_cuda(err, "host step: synchronise");
-    return HC_OK;
+    // The call returns when the results are on the host, or nothing more is on its way.
+    const std::string message = g_last_error;
+    for (cudaStream_t stream : {in, back, s}) {
+        const cudaError_t done = one && stream != s ? cudaSuccess : cudaStreamSynchronize(stream);
+        if (err == cudaSuccess) err = done;
+    }
+    if (st != HC_OK) {
+        g_last_error = message;
+        return st;
+    }
+    return err == cudaSuccess ? HC_OK : check_cuda(err, "host step");
 }
 
 hc_status hc_layer_step_host(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, const void* q, const void* k,
@@ -1478,7 +1533,7 @@ hc_status hc_layer_step_host(hc_context* ctx, hc_kv_cache* cache, int layer, int
     if (tokens > cache->ws.qprep_tokens) {
         return fail(HC_KV_OVERFLOW, "hc_layer_step_host takes at most " + std::to_string(cache->ws.qprep_tokens) + " tokens per call");
     }
-    return host_chunks(ctx, cache, layer, seq, q, k, v, out, tokens, first_position, tokens, params,
+    return host_pieces(ctx, cache, layer, seq, q, k, v, out, tokens, first_position, tokens, params,
                        static_cast<cudaStream_t>(stream));
 }
 
@@ -1492,7 +1547,7 @@ hc_status hc_prefill_host(hc_context* ctx, hc_kv_cache* cache, int layer, int se
     if (chunk > cache->ws.qprep_tokens) {
         return fail(HC_KV_OVERFLOW, "hc_prefill_host takes chunks of at most " + std::to_string(cache->ws.qprep_tokens) + " tokens");
     }
-    return host_chunks(ctx, cache, layer, seq, q, k, v, out, tokens, first_position, chunk, params,
+    return host_pieces(ctx, cache, layer, seq, q, k, v, out, tokens, first_position, chunk, params,
                        static_cast<cudaStream_t>(stream));
 }
 

@@ -534,10 +534,11 @@ HC_API hc_status hc_layer_step_host(hc_context* ctx, hc_kv_cache* cache, int lay
                                     int tokens, int first_position, const hc_attn_params* params,
                                     void* stream);
 
-/* The same for a whole prompt in chunks of `chunk` tokens (at most max(prefill_chunk, max_seqs)): the
- * copy in of chunk i + 1 and the copy out of chunk i - 1 run under the kernels of chunk i (two
- * staging slots, the library's own copy streams, events), and the call returns when every result is
- * on the host.  Use pinned host memory, or the copies serialise. */
+/* The same for a whole prompt in chunks of `chunk` tokens (at most max(prefill_chunk, max_seqs)), whose copies in
+ * and out run under the kernels of the tokens before and after them (the library's own copy streams, events);
+ * the call returns when every result is on the host.  As in hc_prefill_chunks a chunk's size does not show in the
+ * results, and the library takes pieces of its own size, but with params->block_ends.  Use pinned host memory,
+ * or the copies serialise. */
 HC_API hc_status hc_prefill_host(hc_context* ctx, hc_kv_cache* cache, int layer, int seq,
                                  const void* q, const void* k, const void* v, void* out,
                                  int tokens, int first_position, int chunk,
