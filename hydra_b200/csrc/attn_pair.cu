@@ -94,12 +94,14 @@ __device__ __forceinline__ PairItem pair_item(const TcArgs& args, int index) {
     return w;
 }
 struct PairIter {
+    Snake at;
     int item;
     PairItem w;
 };
 template <int D>
 __device__ __forceinline__ void pair_seek(const TcArgs& args, PairIter& it) {
-    for (; it.item < args.n_items; it.item += int(gridDim.x) >> 1) {
+    for (; it.at.item < args.n_items; it.at.next()) {
+        it.item = it.at.item;
         it.w = pair_item<D>(args, it.item);
         if (it.w.n_tiles > 0) return;
     }
@@ -107,15 +109,13 @@ __device__ __forceinline__ void pair_seek(const TcArgs& args, PairIter& it) {
 }
 template <int D>
 __device__ __forceinline__ PairIter pair_begin(const TcArgs& args) {
-    PairIter it;
-    it.item = int(blockIdx.x) >> 1;
-    it.w = PairItem{};
+    PairIter it{Snake(int(blockIdx.x) >> 1, int(gridDim.x) >> 1), 0, PairItem{}};
     pair_seek<D>(args, it);
     return it;
 }
 template <int D>
 __device__ __forceinline__ void pair_next(const TcArgs& args, PairIter& it) {
-    it.item += int(gridDim.x) >> 1;
+    it.at.next();
     pair_seek<D>(args, it);
 }
 

@@ -1,19 +1,18 @@
-// attn_tc.cu — attention on the 5th-generation tensor cores (sm_100a only): chunked prefill and
-// split decode over the bf16 KV cache, one persistent kernel for both.
+// attn_tc.cu — prefill of head_dim 64 and 128 on the 5th-generation tensor cores (sm_100a only) over the
+// bf16 KV cache, one persistent kernel.
 //
-// Replaces attention_prefill (Sources/HydraMetal/Shaders/batch.metal:307-427) and
-// attention_decode_split (Sources/HydraMetal/Shaders/attention.metal:307-415).  Where the reference
+// Replaces attention_prefill (Sources/HydraMetal/Shaders/batch.metal:307-427).  Where the reference
 // gives every (token, query head) its own threadgroup that streams the whole key range, this kernel
 // packs the G query heads that share a KV head and 128/G consecutive tokens into one 128-row tile,
 // so each K/V tile fetched by TMA serves 128 query rows, and both contractions run as tcgen05.mma
 // with accumulators in tensor memory.  A CTA is persistent: it walks a static list of work items
-// (row tile x kv head for prefill; run of key tiles x kv head x sequence for decode) and keeps its
+// (row tile x kv head, or one segment of it) and keeps its
 // TMA ring, tensor memory and barriers across items, so one item's ramp-up hides behind the
 // previous item's tail.
 //
 //   warpgroup 0 (warps 0-3)    control.  Warp 0: TMA loads of K and V tiles (128 keys x d, 128-byte
 //                              swizzle) into a ring.  Warp 1: issues S = Q K^T (A, B from shared
-//                              memory) up to three tiles ahead.  Warp 2: issues O_j = P V (A = P from
+//                              memory) as far ahead as its buffers allow.  Warp 2: issues O_j = P V (A = P from
 //                              tensor memory) and, for d = 64, the row sums of P in the same
 //                              instruction.  Warp 3: copies each item's Q tile into the swizzled
 //                              operand layout, two items ahead.
@@ -21,13 +20,11 @@
 //                              tensor memory, causal / window mask, row maximum, then
 //                              P = bf16(exp2(..)) back into tensor memory over S.  What paces a
 //                              tile is the exp2 unit: 16 results per clock per SM, 1024 clocks for
-//                              128 x 128; the two groups' exp2 phases are left free to overlap.  In decode the 16 real rows are read with the 16x256b shape,
-//                              four threads per row.
+//                              128 x 128; the two groups' exp2 phases are left free to overlap.
 //   warpgroup 3 (warps 12-15)   fold: O_j from tensor memory folded into the row's running (M, L, A)
-//                              in registers (prefill) or written out as the tile's partial
-//                              (decode); the epilogue
+//                              in registers; the epilogue
 //
-// Tensor memory: three S / P buffers of 128 columns and one O buffer.  Registers are moved between
+// Tensor memory: see TcLayout.  Registers are moved between
 // the warpgroups with setmaxnreg (48 / 152 / 152 / 160 per thread at d = 64, 48 / 112 / 112 / 232
 // at d = 128).
 //
@@ -55,11 +52,23 @@ struct TcLayout {
     static constexpr int kBlocks = D / 64;                   // 64-element (128-byte) column blocks
     static constexpr int kTileBytes = kTileKeys * D * 2;     // one K or V tile
     static constexpr int kStages = D == 64 ? 4 : 2;
-    static constexpr int kSBufs = 3;                         // S / P buffers of 128 columns at 0, 128, 256
     static constexpr int kQBytes = kRows * D * 2;            // one Q tile; two are kept
-    static constexpr int kOCol0 = kSBufs * kTileKeys;        // the one O buffer
-    // d = 64 leaves room beside O for 16 columns of row sums computed by the tensor core.
+    // Tensor memory: three buffers, each S and then P of a tile, and O behind them.  d = 64: 96 columns apart, S in
+    // columns 0 .. 127 and P in 32 .. 95 of each: a softmax thread takes its whole row of S into registers, so that
+    // what a buffer shares with its neighbours is S's alone and soon free, and there is room for two O buffers,
+    // each with 16 more columns for the row sums that the tensor core computes.  (With the buffers side by side
+    // and one O buffer 4096 GPT-OSS tokens take 260 us, with these 254.6; one S buffer, three of P and two of O: 270.)
+    static constexpr bool kOverlap = D == 64;
     static constexpr bool kSumOnTensor = D == 64;
+    static constexpr uint32_t kBufs = 3;
+    static constexpr uint32_t kOBufs = kOverlap ? 2 : 1;
+    __device__ static constexpr uint32_t buf(uint32_t t) { return t % kBufs; }
+    __device__ static constexpr uint32_t phase(uint32_t t) { return (t / kBufs) & 1; }
+    __device__ static constexpr uint32_t s_col(uint32_t t) { return buf(t) * (kOverlap ? 96 : kTileKeys); }
+    __device__ static constexpr uint32_t p_col(uint32_t t) { return s_col(t) + (kOverlap ? 32 : 0); }
+    __device__ static constexpr uint32_t o_buf(uint32_t t) { return t % kOBufs; }
+    __device__ static constexpr uint32_t o_phase(uint32_t t) { return (t / kOBufs) & 1; }
+    __device__ static constexpr uint32_t o_col(uint32_t t) { return kOverlap ? 320 + o_buf(t) * 96 : 384; }
     // Registers per thread after setmaxnreg (control / softmax / fold); 128 x their sum with the
     // softmax counted twice is the 64 K register file.
     // With d = 64 the fold needs less and a softmax thread can hold its whole row of S.
@@ -70,17 +79,28 @@ struct TcLayout {
     static constexpr int kTmemCols = 512;
     static constexpr int kOnesBytes = kTileKeys * 128;       // a 128-row block of bf16 1.0 (16 KiB)
     // Staging for the epilogue's coalesced stores: 4 warps x 32 rows x 128 bytes.  With d = 128 the
-    // block of ones is not used by any MMA and serves.
-    static constexpr int kEpiWarpBytes = 32 * 128;
-    static constexpr int kEpiBytes = kSumOnTensor ? 4 * kEpiWarpBytes : 0;
+    // block of ones is not used by any MMA and serves.  With d = 64 a warp has 32 rows x 64 fp32 values there (row minor, 33
+    // apart), which also hold the second fold's values between segments.
+    static constexpr bool kStateInSmem = D == 64;
+    static constexpr int kStateStride = kStateInSmem ? 33 : kRows;
+    static constexpr int kEpiWarpBytes = kStateInSmem ? D * kStateStride * 4 : 32 * 128;
+    static constexpr int kEpiBytes = kStateInSmem ? 4 * kEpiWarpBytes : 0;
     static constexpr int kSmemBytes = 1024 /*align slack*/ + 2 * kQBytes + 2 * kStages * kTileBytes + kOnesBytes + kEpiBytes;
 };
+
+// The items of a CTA, worked out by the warp that stages Q and read by every other role (working them out in each
+// role's own path took 1800 clocks of divisions and cold code an item).  The readers are never 16 items
+// apart: what lies between the Q stager and the fold is 2 items' Q and fewer than 10 tiles.
+constexpr int kItemRing = 16;
 
 struct TcBarriers {
     uint64_t q_full[2], q_empty[2];
     uint64_t k_full[4], k_empty[4], v_full[4], v_empty[4];
-    uint64_t s_full[3], p_full[3], pv_done[3];   // per S buffer; pv_done: P V has read the buffer's P
-    uint64_t o_full, o_free;
+    uint64_t s_full[3], p_full[3], pv_done[3];   // pv_done: P V has read the buffer's P
+    uint64_t s_free[3];                          // d = 64: S is in the softmax group's registers
+    uint64_t o_full[2], o_free[2];
+    uint64_t item_full[kItemRing];
+    TcItem item[kItemRing];
     uint32_t tmem_base;
     int abort_flag;
     float mm[8][kRows];       // per-tile scaled maxima, softmax -> fold (ring of 8 tiles)
@@ -89,16 +109,15 @@ struct TcBarriers {
 };
 
 
-// MODE says what becomes of an item's rows (TcArgs: finish, tile_partials), so that a launch carries
-// the code of its own way only: 0 = the kernel finishes them, 1 = segment partials, 2 = tile partials.
-constexpr int kModeFinish = 0, kModeSegments = 1, kModeTiles = 2;
+// MODE says what becomes of an item's rows (TcArgs: finish), so that a launch carries the code of its
+// own way only: 0 = the kernel finishes them, 1 = segment partials.
+constexpr int kModeFinish = 0, kModeSegments = 1;
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                     const TcArgs args) {
     constexpr bool kFinish = MODE == kModeFinish;
-    constexpr bool kTilePartials = MODE == kModeTiles;
     using LT = TcLayout<D>;
     extern __shared__ unsigned char raw_smem[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
@@ -115,6 +134,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
     const int G = 1 << args.log_group;
     const int world = max(args.map.world, 1);
     volatile int* abort_flag = &bars->abort_flag;
+    // Item `it` of this CTA into w; false behind the last one, or on abort.
+    auto read_item = [&](uint32_t it, TcItem& w) -> bool {
+        if (!mbar_wait(&bars->item_full[it % kItemRing], (it / kItemRing) & 1, abort_flag, args.status, 13)) return false;
+        w = bars->item[it % kItemRing];
+        return w.n_tiles > 0;
+    };
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
@@ -124,11 +149,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         }
         for (int i = 0; i < 3; ++i) {
             mbar_init(&bars->s_full[i], 1);
-            mbar_init(&bars->p_full[i], 128);
+            mbar_init(&bars->p_full[i], 4);
             mbar_init(&bars->pv_done[i], 1);
         }
-        mbar_init(&bars->o_full, 1);
-        mbar_init(&bars->o_free, 128);
+        for (int i = 0; i < 3; ++i) mbar_init(&bars->s_free[i], 4);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->o_full[i], 1);
+            mbar_init(&bars->o_free[i], 4);
+        }
+        for (int i = 0; i < kItemRing; ++i) mbar_init(&bars->item_full[i], 1);
         for (int i = 0; i < 4; ++i) {
             mbar_init(&bars->k_full[i], 1);
             mbar_init(&bars->k_empty[i], 1);
@@ -166,13 +195,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
             // K(t) then V(t), tile by tile.
             uint32_t t = 0;
             bool ok = true;
-            for (TcItemIter walk = items_begin(args); ok && walk.item < args.n_items; items_next(args, walk)) {
-                const TcItem& w = walk.w;
-                const int plane = cache_plane(args.map, w.seq, args.kv_heads, w.kv_head);
+            TcItem w;
+            for (uint32_t it = 0; ok && read_item(it, w); ++it) {
+                const int plane = cache_plane(args.map, args.seq, args.kv_heads, w.kv_head);
                 for (int j = 0; j < w.n_tiles; ++j, ++t) {
                     const int slot = int(t % LT::kStages);
                     const uint32_t round = t / LT::kStages;
-                    const int row0 = cache_row(args.map, w.seq, (w.tile_first + j * world) * kTileKeys);
+                    const int row0 = cache_row(args.map, args.seq, (w.tile_first + j * world) * kTileKeys);
                     if (round > 0 && !mbar_wait(&bars->k_empty[slot], (round - 1) & 1, abort_flag, args.status, 1)) {
                         ok = false;
                         break;
@@ -202,29 +231,23 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         if (LT::kStages < 4 && lane == 0) {
             constexpr int kKeysAhead = 3;
             struct Cursor {
-                TcItemIter walk;
+                TcItem w;
+                bool more;
                 int j;
-                uint32_t t;
+                uint32_t it, t;
             };
-            Cursor ck, cv;
-            ck.walk = items_begin(args);
-            ck.j = 0;
-            ck.t = 0;
-            cv = ck;
-            bool ok = true;
-            while (ok && (ck.walk.item < args.n_items || cv.walk.item < args.n_items)) {
-                const bool keys = ck.walk.item < args.n_items && (ck.t < cv.t + kKeysAhead || cv.walk.item >= args.n_items);
+            Cursor ck{};
+            ck.more = read_item(0, ck.w);
+            Cursor cv = ck;
+            while (ck.more || cv.more) {
+                const bool keys = ck.more && (ck.t < cv.t + kKeysAhead || !cv.more);
                 Cursor& c = keys ? ck : cv;
                 const int slot = int(c.t % LT::kStages);
                 const uint32_t round = c.t / LT::kStages;
                 uint64_t* empty = keys ? &bars->k_empty[slot] : &bars->v_empty[slot];
-                if (round > 0 && !mbar_wait(empty, (round - 1) & 1, abort_flag, args.status, keys ? 1 : 2)) {
-                    ok = false;
-                    break;
-                }
-                const TcItem& w = c.walk.w;
-                const int plane = cache_plane(args.map, w.seq, args.kv_heads, w.kv_head);
-                const int row0 = cache_row(args.map, w.seq, (w.tile_first + c.j * world) * kTileKeys);
+                if (round > 0 && !mbar_wait(empty, (round - 1) & 1, abort_flag, args.status, keys ? 1 : 2)) break;
+                const int plane = cache_plane(args.map, args.seq, args.kv_heads, c.w.kv_head);
+                const int row0 = cache_row(args.map, args.seq, (c.w.tile_first + c.j * world) * kTileKeys);
                 uint64_t* full = keys ? &bars->k_full[slot] : &bars->v_full[slot];
                 unsigned char* dst = (keys ? k_smem : v_smem) + slot * LT::kTileBytes;
                 mbar_expect_tx(full, LT::kTileBytes);
@@ -232,9 +255,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     tma_load_3d(dst + b * (kTileKeys * 128), keys ? &tmap_k : &tmap_v, full, b * 64, row0, plane);
                 }
                 ++c.t;
-                if (++c.j == w.n_tiles) {
+                if (++c.j == c.w.n_tiles) {
                     c.j = 0;
-                    items_next(args, c.walk);
+                    c.more = read_item(++c.it, c.w);
                 }
             }
         }
@@ -245,25 +268,25 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         constexpr uint32_t idesc_qk = instr_desc(kTileKeys, false);
         const uint64_t q_desc0 = smem_desc(smem_u32(q_smem), 16);
         const uint64_t k_desc0 = smem_desc(smem_u32(k_smem), 16);
-        uint32_t t = 0, it = 0;
+        uint32_t t = 0;
         bool ok = true;
-        for (TcItemIter walk = items_begin(args); ok && walk.item < args.n_items; items_next(args, walk), ++it) {
-          const int n_tiles = walk.w.n_tiles;
+        TcItem w;
+        for (uint32_t it = 0; ok && read_item(it, w); ++it) {
+          const int n_tiles = w.n_tiles;
           for (int j = 0; j < n_tiles; ++j, ++t) {
             const int slot = int(t % LT::kStages);
             const int qb = int(it & 1);
-            const int sb = int(t % LT::kSBufs);
-            // The buffer's previous contents, P of tile t - 3, must have been consumed.
-            if (t >= LT::kSBufs &&
-                !mbar_wait(&bars->pv_done[sb], (t / LT::kSBufs - 1) & 1, abort_flag, args.status, 12)) { ok = false; break; }
+            // (Ahead of the waits.)  Descriptors differ from the precomputed bases only in the 16-byte address field.
+            const uint64_t q_desc = warp_uniform(q_desc0 + uint64_t((qb * LT::kQBytes) >> 4));
+            const uint64_t k_desc = warp_uniform(k_desc0 + uint64_t((slot * LT::kTileBytes) >> 4));
+            const uint32_t s_tmem = warp_uniform(tmem + LT::s_col(t));
+            // The buffer's previous contents, P of tile t - 3, must have been consumed, and what its neighbours share with it.
+            if (t >= LT::kBufs && !mbar_wait(&bars->pv_done[LT::buf(t)], LT::phase(t - LT::kBufs), abort_flag, args.status, 12)) { ok = false; break; }
+            if (LT::kOverlap && t >= 1 && !mbar_wait(&bars->s_free[LT::buf(t - 1)], LT::phase(t - 1), abort_flag, args.status, 14)) { ok = false; break; }
             if (j == 0 && !mbar_wait(&bars->q_full[qb], (it >> 1) & 1, abort_flag, args.status, 4)) { ok = false; break; }
             if (!mbar_wait(&bars->k_full[slot], (t / LT::kStages) & 1, abort_flag, args.status, 3)) { ok = false; break; }
             tc_fence_after();
             if (elect_one()) {
-                // Descriptors differ from the precomputed bases only in the 16-byte address field.
-                const uint64_t q_desc = q_desc0 + uint64_t((qb * LT::kQBytes) >> 4);
-                const uint64_t k_desc = k_desc0 + uint64_t((slot * LT::kTileBytes) >> 4);
-                const uint32_t s_tmem = tmem + sb * kTileKeys;
                 #pragma unroll
                 for (int b = 0; b < LT::kBlocks; ++b) {
                     #pragma unroll
@@ -273,7 +296,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     }
                 }
                 tc_commit(&bars->k_empty[slot]);
-                tc_commit(&bars->s_full[sb]);
+                tc_commit(&bars->s_full[LT::buf(t)]);
                 if (j + 1 == n_tiles) tc_commit(&bars->q_empty[qb]);   // the item's Q tile was read for the last time
             }
             __syncwarp();
@@ -290,39 +313,47 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         const uint32_t v_base = smem_u32(v_smem);
         uint32_t t = 0;
         bool ok = true;
-        for (TcItemIter walk = items_begin(args); ok && walk.item < args.n_items; items_next(args, walk)) {
-            const int n_tiles = walk.w.n_tiles;
+        TcItem w;
+        for (uint32_t it = 0; ok && read_item(it, w); ++it) {
+            const int n_tiles = w.n_tiles;
             for (int j = 0; j < n_tiles; ++j, ++t) {
                 const int slot = int(t % LT::kStages);
-                const int sb = int(t % LT::kSBufs);
-                if (!mbar_wait(&bars->p_full[sb], (t / LT::kSBufs) & 1, abort_flag, args.status, 5)) { ok = false; break; }
+                const uint32_t v_addr = v_base + slot * LT::kTileBytes;
+                const uint32_t p_tmem = warp_uniform(tmem + LT::p_col(t));
+                const uint32_t o_tmem = warp_uniform(tmem + LT::o_col(t));
+                const uint32_t block_stride = LT::kSumOnTensor ? ones_addr - v_addr : uint32_t(kTileKeys * 128);
+                const uint64_t v_desc = warp_uniform(smem_desc(v_addr, block_stride));
+                if (!mbar_wait(&bars->p_full[LT::buf(t)], LT::phase(t), abort_flag, args.status, 5)) { ok = false; break; }
                 if (!mbar_wait(&bars->v_full[slot], (t / LT::kStages) & 1, abort_flag, args.status, 6)) { ok = false; break; }
-                if (t >= 1 && !mbar_wait(&bars->o_free, (t - 1) & 1, abort_flag, args.status, 7)) { ok = false; break; }
+                if (t >= LT::kOBufs && !mbar_wait(&bars->o_free[LT::o_buf(t)], LT::o_phase(t - LT::kOBufs), abort_flag, args.status, 7)) { ok = false; break; }
                 tc_fence_after();
                 if (elect_one()) {
-                    const uint32_t v_addr = v_base + slot * LT::kTileBytes;
-                    const uint32_t p_tmem = tmem + sb * kTileKeys;
-                    const uint32_t o_tmem = tmem + LT::kOCol0;
-                    const uint32_t block_stride = LT::kSumOnTensor ? ones_addr - v_addr : uint32_t(kTileKeys * 128);
-                    const uint64_t v_desc = smem_desc(v_addr, block_stride);
                     #pragma unroll
                     for (int ks = 0; ks < kTileKeys / 16; ++ks) {
                         mma_ts(o_tmem, p_tmem + ks * 8, v_desc + uint64_t((ks * 2048) >> 4), idesc_pv, ks != 0 ? 1u : 0u);
                     }
-                    tc_commit(&bars->o_full);
-                    tc_commit(&bars->pv_done[sb]);
+                    tc_commit(&bars->o_full[LT::o_buf(t)]);
+                    tc_commit(&bars->pv_done[LT::buf(t)]);
                     tc_commit(&bars->v_empty[slot]);
                 }
                 __syncwarp();
             }
         }
     } else {
-        // ===== Q stager: copies each item's Q tile (128 rows of the prepared q) into the swizzled
+        // ===== Q stager: publishes the items, and copies each item's Q tile (128 rows of the prepared q) into the swizzled
         // K-major layout, up to two items ahead of the S issuer, so the global-memory latency of a
         // new item never sits in another role's path.  Lane l copies rows l, l + 32, l + 64, l + 96. =====
         uint32_t it = 0;
-        for (TcItemIter walk = items_begin(args); walk.item < args.n_items; items_next(args, walk), ++it) {
+        for (TcItemIter walk = items_begin(args);; items_next(args, walk), ++it) {
+            const bool more = walk.item < args.n_items;
             const TcItem& w = walk.w;
+            if (lane == 0) {
+                TcItem& entry = bars->item[it % kItemRing];
+                entry = w;
+                if (!more) entry.n_tiles = 0;
+                mbar_arrive(&bars->item_full[it % kItemRing]);
+            }
+            if (!more) break;
             const int qb = int(it & 1);
             // The buffer was last read by item it - 2.
             if (it >= 2 && !mbar_wait(&bars->q_empty[qb], ((it >> 1) - 1) & 1, abort_flag, args.status, 10)) break;
@@ -366,108 +397,36 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         const float neg_inf = __int_as_float(0xff800000);
         uint32_t t = 0;
         bool ok = true;
-        for (TcItemIter walk = items_begin(args); ok && walk.item < args.n_items; items_next(args, walk)) {
-            const TcItem& w = walk.w;
+        TcItem w;
+        for (uint32_t it = 0; ok && read_item(it, w); ++it) {
             const bool valid = t_local < w.valid_tokens;
             const bool warp_has_rows = quad * 32 < (w.valid_tokens << args.log_group);   // warp-uniform
             int pos = valid ? w.first_pos + t_local : -1;
             const int lo = args.window > 0 ? max(0, pos - args.window + 1) : 0;
             // From here on `pos` is the last key the row sees: its own, or the end of its bidirectional
             // block (Sources/HydraMetal/Shaders/batch.metal:351-352) as far as keys have been appended.
-            if (!args.decode && args.block_ends != nullptr && valid) {
+            if (args.block_ends != nullptr && valid) {
                 pos = max(pos, min(__ldg(args.block_ends + (w.first_pos - args.first_position) + t_local), args.appended) - 1);
             }
             for (int j = 0; j < w.n_tiles; ++j, ++t) {
                 if (int(t & 1) != parity) continue;
-                const int sb = int(t % LT::kSBufs);
-                const uint32_t s_tmem = tmem + lane_base + sb * kTileKeys;
-                if (!mbar_wait(&bars->s_full[sb], (t / LT::kSBufs) & 1, abort_flag, args.status, 8)) { ok = false; break; }
+                const uint32_t pb = LT::buf(t);
+                const uint32_t s_tmem = tmem + lane_base + LT::s_col(t), p_tmem = tmem + lane_base + LT::p_col(t);
+                if (!mbar_wait(&bars->s_full[pb], LT::phase(t), abort_flag, args.status, 8)) { ok = false; break; }
                 tc_fence_after();
                 if (!warp_has_rows) {
                     // No query row lives in this quadrant: its P rows stay whatever they were and the
                     // O rows they produce are never read (rows are independent).
                     tc_fence_before();
-                    mbar_arrive(&bars->p_full[sb]);
+                    if (LT::kOverlap) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars->s_free[pb]);
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->p_full[pb]);
                     continue;
                 }
                 const int key0 = (w.tile_first + j * world) * kTileKeys;
-                if (args.decode && LT::kSumOnTensor) {
-                    // Decode has at most 16 real rows, all in quadrant 0 and all at one position.  The
-                    // 16x256b shape spreads each row over four threads, so a warp computes 16 x 128
-                    // weights instead of 32 x 128.  Element for element the weights are the
-                    // ones the prefill layout computes; the row sums come from the tensor core either way.
-                    const int q4 = lane & 3;
-                    const int tile_key0 = key0;
-                    const int c_lo = (args.window > 0 ? max(0, w.first_pos - args.window + 1) : 0) - tile_key0;
-                    const int c_hi = w.first_pos - tile_key0;
-                    const bool upper = G > 8;                // rows 8-15 hold heads only when the group is 16
-                    uint32_t v[2][32];
-                    HC_TMEM_LD_16x256b_x8(s_tmem, v[0]);
-                    HC_TMEM_LD_16x256b_x8(s_tmem + 64, v[1]);
-                    tc_wait_ld();
-                    if (!(c_lo <= 0 && c_hi >= kTileKeys - 1)) {
-                        #pragma unroll
-                        for (int hb = 0; hb < 2; ++hb) {
-                            #pragma unroll
-                            for (int n = 0; n < 8; ++n) {
-                                #pragma unroll
-                                for (int e = 0; e < 2; ++e) {
-                                    const int col = 64 * hb + 8 * n + 2 * q4 + e;
-                                    if (col < c_lo || col > c_hi) {
-                                        v[hb][4 * n + e] = __float_as_uint(neg_inf);
-                                        v[hb][4 * n + 2 + e] = __float_as_uint(neg_inf);
-                                    }
-                                }
-                            }
-                        }
-                    }
-                    // Row maxima: this thread's 32 columns, then the four threads of the row.
-                    float neg_mc[2] = {0.0f, 0.0f};
-                    #pragma unroll
-                    for (int rs = 0; rs < 2; ++rs) {
-                        if (rs == 0 || upper) {
-                            float m0 = __uint_as_float(v[0][2 * rs]), m1 = __uint_as_float(v[0][2 * rs + 1]);
-                            float m2 = __uint_as_float(v[1][2 * rs]), m3 = __uint_as_float(v[1][2 * rs + 1]);
-                            #pragma unroll
-                            for (int n = 1; n < 7; n += 2) {
-                                m0 = fmax3(m0, __uint_as_float(v[0][4 * n + 2 * rs]), __uint_as_float(v[0][4 * (n + 1) + 2 * rs]));
-                                m1 = fmax3(m1, __uint_as_float(v[0][4 * n + 2 * rs + 1]), __uint_as_float(v[0][4 * (n + 1) + 2 * rs + 1]));
-                                m2 = fmax3(m2, __uint_as_float(v[1][4 * n + 2 * rs]), __uint_as_float(v[1][4 * (n + 1) + 2 * rs]));
-                                m3 = fmax3(m3, __uint_as_float(v[1][4 * n + 2 * rs + 1]), __uint_as_float(v[1][4 * (n + 1) + 2 * rs + 1]));
-                            }
-                            m0 = fmax3(m0, __uint_as_float(v[0][28 + 2 * rs]), m1);
-                            m2 = fmax3(m2, __uint_as_float(v[1][28 + 2 * rs]), m3);
-                            float m = fmax3(fmaxf(m0, m2), __uint_as_float(v[0][29 + 2 * rs]), __uint_as_float(v[1][29 + 2 * rs]));
-                            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-                            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-                            neg_mc[rs] = -__fmul_rn((m == neg_inf) ? 0.0f : m, args.c);
-                            if (q4 == 0) bars->mm[t & 7][(lane >> 2) + 8 * rs] = __fmul_rn(m, args.c);
-                        }
-                    }
-                    // st[2n + rs]: P column 4n + q4 of row lane/4 + 8 rs, the layout of the 16x128b store.
-                    #pragma unroll
-                    for (int hb = 0; hb < 2; ++hb) {
-                        uint32_t st[16];
-                        #pragma unroll
-                        for (int rs = 0; rs < 2; ++rs) {
-                            #pragma unroll
-                            for (int n = 0; n < 8; ++n) {
-                                if (rs == 0 || upper) {
-                                    const float e0 = tile_weight_raw(__uint_as_float(v[hb][4 * n + 2 * rs]), neg_mc[rs], args.c);
-                                    const float e1 = tile_weight_raw(__uint_as_float(v[hb][4 * n + 2 * rs + 1]), neg_mc[rs], args.c);
-                                    st[2 * n + rs] = pack_bf16x2(e0, e1);
-                                } else {
-                                    st[2 * n + rs] = 0u;
-                                }
-                            }
-                        }
-                        HC_TMEM_ST_16x128b_x8(s_tmem + hb * 32, st);
-                    }
-                    tc_wait_st();
-                    tc_fence_before();
-                    mbar_arrive(&bars->p_full[sb]);
-                    continue;
-                }
                 const int c_lo = lo - key0;                  // visible columns: [c_lo, c_hi]
                 const int c_hi = pos - key0;
                 const bool full = c_lo <= 0 && c_hi >= kTileKeys - 1;
@@ -481,10 +440,20 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     HC_TMEM_LD32(s_tmem + 64, s[2]);
                     HC_TMEM_LD32(s_tmem + 96, s[3]);
                     tc_wait_ld();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->s_free[pb]);
                     if (!full) {
+                        // By bits of a word for each 32 columns: less than half the code of two comparisons a column,
+                        // and it is code that runs cold, once an item (2700 clocks more than an unmasked tile).
                         #pragma unroll
-                        for (int col = 0; col < kTileKeys; ++col) {
-                            if (col < c_lo || col > c_hi) s[col >> 5][col & 31] = __float_as_uint(neg_inf);
+                        for (int q = 0; q < 4; ++q) {
+                            const int from = min(max(c_lo - 32 * q, 0), 32), to = min(max(c_hi + 1 - 32 * q, 0), 32);
+                            const uint32_t visible = uint32_t((1ull << to) - 1) & ~uint32_t((1ull << from) - 1);
+                            #pragma unroll
+                            for (int i = 0; i < 32; ++i) {
+                                if (((visible >> i) & 1u) == 0) s[q][i] = __float_as_uint(neg_inf);
+                            }
                         }
                     }
                     float mx[8];
@@ -514,12 +483,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         for (int i = 0; i < 16; ++i) {
                             packed[i] = pack_bf16x2(__uint_as_float(s[q][2 * i]), __uint_as_float(s[q][2 * i + 1]));
                         }
-                        HC_TMEM_ST16(s_tmem + q * 16, packed);
+                        HC_TMEM_ST16(p_tmem + q * 16, packed);
                     }
                     bars->mm[t & 7][row] = __fmul_rn(m, args.c);
                     tc_wait_st();
                     tc_fence_before();
-                    mbar_arrive(&bars->p_full[sb]);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->p_full[pb]);
                     continue;
                 }
                 // The row is read twice, 32 columns at a time, in rolled loops: the maximum, then the
@@ -575,7 +545,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         packed[i] = pack_bf16x2(e0, e1);
                     }
                     HC_TMEM_ST16(dst, packed);
-                    if (LT::kSumOnTensor) return 0.0f;
                     // Sum of the 32 weights by the butterfly tree (i with i + 16, then + 8, + 4, + 2, + 1).
                     float a[16];
                     #pragma unroll
@@ -617,7 +586,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 bars->mm[t & 7][row] = __fmul_rn(m, args.c);
                 tc_wait_st();
                 tc_fence_before();
-                mbar_arrive(&bars->p_full[sb]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->p_full[pb]);
             }
         }
     } else {
@@ -629,9 +599,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         const int g = row & (G - 1);
         const uint32_t lane_base = uint32_t(quad * 32) << 16;
         // Where this thread's row keeps the values of its second fold between segments.
-        constexpr int kStateStride = kRows;
+        constexpr int kStateStride = LT::kStateStride;
+        float* const warp_state = reinterpret_cast<float*>(epi_smem + quad * LT::kEpiWarpBytes);
         auto state_of_row = [&]() -> float* {
-            return args.row_state + size_t(blockIdx.x) * (D * kRows) + row;
+            return LT::kStateInSmem ? warp_state + lane : args.row_state + size_t(blockIdx.x) * (D * kRows) + row;
         };
         // (M, L) the second fold stands at: what the last segment end left, or the seed.
         auto second_fold_state = [&](bool state_holds, uint16_t sink, float& M2, float& L2) {
@@ -654,63 +625,21 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         };
         uint32_t t = 0, it = 0;
         bool ok = true;
-        TcItemIter walk = items_begin(args);
+        TcItem w, next;
+        bool more = read_item(0, next);
         // The head's sink is fetched one item ahead (only when this kernel runs the second fold), so its
         // latency never sits at an item's start.
         const bool wants_sink = kFinish && args.count_sink && args.sinks != nullptr;
         uint16_t sink_bits = kNoSinkBits;
-        if (wants_sink && walk.item < args.n_items) sink_bits = args.sinks[walk.w.kv_head * G + g];
-        while (ok && walk.item < args.n_items) {
-            const TcItem w = walk.w;
-            items_next(args, walk);
+        if (wants_sink && more) sink_bits = args.sinks[next.kv_head * G + g];
+        while (ok && more) {
+            w = next;
+            more = read_item(++it, next);
             const int head = w.kv_head * G + g;
             const bool valid = t_local < w.valid_tokens;
             const bool warp_has_rows = quad * 32 < (w.valid_tokens << args.log_group);   // warp-uniform
             const uint16_t item_sink = sink_bits;
-            if (wants_sink && walk.item < args.n_items) sink_bits = args.sinks[walk.w.kv_head * G + g];
-            if constexpr (kTilePartials) {
-                // Finely split decode: every tile's own partial goes to the workspace, both folds to the merge.
-                for (int j = 0; j < w.n_tiles; ++j, ++t) {
-                    if (!mbar_wait(&bars->o_full, t & 1, abort_flag, args.status, 9)) { ok = false; break; }
-                    tc_fence_after();
-                    if (!warp_has_rows) {
-                        tc_fence_before();
-                        mbar_arrive(&bars->o_free);
-                        continue;
-                    }
-                    const uint32_t o_tmem = tmem + lane_base + LT::kOCol0;
-                    const uint32_t l_bits = tile_sum(o_tmem, t);   // valid after the first wait below
-                    const size_t prow = (size_t(w.row0) * args.q_heads + head) * args.slots + (w.slot + j);
-                    #pragma unroll
-                    for (int hb = 0; hb < D / 64; ++hb) {
-                        uint32_t o[2][32];
-                        HC_TMEM_LD32(o_tmem + hb * 64, o[0]);
-                        HC_TMEM_LD32(o_tmem + hb * 64 + 32, o[1]);
-                        tc_wait_ld();
-                        if (hb == D / 64 - 1) {
-                            tc_fence_before();
-                            mbar_arrive(&bars->o_free);
-                        }
-                        if (valid) {
-                            float* dst = args.part_o + prow * D + hb * 64;
-                            #pragma unroll
-                            for (int u = 0; u < 2; ++u) {
-                                #pragma unroll
-                                for (int i = 0; i < 32; i += 4) {
-                                    *reinterpret_cast<uint4*>(dst + u * 32 + i) =
-                                        make_uint4(o[u][i], o[u][i + 1], o[u][i + 2], o[u][i + 3]);
-                                }
-                            }
-                        }
-                    }
-                    if (valid) {
-                        *reinterpret_cast<float2*>(args.part_ml + prow * 2) =
-                            make_float2(bars->mm[t & 7][row], __uint_as_float(l_bits));
-                    }
-                }
-                ++it;
-                continue;
-            }
+            if (wants_sink && more) sink_bits = args.sinks[next.kv_head * G + g];
             // The running segment's partial: a fold over its tiles from the empty state.
             float M = kEmptyMax, L = 0.0f;
             float A[D];
@@ -718,23 +647,24 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
             for (int i = 0; i < D; ++i) A[i] = 0.0f;
             // One pass per segment the item touches.  With finish, the row's second fold runs between
             // the passes.  Its state is kept out of the registers: (M2, L2) in shared memory, the values
-            // in global memory (element i of this thread's row at state[i * kStateStride]; it stays in L2);
-            // both are untouched
-            // until the item's first segment is complete, which a tile's segment index tells.
+            // there too (d = 64) or in global memory (d = 128, it stays in L2), element i of this thread's row at
+            // state[i * kStateStride]; both are untouched until the item's first segment is complete, which a
+            // tile's segment index tells.
             for (int j = 0; ok && j < w.n_tiles;) {
                 const int pass_tile = w.tile_first + j * world;
                 const int pass_last = (((pass_tile >> args.map.log_segment) + 1) << args.map.log_segment) - 1;
                 const int pass_end = min(w.n_tiles, j + (pass_last - pass_tile) / world + 1);
                 // The first fold over the segment's tiles.
                 for (; j < pass_end; ++j, ++t) {
-                    if (!mbar_wait(&bars->o_full, t & 1, abort_flag, args.status, 9)) { ok = false; break; }
+                    if (!mbar_wait(&bars->o_full[LT::o_buf(t)], LT::o_phase(t), abort_flag, args.status, 9)) { ok = false; break; }
                     tc_fence_after();
                     if (!warp_has_rows) {
                         tc_fence_before();
-                        mbar_arrive(&bars->o_free);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars->o_free[LT::o_buf(t)]);
                         continue;
                     }
-                    const uint32_t o_tmem = tmem + lane_base + LT::kOCol0;
+                    const uint32_t o_tmem = tmem + lane_base + LT::o_col(t);
                     const uint32_t l_bits = tile_sum(o_tmem, t);   // valid after the first wait below
                     float Mn, a, b;
                     #pragma unroll
@@ -746,7 +676,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         tc_wait_ld();
                         if (hb == D / 64 - 1) {
                             tc_fence_before();
-                            mbar_arrive(&bars->o_free);
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&bars->o_free[LT::o_buf(t)]);
                         }
                         if (hb == 0) {
                             L = __fmaf_rn(L, a, __fmul_rn(__uint_as_float(l_bits), b));
@@ -811,10 +742,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
             }
             if (!ok) break;
             const size_t out_row = size_t(w.row0 + t_local);
-            if constexpr (!kFinish) {
-                ++it;
-                continue;
-            }
+            if constexpr (!kFinish) continue;
             // The row's last segment: the last step of the second fold, which started from the sink (or,
             // on the ranks of a sequence-sharded cache that do not count it, from the empty state).
             {
@@ -826,8 +754,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 fold_coefficients(M2, M, Mn, a, b);
                 L = __fmaf_rn(L2, a, __fmul_rn(L, b));
                 M = Mn;
-                const float* const state = state_of_row();
-                if (state_holds) {
+                float* const state = state_of_row();
+                if constexpr (LT::kStateInSmem) {
+                    // The rows' final values to the staging (in place of the state's), then out from there in a
+                    // rolled loop, eight lanes a row: coalesced, and little code (unrolled, with 64 divisions in a row,
+                    // it took 2400 clocks an item, most of them for fetching instructions).
+                    #pragma unroll
+                    for (int i = 0; i < D; ++i) {
+                        const float before = state_holds ? state[i * kStateStride] : 0.0f;
+                        state[i * kStateStride] = fold_value(before, a, A[i], b);
+                    }
+                } else if (state_holds) {
                     #pragma unroll
                     for (int i0 = 0; i0 < D; i0 += 16) {
                         float before[16];
@@ -842,6 +779,48 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     #pragma unroll
                     for (int i = 0; i < D; ++i) A[i] = __fmul_rn(A[i], b);
                 }
+            }
+            if constexpr (LT::kStateInSmem) {
+                __syncwarp();
+                if (warp_has_rows) {
+                    const bool gated = args.ep.gate_layout != HC_GATE_NONE;
+                    const int column = (lane & 7) * 8;
+                    #pragma unroll 1
+                    for (int k = 0; k < 8; ++k) {
+                        const int rl = k * 4 + (lane >> 3);
+                        const float row_l = __shfl_sync(0xffffffffu, L, rl);
+                        const float row_m = __shfl_sync(0xffffffffu, M, rl);
+                        const int t2 = (quad * 32 + rl) >> args.log_group;
+                        if (t2 >= w.valid_tokens) continue;
+                        const size_t vec = size_t(w.row0 + t2) * args.q_heads + size_t(w.kv_head) * G + ((quad * 32 + rl) & (G - 1));
+                        float r[8];
+                        #pragma unroll
+                        for (int u = 0; u < 8; ++u) r[u] = warp_state[(column + u) * kStateStride + rl];
+                        if (args.ep.write_partial) {
+                            // A partial row is D + 2 floats: its start is 8-byte aligned, not 16.
+                            float* dst = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2);
+                            #pragma unroll
+                            for (int u = 0; u < 8; u += 2) *reinterpret_cast<float2*>(dst + column + u) = make_float2(r[u], r[u + 1]);
+                            if (column == 0) *reinterpret_cast<float2*>(dst + D) = make_float2(row_m, row_l);
+                            continue;
+                        }
+                        const size_t gate = (args.ep.gate_layout == HC_GATE_INTERLEAVED ? vec * size_t(2 * D) + D : vec * size_t(D)) + column;
+                        #pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            r[u] = finish_value(r[u], row_l, gated, gated ? load_io(args.ep.gate, gate + u, args.ep.io_dtype) : 0.0f);
+                        }
+                        if (args.ep.io_dtype == HC_F32) {
+                            float* dst = reinterpret_cast<float*>(args.ep.out) + vec * D + column;
+                            *reinterpret_cast<float4*>(dst) = make_float4(r[0], r[1], r[2], r[3]);
+                            *reinterpret_cast<float4*>(dst + 4) = make_float4(r[4], r[5], r[6], r[7]);
+                        } else {
+                            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(args.ep.out) + vec * D + column) =
+                                make_uint4(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]), pack_bf16x2(r[4], r[5]), pack_bf16x2(r[6], r[7]));
+                        }
+                    }
+                    __syncwarp();
+                }
+                continue;
             }
             if (warp_has_rows && !args.ep.write_partial && args.ep.gate_layout == HC_GATE_NONE &&
                 args.ep.io_dtype != HC_F32) {
@@ -915,7 +894,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     }
                 }
             }
-            ++it;
         }
     }
 
@@ -1040,7 +1018,6 @@ static hc_status launch_tc_mode(hc_context* ctx, const TcArgs& args, const hc_la
 template <int D>
 static hc_status launch_tc(hc_context* ctx, const TcArgs& args, const hc_layer_store& layer, cudaStream_t stream) {
     if (args.finish) return launch_tc_mode<D, kModeFinish>(ctx, args, layer, stream);
-    if (args.tile_partials) return launch_tc_mode<D, kModeTiles>(ctx, args, layer, stream);
     return launch_tc_mode<D, kModeSegments>(ctx, args, layer, stream);
 }
 
@@ -1065,9 +1042,9 @@ static void fill_common_args(TcArgs& args, hc_context* ctx, const AttnShape& sha
     args.row_state = ws.part_o;       // a launch uses one or the other
 }
 
-// Floats of row state a whole-row launch needs.
+// Floats of row state a whole-row launch needs (head_dim 64 keeps it in shared memory).
 static size_t row_state_floats(const hc_context* ctx, const AttnShape& shape) {
-    return size_t(std::max(ctx->sm_count, 1)) * std::min(shape.head_dim, 256) * kRows;
+    return shape.head_dim == 64 ? 0 : size_t(std::max(ctx->sm_count, 1)) * std::min(shape.head_dim, 256) * kRows;
 }
 
 static hc_status launch_any(hc_context* ctx, const AttnShape& shape, const TcArgs& args, const hc_layer_store& layer,
@@ -1087,7 +1064,6 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
     args.tokens = tokens;
     args.first_position = first_position;
     args.seq = seq;
-    args.log_run = cache.map.log_segment;
     // Head_dim 256 and 512: row tiles of 256 rows on pairs of SMs.
     const bool pairs = shape.head_dim >= 256;
     const int tokens_per_tile = (pairs ? 2 : 1) * kRows / shape.group;

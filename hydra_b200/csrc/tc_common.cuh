@@ -10,7 +10,7 @@ namespace {
 
 struct TcArgs {
     const uint16_t* q;        // bf16 [rows][q_heads][d], prepared
-    int tokens;               // prefill: tokens of the chunk; decode: batch entries
+    int tokens;
     int first_position;
     int q_heads;
     int kv_heads;
@@ -24,35 +24,21 @@ struct TcArgs {
     EpilogueArgs ep;
     int* status;
     int n_items;              // work items in the list
-    int mtiles;               // prefill: row tiles per kv head
+    int mtiles;               // row tiles per kv head
     // How a launch cuts its rows' keys into items (the bits are the same whichever the host picks):
-    //   finish != 0       an item is all the key tiles of one row tile and kv head (prefill) or of one
-    //                     sequence and kv head (decode).  The kernel runs both folds and the epilogue,
-    //                     keeping the second fold's values between segments in row_state.
-    //   otherwise         the kernel writes partials to the workspace, `slots` per row at most, and a
-    //                     merge kernel finishes the rows.  With tile_partials == 0 an item is a run of
-    //                     whole segments (one in prefill; seq_run[b] in decode, so that a sequence's
-    //                     items are of one size) and leaves each segment's partial, slot = ordinal of
-    //                     the segment.  With tile_partials != 0 (decode only) an item is an aligned run
-    //                     of 2^log_run tiles, log_run < map.log_segment, and leaves every tile's own
-    //                     partial, slot = ordinal of the tile among the row's tiles.
-    int decode;
+    //   finish != 0       an item is all the key tiles of one row tile and kv head.  The kernel runs both folds
+    //                     and the epilogue, keeping the second fold's values between segments in row_state
+    //                     (head_dim 64: in shared memory).
+    //   otherwise         an item is one segment of those and leaves its partial in the workspace, `slots`
+    //                     per row at most (slot = ordinal of the segment); a merge kernel finishes the rows.
     int slots;
     int finish;
-    int log_run;
-    int tile_partials;
     float* part_o;            // fp32 [rows][slots][d]
     float* part_ml;           // fp32 [rows][slots][2]
     float* row_state;         // fp32 [thread blocks][d][128], finish only
-    // Multipliers for the divisions of decode_item (see fast_div); 0 = divide the ordinary way.
+    // Multipliers for the divisions of tc_item (see fast_div); 0 = divide the ordinary way.
     uint32_t magic_slots, magic_kv_heads;
-    // Decode: sequence b has seq_slots[b] runs; its items, kv head major, start at item_start[b].
-    int item_start[kMaxBatch + 1];
-    unsigned short seq_slots[kMaxBatch];
-    unsigned short seq_run[kMaxBatch];   // segments per run of sequence b (decode, segment partials)
-    uint32_t seq_magic[kMaxBatch];       // division by seq_slots[b]
-    BatchMeta meta;
-    // Prefill with bidirectional blocks: per token of the call, one past the end of its block (0 =
+    // Bidirectional blocks: per token of the call, one past the end of its block (0 =
     // none), and the position one past the last key appended.  Every item then reaches to the last
     // appended key's tile; rows that see nothing of a tile fold its empty partial, a no-op.
     const int* block_ends;
@@ -72,90 +58,69 @@ __device__ __forceinline__ int fast_div(int n, int d, uint32_t magic) {
 
 struct TcItem {
     int kv_head;
-    int seq;
-    int row0;          // first row of q / out (token index of the chunk, or batch entry)
+    int row0;          // first row of q / out (token index of the chunk)
     int valid_tokens;  // query tokens in this row tile
     int first_pos;     // position of the first query token
     int tile_first;    // absolute index of the first key tile
     int n_tiles;       // key tiles to visit (stride `world` apart); <= 0: nothing to do
-    int slot;          // ordinal of the item's run among the rows' runs; with tile partials, the row's
-                       // partial slot of the item's first tile
     int first_segment; // absolute index of the first segment the rows see (segment partials go to
                        // slot = segment - first_segment)
 };
 
-__device__ __forceinline__ TcItem decode_item(const TcArgs& args, int index) {
+__device__ __forceinline__ TcItem tc_item(const TcArgs& args, int index) {
     TcItem w;
     const int tokens_per_tile = kRows >> args.log_group;
-    if (args.decode) {
-        int lo = 0, hi = args.tokens;                 // item_start[lo] <= index < item_start[hi]
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (index >= args.item_start[mid]) lo = mid; else hi = mid;
-        }
-        const int b = lo;
-        const int local = index - args.item_start[b];
-        const int slots = args.seq_slots[b];
-        w.kv_head = fast_div(local, slots, args.seq_magic[b]);
-        w.slot = local - w.kv_head * slots;
-        w.row0 = b;
-        w.valid_tokens = 1;
-        w.first_pos = args.meta.pos[b];
-        w.seq = args.meta.seq[b];
-    } else {
-        // Longest key ranges first: descending row tile; a row tile's segments and kv heads adjacent.
-        const int rest = fast_div(index, args.slots, args.magic_slots);
-        w.slot = index - rest * args.slots;
-        const int tile_index = fast_div(rest, args.kv_heads, args.magic_kv_heads);
-        w.kv_head = rest - tile_index * args.kv_heads;
-        const int mtile = args.mtiles - 1 - tile_index;
-        w.row0 = mtile * tokens_per_tile;
-        w.valid_tokens = min(tokens_per_tile, args.tokens - w.row0);
-        w.first_pos = args.first_position + w.row0;
-        w.seq = args.seq;
-    }
-    const int last_pos = (!args.decode && args.block_ends != nullptr) ? args.appended - 1 : w.first_pos + w.valid_tokens - 1;
-    TileRange tiles;
-    if (args.finish) {
-        tiles = row_tiles(args.map, w.first_pos, last_pos, args.window);
-    } else if (args.decode && !args.tile_partials) {
-        const int run = args.seq_run[w.row0];           // the sequence's segments in runs of one size
-        tiles = segment_run_tiles(args.map, w.first_pos, last_pos, args.window, w.slot * run, run);
-    } else {
-        tiles = group_tiles(args.map, w.first_pos, last_pos, args.window, w.slot, args.log_run);
-    }
+    // Longest key ranges first: descending row tile; a row tile's segments and kv heads adjacent.
+    const int rest = fast_div(index, args.slots, args.magic_slots);
+    const int slot = index - rest * args.slots;
+    const int tile_index = fast_div(rest, args.kv_heads, args.magic_kv_heads);
+    w.kv_head = rest - tile_index * args.kv_heads;
+    const int mtile = args.mtiles - 1 - tile_index;
+    w.row0 = mtile * tokens_per_tile;
+    w.valid_tokens = min(tokens_per_tile, args.tokens - w.row0);
+    w.first_pos = args.first_position + w.row0;
+    const int last_pos = args.block_ends != nullptr ? args.appended - 1 : w.first_pos + w.valid_tokens - 1;
+    const TileRange tiles = args.finish ? row_tiles(args.map, w.first_pos, last_pos, args.window)
+                                        : group_tiles(args.map, w.first_pos, last_pos, args.window, slot, args.map.log_segment);
     w.tile_first = tiles.first;
     w.n_tiles = tiles.count;
     w.first_segment = first_visible_tile(w.first_pos, args.window) >> args.map.log_segment;
-    if (args.tile_partials && tiles.count > 0) {
-        const int world = args.map.world > 1 ? args.map.world : 1;
-        w.slot = (tiles.first - row_tiles(args.map, w.first_pos, last_pos, args.window).first) / world;
-    }
     return w;
 }
+
+// A worker's way through a list of items, longest first: forwards through the workers in one round, backwards in the
+// next, so that the first of them does not get the longest item of every round.
+struct Snake {
+    int item, step, twice;
+    __device__ __forceinline__ Snake(int worker, int workers) : item(worker), step(2 * (workers - worker) - 1), twice(2 * workers) {}
+    __device__ __forceinline__ void next() {
+        item += step;
+        step = twice - step;
+    }
+};
 
 // The walk over a CTA's items: each item is decoded once per role (its decoding costs a few integer
 // divisions, which a role pays on its critical path at every item boundary).
 struct TcItemIter {
+    Snake at;
     int item;          // index in the work list, or n_items at the end
     TcItem w;
 };
 __device__ __forceinline__ void items_seek(const TcArgs& args, TcItemIter& it) {
-    for (; it.item < args.n_items; it.item += gridDim.x) {
-        it.w = decode_item(args, it.item);
+    for (; it.at.item < args.n_items; it.at.next()) {
+        it.item = it.at.item;
+        it.w = tc_item(args, it.item);
         if (it.w.n_tiles > 0) return;
     }
     it.item = args.n_items;
 }
 __device__ __forceinline__ TcItemIter items_begin(const TcArgs& args) {
-    TcItemIter it;
-    it.item = blockIdx.x;
-    it.w = TcItem{};
+    TcItemIter it{Snake(int(blockIdx.x), int(gridDim.x)), 0, TcItem{}};
     items_seek(args, it);
     return it;
 }
 __device__ __forceinline__ void items_next(const TcArgs& args, TcItemIter& it) {
-    it.item += gridDim.x;
+    it.at.next();
     items_seek(args, it);
 }
 
