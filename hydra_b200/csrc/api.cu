@@ -363,7 +363,8 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
     // A launch takes as many sequences as the prepared-query buffer has rows for.
     // (The tcgen05 decode kernel lists its rows, 512 of them at most, in shared memory.)
     int per_launch = prep ? std::min(kMaxBatch, cache->ws.qprep_tokens) : kMaxBatch;
-    if (tensor) per_launch = std::max(1, std::min(per_launch, 512 / p->kv_heads));
+    // The workspace holds any cut of max_seqs rows; more, some of the same sequence, go in several launches.
+    if (tensor) per_launch = std::max(1, std::min({per_launch, 512 / p->kv_heads, cache->max_seqs}));
 
     for (int start = 0; start < n_seq; start += per_launch) {
         const int count = std::min(per_launch, n_seq - start);

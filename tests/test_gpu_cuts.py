@@ -1,0 +1,181 @@
+"""Every way the kernels cut their work, at the sizes where a cut can go wrong: rows and keys on both sides of a tile,
+a segment and a row tile, ragged batches, column widths of the projections, pieces of a host prompt.  The
+reference is the oracle, plain PyTorch in fp32 for the projections, and the path's own invariant: a position's
+result is the same bits whether it came in a prompt or as a decoded token."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import hydra_oracle as ho
+from tests import hydra_testlib as tl
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def hb():
+    import hydra_b200
+    return hydra_b200
+
+
+@pytest.fixture(scope="module")
+def ctx(hb):
+    c = hb.Context(0)
+    yield c
+    c.close()
+
+
+def _filled(hb, ctx, d, qh, kvh, window, tokens, seqs=1, io="bf16", gated=False):
+    rng = np.random.default_rng(d * 31 + qh + tokens)
+    q = tl.normal_bf16(rng, (tokens, qh, d))
+    k = tl.normal_bf16(rng, (tokens, kvh, d))
+    v = tl.normal_bf16(rng, (tokens, kvh, d))
+    sinks = tl.normal_bf16(rng, (qh,))
+    gate = tl.normal_bf16(rng, (tokens, qh, d)) if gated else None
+    layer = tl.Layer(hb, ctx, qh, kvh, d, 4608, window=window, sinks=sinks, io=io, max_seqs=seqs,
+                     storage=hb.capi.HC_STORAGE_LINEAR)
+    for seq in range(seqs):
+        layer.append(k, v, 0, seq=seq)
+    return layer, q, k, v, sinks, gate
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, tokens, io, gated", [
+    (64, 64, 8, 0, 2203, "bf16", False),       # three segments of 1024, a last row tile of 11 tokens
+    (64, 64, 8, 128, 1100, "f32", False),      # two tiles a row
+    (64, 8, 8, 0, 1153, "bf16", True),         # one head a group: 128 tokens a row tile
+    (128, 16, 2, 0, 1290, "bf16", False),
+    (256, 16, 8, 1024, 2180, "bf16", False),   # pairs of SMs; the window crosses a segment of 2048
+    (256, 16, 2, 0, 2305, "bf16", True),       # the gated epilogue
+    (256, 4, 4, 0, 383, "f32", False),
+    (512, 16, 1, 0, 1031, "bf16", False),      # two halves of O, segments of 2048 for decode and prefill alike
+    (512, 8, 1, 0, 130, "bf16", False),
+])
+def test_prompt_rows_equal_decoded_tokens_and_the_oracle(hb, ctx, d, qh, kvh, window, tokens, io, gated):
+    layer, q, k, v, sinks, gate = _filled(hb, ctx, d, qh, kvh, window, tokens, io=io, gated=gated)
+    prompt = layer.prefill(q, 0, gate=gate)
+    edges = [0, 1, 15, 16, 127, 128, 129, 255, 256, 1023, 1024, 1151, 1152, 2047, 2048, 2049, tokens - 2, tokens - 1]
+    rows = sorted({r for r in edges if r < tokens})
+    for r in rows:
+        one = layer.decode(q[r:r + 1], [r], gate=None if gate is None else gate[r:r + 1])
+        assert np.array_equal(one[0], prompt[r]), r
+    want = ho.attention_rows(q[rows], np.asarray(rows), k, v, 1 / np.sqrt(d), window, sinks=sinks,
+                             gate=None if gate is None else gate[rows])
+    assert tl.within_tolerance(prompt[rows], want, bf16_output=io == "bf16")
+    # the same rows as the end of a later chunk
+    tail = min(tokens, 37)
+    assert np.array_equal(layer.prefill(q[-tail:], tokens - tail, gate=None if gate is None else gate[-tail:]), prompt[-tail:])
+    layer.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window", [(64, 64, 8, 0), (64, 64, 8, 128), (128, 16, 2, 0), (256, 16, 2, 0), (512, 16, 1, 0)])
+@pytest.mark.parametrize("n_seq", [2, 13, 64])
+def test_ragged_batches_equal_their_rows_alone(hb, ctx, d, qh, kvh, window, n_seq):
+    tokens = 2305
+    layer, q, k, v, sinks, _ = _filled(hb, ctx, d, qh, kvh, window, tokens, seqs=4)
+    rng = np.random.default_rng(n_seq)
+    positions = [0, 127, 128, 1023, 1024, 2047, 2048, tokens - 1] + [int(p) for p in rng.integers(0, tokens, 64)]
+    positions = positions[-n_seq:] if n_seq < 8 else positions[:n_seq]
+    ids = [b % 4 for b in range(n_seq)]
+    got = layer.decode(q[positions], positions, seq_ids=ids)
+    for b in range(0, n_seq, max(1, n_seq // 6)):
+        alone = layer.decode(q[positions[b]:positions[b] + 1], positions[b:b + 1], seq_ids=ids[b:b + 1])
+        assert np.array_equal(alone[0], got[b]), b
+    want = ho.attention_rows(q[positions], np.asarray(positions), k, v, 1 / np.sqrt(d), window, sinks=sinks)
+    assert tl.within_tolerance(got, want)
+    layer.close()
+
+
+@pytest.mark.parametrize("tokens", [1, 16, 17, 64, 65, 128, 129, 257, 900])
+@pytest.mark.parametrize("n_in, widths", [(2880, (4096, 512, 512)), (2048, (9216,)), (64, (40,)), (192, (2880, 72)), (4096, (2888,))])
+def test_projections_of_every_tile_shape(hb, ctx, tokens, n_in, widths):
+    """Up to 128 tokens one column tile per SM (16 to 64 wide), above that pairs of SMs with 128 to 256 columns:
+    token counts and widths around all of them, K steps that do not fill a stage."""
+    import torch
+    backend = hb.AttentionBackend(ctx)
+    gen = torch.Generator(device="cuda").manual_seed(tokens + n_in)
+
+    def bf16(*shape, scale=1.0):
+        return (torch.randn(shape, generator=gen, device="cuda") * scale).to(torch.bfloat16)
+
+    x = bf16(tokens, n_in)
+    w = [bf16(n, n_in, scale=0.02) for n in widths]
+    b = [bf16(n) for n in widths]
+    want = [x.float() @ wi.float().T + bi.float() for wi, bi in zip(w, b)]
+    out = [torch.empty((tokens, n), device="cuda") for n in widths]
+    backend.linear_group(x, w, b, out, tokens, n_in, y_dtype=hb.capi.HC_F32)
+    residual = torch.randn((tokens, widths[0]), generator=gen, device="cuda")
+    updated = residual.clone()
+    backend.linear(x, w[0], b[0], updated, tokens, n_in, widths[0], y_dtype=hb.capi.HC_F32, residual=updated)
+    ctx.check()
+    for got, ref in zip(out, want):
+        assert float((got - ref).abs().max()) <= 1e-3 * max(1.0, float(ref.abs().max()))
+    assert torch.equal(updated, out[0] + residual)
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, tokens, io", [
+    (64, 64, 8, 0, 40, "bf16"), (64, 64, 8, 0, 2500, "bf16"), (64, 64, 8, 128, 1700, "bf16"),
+    (64, 64, 8, 0, 700, "f32"), (256, 16, 8, 256, 3000, "bf16"), (128, 16, 2, 0, 4096, "bf16"),
+])
+def test_host_prompts_in_pieces_equal_device_prompts(hb, ctx, d, qh, kvh, window, tokens, io):
+    import torch
+    rng = np.random.default_rng(tokens)
+    dtype = torch.bfloat16 if io == "bf16" else torch.float32
+    host = [torch.from_numpy(tl.normal_bf16(rng, (tokens, h, d))).to(dtype).pin_memory() for h in (qh, kvh, kvh)]
+    outs = []
+    for on_host in (False, True):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 4608, window=window, io=io, prefill_chunk=256,
+                         rope_inv_freq=ho.inverse_frequencies(d, 10000.0))
+        q, k, v = host if on_host else [t.cuda() for t in host]
+        out = torch.zeros((tokens, qh, d), dtype=dtype)
+        out = out.pin_memory() if on_host else out.cuda()
+        call = layer.backend.prefill_host if on_host else layer.backend.prefill_chunks
+        call(layer.cache, 0, q, k, v, out, tokens, 0, 256, layer.params)
+        ctx.check()
+        outs.append(tl.to_host(out))
+        layer.close()
+    assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("tokens", [1, 5, 200])
+def test_stack_call_equals_its_parts(hb, ctx, tokens):
+    """hc_attention_stack_host over two gated layers of different windows against the same calls one by one."""
+    import torch
+    capi, width, qh, kvh, d = hb.capi, 320, 8, 2, 64
+    backend = hb.AttentionBackend(ctx)
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+
+    def bf16(*shape, scale=0.05):
+        return (torch.randn(shape, generator=gen, device="cuda") * scale).to(torch.bfloat16)
+
+    windows = (128, 0)
+    shapes = dict(input_norm=(width,), wq=(2 * qh * d, width), bq=(2 * qh * d,), wk=(kvh * d, width), bk=(kvh * d,),
+                  wv=(kvh * d, width), bv=(kvh * d,), wo=(width, qh * d), bo=(width,))
+    layers = [{name: bf16(*shape) for name, shape in shapes.items()} for _ in windows]
+    params = [hb.AttnParams(q_heads=qh, kv_heads=kvh, head_dim=d, window=w, sm_scale=0.125, io_dtype=capi.HC_BF16,
+                            gate_layout=capi.HC_GATE_INTERLEAVED) for w in windows]
+    states = torch.randn((tokens, width), generator=gen, device="cuda")
+    caches = [hb.KVCache(ctx, [dict(q_heads=qh, kv_heads=kvh, head_dim=d, window=w) for w in windows], 512) for _ in range(2)]
+    want = states.clone()
+    for i, (w, p) in enumerate(zip(layers, params)):
+        normed = torch.empty((tokens, width), device="cuda", dtype=torch.bfloat16)
+        q, k, v, attended = (torch.empty((tokens, n * d), device="cuda", dtype=torch.bfloat16) for n in (2 * qh, kvh, kvh, qh))
+        backend.rms_norm(want, w["input_norm"], normed, tokens, width, 1e-5)
+        backend.linear_group(normed, [w["wq"], w["wk"], w["wv"]], [w["bq"], w["bk"], w["bv"]], [q, k, v], tokens, width,
+                             y_dtype=capi.HC_BF16)
+        backend.layer_step(caches[0], i, q, k, v, attended, tokens, 0, p)
+        backend.linear(attended, w["wo"], w["bo"], want, tokens, qh * d, width, y_dtype=capi.HC_F32, residual=want)
+    blocks = (capi.BlockWeightsStruct * 2)()
+    for block, w, p in zip(blocks, layers, params):
+        for name, tensor in w.items():
+            setattr(block, name, tensor.data_ptr())
+        block.params = p.struct()
+    lib = capi.load()
+    workspace = torch.empty(lib.hc_attention_stack_bytes(blocks, 2, tokens, width), dtype=torch.uint8, device="cuda")
+    host = states.cpu().numpy().copy()
+    status = lib.hc_attention_stack_host(ctx.handle, caches[1].handle, blocks, 2, 0, host.ctypes.data, host.ctypes.data, tokens,
+                                         width, 0, ctypes.c_float(1e-5), workspace.data_ptr(), None)
+    assert status == 0
+    assert np.array_equal(host, want.cpu().numpy())
+    for cache in caches:
+        cache.close()
