@@ -181,6 +181,7 @@ struct hc_kv_cache {
     hc::Workspace ws;
     // hc_layer_step_host / hc_prefill_host: two device staging slots, a stream for the copies in and
     // one for the copies out, and the events that order them against the caller's stream.
+    void* workspace_dev = nullptr;   // ws and the staging slots
     void* stage_dev = nullptr;
     size_t stage_bytes = 0;       // of one slot
     cudaStream_t copy_in = nullptr;
