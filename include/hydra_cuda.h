@@ -234,7 +234,7 @@ HC_API hc_status hc_rms_norm(hc_context* ctx, const void* x, const void* scale_b
  * margin longer (hc_layer_info.capacity), which lets hc_prefill_chunks take several chunks at once.
  * `shard` may be NULL.
  *
- * The call also fixes how each layer groups its 128-key tiles into segments (1024 or 4096 keys),
+ * The call also fixes how each layer groups its 128-key tiles into segments (1024, 2048 or 4096 keys),
  * from the layer's head counts, prefill_chunk, max_seqs and the device's SM count: the attention
  * kernels fold tiles into segment partials and segment partials into rows, and a launch may spread
  * a row's segments over thread blocks.  All calls on one cache agree bit for bit (chunked prefill,
@@ -355,7 +355,7 @@ HC_API hc_status hc_attention_decode(hc_context* ctx, hc_kv_cache* cache, int la
  *   - q must be bf16, already normalised and rotated: io_dtype HC_BF16, norm_q 0, rope NULL, gate
  *     none or HC_GATE_SEPARATE.  1 to 64 sequences; not for sequence-sharded caches.
  *   - A call whose partials (n_seq * q_heads * slots * (head_dim + 2) floats, where slots is the
- *     number of segments of 1024 or 4096 keys, or of 128-key tiles, that the library cuts the longest
+ *     number of segments of 1024, 2048 or 4096 keys, or of 128-key tiles, that the library cuts the longest
  *     sequence into for this batch) exceed the limit is refused with HC_KV_OVERFLOW and a message
  *     that states both sizes.
  *   - It runs the same kernels as hc_attention_decode (tcgen05 for head_dim 64, 128, 256, CUDA
