@@ -70,7 +70,7 @@ def _ptr(buffer) -> Optional[int]:
         return None
     if isinstance(buffer, int):
         return buffer
-    return int(buffer.data_ptr())
+    return buffer.data_ptr()
 
 
 def _stream(stream) -> Optional[int]:
@@ -189,18 +189,29 @@ class AttnParams:
     block_ends: object = None       # int32 [tokens] device buffer (blockEnds of BatchEncoder.attention), or None
     _keep: list = field(default_factory=list, repr=False)
 
+    def __setattr__(self, name, value) -> None:
+        object.__setattr__(self, name, value)
+        object.__setattr__(self, "_struct", None)
+
     def struct(self) -> capi.AttnParamsStruct:
-        s = capi.AttnParamsStruct()
-        s.q_heads, s.kv_heads, s.head_dim, s.window = self.q_heads, self.kv_heads, self.head_dim, self.window
-        s.sm_scale, s.io_dtype = float(self.sm_scale), int(self.io_dtype)
-        s.sinks = _ptr(self.sinks)
-        s.norm_q, s.norm_k, s.norm_v = self.norm_q, self.norm_k, self.norm_v
-        s.q_norm_weight, s.k_norm_weight = _ptr(self.q_norm_weight), _ptr(self.k_norm_weight)
-        s.norm_eps = float(self.norm_eps)
-        s.rope = self.rope.handle if self.rope is not None else None
-        s.gate_layout, s.gate = int(self.gate_layout), _ptr(self.gate)
-        s.kernel_path = int(self.kernel_path)
-        s.block_ends = _ptr(self.block_ends)
+        """The C struct, filled once and again after any attribute changes (filling it takes as long as the library
+        takes to launch a decode step).  What buffers point at is looked up on every call."""
+        s = self._struct
+        if s is None:
+            s = capi.AttnParamsStruct()
+            s.q_heads, s.kv_heads, s.head_dim, s.window = self.q_heads, self.kv_heads, self.head_dim, self.window
+            s.sm_scale, s.io_dtype = float(self.sm_scale), int(self.io_dtype)
+            s.norm_q, s.norm_k, s.norm_v = self.norm_q, self.norm_k, self.norm_v
+            s.norm_eps = float(self.norm_eps)
+            s.gate_layout = int(self.gate_layout)
+            s.kernel_path = int(self.kernel_path)
+            buffers = [(name, getattr(self, name)) for name in ("sinks", "q_norm_weight", "k_norm_weight", "gate", "block_ends")]
+            object.__setattr__(self, "_buffers", [(name, buffer) for name, buffer in buffers if buffer is not None])
+            object.__setattr__(self, "_struct", s)
+        for name, buffer in self._buffers:
+            setattr(s, name, _ptr(buffer))
+        if self.rope is not None:
+            s.rope = self.rope.handle
         return s
 
 
