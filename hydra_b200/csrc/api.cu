@@ -715,9 +715,8 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         if (ring && sequence) { st = fail(HC_UNSUPPORTED, "ring storage cannot be sequence-sharded"); break; }
         // The reference's ring holds window + prefill_chunk rows (KVCache.swift:160-167; here rounded up
         // to whole tiles): that is what the margin, the reported ring size and the rewind floor
-        // follow.  The stored ring is one margin longer, so that the rows a chunk appends never
-        // overwrite keys the previous chunk still attends to and hc_prefill_chunks may run a chunk's
-        // prologue while the previous chunk's attention is finishing.
+        // follow.  The stored ring is one margin longer, so that hc_prefill_chunks can append more than a
+        // chunk before its first token attends.
         const int reference_ring = ring ? round_up(L.desc.window + prefill_chunk, kTileKeys) : 0;
         L.ring_margin = ring ? reference_ring - L.desc.window : 0;
         L.ring = ring ? round_up(reference_ring + L.ring_margin, kTileKeys) : 0;

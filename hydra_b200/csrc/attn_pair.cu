@@ -142,9 +142,11 @@ __device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
     return r;
 }
 
-// FINISH: the kernel finishes an item's rows; otherwise it leaves segment partials (a template argument, so that a
-// launch carries only its own code).
-template <int D, bool FINISH>
+// MODE: what becomes of an item's rows, a template argument so that a launch carries the code (and the registers) of its
+// own way only: bf16 rows (or, sequence-sharded, row partials; head_dim 512: all finished rows); rows with a gate or
+// in fp32; segment partials.
+constexpr int kPairRowsOut = 0, kPairGatedOut = 1, kPairSegments = 2;
+template <int D, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                       const __grid_constant__ CUtensorMap tmap_q, const TcArgs args) {
@@ -448,6 +450,8 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                 L2 = 0.0f;
             }
         };
+        // The gated epilogue uses an item's last O buffer and frees it.
+        constexpr bool keep_o = MODE == kPairGatedOut;
         uint32_t t = 0;
         bool ok = true;
         for (PairIter walk = pair_begin<D>(args); ok && walk.item < args.n_items; pair_next<D>(args, walk)) {
@@ -478,7 +482,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                         uint32_t o[16];
                         HC_TMEM_LD16(o_tmem + chunk * 16, o);
                         tc_wait_ld();
-                        if (chunk == 7) {
+                        if (chunk == 7 && !(keep_o && j + 1 == w.n_tiles)) {
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) mbar_arrive_cluster_relaxed(o_free);      // nothing but tensor memory was read
@@ -490,7 +494,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     if (lane == 0) mbar_arrive_cluster_relaxed(o_free);
                 }
                 const int tile = w.tile_first + j * world;
-                if (!FINISH || j + 1 == w.n_tiles || (tile >> args.map.log_segment) == ((tile + world) >> args.map.log_segment)) continue;
+                if (MODE == kPairSegments || j + 1 == w.n_tiles || (tile >> args.map.log_segment) == ((tile + world) >> args.map.log_segment)) continue;
                 // A segment is complete and another follows: fold it into the row's state, which is kept out of the
                 // registers ((M2, L2) in shared memory, the values in global memory), and start over.
                 if (!warp_has_rows) continue;
@@ -520,7 +524,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
             }
             if (!ok) break;
             const int col0 = w.half * kPairO + half * 128;
-            if constexpr (!FINISH) {
+            if constexpr (MODE == kPairSegments) {
                 // The segment's partial goes to the workspace (a merge kernel runs the second fold).
                 if (valid) {
                     const size_t prow = vec * args.slots + w.slot;
@@ -564,7 +568,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     for (int i = 0; i < 128; ++i) A[i] = __fmul_rn(A[i], b);
                 }
             }
-            if (args.ep.write_partial) {
+            if (MODE == kPairRowsOut && args.ep.write_partial) {
                 if (!valid) continue;
                 float* dst = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2) + col0;
                 #pragma unroll
@@ -590,7 +594,73 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                 out_row = size_t(w.row0 + token) * args.q_heads + size_t(w.kv_head) * G + (r & (G - 1));
                 return token < w.valid_tokens;
             };
-            if (args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32) {
+            if constexpr (MODE == kPairGatedOut) {
+                // With a gate, or fp32 rows.  The values go back to tensor memory, in place of the last O, so that the
+                // rest can be a rolled loop, thread = row, with registers to spare for the next 16 columns' gates: eight
+                // copies of it, fetched cold, and gate loads that waited for one another were 17 us of a launch
+                // (777 tokens behind 1291, 16 gated heads of 256: 97 us, now 83).
+                #pragma unroll
+                for (int i = 0; i < 128; i += 16) {
+                    uint32_t v[16];
+                    #pragma unroll
+                    for (int u = 0; u < 16; ++u) v[u] = __float_as_uint(__fmul_rn(A[i + u], inverse));
+                    HC_TMEM_ST16(o_tmem + i, v);
+                }
+                tc_wait_st();
+                asm volatile("" ::: "memory");
+                const bool gated = args.ep.gate_layout != HC_GATE_NONE, fp32 = args.ep.io_dtype == HC_F32;
+                const int bytes = fp32 ? 4 : 2;
+                const size_t gate_at = args.ep.gate_layout == HC_GATE_INTERLEAVED ? vec * size_t(2 * D) + D : vec * size_t(D);
+                const unsigned char* gate = static_cast<const unsigned char*>(args.ep.gate) + (gate_at + col0) * bytes;
+                unsigned char* out = static_cast<unsigned char*>(args.ep.out) + (vec * D + col0) * bytes;
+                const bool aligned = (reinterpret_cast<uintptr_t>(gate) & 15) == 0;
+                // Four columns of the thread's row as fp32.
+                auto gate4 = [&](int i) -> float4 {
+                    if (!gated || !valid) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (fp32) {
+                        const float* from = reinterpret_cast<const float*>(gate) + i;
+                        return aligned ? *reinterpret_cast<const float4*>(from) : make_float4(from[0], from[1], from[2], from[3]);
+                    }
+                    const uint16_t* from = reinterpret_cast<const uint16_t*>(gate) + i;
+                    const uint2 two = aligned ? *reinterpret_cast<const uint2*>(from)
+                                              : make_uint2(from[0] | uint32_t(from[1]) << 16, from[2] | uint32_t(from[3]) << 16);
+                    return make_float4(__uint_as_float(two.x << 16), __uint_as_float(two.x & 0xffff0000u),
+                                       __uint_as_float(two.y << 16), __uint_as_float(two.y & 0xffff0000u));
+                };
+                float4 now[4], next[4];
+                #pragma unroll
+                for (int u = 0; u < 4; ++u) now[u] = gate4(4 * u);
+                #pragma unroll 1
+                for (int i = 0; i < 128; i += 16) {
+                    uint32_t v[16];
+                    HC_TMEM_LD16(o_tmem + i, v);
+                    #pragma unroll
+                    for (int u = 0; u < 4; ++u) next[u] = gate4(i < 112 ? i + 16 + 4 * u : 0);
+                    tc_wait_ld();
+                    #pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        float r[4] = {__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1]), __uint_as_float(v[4 * u + 2]), __uint_as_float(v[4 * u + 3])};
+                        if (gated) {
+                            r[0] = __fmul_rn(r[0], sigmoid_gate(now[u].x));
+                            r[1] = __fmul_rn(r[1], sigmoid_gate(now[u].y));
+                            r[2] = __fmul_rn(r[2], sigmoid_gate(now[u].z));
+                            r[3] = __fmul_rn(r[3], sigmoid_gate(now[u].w));
+                        }
+                        now[u] = next[u];
+                        if (!valid) continue;
+                        if (fp32) {
+                            *reinterpret_cast<float4*>(out + (i + 4 * u) * 4) = make_float4(r[0], r[1], r[2], r[3]);
+                        } else {
+                            *reinterpret_cast<uint2*>(out + (i + 4 * u) * 2) = make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster_relaxed(o_free);
+                continue;
+            }
+            if (D == 256 || (args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32)) {
                 uint16_t* out = reinterpret_cast<uint16_t*>(args.ep.out) + col0 + c * 8;
                 #pragma unroll
                 for (int i = 0; i < 128; i += 32) {
@@ -610,7 +680,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     }
                     __syncwarp();
                 }
-            } else {
+            } else if constexpr (D == 512) {
                 const int gate_layout = args.ep.gate_layout;
                 const size_t gate_stride = gate_layout == HC_GATE_INTERLEAVED ? size_t(2 * D) : size_t(D);
                 const size_t gate_first = (gate_layout == HC_GATE_INTERLEAVED ? D : 0) + col0 + c * 4;
@@ -660,18 +730,18 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     if (warp == 1) tmem_dealloc_pair(tmem, 512);
 }
 
-template <int D, bool FINISH>
+template <int D, int MODE>
 hc_status launch_pair_kernel(hc_context* ctx, const hc_layer_store& layer, const CUtensorMap& tmap_q, const TcArgs& args, cudaStream_t stream) {
     constexpr int smem = PairLayout<D>::kSmemBytes + int(sizeof(PairBarriers));
     static_assert(smem <= 227 * 1024, "shared memory of one CTA");
     static bool configured[64] = {};
     if (!configured[ctx->device & 63]) {
-        const cudaError_t err = cudaFuncSetAttribute(attention_pair_kernel<D, FINISH>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t err = cudaFuncSetAttribute(attention_pair_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (err != cudaSuccess) return check_cuda(err, "attention_pair_kernel shared memory");
         configured[ctx->device & 63] = true;
     }
     const int grid = 2 * std::max(1, std::min(args.n_items, std::max(ctx->sm_count / 2, 1)));
-    const cudaError_t launched = launch_pdl(attention_pair_kernel<D, FINISH>, grid, kPairThreads, size_t(smem), stream,
+    const cudaError_t launched = launch_pdl(attention_pair_kernel<D, MODE>, grid, kPairThreads, size_t(smem), stream,
                                             *static_cast<const CUtensorMap*>(layer.tmap_k64),
                                             *static_cast<const CUtensorMap*>(layer.tmap_v), tmap_q, args);
     ctx->launches += 1;
@@ -690,12 +760,12 @@ hc_status launch_attention_pair(hc_context* ctx, const hc_layer_store& layer, co
     const hc_status st = tc_encode_3d(&tmap_q, args.q, uint64_t(head_dim), uint64_t(args.q_heads), uint64_t(args.tokens), uint32_t(group),
                                       uint32_t(kRows / group));
     if (st != HC_OK) return st;
-    if (head_dim == 256) {
-        return args.finish ? launch_pair_kernel<256, true>(ctx, layer, tmap_q, args, stream)
-                           : launch_pair_kernel<256, false>(ctx, layer, tmap_q, args, stream);
-    }
-    return args.finish ? launch_pair_kernel<512, true>(ctx, layer, tmap_q, args, stream)
-                       : launch_pair_kernel<512, false>(ctx, layer, tmap_q, args, stream);
+    // (Head_dim 512 has one epilogue for all: apart, its kernel for bf16 rows came out 6 % slower.)
+    const bool gated = !args.ep.write_partial && (args.ep.gate_layout != HC_GATE_NONE || args.ep.io_dtype == HC_F32);
+    auto launch = head_dim == 512 ? (args.finish ? launch_pair_kernel<512, kPairRowsOut> : launch_pair_kernel<512, kPairSegments>)
+                : !args.finish    ? launch_pair_kernel<256, kPairSegments>
+                : gated           ? launch_pair_kernel<256, kPairGatedOut> : launch_pair_kernel<256, kPairRowsOut>;
+    return launch(ctx, layer, tmap_q, args, stream);
 }
 
 }  // namespace hc
