@@ -617,7 +617,7 @@ def run_cuda(args):
               "kv_gbs": dec_gbs, "frac_of_8tbs": dec_gbs / (NOMINAL_HBM_GBS * world),
               "frac_of_measured": dec_gbs / (peaks["hbm_gbs"] * world),
               "timer_floor_us": floor_us, "us_per_step_l2_resident": resident_us,
-              "note": "call = q prologue + split kernel + merge; L2 flushed before each timed call.  timer_floor_us: a "
+              "note": "call = one launch (query prologue, attention over the split keys, merge); L2 flushed before each timed call.  timer_floor_us: a "
                       "one-row hc_rms_norm under the same timer and flush; us_per_step_l2_resident: 32 calls back to "
                       "back without the flush (K/V in L2: latency, not an HBM figure)"}
 
@@ -641,8 +641,8 @@ def run_cuda(args):
     e2e = {"value": cfg.prompt / (e2e_ms * 1e-3), "unit": "tok/s",
            "h2d_bytes_per_step": cfg.prompt * (cfg.q_heads + 2 * cfg.kv_heads) * d * 2,
            "d2h_bytes_per_step": cfg.prompt * cfg.q_heads * d * 2, "ms_per_step": e2e_ms,
-           "note": "per rank bytes; hc_prefill_host: pinned host buffers, the copies of chunk i+1 / i-1 overlap the "
-                   "kernels of chunk i"}
+           "note": "per rank bytes; hc_prefill_host: pinned host buffers, the copies in and out overlap the "
+                   "kernels of the tokens before and after"}
     clocks = sampler.stop() if rank == 0 else None
     run.close()
 
