@@ -149,13 +149,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         }
         for (int i = 0; i < 3; ++i) {
             mbar_init(&bars->s_full[i], 1);
-            mbar_init(&bars->p_full[i], 4);
+            mbar_init(&bars->p_full[i], 128);
             mbar_init(&bars->pv_done[i], 1);
         }
-        for (int i = 0; i < 3; ++i) mbar_init(&bars->s_free[i], 4);
+        for (int i = 0; i < 3; ++i) mbar_init(&bars->s_free[i], 128);
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bars->o_full[i], 1);
-            mbar_init(&bars->o_free[i], 4);
+            mbar_init(&bars->o_free[i], 128);
         }
         for (int i = 0; i < kItemRing; ++i) mbar_init(&bars->item_full[i], 1);
         for (int i = 0; i < 4; ++i) {
@@ -419,11 +419,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     // O rows they produce are never read (rows are independent).
                     tc_fence_before();
                     if (LT::kOverlap) {
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&bars->s_free[pb]);
+                        mbar_arrive(&bars->s_free[pb]);
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->p_full[pb]);
+                    mbar_arrive(&bars->p_full[pb]);
                     continue;
                 }
                 const int key0 = (w.tile_first + j * world) * kTileKeys;
@@ -441,8 +439,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     HC_TMEM_LD32(s_tmem + 96, s[3]);
                     tc_wait_ld();
                     tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->s_free[pb]);
+                    mbar_arrive(&bars->s_free[pb]);
                     if (!full) {
                         // By bits of a word for each 32 columns: less than half the code of two comparisons a column,
                         // and it is code that runs cold, once an item (2700 clocks more than an unmasked tile).
@@ -488,8 +485,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     bars->mm[t & 7][row] = __fmul_rn(m, args.c);
                     tc_wait_st();
                     tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->p_full[pb]);
+                    mbar_arrive(&bars->p_full[pb]);
                     continue;
                 }
                 // The row is read twice, 32 columns at a time, in rolled loops: the maximum, then the
@@ -586,8 +582,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 bars->mm[t & 7][row] = __fmul_rn(m, args.c);
                 tc_wait_st();
                 tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->p_full[pb]);
+                mbar_arrive(&bars->p_full[pb]);
             }
         }
     } else {
@@ -660,8 +655,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     tc_fence_after();
                     if (!warp_has_rows) {
                         tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&bars->o_free[LT::o_buf(t)]);
+                        mbar_arrive(&bars->o_free[LT::o_buf(t)]);
                         continue;
                     }
                     const uint32_t o_tmem = tmem + lane_base + LT::o_col(t);
@@ -676,8 +670,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         tc_wait_ld();
                         if (hb == D / 64 - 1) {
                             tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&bars->o_free[LT::o_buf(t)]);
+                            mbar_arrive(&bars->o_free[LT::o_buf(t)]);
                         }
                         if (hb == 0) {
                             L = __fmaf_rn(L, a, __fmul_rn(__uint_as_float(l_bits), b));
