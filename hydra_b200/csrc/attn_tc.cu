@@ -57,7 +57,7 @@ struct TcLayout {
     // columns 0 .. 127 and P in 32 .. 95 of each: a softmax thread takes its whole row of S into registers, so that
     // what a buffer shares with its neighbours is S's alone and soon free, and there is room for two O buffers,
     // each with 16 more columns for the row sums that the tensor core computes.  (With the buffers side by side
-    // and one O buffer 4096 GPT-OSS tokens take 260 us, with these 254.6; one S buffer, three of P and two of O: 270.)
+    // and one O buffer 4096 GPT-OSS tokens take 2 % longer; with one S buffer, three of P and two of O 6 %.)
     static constexpr bool kOverlap = D == 64;
     static constexpr bool kSumOnTensor = D == 64;
     static constexpr uint32_t kBufs = 3;
@@ -276,10 +276,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
           for (int j = 0; j < n_tiles; ++j, ++t) {
             const int slot = int(t % LT::kStages);
             const int qb = int(it & 1);
-            // (Ahead of the waits.)  Descriptors differ from the precomputed bases only in the 16-byte address field.
-            const uint64_t q_desc = warp_uniform(q_desc0 + uint64_t((qb * LT::kQBytes) >> 4));
-            const uint64_t k_desc = warp_uniform(k_desc0 + uint64_t((slot * LT::kTileBytes) >> 4));
-            const uint32_t s_tmem = warp_uniform(tmem + LT::s_col(t));
+            // Descriptors differ from the precomputed bases only in the 16-byte address field.
+            const uint64_t q_desc = q_desc0 + uint64_t((qb * LT::kQBytes) >> 4);
+            const uint64_t k_desc = k_desc0 + uint64_t((slot * LT::kTileBytes) >> 4);
+            const uint32_t s_tmem = tmem + LT::s_col(t);
             // The buffer's previous contents, P of tile t - 3, must have been consumed, and what its neighbours share with it.
             if (t >= LT::kBufs && !mbar_wait(&bars->pv_done[LT::buf(t)], LT::phase(t - LT::kBufs), abort_flag, args.status, 12)) { ok = false; break; }
             if (LT::kOverlap && t >= 1 && !mbar_wait(&bars->s_free[LT::buf(t - 1)], LT::phase(t - 1), abort_flag, args.status, 14)) { ok = false; break; }
@@ -319,10 +319,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
             for (int j = 0; j < n_tiles; ++j, ++t) {
                 const int slot = int(t % LT::kStages);
                 const uint32_t v_addr = v_base + slot * LT::kTileBytes;
-                const uint32_t p_tmem = warp_uniform(tmem + LT::p_col(t));
-                const uint32_t o_tmem = warp_uniform(tmem + LT::o_col(t));
+                const uint32_t p_tmem = tmem + LT::p_col(t);
+                const uint32_t o_tmem = tmem + LT::o_col(t);
                 const uint32_t block_stride = LT::kSumOnTensor ? ones_addr - v_addr : uint32_t(kTileKeys * 128);
-                const uint64_t v_desc = warp_uniform(smem_desc(v_addr, block_stride));
+                const uint64_t v_desc = smem_desc(v_addr, block_stride);
                 if (!mbar_wait(&bars->p_full[LT::buf(t)], LT::phase(t), abort_flag, args.status, 5)) { ok = false; break; }
                 if (!mbar_wait(&bars->v_full[slot], (t / LT::kStages) & 1, abort_flag, args.status, 6)) { ok = false; break; }
                 if (t >= LT::kOBufs && !mbar_wait(&bars->o_free[LT::o_buf(t)], LT::o_phase(t - LT::kOBufs), abort_flag, args.status, 7)) { ok = false; break; }
