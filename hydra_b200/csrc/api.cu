@@ -214,9 +214,6 @@ bool use_tensor_path(const hc_attn_params* p, const AttnShape& shape, hc_status*
     return ok;
 }
 
-// The body shared by hc_attention_prefill and hc_attention_prefill_partial.
-// With k_fused / v_fused set (hc_layer_step; one pass, tokens <= the prologue workspace) the K/V
-// append of the same tokens rides in the Q prologue's launch.
 // Paged storage: every 128-key tile of [first, first + tokens) of `seq` gets a page (all layers share
 // the table, so whichever layer appends a position first assigns it), and the new entries are copied
 // to the device table on `stream`, ahead of the kernel that writes the rows.
@@ -254,6 +251,9 @@ void release_pages(hc_kv_cache* cache, int seq, int first_tile) {
     }
 }
 
+// The body shared by hc_attention_prefill and hc_attention_prefill_partial.  With k_fused / v_fused set
+// (hc_layer_step, tokens <= the prologue workspace) the K/V append of the same tokens rides in the Q
+// prologue's launch, pass by pass: one pass, but with bidirectional blocks, which go chunk by chunk.
 // `most_in_ring`: how many tokens a ring layer may take at once (its margin by default).
 hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, const void* q,
                        void* out, int tokens, int first_position, const hc_attn_params* p,
@@ -297,7 +297,9 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
             uint16_t* prepared = cache->ws.qprep;
             if (prep) fill_q_job(args.job[jobs++], p, q_rows, prepared);
             if (k_fused) {
-                fill_kv_jobs(args, jobs, p, k_fused, v_fused);
+                const size_t kv_row = size_t(p->kv_heads) * d;
+                fill_kv_jobs(args, jobs, p, offset_rows(k_fused, size_t(start), kv_row, p->io_dtype),
+                             offset_rows(v_fused, size_t(start), kv_row, p->io_dtype));
                 jobs += 2;
             }
             args.n_jobs = jobs;

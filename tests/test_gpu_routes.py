@@ -1,0 +1,60 @@
+"""Calls that take another way through the library than the one they are usually made in: each has to give what the
+plain sequence of calls gives, bit for bit, or what the oracle gives."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from oracle import hydra_oracle as ho
+from tests import hydra_testlib as tl
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def hb():
+    import hydra_b200
+    return hydra_b200
+
+
+@pytest.fixture(scope="module")
+def ctx(hb):
+    c = hb.Context(0)
+    yield c
+    c.close()
+
+
+def _inputs(seed, tokens, qh, kvh, d):
+    rng = np.random.default_rng(seed)
+    return [tl.normal_bf16(rng, (tokens, h, d)) for h in (qh, kvh, kvh)]
+
+
+@pytest.mark.parametrize("call", ["layer_step", "prefill_chunks"])
+@pytest.mark.parametrize("d, rope", [(64, False), (256, True)])
+def test_blocks_in_a_call_of_several_cache_chunks(hb, ctx, call, d, rope):
+    """With bidirectional blocks a call is worked in chunks of the cache's prefill_chunk: the keys and values that are
+    appended with a later chunk's queries are that chunk's own rows."""
+    import torch
+    qh, kvh, tokens, chunk = 8, 2, 300, 128
+    q, k, v = _inputs(d, tokens, qh, kvh, d)
+    ends = np.zeros(tokens, np.int32)
+    ends[20:90], ends[140:200] = 90, 200
+    outs, rows = [], []
+    for fused in (False, True):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 1024, prefill_chunk=chunk,
+                         rope_inv_freq=ho.inverse_frequencies(d, 10000.0) if rope else None)
+        params = dataclasses.replace(layer.params, block_ends=torch.from_numpy(ends).cuda())
+        qd, kd, vd, out = tl.to_device(q), tl.to_device(k), tl.to_device(v), tl.device_empty((tokens, qh, d))
+        if not fused:
+            layer.backend.write_key_value(layer.cache, 0, kd, vd, tokens, 0, layer.params)
+            layer.backend.attention_prefill(layer.cache, 0, qd, out, tokens, 0, params)
+        elif call == "layer_step":
+            layer.backend.layer_step(layer.cache, 0, qd, kd, vd, out, tokens, 0, params)
+        else:
+            layer.backend.prefill_chunks(layer.cache, 0, qd, kd, vd, out, tokens, 0, tokens, params)
+        ctx.check()
+        outs.append(tl.to_host(out))
+        rows.append(tl.read_cache(layer.cache, 0, tokens, kvh, d))
+        layer.close()
+    assert np.array_equal(rows[0][0], rows[1][0]) and np.array_equal(rows[0][1], rows[1][1])
+    assert np.array_equal(outs[0], outs[1])
