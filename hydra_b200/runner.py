@@ -21,13 +21,16 @@ comes from torch; nothing here computes.
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
 import numpy as np
 
 from . import capi
-from .backend import AttentionBackend, AttnParams, Context, KVCache, RopeTable, _check
+from .backend import AttentionBackend, AttnParams, Context, KVCache, RopeTable, _check, _ptr
+
+_WEIGHTS = ("input_norm", "wq", "bq", "wk", "bk", "wv", "bv", "wo", "bo")       # as hc_block_weights has them
 
 
 @dataclass
@@ -72,7 +75,7 @@ class AttentionStackRunner:
 
         self.weights, self.tables, self.params = [], [], []
         for w in layers:
-            t = {name: dev(getattr(w, name)) for name in ("input_norm", "wq", "bq", "wk", "bk", "wv", "bv", "wo", "bo")}
+            t = {name: dev(getattr(w, name)) for name in _WEIGHTS}
             t["sinks"] = dev(w.sinks) if w.sinks is not None else None
             self.weights.append(t)
             table = RopeTable(ctx, list(w.inv_freq), context_length, w.rope_concentration) if w.inv_freq is not None else None
@@ -81,13 +84,12 @@ class AttentionStackRunner:
                                           sm_scale=1.0 / np.sqrt(head_dim), io_dtype=capi.HC_BF16, sinks=t["sinks"],
                                           rope=table))
 
-        # What a call needs besides the hidden states, laid out once: the layers' pointers and parameters, the
+        # What a call needs besides the hidden states: the C structs of the layers (filled on every pass), the
         # device workspace, and pinned host buffers (a copy from or to pageable memory is two).
         self._blocks = (capi.BlockWeightsStruct * len(layers))()
-        for block, t, params in zip(self._blocks, self.weights, self.params):
-            for name in ("input_norm", "wq", "bq", "wk", "bk", "wv", "bv", "wo", "bo"):
-                setattr(block, name, t[name].data_ptr())
-            block.params = params.struct()
+        # A block begins with the nine weight pointers; as one array they are stored by one assignment.
+        self._parts = [(block, (ctypes.c_void_p * len(_WEIGHTS)).from_buffer(block)) for block in self._blocks]
+        self._fill_blocks()
         self._lib = capi.load()
         chunk = self.prefill_chunk_tokens
         need = self._lib.hc_attention_stack_bytes(self._blocks, len(layers), chunk, hidden)
@@ -110,11 +112,21 @@ class AttentionStackRunner:
         self.kv_cache.reset()
 
     # -- the passes -------------------------------------------------------------------------------
+    def _fill_blocks(self) -> None:
+        """The layers' weights and parameters as they are now: a program may have put other tensors in the lists."""
+        for (block, pointers), t, params in zip(self._parts, self.weights, self.params):
+            try:
+                pointers[:] = [t[name].data_ptr() for name in _WEIGHTS]
+            except AttributeError:                             # no bias, or a plain address
+                pointers[:] = [_ptr(t[name]) for name in _WEIGHTS]
+            block.params = params.struct()
+
     def _layers(self, tokens: int, first_position: int) -> None:
         """`tokens` hidden states from the first pinned buffer through every layer's attention block to the second."""
+        self._fill_blocks()
         _check(self._lib.hc_attention_stack_host(
-            self.ctx.handle, self.kv_cache.handle, self._blocks, len(self._blocks), 0, self._host[0].ctypes.data,
-            self._host[1].ctypes.data, tokens, self.hidden, first_position, self.eps, self._workspace.data_ptr(), None))
+            self.ctx.handle, self.kv_cache.handle, self._blocks, len(self._parts), 0, self._pinned[0].data_ptr(),
+            self._pinned[1].data_ptr(), tokens, self.hidden, first_position, self.eps, self._workspace.data_ptr(), None))
 
     def prefill(self, hidden_states: np.ndarray) -> np.ndarray:
         """A prompt's hidden states [tokens][hidden] in chunks, each chunk through every layer before

@@ -58,3 +58,46 @@ def test_blocks_in_a_call_of_several_cache_chunks(hb, ctx, call, d, rope):
         layer.close()
     assert np.array_equal(rows[0][0], rows[1][0]) and np.array_equal(rows[0][1], rows[1][1])
     assert np.array_equal(outs[0], outs[1])
+
+
+def test_runner_reads_its_weights_where_they_are_now(hb, ctx):
+    """A program may put other tensors, sinks or parameters in a runner's lists between passes: what a pass reads is
+    what they hold then."""
+    from hydra_b200.runner import AttentionLayerWeights, AttentionStackRunner
+    rng = np.random.default_rng(3)
+    width, qh, kvh, d, tokens = 128, 4, 2, 64, 9
+    shapes = dict(wq=(qh * d, width), bq=(qh * d,), wk=(kvh * d, width), bk=(kvh * d,), wv=(kvh * d, width),
+                  bv=(kvh * d,), wo=(width, qh * d), bo=(width,))
+
+    def layer():
+        weights = {name: ho.bf16_round(rng.normal(0, 0.1, shape)) for name, shape in shapes.items()}
+        return AttentionLayerWeights(input_norm=ho.bf16_round(1 + 0.1 * rng.standard_normal(width)), window=0,
+                                     sinks=tl.normal_bf16(rng, (qh,)), **weights)
+
+    def runner(layers):
+        return AttentionStackRunner(ctx, layers, width, qh, kvh, d, context_length=256, prefill_chunk_tokens=128)
+
+    states = rng.standard_normal((tokens, width)).astype(np.float32)
+    first, second = [layer(), layer()], [layer(), layer()]
+    changed, fresh = runner(first), runner(second)
+    before = changed.verify(states)
+    kept = list(changed.weights)                 # (the old tensors stay alive: nothing here reads freed memory)
+    for index in range(2):
+        changed.weights[index] = dict(fresh.weights[index])
+        changed.params[index].sinks = fresh.weights[index]["sinks"]
+    changed.reset()
+    got, want = changed.verify(states), fresh.verify(states)
+    assert not np.array_equal(before, want) and len(kept) == 2
+    assert np.array_equal(got, want)
+    changed.params[1].sm_scale = 0.5
+    changed.reset()
+    assert not np.array_equal(changed.verify(states), want)
+    changed.params[1].sm_scale = fresh.params[1].sm_scale
+    for weights in (changed.weights[0], fresh.weights[0]):
+        weights["bk"] = None                     # a projection without a bias
+    changed.reset()
+    fresh.reset()
+    without = changed.verify(states)
+    assert np.array_equal(without, fresh.verify(states)) and not np.array_equal(without, want)
+    changed.close()
+    fresh.close()
