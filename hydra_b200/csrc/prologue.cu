@@ -328,8 +328,9 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
     }
     if (vector_ok) {
         const int per_warp = d >= 256 ? 1 : 256 / d;
-        const long long groups = (long long)args.tokens * ((total_heads + per_warp - 1) / per_warp);
-        const int grid = int(std::min<long long>((groups + kPrepWarps - 1) / kPrepWarps, cap));
+        const long long head_groups = (total_heads + per_warp - 1) / per_warp, groups = args.tokens * head_groups;
+        // (A warp stays with its heads, so there are never fewer warps than a token has groups of them.)
+        const int grid = int((std::max(std::min(groups, cap * kPrepWarps), head_groups) + kPrepWarps - 1) / kPrepWarps);
         auto kernel = d == 64 ? prepare_heads_vec_kernel<64> : d == 128 ? prepare_heads_vec_kernel<128>
                     : d == 256 ? prepare_heads_vec_kernel<256> : prepare_heads_vec_kernel<512>;
         launch_pdl(kernel, grid, kPrepWarps * 32, 0, stream, args, total_heads);

@@ -101,3 +101,28 @@ def test_runner_reads_its_weights_where_they_are_now(hb, ctx):
     assert np.array_equal(without, fresh.verify(states)) and not np.array_equal(without, want)
     changed.close()
     fresh.close()
+
+
+@pytest.mark.parametrize("d, heads", [(64, 80000), (256, 20000), (512, 19000)])
+def test_one_token_of_very_many_heads(hb, ctx, d, heads):
+    """The element-wise entry points take the rows of a matrix as one token's heads: more of them than the launch has
+    warps."""
+    import torch
+    be = hb.AttentionBackend(ctx)
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    x = torch.randn((heads, d), device="cuda", generator=gen)
+    weight = torch.randn(d, device="cuda", generator=gen).to(torch.bfloat16)
+    table = hb.RopeTable(ctx, list(ho.inverse_frequencies(d, 10000.0)), 8)
+    rows, one = x.clone(), x.clone()
+    be.rms_norm_heads(rows, weight, heads, 1, d, 1e-6, hb.capi.HC_F32)
+    be.rms_norm_heads(one, weight, 1, heads, d, 1e-6, hb.capi.HC_F32)
+    ctx.check()
+    assert torch.equal(rows, one) and not torch.equal(rows, x)
+    parts, one = x.clone(), x.clone()
+    for start in range(0, heads, 5000):
+        count = min(5000, heads - start)
+        be.apply_rope(parts[start:start + count], table, 1, count, d, 5, hb.capi.HC_F32)
+    be.apply_rope(one, table, 1, heads, d, 5, hb.capi.HC_F32)
+    ctx.check()
+    assert torch.equal(parts, one) and not torch.equal(parts, x)
+    table.close()
