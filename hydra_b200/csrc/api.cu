@@ -1454,7 +1454,8 @@ static hc_status host_pieces(hc_context* ctx, hc_kv_cache* cache, int layer, int
         return check_positions(cache, L, first_position, std::min(chunk, tokens), params);
     }
     int most = int(std::min<size_t>((slot_bytes - 5 * 256) / piece_row, size_t(tokens)));
-    if (L.ring > 0) most = std::min(most, std::max(L.ring - L.desc.window, std::min(chunk, tokens)));
+    // (A piece beyond the prepared-query buffer is appended by a call of its own, which takes the ring's margin at most.)
+    if (L.ring > 0) most = std::min(most, std::max(std::min(L.ring - L.desc.window, cache->ws.qprep_capacity), std::min(chunk, tokens)));
     if (params->block_ends) most = chunk;
     const int quantum = int(((size_t(2) << 20) / q_row / kTileKeys + 1) * kTileKeys);
     auto end_of = [&](int start) {

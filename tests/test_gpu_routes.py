@@ -126,3 +126,28 @@ def test_one_token_of_very_many_heads(hb, ctx, d, heads):
     ctx.check()
     assert torch.equal(parts, one) and not torch.equal(parts, x)
     table.close()
+
+
+@pytest.mark.parametrize("context, chunk, tokens", [(200, 64, 2000), (4096, 64, 700)])
+def test_host_prompt_on_a_ring(hb, ctx, context, chunk, tokens):
+    """A ring takes prompts longer than the context the cache was made for; the pieces of a host prompt are as long as
+    both the ring and the prepared-query buffer allow."""
+    import torch
+    qh, kvh, d, window = 8, 2, 64, 128
+    q, k, v = _inputs(tokens, tokens, qh, kvh, d)
+    outs = []
+    for on_host in (False, True):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, context, window=window, storage=hb.capi.HC_STORAGE_RING, prefill_chunk=chunk)
+        if on_host:
+            host = [torch.from_numpy(a).to(torch.bfloat16).pin_memory() for a in (q, k, v)]
+            out = torch.zeros((tokens, qh, d), dtype=torch.bfloat16).pin_memory()
+            layer.backend.prefill_host(layer.cache, 0, *host, out, tokens, 0, chunk, layer.params)
+        else:
+            qd, kd, vd, out = tl.to_device(q), tl.to_device(k), tl.to_device(v), tl.device_empty((tokens, qh, d))
+            for at in range(0, tokens, chunk):
+                n = min(chunk, tokens - at)
+                layer.backend.layer_step(layer.cache, 0, qd[at:], kd[at:], vd[at:], out[at:], n, at, layer.params)
+        ctx.check()
+        outs.append(tl.to_host(out))
+        layer.close()
+    assert np.array_equal(outs[0], outs[1])
