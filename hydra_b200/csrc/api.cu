@@ -108,6 +108,9 @@ bool needs_q_prepare(const hc_attn_params* p) {
            p->gate_layout == HC_GATE_INTERLEAVED;
 }
 
+// What aligning the five parts of a staging slot to 256 bytes may cost.
+constexpr size_t kStageSlack = 5 * 256;
+
 // Rows a position range needs; checks capacity the way KVCache.advance does (KVCache.swift:202-213).
 hc_status check_positions(const hc_kv_cache* cache, const hc_layer_store& L, int first, int tokens,
                           const hc_attn_params* p, int most_in_ring = -1) {
@@ -795,8 +798,8 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         // Prepared queries: a call's, up to 64 MB of them, so that a prompt is one prologue and one attention launch.
         ws.qprep_capacity = std::max(ws.qprep_tokens, int(std::min<size_t>((size_t(32) << 20) / max_q_elems, size_t(context_length))));
         // Staging for the host-buffer entry points, two slots: q (twice as wide when the gate is
-        // interleaved), gate, out, k, v.
-        cache->stage_bytes = (size_t(ws.qprep_tokens) * (4 * max_q_elems + 2 * max_kv_elems) * 4 + 1023) & ~size_t(1023);
+        // interleaved), gate, out, k, v, each on a 256-byte boundary.
+        cache->stage_bytes = (size_t(ws.qprep_tokens) * (4 * max_q_elems + 2 * max_kv_elems) * 4 + kStageSlack + 1023) & ~size_t(1023);
         ws.n_tickets = n_tickets;
         // All of it in one allocation, each part on a 1 KB boundary.
         auto align = [](size_t x) { return (x + 1023) & ~size_t(1023); };
@@ -1443,17 +1446,17 @@ static hc_status host_pieces(hc_context* ctx, hc_kv_cache* cache, int layer, int
     const size_t g_row = sep_gate ? o_row : 0;
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t kv_all = align(kv_row * tokens);
-    const size_t least = 5 * 256 + (q_row + g_row + o_row) * std::min(chunk, tokens);
+    const size_t least = kStageSlack + (q_row + g_row + o_row) * std::min(chunk, tokens);
     const bool kv_ahead = kv_all <= cache->stage_bytes / 2 && cache->stage_bytes - kv_all >= least + 256;
     const size_t slots_at = kv_ahead ? 2 * kv_all : 0;
     const size_t slot_bytes = (cache->stage_bytes - slots_at / 2) & ~size_t(255);
     const size_t piece_row = q_row + g_row + o_row + (kv_ahead ? 0 : 2 * kv_row);
-    if (slot_bytes < 5 * 256 + piece_row * std::min(chunk, tokens)) return fail(HC_KV_OVERFLOW, "staging buffer too small for this chunk");
+    if (slot_bytes < kStageSlack + piece_row * std::min(chunk, tokens)) return fail(HC_KV_OVERFLOW, "staging buffer too small for this chunk");
     const hc_layer_store& L = cache->layers[size_t(layer)];
     if (L.ring > 0 && std::min(chunk, tokens) > L.ring_margin) {
         return check_positions(cache, L, first_position, std::min(chunk, tokens), params);
     }
-    int most = int(std::min<size_t>((slot_bytes - 5 * 256) / piece_row, size_t(tokens)));
+    int most = int(std::min<size_t>((slot_bytes - kStageSlack) / piece_row, size_t(tokens)));
     // (A piece beyond the prepared-query buffer is appended by a call of its own, which takes the ring's margin at most.)
     if (L.ring > 0) most = std::min(most, std::max(std::min(L.ring - L.desc.window, cache->ws.qprep_capacity), std::min(chunk, tokens)));
     if (params->block_ends) most = chunk;

@@ -151,3 +151,23 @@ def test_host_prompt_on_a_ring(hb, ctx, context, chunk, tokens):
         outs.append(tl.to_host(out))
         layer.close()
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("qh, d, io", [(1, 8, "bf16"), (1, 64, "f32"), (2, 64, "bf16")])
+def test_host_step_of_the_smallest_caches(hb, ctx, qh, d, io):
+    """The staging buffer holds a chunk of the cache's own size whatever that is."""
+    import torch
+    rng = np.random.default_rng(d)
+    layer = tl.Layer(hb, ctx, qh, 1, d, 256, prefill_chunk=1, io=io)
+    dtype = torch.bfloat16 if io == "bf16" else torch.float32
+    k_rows, v_rows = [], []
+    for position in range(3):
+        q, k, v = (tl.normal_bf16(rng, (1, h, d)) for h in (qh, 1, 1))
+        k_rows.append(k)
+        v_rows.append(v)
+        out = torch.zeros((1, qh, d), dtype=dtype)
+        host = [torch.from_numpy(a).to(dtype) for a in (q, k, v)]
+        layer.backend.layer_step_host(layer.cache, 0, *host, out, 1, position, layer.params)
+        want = ho.attention_rows(q, np.asarray([position]), np.concatenate(k_rows), np.concatenate(v_rows), 1 / np.sqrt(d))
+        assert tl.within_tolerance(tl.to_host(out), want, bf16_output=io == "bf16")
+    layer.close()
