@@ -365,24 +365,23 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
     const int d = p->head_dim;
     const int mult = p->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
     const bool prep = needs_q_prepare(p);
-    // A launch takes as many sequences as the prepared-query buffer has rows for.
-    // (The tcgen05 decode kernel lists its rows, 512 of them at most, in shared memory.)
-    int per_launch = prep ? std::min(kMaxBatch, cache->ws.qprep_tokens) : kMaxBatch;
-    // The workspace holds any cut of max_seqs rows; more, some of the same sequence, go in several launches.
-    if (tensor) per_launch = std::max(1, std::min({per_launch, 512 / p->kv_heads, cache->max_seqs}));
-
-    for (int start = 0; start < n_seq; start += per_launch) {
-        const int count = std::min(per_launch, n_seq - start);
-        BatchMeta meta{};
-        for (int b = 0; b < count; ++b) {
-            meta.seq[b] = seq_ids[start + b];
-            meta.pos[b] = positions[start + b];
-        }
+    for (int start = 0, served = 0; start < n_seq; start += served) {
+        // As many rows as a launch takes: on the tensor cores what tc_decode says, elsewhere what the prepared-query buffer
+        // has room for.
+        int count = std::min(kMaxBatch, n_seq - start);
         const unsigned char* q_rows = offset_rows(q, size_t(start), size_t(p->q_heads) * d * mult, p->io_dtype);
         const uint16_t* q_bf16 = reinterpret_cast<const uint16_t*>(q_rows);
         const size_t kv_row = size_t(p->kv_heads) * d;
         const void* k_rows = k_fused ? offset_rows(k_fused, size_t(start), kv_row, p->io_dtype) : nullptr;
         const void* v_rows = k_fused ? offset_rows(v_fused, size_t(start), kv_row, p->io_dtype) : nullptr;
+        const bool in_kernel = tensor && decode_takes_raw(p, q_rows, k_rows, v_rows);
+        if (prep && !in_kernel) count = std::min(count, cache->ws.qprep_tokens);
+        served = count;
+        BatchMeta meta{};
+        for (int b = 0; b < count; ++b) {
+            meta.seq[b] = seq_ids[start + b];
+            meta.pos[b] = positions[start + b];
+        }
         if (k_fused) {
             for (int b = 0; b < count; ++b) {
                 st = ensure_pages(cache, L, meta.seq[b], meta.pos[b], 1, stream);
@@ -392,7 +391,6 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
         DecodeSource src{};
         src.dtype = HC_BF16;
         src.q_head_stride = d;
-        const bool in_kernel = tensor && decode_takes_raw(p, q_rows, k_rows, v_rows);
         if (in_kernel) {
             src = raw_source(p, q_rows, k_rows, v_rows);
         } else if (prep || k_fused) {
@@ -428,7 +426,7 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
             ep.gate = q_rows;
         }
         if (!in_kernel) src.q = q_bf16;
-        if (tensor) st = tc_decode(ctx, shape, L, view, meta, count, src, cache->ws, ep, stream);
+        if (tensor) st = tc_decode(ctx, shape, L, view, meta, count, src, cache->ws, ep, stream, &served);
         else st = simt_decode(ctx, shape, view, meta, count, q_bf16, cache->ws, ep, stream);
         if (st != HC_OK) return st;
     }
@@ -768,7 +766,13 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         const size_t decode_rows = size_t(std::min(max_seqs, kMaxBatch)) * L.desc.q_heads;
         part_o_floats = std::max(part_o_floats, decode_rows * decode_slots * d);
         part_ml_floats = std::max(part_ml_floats, decode_rows * decode_slots * 2 + 4);
-        n_tickets = std::max(n_tickets, size_t(std::min(max_seqs, kMaxBatch)) * L.desc.kv_heads * 16);
+        n_tickets = std::max(n_tickets, size_t(kMaxBatch) * L.desc.kv_heads * 16);
+        // A launch may have more rows than the cache has sequences (several positions of one): room for the segment partials
+        // of a full one, 32 MB at most, beyond which it goes in parts.
+        const size_t decode_segments = size_t((((decode_reach + kTileKeys - 1) / kTileKeys) >> L.log_segment) + 2);
+        const size_t most_parts = std::min(size_t(kMaxBatch) * L.desc.q_heads * decode_segments, (size_t(8) << 20) / d);
+        part_o_floats = std::max(part_o_floats, most_parts * d);
+        part_ml_floats = std::max(part_ml_floats, most_parts * 2 + 4);
         if (few_rows || pairs) {
             const size_t prefill_slots = size_t((((reach + kTileKeys - 1) / kTileKeys) >> kLogSegmentSmall) + 2);
             const size_t prefill_rows = size_t(prefill_chunk) * L.desc.q_heads;

@@ -129,7 +129,7 @@ struct DecItem {
 };
 
 // b with start[b] <= index < start[b + 1]
-__device__ __forceinline__ int dec_search(const DecArgs& args, int index) {
+__host__ __device__ __forceinline__ int dec_search(const DecArgs& args, int index) {
     int lo = 0, hi = args.n_seq;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -138,17 +138,17 @@ __device__ __forceinline__ int dec_search(const DecArgs& args, int index) {
     return lo;
 }
 
-// Where thread block c's stretch of the line begins: a row and a tile of it, the equal share's end moved to the nearest
-// segment boundary.
+// Where the stretch of the line begins that block c of `blocks` takes: a row and a tile of it, the equal share's end moved to
+// the nearest segment boundary.  (The host asks too, for the rows that the longest list holds.)
 struct DecPlace {
     int row, t;
 };
-__device__ __forceinline__ DecPlace dec_place(const DecArgs& args, int c) {
+__host__ __device__ __forceinline__ DecPlace dec_place(const DecArgs& args, int c, int blocks) {
     DecPlace p;
     p.row = args.n_seq * args.cache.kv_heads;
     p.t = 0;
-    if (c >= int(gridDim.x)) return p;
-    const int at = int((long long)c * args.n_tiles / int(gridDim.x));
+    if (c >= blocks) return p;
+    const int at = int((long long)c * args.n_tiles / blocks);
     const int b = dec_search(args, at);
     const int world = args.cache.map.world > 1 ? args.cache.map.world : 1;
     const int log_segment = args.cache.map.log_segment;
@@ -158,7 +158,8 @@ __device__ __forceinline__ DecPlace dec_place(const DecArgs& args, int c) {
     const int t = at - args.start[b] - head * row.count;
     const int segment_tile = ((row.first + t * world) >> log_segment) << log_segment;
     const int before = segment_tile <= row.first ? 0 : (segment_tile - row.first + world - 1) / world;
-    const int after = min(row.count, (segment_tile + (1 << log_segment) - row.first + world - 1) / world);
+    const int next = (segment_tile + (1 << log_segment) - row.first + world - 1) / world;
+    const int after = next < row.count ? next : row.count;
     p.row = b * args.cache.kv_heads + head;
     p.t = t - before <= after - t ? before : after;
     if (p.t == row.count) {
@@ -166,6 +167,10 @@ __device__ __forceinline__ DecPlace dec_place(const DecArgs& args, int c) {
         ++p.row;
     }
     return p;
+}
+// The list of the block that starts at `from` and ends at `to`.
+__host__ __device__ __forceinline__ int dec_items(const DecPlace& from, const DecPlace& to) {
+    return to.row - from.row + (to.t > 0 ? 1 : 0);
 }
 
 // A thread block's items, worked out once by all its threads side by side (finding an item takes a search and
@@ -219,8 +224,8 @@ __device__ __forceinline__ void dec_list_build(const DecArgs& args, DecList* lis
         list->span_tiles = max(tiles.count, 0);
         return;
     }
-    const DecPlace from = dec_place(args, int(blockIdx.x)), to = dec_place(args, int(blockIdx.x) + 1);
-    const int count = min(to.row - from.row + (to.t > 0 ? 1 : 0), kDecItems);
+    const DecPlace from = dec_place(args, int(blockIdx.x), int(gridDim.x)), to = dec_place(args, int(blockIdx.x) + 1, int(gridDim.x));
+    const int count = min(dec_items(from, to), kDecItems);
     if (threadIdx.x == 0) list->count = count;
     for (int i = threadIdx.x; i < count; i += kTcThreads) {
         DecItem w;
@@ -1463,15 +1468,53 @@ TcDecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const
     return plan;
 }
 
+// A launch's arguments as far as they follow from its rows: where the rows lie on the line, or in clusters.
+static long long dec_lay_out(DecArgs& args, const TcDecodePlan& plan, const BatchMeta& meta, int n_seq, const AttnShape& shape) {
+    args.n_seq = n_seq;
+    args.cluster = plan.cluster;
+    args.slots = plan.slots;
+    args.meta = meta;
+    long long next = 0;
+    for (int b = 0; b < n_seq; ++b) {
+        args.start[b] = int(std::min(next, 0x7fffffffLL));
+        if (plan.cluster == 1) {
+            next += (long long)std::max(row_tiles(args.cache.map, meta.pos[b], meta.pos[b], shape.window).count, 0) * shape.kv_heads;
+        } else {
+            // Spans of one size, plan.run_segments each at most.
+            const int segments = visible_groups(meta.pos[b], meta.pos[b], shape.window, args.cache.map.log_segment);
+            const int want = (segments + plan.run_segments - 1) / plan.run_segments;
+            const int run = (segments + want - 1) / want;
+            args.seq_run[b] = static_cast<unsigned short>(run);
+            args.seq_spans[b] = static_cast<unsigned short>((segments + run - 1) / run);
+            next += (long long)args.seq_spans[b] * shape.kv_heads;
+        }
+    }
+    for (int b = n_seq; b <= kMaxBatch; ++b) args.start[b] = int(std::min(next, 0x7fffffffLL));
+    args.n_tiles = args.start[n_seq];
+    return next;
+}
+
+// Whether the longest of the blocks' lists has room in shared memory.
+static bool dec_lists_fit(const DecArgs& args, int blocks, const AttnShape& shape) {
+    // (Most launches: no more rows than a list holds, or no more tiles to a stretch, where every row has one.)
+    const long long rows = (long long)args.n_seq * shape.kv_heads;
+    if (args.cluster > 1 || rows <= kDecItems) return true;
+    if (args.cache.map.world <= 1 && args.n_tiles / blocks + 2 * (1 << args.cache.map.log_segment) + 2 <= kDecItems) return true;
+    DecPlace from = dec_place(args, 0, blocks);
+    for (int c = 0; c < blocks; ++c) {
+        const DecPlace to = dec_place(args, c + 1, blocks);
+        if (dec_items(from, to) > kDecItems) return false;
+        from = to;
+    }
+    return true;
+}
+
 hc_status tc_decode(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
                     const BatchMeta& meta, int n_seq, const DecodeSource& src, const Workspace& ws, const EpilogueArgs& ep,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, int* served) {
+    *served = 0;
     if (!layer.tmap_k || !layer.tmap_v) return fail(HC_UNSUPPORTED, "this layer has no tensor maps");
     if (n_seq <= 0) return HC_OK;
-    const TcDecodePlan plan = tc_plan_decode(ctx, shape, cache.map, meta, n_seq);
-    if (plan.part_o_floats > ws.part_o_floats || plan.part_ml_floats > ws.part_ml_floats || plan.tickets > ws.n_tickets) {
-        return fail(HC_KV_OVERFLOW, "decode: the split-attention workspace is too small for this call");
-    }
     DecArgs args{};
     args.q = src.q;
     args.k_new = src.k;
@@ -1496,37 +1539,23 @@ hc_status tc_decode(hc_context* ctx, const AttnShape& shape, const hc_layer_stor
     args.count_sink = shape.count_sink;
     args.ep = ep;
     args.status = ctx->status_dev;
-    args.n_seq = n_seq;
-    args.cluster = plan.cluster;
-    args.slots = plan.slots;
     args.part_o = ws.part_o;
     args.part_ml = ws.part_ml;
     args.tickets = ws.tickets;
-    args.meta = meta;
-    long long next = 0;
-    for (int b = 0; b < n_seq; ++b) {
-        args.start[b] = int(next);
-        if (plan.cluster == 1) {
-            next += (long long)std::max(row_tiles(cache.map, meta.pos[b], meta.pos[b], shape.window).count, 0) * shape.kv_heads;
-        } else {
-            // Spans of one size, plan.run_segments each at most.
-            const int segments = visible_groups(meta.pos[b], meta.pos[b], shape.window, cache.map.log_segment);
-            const int want = (segments + plan.run_segments - 1) / plan.run_segments;
-            const int run = (segments + want - 1) / want;
-            args.seq_run[b] = static_cast<unsigned short>(run);
-            args.seq_spans[b] = static_cast<unsigned short>((segments + run - 1) / run);
-            next += (long long)args.seq_spans[b] * shape.kv_heads;
-        }
+    // As many of the rows as the workspace has partials for and the blocks' lists hold: all of them, but for many rows
+    // of a cache that was made for few sequences, or for thousands of short ones.
+    TcDecodePlan plan{};
+    for (;; n_seq = (n_seq + 1) / 2) {
+        plan = tc_plan_decode(ctx, shape, cache.map, meta, n_seq);
+        const bool room = plan.part_o_floats <= ws.part_o_floats && plan.part_ml_floats <= ws.part_ml_floats && plan.tickets <= ws.n_tickets;
+        if (!room && n_seq == 1) return fail(HC_KV_OVERFLOW, "decode: the split-attention workspace is too small for this call");
+        if (!room) continue;
+        const long long tiles = dec_lay_out(args, plan, meta, n_seq, shape);
+        if (tiles <= 0x7fffffffLL && dec_lists_fit(args, plan.blocks, shape)) break;
+        if (n_seq == 1) return fail(HC_UNSUPPORTED, "decode: too many key tiles or rows for one launch");
     }
-    for (int b = n_seq; b <= kMaxBatch; ++b) args.start[b] = int(next);
-    args.n_tiles = int(next);
+    *served = n_seq;
     const int grid = plan.blocks;
-    // A thread block's stretch of the line touches no more rows than it has tiles, nor more than there are.
-    const long long rows = (long long)n_seq * shape.kv_heads;
-    const long long stretch = next / grid + 2 * (1 << cache.map.log_segment) + 2;
-    if (next > 0x7fffffffLL || (plan.cluster == 1 && std::min(rows, stretch) > kDecItems)) {
-        return fail(HC_UNSUPPORTED, "decode: too many key tiles or rows for one launch");
-    }
     switch (shape.head_dim) {
         case 64: return launch_decode_dim<64>(ctx, args, grid, layer, stream);
         case 128: return launch_decode_dim<128>(ctx, args, grid, layer, stream);

@@ -901,7 +901,10 @@ hc_status hc_attention_decode_static(hc_context* ctx, hc_kv_cache* cache, int la
         src.q = q;
         src.dtype = HC_BF16;
         src.q_head_stride = shape.head_dim;
-        return tc_decode(ctx, shape, *store, view, meta, n_seq, src, ws, ep, static_cast<cudaStream_t>(stream));
+        int served = 0;
+        st = tc_decode(ctx, shape, *store, view, meta, n_seq, src, ws, ep, static_cast<cudaStream_t>(stream), &served);
+        if (st == HC_OK && served < n_seq) return fail(HC_UNSUPPORTED, "hc_attention_decode_static: too many rows for one launch");
+        return st;
     }
     return simt_decode(ctx, shape, view, meta, n_seq, static_cast<const uint16_t*>(q), ws, ep,
                        static_cast<cudaStream_t>(stream));

@@ -262,9 +262,10 @@ struct TcDecodePlan {
 };
 hc_status decode_cluster_slots(hc_context* ctx);
 TcDecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const RowMap& map, const BatchMeta& meta, int n_seq);
+// One launch, for the first *served of the n_seq rows: as many as it takes (see there); the caller comes back for the rest.
 hc_status tc_decode(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer,
                     const CacheView& cache, const BatchMeta& meta, int n_seq, const DecodeSource& src,
-                    const Workspace& ws, const EpilogueArgs& ep, cudaStream_t stream);
+                    const Workspace& ws, const EpilogueArgs& ep, cudaStream_t stream, int* served);
 // linear_tc.cu
 // n_jobs (1 to 4) projections of the same x in one launch; bias / residual may be null, or hold nulls.
 hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* const* w, const void* const* bias,

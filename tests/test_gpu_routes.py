@@ -171,3 +171,56 @@ def test_host_step_of_the_smallest_caches(hb, ctx, qh, d, io):
         want = ho.attention_rows(q, np.asarray([position]), np.concatenate(k_rows), np.concatenate(v_rows), 1 / np.sqrt(d))
         assert tl.within_tolerance(tl.to_host(out), want, bf16_output=io == "bf16")
     layer.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, rows", [(64, 64, 8, 0, 8), (64, 64, 8, 128, 16), (256, 16, 2, 0, 8),
+                                                      (512, 16, 2, 0, 8), (64, 16, 16, 0, 40)])
+def test_rows_of_one_sequence_in_one_launch(hb, ctx, d, qh, kvh, window, rows):
+    """Several positions of one sequence decoded together: one launch as long as the workspace holds its partials."""
+    tokens = 2100
+    q, k, v = _inputs(d + rows, tokens, qh, kvh, d)
+    layer = tl.Layer(hb, ctx, qh, kvh, d, 4608, window=window)
+    layer.append(k, v, 0)
+    positions = [0, 127, 128, 1023, 1024, 2047, 2048, tokens - 1] + list(range(100, 100 + 40 * (rows - 8), 40))
+    before = ctx.launch_count
+    got = layer.decode(q[positions], positions, seq_ids=[0] * rows)
+    assert ctx.launch_count - before == 1
+    for b in range(rows):
+        alone = layer.decode(q[positions[b]:positions[b] + 1], positions[b:b + 1])
+        assert np.array_equal(alone[0], got[b]), b
+    layer.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, paged", [(64, 64, 8, 0, False), (64, 64, 8, 128, True), (128, 16, 2, 0, True),
+                                                       (256, 16, 2, 0, True), (512, 16, 1, 0, False), (64, 16, 16, 0, False)])
+def test_a_full_batch_is_one_launch(hb, ctx, d, qh, kvh, window, paged):
+    """64 ragged sequences in a cache made for them: one launch cut as one line, long lists of rows a block (1024 rows
+    in the last case), the search over a full table of sequences, segments of 1024 keys."""
+    tokens, n_seq = 2305, 64
+    q, k, v = _inputs(d + kvh, tokens, qh, kvh, d)
+    rng = np.random.default_rng(d)
+    lengths = [1, 128, 129, 1024, 1025, 2048, 2049, tokens] + [int(n) for n in rng.integers(1, 700, n_seq - 8)]
+    pages = sum((n + 127) // 128 for n in lengths) if paged else 0
+    cache = hb.KVCache(ctx, [dict(q_heads=qh, kv_heads=kvh, head_dim=d, window=window)], 2432, max_seqs=n_seq, total_pages=pages)
+    be = hb.AttentionBackend(ctx)
+    params = hb.AttnParams(q_heads=qh, kv_heads=kvh, head_dim=d, window=window, sm_scale=1 / np.sqrt(d), io_dtype=hb.capi.HC_BF16)
+    kd, vd = tl.to_device(k), tl.to_device(v)
+    for seq, n in enumerate(lengths):
+        if n > 1:
+            be.write_key_value(cache, 0, kd, vd, n - 1, 0, params, seq=seq)
+    positions, ids = [n - 1 for n in lengths], list(range(n_seq))
+    be.write_key_value_batch(cache, 0, kd[positions], vd[positions], ids, positions, params)
+    qd, out = tl.to_device(q[positions]), tl.device_empty((n_seq, qh, d))
+    before = ctx.launch_count
+    be.attention(cache, 0, qd, out, positions, params, seq_ids=ids)
+    assert ctx.launch_count - before == 1
+    ctx.check()
+    got = tl.to_host(out)
+    for b in list(range(10)) + [37, 63]:
+        alone = tl.device_empty((1, qh, d))
+        be.attention(cache, 0, qd[b:b + 1], alone, positions[b:b + 1], params, seq_ids=ids[b:b + 1])
+        ctx.check()
+        assert np.array_equal(tl.to_host(alone)[0], got[b]), b
+    want = ho.attention_rows(q[positions], np.asarray(positions), k, v, 1 / np.sqrt(d), window)
+    assert tl.within_tolerance(got, want)
+    cache.close()
