@@ -175,26 +175,35 @@ __host__ __device__ __forceinline__ int dec_items(const DecPlace& from, const De
 
 // A thread block's items, worked out once by all its threads side by side (finding an item takes a search and
 // a few divisions, thousands of clocks for a single thread, and every role needs every item) and packed
-// into eight bytes each.
-constexpr int kDecItems = 512;       // of one thread block, at most
+// into twelve bytes each; a tile's index takes 24 bits, positions being ints.  (Eight bytes, with the first tile worked
+// out from the position again by every reader: batches of 64 long sequences 2 % slower.)
+constexpr int kDecItems = 340;       // of one thread block, at most: what head_dim 256 leaves of shared memory
+struct DecPacked {
+    uint32_t what;                   // sequence, kv head, flags
+    int tile_first, n_tiles;
+};
+static_assert(kMaxBatch <= 64, "the sequence has six bits");
 struct DecList {
-    uint2 packed[kDecItems];
+    DecPacked packed[kDecItems];
     int pos[kMaxBatch], seq[kMaxBatch];
     int count;
     int span_first, span_tiles;      // of the cluster
 };
-__device__ __forceinline__ uint2 dec_pack(const DecItem& w) {
-    return make_uint2(uint32_t(w.b) | (uint32_t(w.kv_head) << 8) | (w.whole ? 0x40000000u : 0u) | (w.last ? 0x80000000u : 0u),
-                      uint32_t(w.tile_first) | (uint32_t(w.n_tiles) << 16));
+__device__ __forceinline__ DecPacked dec_pack(const DecItem& w) {
+    DecPacked p;
+    p.what = uint32_t(w.b) | (uint32_t(w.kv_head) << 6) | (w.whole ? 0x40000000u : 0u) | (w.last ? 0x80000000u : 0u);
+    p.tile_first = w.tile_first;
+    p.n_tiles = w.n_tiles;
+    return p;
 }
-__device__ __forceinline__ DecItem dec_unpack(const uint2& p) {
+__device__ __forceinline__ DecItem dec_unpack(const DecPacked& p) {
     DecItem w;
-    w.b = int(p.x & 0xffu);
-    w.kv_head = int((p.x >> 8) & 0x3fffffu);
-    w.whole = (p.x & 0x40000000u) != 0;
-    w.last = (p.x >> 31) != 0;
-    w.tile_first = int(p.y & 0xffffu);
-    w.n_tiles = int(p.y >> 16);
+    w.b = int(p.what & 0x3fu);
+    w.kv_head = int((p.what >> 6) & 0xffffffu);
+    w.whole = (p.what & 0x40000000u) != 0;
+    w.last = (p.what >> 31) != 0;
+    w.tile_first = p.tile_first;
+    w.n_tiles = p.n_tiles;
     return w;
 }
 __device__ __forceinline__ void dec_list_build(const DecArgs& args, DecList* list) {
@@ -1440,6 +1449,7 @@ TcDecodePlan tc_plan_decode(const hc_context* ctx, const AttnShape& shape, const
                 const int fit = most_span / segment_tiles;
                 if (fit < 1) continue;
                 const int spans = (most_segments + fit - 1) / fit;
+                if (spans > 0xffff) continue;                          // (DecArgs counts a row's spans in 16 bits)
                 run = (most_segments + spans - 1) / spans;
             }
             long long clusters = 0;

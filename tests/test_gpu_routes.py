@@ -224,3 +224,26 @@ def test_a_full_batch_is_one_launch(hb, ctx, d, qh, kvh, window, paged):
     want = ho.attention_rows(q[positions], np.asarray(positions), k, v, 1 / np.sqrt(d), window)
     assert tl.within_tolerance(got, want)
     cache.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window", [(64, 8, 2, 128), (64, 64, 8, 1000), (256, 16, 8, 1024), (512, 8, 1, 300)])
+def test_positions_beyond_eight_million(hb, ctx, d, qh, kvh, window):
+    """A ring takes any position.  Without a rotation the results depend on where the keys lie in their tiles and
+    segments only: far up the sequence they are what they are at its beginning, bit for bit."""
+    rows, batch = window + 140, 12
+    q, k, v = _inputs(d + window, rows, qh, kvh, d)
+    got = []
+    for base in (3 * 4096 + 77, (1 << 23) + 5 * 4096 + 77, (1 << 30) + 77):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 16384, window=window, storage=hb.capi.HC_STORAGE_RING, prefill_chunk=128)
+        for at in range(0, rows, 128):
+            layer.append(k[at:at + 128], v[at:at + 128], base + at)
+        positions = [base + rows - 1 - 3 * b for b in range(batch)]
+        take = [rows - 1 - 3 * b for b in range(batch)]
+        together = layer.decode(q[take], positions, seq_ids=[0] * batch)
+        alone = layer.decode(q[take[:1]], positions[:1])
+        prompt = layer.prefill(q[-9:], base + rows - 9)
+        assert np.array_equal(alone[0], together[0]) and np.array_equal(prompt[-1], alone[0])
+        got.append((together, prompt))
+        layer.close()
+    for other in got[1:]:
+        assert np.array_equal(got[0][0], other[0]) and np.array_equal(got[0][1], other[1])
