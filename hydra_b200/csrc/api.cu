@@ -748,15 +748,19 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         //            sequence of 32768 keys, head_dim 256: 4096-key segments made two waves of clusters
         //            of what is one with 2048).
         const bool pairs = d == 256 || d == 512;               // row tiles of 256 rows on pairs of SMs
-        const int tokens_per_tile = (pairs ? 2 : 1) * kTileKeys / (L.desc.q_heads / L.desc.kv_heads);
+        const int group = L.desc.q_heads / L.desc.kv_heads;
+        const int tokens_per_tile = (pairs ? 2 : 1) * kTileKeys / group;
         const int chunk_row_tiles = (prefill_chunk + tokens_per_tile - 1) / tokens_per_tile;
         const int reach = windowed ? std::min(L.desc.window + prefill_chunk, context_length) : context_length;
         const bool few_rows = 2 * chunk_row_tiles * L.desc.kv_heads * (pairs ? d / 256 : 1) <= std::max(ctx->sm_count, 1) / (pairs ? 2 : 1) &&
                               reach > (2 * kTileKeys << kLogSegmentSmall);
         const bool batched = max_seqs >= 8;
-        L.log_segment_general = few_rows || batched ? kLogSegmentSmall : kLogSegmentLarge;
         // (A whole row of 256 columns pays 6000 clocks, two key tiles, for every segment it spans.)
-        L.log_segment = pairs && !batched ? kLogSegmentWide : L.log_segment_general;
+        L.log_segment = pairs && !batched ? kLogSegmentWide : few_rows || batched ? kLogSegmentSmall : kLogSegmentLarge;
+        // The grouping by row tiles of 128 rows whatever the head_dim, in which hc_attention_decode_static states its limit.
+        const int general_rows = (prefill_chunk + kTileKeys / group - 1) / (kTileKeys / group) * L.desc.kv_heads;
+        const bool general_few = (d == 256 ? 4 : 2) * general_rows <= std::max(ctx->sm_count, 1) && reach > (2 * kTileKeys << kLogSegmentSmall);
+        L.log_segment_general = general_few || batched ? kLogSegmentSmall : kLogSegmentLarge;
         // Workspace for the partials of split launches.  Decode, at its finest cut: one per (batch
         // entry, query head, key tile of this rank).  Prefill, layers with short segments only: one
         // per (query token, query head, segment).

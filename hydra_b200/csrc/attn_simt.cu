@@ -843,6 +843,31 @@ hc_status static_decode_inputs(hc_context* ctx, hc_kv_cache* cache, int layer, c
                                const hc_attn_params* p, AttnShape* shape, CacheView* view, BatchMeta* meta,
                                EpilogueArgs* ep, const hc_layer_store** store, bool* tensor);
 
+// Floats of partials that a call's general cut into tiles and segments leaves (the header puts the limit this way), whichever
+// kernels run and however they cut: a caller's program is not refused by one build and served by the next.
+static size_t static_need(const hc_context* ctx, const AttnShape& shape, const hc_layer_store& store, const RowMap& map,
+                          const BatchMeta& meta, int n_seq, bool tensor) {
+    RowMap general = map;
+    general.log_segment = store.log_segment_general;
+    const int sms = std::max(ctx->sm_count, 1);
+    DecodePlan plan;
+    if (tensor && shape.head_dim <= 256) {
+        const int target = (shape.head_dim == 256 ? 1 : 6) * sms;
+        plan = plan_decode(shape, general, meta, n_seq, target, true, 64);
+        bool spans = false;
+        for (int b = 0; b < n_seq; ++b) spans = spans || visible_groups(meta.pos[b], meta.pos[b], shape.window, general.log_segment) > 1;
+        // Whole rows of several segments would keep a state of head_dim x 128 floats a thread block.
+        if (plan.finish && spans && size_t(sms) * shape.head_dim * kTileKeys > kStaticScratchFloats) {
+            plan = plan_decode(shape, general, meta, n_seq, target, false, 64);
+        }
+    } else {
+        plan = simt_plan_decode(ctx, shape, general, meta, n_seq);
+    }
+    if (plan.finish) return 0;
+    const size_t parts = size_t(n_seq) * shape.q_heads * plan.slots;
+    return ((parts * 2 + 3) & ~size_t(3)) + parts * shape.head_dim;
+}
+
 }  // namespace hc
 
 extern "C" {
@@ -863,51 +888,59 @@ hc_status hc_attention_decode_static(hc_context* ctx, hc_kv_cache* cache, int la
                                         &view, &meta, &ep, &store, &tensor);
     if (st != HC_OK) return st;
     if (!ctx->static_scratch) return fail(HC_CUDA_ERROR, "this context has no static scratch address");
-    // What a call may be is stated in terms of the general cut of its rows' keys into tiles and segments (as the header
-    // puts it), whichever kernels run: a caller's program is not refused by one build and served by the next.
-    const size_t rows = size_t(n_seq) * shape.q_heads;
-    const int target = tensor ? (shape.head_dim == 256 ? 1 : 6) * std::max(ctx->sm_count, 1) : 0;
-    RowMap general = view.map;
-    general.log_segment = store->log_segment_general;
-    const DecodePlan plan = tensor ? plan_decode(shape, general, meta, n_seq, target, true, 64)
-                                   : simt_plan_decode(ctx, shape, view.map, meta, n_seq);
-    size_t ml_floats = plan.finish ? 0 : (rows * plan.slots * 2 + 3) & ~size_t(3);
-    size_t o_floats = plan.finish ? 0 : rows * plan.slots * shape.head_dim;
-    TcDecodePlan tc{};
-    if (tensor) {
-        // The tensor-core kernel's own cut leaves fewer partials, if any.
-        tc = tc_plan_decode(ctx, shape, view.map, meta, n_seq);
-        ml_floats = std::max(ml_floats, tc.part_ml_floats);
-        o_floats = std::max(o_floats, tc.part_o_floats);
-    }
-    if (ml_floats + o_floats > kStaticScratchFloats || tc.tickets > kStaticTickets) {
-        return fail(HC_KV_OVERFLOW, "hc_attention_decode_static: this call needs " + std::to_string((ml_floats + o_floats) * 4) +
+    const size_t need = static_need(ctx, shape, *store, view.map, meta, n_seq, tensor);
+    if (need > kStaticScratchFloats) {
+        return fail(HC_KV_OVERFLOW, "hc_attention_decode_static: this call needs " + std::to_string(need * 4) +
                                         " bytes of partials, the fixed scratch holds " +
                                         std::to_string(kStaticScratchFloats * 4));
     }
     // Every partial the merge reads is written by this call first, so nothing in the array has to start
     // at zero but the tickets behind it, which every launch leaves at zero.
     Workspace ws;
+    ws.part_ml_floats = (kStaticScratchFloats * 2 / (shape.head_dim + 2)) & ~size_t(3);
+    ws.part_o_floats = kStaticScratchFloats - ws.part_ml_floats;
     ws.part_ml = ctx->static_scratch;
-    ws.part_ml_floats = ml_floats;
-    ws.part_o = ctx->static_scratch + ml_floats;
-    ws.part_o_floats = kStaticScratchFloats - ml_floats;
+    ws.part_o = ctx->static_scratch + ws.part_ml_floats;
     ws.tickets = reinterpret_cast<unsigned*>(ctx->static_scratch + kStaticScratchFloats);
     ws.n_tickets = kStaticTickets;
-    // The same kernels, in the same order, as hc_attention_decode: only the partials live elsewhere,
-    // so the two entry points return the same bits.
-    if (tensor) {
-        DecodeSource src{};
-        src.q = q;
-        src.dtype = HC_BF16;
-        src.q_head_stride = shape.head_dim;
-        int served = 0;
-        st = tc_decode(ctx, shape, *store, view, meta, n_seq, src, ws, ep, static_cast<cudaStream_t>(stream), &served);
-        if (st == HC_OK && served < n_seq) return fail(HC_UNSUPPORTED, "hc_attention_decode_static: too many rows for one launch");
-        return st;
+    // The same kernels as hc_attention_decode: only the partials live elsewhere, so the two entry points return the same
+    // bits.  The cut they make of the rows may be finer than the one the limit is stated in: then the rows go in
+    // parts, and a row whose partials alone are too many borrows the cache's own workspace.
+    const size_t row_elems = size_t(shape.q_heads) * shape.head_dim;
+    for (int start = 0, served = 0; start < n_seq; start += served) {
+        BatchMeta part{};
+        int count = n_seq - start;
+        for (int b = 0; b < count; ++b) {
+            part.seq[b] = meta.seq[start + b];
+            part.pos[b] = meta.pos[start + b];
+        }
+        const uint16_t* q_rows = static_cast<const uint16_t*>(q) + size_t(start) * row_elems;
+        EpilogueArgs part_ep = ep;
+        part_ep.out = static_cast<uint16_t*>(ep.out) + size_t(start) * row_elems;
+        if (ep.gate) part_ep.gate = static_cast<const uint16_t*>(ep.gate) + size_t(start) * row_elems;
+        if (tensor) {
+            DecodeSource src{};
+            src.q = q_rows;
+            src.dtype = HC_BF16;
+            src.q_head_stride = shape.head_dim;
+            st = tc_decode(ctx, shape, *store, view, part, count, src, ws, part_ep, static_cast<cudaStream_t>(stream), &served);
+            if (st == HC_KV_OVERFLOW && served == 0) {
+                st = tc_decode(ctx, shape, *store, view, part, 1, src, cache->ws, part_ep, static_cast<cudaStream_t>(stream), &served);
+            }
+        } else {
+            bool room = false;
+            for (;; count = (count + 1) / 2) {
+                const DecodePlan plan = simt_plan_decode(ctx, shape, view.map, part, count);
+                const size_t parts = size_t(count) * shape.q_heads * plan.slots;
+                room = parts * shape.head_dim <= ws.part_o_floats && parts * 2 <= ws.part_ml_floats;
+                if (room || count == 1) break;
+            }
+            served = count;
+            st = simt_decode(ctx, shape, view, part, count, q_rows, room ? ws : cache->ws, part_ep, static_cast<cudaStream_t>(stream));
+        }
+        if (st != HC_OK) return st;
     }
-    return simt_decode(ctx, shape, view, meta, n_seq, static_cast<const uint16_t*>(q), ws, ep,
-                       static_cast<cudaStream_t>(stream));
+    return HC_OK;
 }
 
 }  // extern "C"

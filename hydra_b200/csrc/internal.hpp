@@ -155,7 +155,7 @@ struct hc_layer_store {
                                   // append at once and how far a rewind may reach
     int capacity = 0;
     int log_segment = 0;          // key tiles per segment, as a power of two (see common.cuh)
-    int log_segment_general = 0;  // the same by the head counts alone: what hc_attention_decode_static's limit goes by
+    int log_segment_general = 0;  // the grouping that hc_attention_decode_static's limit is stated in
     bool keeps_history = false;
     void* tmap_k = nullptr;       // tensor maps of the tcgen05 path (host copies), or null
     void* tmap_v = nullptr;

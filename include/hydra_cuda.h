@@ -348,26 +348,27 @@ HC_API hc_status hc_attention_decode(hc_context* ctx, hc_kv_cache* cache, int la
  * Who needs it: a runner that has already given every free byte of the device to its weight and KV
  * pools, a plugin that must not touch its host process's allocator, or code running where
  * cudaMalloc is not allowed.  The split-decode partials of this call live in one fixed array
- * inside the library (hc_attention_decode_static_limit() bytes, 8 MiB, held by every GPU that
- * loads the library until the process exits) and the call performs no cudaMalloc, cudaFree or any
- * other allocating routine.
+ * inside the library (hc_attention_decode_static_limit() bytes, 8 MiB, and 256 KiB of counters, held by
+ * every GPU that loads the library until the process exits) and the call performs no cudaMalloc, cudaFree
+ * or any other allocating routine.
  *
  *   - q must be bf16, already normalised and rotated: io_dtype HC_BF16, norm_q 0, rope NULL, gate
  *     none or HC_GATE_SEPARATE.  1 to 64 sequences; not for sequence-sharded caches.
  *   - A call whose partials (n_seq * q_heads * slots * (head_dim + 2) floats, where slots is the
- *     number of segments of 1024, 2048 or 4096 keys, or of 128-key tiles, that the library cuts the longest
- *     sequence into for this batch) exceed the limit is refused with HC_KV_OVERFLOW and a message
- *     that states both sizes.
- *   - It runs the same kernels as hc_attention_decode (tcgen05 for head_dim 64, 128, 256, CUDA
+ *     number of segments of 1024 or 4096 keys, or of 128-key tiles, that a general cut makes of the longest
+ *     sequence for this batch) exceed the limit is refused with HC_KV_OVERFLOW and a message
+ *     that states both sizes.  Where the kernels' own cut leaves more partials than that, the rows go in
+ *     several launches, and a single row beyond the array uses the cache's workspace.
+ *   - It runs the same kernels as hc_attention_decode (tcgen05 for head_dim 64, 128, 256, 512, CUDA
  *     cores otherwise, params->kernel_path honoured) with the partials redirected, so its output
  *     equals hc_attention_decode's bit for bit.
  *   - The array's device address is looked up by hc_context_create (cudaGetSymbolAddress, with the
  *     context's device current), which also makes the CUDA runtime load the module that holds the
  *     array: the 8 MiB are reserved when the context is created, not inside a later call.  Create
  *     the context before starting a stream capture and before handing the device's memory away.
- *   - All calls share the array and it keeps the last call's contents.  Nothing in it needs to be
- *     zero beforehand: each call writes every partial before reading it.  Two calls that overlap on
- *     the GPU (different streams, no dependency) race on it: serialise them. */
+ *   - All calls share the array and it keeps the last call's contents: each call writes every partial
+ *     before reading it.  The counters begin at zero and every launch leaves them there.  Two calls that
+ *     overlap on the GPU (different streams, no dependency) race on both: serialise them. */
 HC_API size_t hc_attention_decode_static_limit(void);
 HC_API hc_status hc_attention_decode_static(hc_context* ctx, hc_kv_cache* cache, int layer,
                                             const int* seq_ids, const int* positions, int n_seq,

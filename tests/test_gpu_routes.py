@@ -247,3 +247,28 @@ def test_positions_beyond_eight_million(hb, ctx, d, qh, kvh, window):
         layer.close()
     for other in got[1:]:
         assert np.array_equal(got[0][0], other[0]) and np.array_equal(got[0][1], other[1])
+
+
+@pytest.mark.parametrize("d, qh, kvh, n_seq, longest", [
+    (64, 16, 16, 64, 12200),     # 1024 rows of some 90 key tiles: more rows than a launch lists
+    (256, 16, 16, 64, 28600),    # the partials of its 2048-key segments take several launches
+    (512, 2, 2, 64, 6100),
+])
+def test_static_decode_serves_what_its_limit_allows(hb, ctx, d, qh, kvh, n_seq, longest):
+    """hc_attention_decode_static refuses by the general cut of the rows' keys, not by how the kernels cut them."""
+    import torch
+    rng = np.random.default_rng(d)
+    layer = tl.Layer(hb, ctx, qh, kvh, d, longest + 60)
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    k, v = (torch.randn((longest, kvh, d), device="cuda", generator=gen).to(torch.bfloat16) for _ in range(2))
+    layer.backend.write_key_value(layer.cache, 0, k, v, longest, 0, layer.params)
+    positions = [int(p) for p in rng.integers(longest - longest // 10, longest, n_seq)]
+    q = tl.normal_bf16(rng, (n_seq, qh, d))
+    out = tl.device_empty((n_seq, qh, d))
+    layer.backend.attention_static(layer.cache, 0, tl.to_device(q), out, positions, layer.params, seq_ids=[0] * n_seq)
+    ctx.check()
+    got = tl.to_host(out)
+    assert np.array_equal(got, layer.decode(q, positions, seq_ids=[0] * n_seq))
+    for b in (0, n_seq // 2, n_seq - 1):
+        assert np.array_equal(layer.decode(q[b:b + 1], positions[b:b + 1])[0], got[b]), b
+    layer.close()
