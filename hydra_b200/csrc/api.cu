@@ -103,9 +103,11 @@ hc_status check_shard_mode(const hc_kv_cache* cache, bool partial_mode) {
     return HC_OK;
 }
 
-bool needs_q_prepare(const hc_attn_params* p) {
+// Whether queries go through the prologue: what is asked of them, or, for the tensor-core kernels, which read them 8 and 16
+// bytes at a time, to be moved to a 16-byte boundary.
+bool needs_q_prepare(const hc_attn_params* p, const void* q, bool tensor) {
     return p->io_dtype != HC_BF16 || p->norm_q != 0 || p->rope != nullptr ||
-           p->gate_layout == HC_GATE_INTERLEAVED;
+           p->gate_layout == HC_GATE_INTERLEAVED || (tensor && (reinterpret_cast<uintptr_t>(q) & 15) != 0);
 }
 
 // What aligning the five parts of a staging slot to 256 bytes may cost.
@@ -279,7 +281,7 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
     if (st != HC_OK) return st;
     const int d = p->head_dim;
     const int mult = p->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
-    const bool prep = needs_q_prepare(p);
+    const bool prep = needs_q_prepare(p, q, tensor);
     int step = prep ? cache->ws.qprep_capacity : tokens;
     // Bidirectional blocks: chunk by chunk (a block ends with its token's chunk).
     const int* blocks = p->block_ends;
@@ -364,7 +366,7 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
     if (st != HC_OK) return st;
     const int d = p->head_dim;
     const int mult = p->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
-    const bool prep = needs_q_prepare(p);
+    const bool prep = needs_q_prepare(p, q, tensor);
     for (int start = 0, served = 0; start < n_seq; start += served) {
         // As many rows as a launch takes: on the tensor cores what tc_decode says, elsewhere what the prepared-query buffer
         // has room for.
@@ -434,6 +436,17 @@ hc_status decode_impl(hc_context* ctx, hc_kv_cache* cache, int layer, const int*
 }
 
 }  // namespace
+
+// `count` bf16 queries that need nothing but a 16-byte boundary, into the cache's prepared-query buffer (which has room for
+// qprep_capacity tokens).
+hc_status align_queries(hc_context* ctx, hc_kv_cache* cache, const hc_attn_params* p, const void* q, int count, cudaStream_t stream) {
+    PrepArgs args{};
+    fill_common(args, p);
+    fill_q_job(args.job[0], p, q, cache->ws.qprep);
+    args.n_jobs = 1;
+    args.tokens = count;
+    return launch_prepare(ctx, args, stream);
+}
 
 // Argument checking and kernel arguments for hc_attention_decode_static (attn_simt.cu).  Nothing
 // here allocates.

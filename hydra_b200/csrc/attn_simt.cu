@@ -843,6 +843,8 @@ hc_status static_decode_inputs(hc_context* ctx, hc_kv_cache* cache, int layer, c
                                const hc_attn_params* p, AttnShape* shape, CacheView* view, BatchMeta* meta,
                                EpilogueArgs* ep, const hc_layer_store** store, bool* tensor);
 
+hc_status align_queries(hc_context* ctx, hc_kv_cache* cache, const hc_attn_params* p, const void* q, int count, cudaStream_t stream);
+
 // Floats of partials that a call's general cut into tiles and segments leaves (the header puts the limit this way), whichever
 // kernels run and however they cut: a caller's program is not refused by one build and served by the next.
 static size_t static_need(const hc_context* ctx, const AttnShape& shape, const hc_layer_store& store, const RowMap& map,
@@ -907,9 +909,11 @@ hc_status hc_attention_decode_static(hc_context* ctx, hc_kv_cache* cache, int la
     // bits.  The cut they make of the rows may be finer than the one the limit is stated in: then the rows go in
     // parts, and a row whose partials alone are too many borrows the cache's own workspace.
     const size_t row_elems = size_t(shape.q_heads) * shape.head_dim;
+    const bool align = tensor && (reinterpret_cast<uintptr_t>(q) & 15) != 0;
     for (int start = 0, served = 0; start < n_seq; start += served) {
         BatchMeta part{};
         int count = n_seq - start;
+        if (align) count = std::min(count, cache->ws.qprep_capacity);
         for (int b = 0; b < count; ++b) {
             part.seq[b] = meta.seq[start + b];
             part.pos[b] = meta.pos[start + b];
@@ -919,8 +923,12 @@ hc_status hc_attention_decode_static(hc_context* ctx, hc_kv_cache* cache, int la
         part_ep.out = static_cast<uint16_t*>(ep.out) + size_t(start) * row_elems;
         if (ep.gate) part_ep.gate = static_cast<const uint16_t*>(ep.gate) + size_t(start) * row_elems;
         if (tensor) {
+            if (align) {
+                st = align_queries(ctx, cache, params, q_rows, count, static_cast<cudaStream_t>(stream));
+                if (st != HC_OK) return st;
+            }
             DecodeSource src{};
-            src.q = q_rows;
+            src.q = align ? cache->ws.qprep : q_rows;
             src.dtype = HC_BF16;
             src.q_head_stride = shape.head_dim;
             st = tc_decode(ctx, shape, *store, view, part, count, src, ws, part_ep, static_cast<cudaStream_t>(stream), &served);

@@ -353,7 +353,8 @@ HC_API hc_status hc_attention_decode(hc_context* ctx, hc_kv_cache* cache, int la
  * or any other allocating routine.
  *
  *   - q must be bf16, already normalised and rotated: io_dtype HC_BF16, norm_q 0, rope NULL, gate
- *     none or HC_GATE_SEPARATE.  1 to 64 sequences; not for sequence-sharded caches.
+ *     none or HC_GATE_SEPARATE.  1 to 64 sequences; not for sequence-sharded caches.  (A q off a 16-byte
+ *     boundary is first moved to the cache's prepared-query buffer.)
  *   - A call whose partials (n_seq * q_heads * slots * (head_dim + 2) floats, where slots is the
  *     number of segments of 1024 or 4096 keys, or of 128-key tiles, that a general cut makes of the longest
  *     sequence for this batch) exceed the limit is refused with HC_KV_OVERFLOW and a message

@@ -272,3 +272,41 @@ def test_static_decode_serves_what_its_limit_allows(hb, ctx, d, qh, kvh, n_seq, 
     for b in (0, n_seq // 2, n_seq - 1):
         assert np.array_equal(layer.decode(q[b:b + 1], positions[b:b + 1])[0], got[b]), b
     layer.close()
+
+
+def _off_by_one(array, io="bf16"):
+    """The array on the device, one element behind a 16-byte boundary."""
+    import torch
+    flat = tl.to_device(array, io).reshape(-1)
+    room = torch.empty(flat.numel() + 8, device="cuda", dtype=flat.dtype)
+    room[1:1 + flat.numel()] = flat
+    return room[1:1 + flat.numel()].view(array.shape)
+
+
+@pytest.mark.parametrize("d, qh, kvh, window", [(64, 16, 2, 0), (64, 16, 2, 128), (128, 8, 2, 0), (256, 16, 2, 0), (512, 16, 2, 0)])
+def test_queries_off_a_16_byte_boundary(hb, ctx, d, qh, kvh, window):
+    """Queries that need no prologue, anywhere: the bits of the same queries on a boundary."""
+    tokens, rows = 300, 5
+    q, k, v = _inputs(d + window, tokens, qh, kvh, d)
+    layer = tl.Layer(hb, ctx, qh, kvh, d, 512, window=window)
+    kd, vd = _off_by_one(k), _off_by_one(v)
+    layer.backend.write_key_value(layer.cache, 0, kd, vd, tokens, 0, layer.params)
+    be, cache, params = layer.backend, layer.cache, layer.params
+    positions, ids = [3, 127, 128, 256, tokens - 1], [0] * rows
+    moved, out = _off_by_one(q), tl.device_empty((tokens, qh, d))
+    assert moved.data_ptr() % 16 == 2
+    be.attention_prefill(cache, 0, moved, out, tokens, 0, params)
+    ctx.check()
+    prompt = tl.to_host(out)
+    assert np.array_equal(prompt, layer.prefill(q, 0))
+    for call in (be.attention, be.attention_static):
+        out = tl.device_empty((rows, qh, d))
+        call(cache, 0, _off_by_one(q[positions]), out, positions, params, seq_ids=ids)
+        ctx.check()
+        assert np.array_equal(tl.to_host(out), prompt[positions])
+    # a token's own rows, appended by its step
+    out = tl.device_empty((1, qh, d))
+    be.layer_step(cache, 0, _off_by_one(q[-1:]), _off_by_one(k[-1:]), _off_by_one(v[-1:]), out, 1, tokens - 1, params)
+    ctx.check()
+    assert np.array_equal(tl.to_host(out)[0], prompt[-1])
+    layer.close()
