@@ -454,6 +454,7 @@ struct MergeRows {
     int first_position;      // prefill
     int tokens;              // query tokens, or batch entries
     int tokens_per_tile;     // prefill: tokens of a row tile, which share their slots
+    int last_of_all;         // prefill: the key that all of them reach to with bidirectional blocks, else -1
     BatchMeta meta;
 };
 
@@ -480,7 +481,7 @@ merge_rows_kernel(const AttnShape shape, const RowMap map, const MergeRows rows,
     } else {
         const int tile_row0 = (r / rows.tokens_per_tile) * rows.tokens_per_tile;
         first_pos = rows.first_position + tile_row0;
-        last_pos = rows.first_position + min(tile_row0 + rows.tokens_per_tile, rows.tokens) - 1;
+        last_pos = rows.last_of_all >= 0 ? rows.last_of_all : rows.first_position + min(tile_row0 + rows.tokens_per_tile, rows.tokens) - 1;
     }
     const int n_parts = min(visible_groups(first_pos, last_pos, shape.window, map.log_segment), slots);
 
@@ -789,11 +790,13 @@ hc_status launch_merge_decode(hc_context* ctx, const AttnShape& shape, const Row
 }
 
 hc_status launch_merge_prefill(hc_context* ctx, const AttnShape& shape, const RowMap& map, int tokens, int first_position,
-                               int tokens_per_tile, const Workspace& ws, int slots, const EpilogueArgs& ep, cudaStream_t stream) {
+                               int tokens_per_tile, int last_of_all, const Workspace& ws, int slots, const EpilogueArgs& ep,
+                               cudaStream_t stream) {
     MergeRows rows{};
     rows.first_position = first_position;
     rows.tokens = tokens;
     rows.tokens_per_tile = tokens_per_tile;
+    rows.last_of_all = last_of_all;
     return launch_merge_rows(ctx, shape, map, rows, ws, slots, ep, stream);
 }
 

@@ -1047,48 +1047,61 @@ static hc_status launch_any(hc_context* ctx, const AttnShape& shape, const TcArg
     return launch_attention_pair(ctx, layer, &args, shape.head_dim, stream);
 }
 
-hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
-                     int seq, const uint16_t* q, int tokens, int first_position, const Workspace& ws,
-                     const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends) {
-    if (!layer.tmap_k || !layer.tmap_v) return fail(HC_UNSUPPORTED, "this layer has no tensor maps");
-    if (tokens <= 0) return HC_OK;
+// Segments and key tiles that a row tile of the pass spans, at most.  `last_of_all`: where every item reaches with
+// bidirectional blocks (else -1).
+struct PrefillSpan {
+    int tokens_per_tile, mtiles, slots, tiles;
+};
+static PrefillSpan prefill_span(const AttnShape& shape, const RowMap& map, int tokens, int first_position, int last_of_all) {
+    PrefillSpan s;
+    // Head_dim 256 and 512: row tiles of 256 rows on pairs of SMs.
+    s.tokens_per_tile = (shape.head_dim >= 256 ? 2 : 1) * kRows / shape.group;
+    s.mtiles = (tokens + s.tokens_per_tile - 1) / s.tokens_per_tile;
+    s.slots = s.tiles = 1;
+    for (int mtile = 0; mtile < s.mtiles; ++mtile) {
+        const int first = first_position + mtile * s.tokens_per_tile;
+        const int last = last_of_all >= 0 ? last_of_all : first_position + std::min((mtile + 1) * s.tokens_per_tile, tokens) - 1;
+        s.slots = std::max(s.slots, visible_groups(first, last, shape.window, map.log_segment));
+        s.tiles = std::max(s.tiles, row_tiles(map, first, last, shape.window).count);
+    }
+    return s;
+}
+
+// One attention launch (and its merge) for `tokens` tokens, with keys appended up to position appended - 1.
+// `merged`: the rows have to leave through the merge kernel, which stores element by element.
+static hc_status prefill_pass(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
+                              int seq, const uint16_t* q, int tokens, int first_position, int appended, const Workspace& ws,
+                              const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends, bool merged) {
     TcArgs args{};
     fill_common_args(args, ctx, shape, cache, q, ws, ep);
     args.tokens = tokens;
     args.first_position = first_position;
     args.seq = seq;
-    // Head_dim 256 and 512: row tiles of 256 rows on pairs of SMs.
     const bool pairs = shape.head_dim >= 256;
-    const int tokens_per_tile = (pairs ? 2 : 1) * kRows / shape.group;
-    args.mtiles = (tokens + tokens_per_tile - 1) / tokens_per_tile;
-    // Segments and key tiles a row tile spans, at most.
-    int slots = 1, most_tiles = 1;
-    for (int mtile = 0; mtile < args.mtiles; ++mtile) {
-        const int first = first_position + mtile * tokens_per_tile;
-        const int last = first_position + (block_ends ? tokens : std::min((mtile + 1) * tokens_per_tile, tokens)) - 1;
-        slots = std::max(slots, visible_groups(first, last, shape.window, cache.map.log_segment));
-        most_tiles = std::max(most_tiles, row_tiles(cache.map, first, last, shape.window).count);
-    }
+    const int last_of_all = block_ends ? appended - 1 : -1;
+    const PrefillSpan span = prefill_span(shape, cache.map, tokens, first_position, last_of_all);
+    args.mtiles = span.mtiles;
+    int slots = span.slots;
     // Whole rows per item, or one item per (row tile, kv head, segment) merged afterwards: whichever
     // the longest thread block (or pair) finishes first, in units of one key tile's time.  An item costs its
     // tiles plus a start and an end (about four tiles' worth at head_dim 64, two of a pair's longer ones), the merge
     // and its launch about ten of the former, five of the latter.
     const int whole_items = args.mtiles * shape.kv_heads * (pairs ? pair_items_per_row_tile(shape.head_dim) : 1);
     const size_t rows = size_t(tokens) * shape.q_heads;
-    const bool can_split = slots > 1 && rows * slots * shape.head_dim <= ws.part_o_floats && rows * slots * 2 <= ws.part_ml_floats;
-    const bool can_finish = slots == 1 || row_state_floats(ctx, shape) <= ws.part_o_floats;
+    const bool can_split = (slots > 1 || merged) && rows * slots * shape.head_dim <= ws.part_o_floats && rows * slots * 2 <= ws.part_ml_floats;
+    const bool can_finish = !merged && (slots == 1 || row_state_floats(ctx, shape) <= ws.part_o_floats);
     const int workers = std::max(pairs ? ctx->sm_count / 2 : ctx->sm_count, 1);
     const int item_cost = pairs ? 2 : 4;
-    const int whole_time = ((whole_items + workers - 1) / workers) * (most_tiles + item_cost);
-    const int split_time = ((whole_items * slots + workers - 1) / workers) * (std::min(most_tiles, 1 << cache.map.log_segment) + item_cost) +
+    const int whole_time = ((whole_items + workers - 1) / workers) * (span.tiles + item_cost);
+    const int split_time = ((whole_items * slots + workers - 1) / workers) * (std::min(span.tiles, 1 << cache.map.log_segment) + item_cost) +
                            (pairs ? 5 : 10);
-    // With bidirectional blocks a row's last key is known on the device only: whole rows per item, no
-    // merge over per-row segment lists (or the general kernel, if the row state does not fit).
-    if (block_ends && !can_finish) return simt_prefill(ctx, shape, cache, seq, q, tokens, first_position, ep, stream, block_ends);
+    // With bidirectional blocks every row tile reaches to the last key: whole rows per item (or the general kernel, if the
+    // row state does not fit).
+    if (block_ends && !merged && !can_finish) return simt_prefill(ctx, shape, cache, seq, q, tokens, first_position, ep, stream, block_ends);
     args.block_ends = block_ends;
-    args.appended = first_position + tokens;
-    const bool whole = block_ends != nullptr || !can_split || (can_finish && whole_time <= split_time);
-    if (whole && !can_finish) {
+    args.appended = appended;
+    const bool whole = !merged && (block_ends != nullptr || !can_split || (can_finish && whole_time <= split_time));
+    if (whole ? !can_finish : !can_split) {
         return fail(HC_KV_OVERFLOW, "prefill: the attention workspace is too small for this chunk (" + std::to_string(tokens) +
                                         " tokens over " + std::to_string(slots) + " segments)");
     }
@@ -1100,7 +1113,36 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
     args.magic_kv_heads = division_magic(uint32_t(shape.kv_heads), uint32_t(args.n_items));
     const hc_status st = launch_any(ctx, shape, args, layer, stream);
     if (st != HC_OK || args.finish) return st;
-    return launch_merge_prefill(ctx, shape, cache.map, tokens, first_position, tokens_per_tile, ws, slots, ep, stream);
+    return launch_merge_prefill(ctx, shape, cache.map, tokens, first_position, span.tokens_per_tile, last_of_all, ws, slots, ep, stream);
+}
+
+hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
+                     int seq, const uint16_t* q, int tokens, int first_position, const Workspace& ws,
+                     const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends) {
+    if (!layer.tmap_k || !layer.tmap_v) return fail(HC_UNSUPPORTED, "this layer has no tensor maps");
+    if (tokens <= 0) return HC_OK;
+    const int appended = first_position + tokens;
+    // The kernels store whole rows 16 bytes at a time (row partials 8).  An output off that boundary leaves through the
+    // merge kernel instead, as many tokens at a time as the workspace has partials for.
+    if ((reinterpret_cast<uintptr_t>(ep.out) & (ep.write_partial ? 7 : 15)) == 0) {
+        return prefill_pass(ctx, shape, layer, cache, seq, q, tokens, first_position, appended, ws, ep, stream, block_ends, false);
+    }
+    const size_t out_row = size_t(shape.q_heads) * (ep.write_partial ? (shape.head_dim + 2) * 4 : shape.head_dim * (ep.io_dtype == HC_F32 ? 4 : 2));
+    const size_t gate_row = size_t(shape.q_heads) * shape.head_dim * (ep.gate_layout == HC_GATE_INTERLEAVED ? 2 : 1) * (ep.io_dtype == HC_F32 ? 4 : 2);
+    for (int start = 0, count = 0; start < tokens; start += count) {
+        for (count = tokens - start; count > 1; count = (count + 1) / 2) {
+            const PrefillSpan span = prefill_span(shape, cache.map, count, first_position + start, block_ends ? appended - 1 : -1);
+            const size_t parts = size_t(count) * shape.q_heads * span.slots;
+            if (parts * shape.head_dim <= ws.part_o_floats && parts * 2 <= ws.part_ml_floats) break;
+        }
+        EpilogueArgs part = ep;
+        part.out = static_cast<unsigned char*>(ep.out) + size_t(start) * out_row;
+        if (ep.gate) part.gate = static_cast<const unsigned char*>(ep.gate) + size_t(start) * gate_row;
+        const hc_status st = prefill_pass(ctx, shape, layer, cache, seq, q + size_t(start) * shape.q_heads * shape.head_dim, count,
+                                          first_position + start, appended, ws, part, stream, block_ends ? block_ends + start : nullptr, true);
+        if (st != HC_OK) return st;
+    }
+    return HC_OK;
 }
 
 }  // namespace hc

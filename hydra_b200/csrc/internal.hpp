@@ -234,7 +234,7 @@ hc_status launch_merge_decode(hc_context* ctx, const AttnShape& shape, const Row
                               int n_seq, const Workspace& ws, const DecodePlan& plan, const EpilogueArgs& ep,
                               cudaStream_t stream);
 hc_status launch_merge_prefill(hc_context* ctx, const AttnShape& shape, const RowMap& map, int tokens,
-                               int first_position, int tokens_per_tile, const Workspace& ws, int slots,
+                               int first_position, int tokens_per_tile, int last_of_all, const Workspace& ws, int slots,
                                const EpilogueArgs& ep, cudaStream_t stream);
 hc_status launch_combine(hc_context* ctx, const float* gathered, int world, int rows, int q_heads,
                          int d, const EpilogueArgs& ep, cudaStream_t stream);

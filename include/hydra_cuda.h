@@ -17,7 +17,9 @@
  *   - Activations (q, k, v, gate, out) are device buffers of `io_dtype` (fp32, as the reference's
  *     buffers are, or bf16).  The cache is bf16.  Sinks and norm weights are bf16 device pointers
  *     read in place, as the reference reads them from the mapped checkpoint.  RoPE tables are fp32.
- *   - Shapes: q/out/gate [tokens][q_heads][head_dim]; k/v [tokens][kv_heads][head_dim].
+ *   - Shapes: q/out/gate [tokens][q_heads][head_dim]; k/v [tokens][kv_heads][head_dim].  Buffers need no
+ *     alignment beyond their elements' (but where an entry says so); off a 16-byte boundary a call takes
+ *     slower kernels or an extra launch.
  *     head_dim must be a multiple of 8 and at most 512 (the reference's own bound,
  *     Sources/HydraMetal/Shaders/attention.metal:115); q_heads / kv_heads must be a power of two
  *     no larger than 16.

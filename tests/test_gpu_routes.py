@@ -310,3 +310,65 @@ def test_queries_off_a_16_byte_boundary(hb, ctx, d, qh, kvh, window):
     ctx.check()
     assert np.array_equal(tl.to_host(out)[0], prompt[-1])
     layer.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, io, gated, blocks", [
+    (64, 16, 2, 0, "bf16", False, False), (64, 64, 8, 128, "f32", True, True), (128, 8, 2, 0, "bf16", True, True),
+    (256, 16, 2, 0, "f32", True, False), (256, 16, 8, 300, "bf16", False, True), (512, 16, 2, 0, "bf16", False, False),
+    (512, 8, 1, 0, "f32", True, True),
+])
+def test_outputs_off_a_16_byte_boundary(hb, ctx, d, qh, kvh, window, io, gated, blocks):
+    """A prompt's rows stored element by element, in one pass or (the small workspace of a cache made for chunks of 16)
+    several: the bits of the same call on a boundary, bidirectional blocks and gates included."""
+    import torch
+    tokens, first = 700, 1900
+    rng = np.random.default_rng(d + tokens)
+    q = tl.normal_bf16(rng, (tokens, qh, d))
+    k, v = (tl.normal_bf16(rng, (first + tokens, kvh, d)) for _ in range(2))
+    gate = tl.normal_bf16(rng, (tokens, qh, d))
+    ends = np.zeros(tokens, np.int32)
+    ends[100:230], ends[600:690] = first + 230, first + 690
+    for chunk in (1024, 16):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 2816, window=window, io=io, prefill_chunk=chunk)
+        layer.append(k, v, 0)
+        more = dict(block_ends=torch.from_numpy(ends).cuda()) if blocks else {}
+        if gated:
+            more.update(gate_layout=hb.capi.HC_GATE_SEPARATE, gate=_off_by_one(gate, io))
+        params = dataclasses.replace(layer.params, **more)
+        qd = tl.to_device(q, io)
+        outs = []
+        for shift in (0, 1):
+            room = torch.full((tokens * qh * d + 8,), 7.0, device="cuda", dtype=qd.dtype)
+            out = room[shift:shift + tokens * qh * d].view(tokens, qh, d)
+            layer.backend.attention_prefill(layer.cache, 0, qd, out, tokens, first, params)
+            ctx.check()
+            outs.append(tl.to_host(out))
+            assert bool((room[:shift] == 7).all()) and bool((room[shift + tokens * qh * d:] == 7).all())
+            one = room[shift:shift + qh * d].view(1, qh, d)
+            layer.backend.attention(layer.cache, 0, qd[-1:], one, [first + tokens - 1],
+                                    dataclasses.replace(params, gate=params.gate[-1:]) if gated else params)
+            ctx.check()
+            assert np.array_equal(tl.to_host(one)[0], outs[0][-1])
+        assert np.array_equal(outs[0], outs[1])
+        layer.close()
+
+
+def test_partials_off_an_8_byte_boundary(hb, ctx):
+    """The same for the row partials of a sequence shard."""
+    import torch
+    qh, kvh, d, tokens, first = 8, 2, 512, 300, 256
+    q, k, v = _inputs(9, first + tokens, qh, kvh, d)
+    q = q[first:]
+    for rank in range(2):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 1024, shard=(hb.capi.HC_SHARD_SEQUENCE, rank, 2), prefill_chunk=1024)
+        layer.append(k, v, 0)
+        size = tokens * qh * (d + 2)
+        outs = []
+        for shift in (0, 1):
+            room = torch.zeros(size + 4, device="cuda")
+            partial = room[shift:shift + size]
+            layer.backend.attention_prefill_partial(layer.cache, 0, tl.to_device(q), partial, tokens, first, layer.params)
+            ctx.check()
+            outs.append(partial.cpu().numpy())
+        assert np.array_equal(outs[0], outs[1])
+        layer.close()
