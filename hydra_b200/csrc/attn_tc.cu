@@ -1068,7 +1068,7 @@ static PrefillSpan prefill_span(const AttnShape& shape, const RowMap& map, int t
 }
 
 // One attention launch (and its merge) for `tokens` tokens, with keys appended up to position appended - 1.
-// `merged`: the rows have to leave through the merge kernel, which stores element by element.
+// `merged`: the rows have to leave through the merge kernel.
 static hc_status prefill_pass(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
                               int seq, const uint16_t* q, int tokens, int first_position, int appended, const Workspace& ws,
                               const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends, bool merged) {
@@ -1122,15 +1122,27 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
     if (!layer.tmap_k || !layer.tmap_v) return fail(HC_UNSUPPORTED, "this layer has no tensor maps");
     if (tokens <= 0) return HC_OK;
     const int appended = first_position + tokens;
-    // The kernels store whole rows 16 bytes at a time (row partials 8).  An output off that boundary leaves through the
-    // merge kernel instead, as many tokens at a time as the workspace has partials for.
-    if ((reinterpret_cast<uintptr_t>(ep.out) & (ep.write_partial ? 7 : 15)) == 0) {
-        return prefill_pass(ctx, shape, layer, cache, seq, q, tokens, first_position, appended, ws, ep, stream, block_ends, false);
+    const int tokens_per_tile = (shape.head_dim >= 256 ? 2 : 1) * kRows / shape.group;
+    // The first `merged` tokens leave through the merge kernel, as many at a time as the workspace has partials for.
+    int merged = 0;
+    if ((reinterpret_cast<uintptr_t>(ep.out) & (ep.write_partial ? 7 : 15)) != 0) {
+        // The kernels store whole rows 16 bytes at a time (row partials 8); the merge kernel element by element.
+        merged = tokens;
+    } else if (ep.write_partial && cache.map.world > 1) {
+        // A row tile that sees no key tile of this rank is nobody's item: its rows' partials are the empty fold, which the
+        // merge kernel writes.
+        for (int start = 0; start < tokens; start += tokens_per_tile) {
+            const int last = block_ends ? appended - 1 : first_position + std::min(start + tokens_per_tile, tokens) - 1;
+            if (row_tiles(cache.map, first_position + start, last, shape.window).count <= 0) merged = std::min(start + tokens_per_tile, tokens);
+        }
     }
-    const size_t out_row = size_t(shape.q_heads) * (ep.write_partial ? (shape.head_dim + 2) * 4 : shape.head_dim * (ep.io_dtype == HC_F32 ? 4 : 2));
-    const size_t gate_row = size_t(shape.q_heads) * shape.head_dim * (ep.gate_layout == HC_GATE_INTERLEAVED ? 2 : 1) * (ep.io_dtype == HC_F32 ? 4 : 2);
+    const size_t q_row = size_t(shape.q_heads) * shape.head_dim;
+    const size_t out_row = ep.write_partial ? size_t(shape.q_heads) * (shape.head_dim + 2) * 4 : q_row * (ep.io_dtype == HC_F32 ? 4 : 2);
+    const size_t gate_row = q_row * (ep.gate_layout == HC_GATE_INTERLEAVED ? 2 : 1) * (ep.io_dtype == HC_F32 ? 4 : 2);
     for (int start = 0, count = 0; start < tokens; start += count) {
-        for (count = tokens - start; count > 1; count = (count + 1) / 2) {
+        const bool merge = start < merged;
+        count = (merge ? merged : tokens) - start;
+        for (; merge && count > 1; count = (count + 1) / 2) {
             const PrefillSpan span = prefill_span(shape, cache.map, count, first_position + start, block_ends ? appended - 1 : -1);
             const size_t parts = size_t(count) * shape.q_heads * span.slots;
             if (parts * shape.head_dim <= ws.part_o_floats && parts * 2 <= ws.part_ml_floats) break;
@@ -1138,8 +1150,8 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
         EpilogueArgs part = ep;
         part.out = static_cast<unsigned char*>(ep.out) + size_t(start) * out_row;
         if (ep.gate) part.gate = static_cast<const unsigned char*>(ep.gate) + size_t(start) * gate_row;
-        const hc_status st = prefill_pass(ctx, shape, layer, cache, seq, q + size_t(start) * shape.q_heads * shape.head_dim, count,
-                                          first_position + start, appended, ws, part, stream, block_ends ? block_ends + start : nullptr, true);
+        const hc_status st = prefill_pass(ctx, shape, layer, cache, seq, q + size_t(start) * q_row, count, first_position + start, appended,
+                                          ws, part, stream, block_ends ? block_ends + start : nullptr, merge);
         if (st != HC_OK) return st;
     }
     return HC_OK;

@@ -372,3 +372,30 @@ def test_partials_off_an_8_byte_boundary(hb, ctx):
             outs.append(partial.cpu().numpy())
         assert np.array_equal(outs[0], outs[1])
         layer.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window", [(64, 16, 2, 0), (256, 8, 2, 0), (512, 8, 1, 0), (64, 16, 2, 200), (128, 8, 2, 130)])
+def test_prompt_partials_of_ranks_without_a_key(hb, ctx, d, qh, kvh, window):
+    """The first tokens of a prompt (and on a window layer any) see no key tile of some ranks: those ranks' partials are
+    the empty fold, whatever the buffer held."""
+    import torch
+    world, tokens = 4, 700
+    q, k, v = _inputs(d + window, tokens, qh, kvh, d)
+    sinks = tl.normal_bf16(np.random.default_rng(d), (qh,))
+    gathered = None
+    for rank in range(world):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 1024, window=window, sinks=sinks, prefill_chunk=1024,
+                         shard=(hb.capi.HC_SHARD_SEQUENCE, rank, world), storage=hb.capi.HC_STORAGE_LINEAR)
+        layer.append(k, v, 0)
+        if gathered is None:
+            gathered = torch.full((world, layer.backend.partial_bytes(layer.params, tokens) // 4), 1e30, device="cuda")
+        layer.backend.attention_prefill_partial(layer.cache, 0, tl.to_device(q), gathered[rank], tokens, 0, layer.params)
+        ctx.check()
+        if rank + 1 < world:
+            layer.close()
+    out = tl.device_empty((tokens, qh, d))
+    layer.backend.attention_combine(gathered, world, tokens, out, layer.params)
+    ctx.check()
+    want = ho.attention_rows(q, np.arange(tokens), k, v, 1 / np.sqrt(d), window, sinks=sinks)
+    assert tl.within_tolerance(tl.to_host(out), want)
+    layer.close()
