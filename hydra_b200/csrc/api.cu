@@ -1406,10 +1406,25 @@ hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_
                                   void* workspace, void* stream) {
     if (!ctx || !cache || !layers || !hidden_in || !hidden_out || !workspace) return fail(HC_INVALID_ARGUMENT, "null context or buffer");
     if (n_layers <= 0 || n_layers > int(cache->layers.size()) || tokens <= 0 || width <= 0) return fail(HC_INVALID_ARGUMENT, "bad sizes");
+    if (width % 64 != 0) return fail(HC_DIM_MISMATCH, "hc_attention_stack_host: width " + std::to_string(width) + " must be a multiple of 64");
+    if (!seq_ok(cache, seq)) return fail(HC_INVALID_ARGUMENT, "sequence index out of range");
+    if (reinterpret_cast<uintptr_t>(workspace) & 15) return fail(HC_INVALID_ARGUMENT, "hc_attention_stack_host: the workspace is not aligned");
+    // Everything that a layer's calls would refuse is refused before anything is queued.
     for (int i = 0; i < n_layers; ++i) {
-        const hc_status st = validate_params(cache, i, &layers[i].params);
+        const hc_block_weights& w = layers[i];
+        hc_status st = validate_params(cache, i, &w.params);
+        if (st == HC_OK) st = check_positions(cache, cache->layers[size_t(i)], first_position, tokens, &w.params);
+        if (st == HC_OK) st = check_shard_mode(cache, false);
         if (st != HC_OK) return st;
-        if (layers[i].params.io_dtype != HC_BF16) return fail(HC_INVALID_ARGUMENT, "hc_attention_stack_host: io_dtype must be HC_BF16");
+        if (w.params.io_dtype != HC_BF16) return fail(HC_INVALID_ARGUMENT, "hc_attention_stack_host: io_dtype must be HC_BF16");
+        const void* weights[4] = {w.wq, w.wk, w.wv, w.wo};
+        for (const void* weight : weights) {
+            if (!weight) return fail(HC_INVALID_ARGUMENT, "hc_attention_stack_host: layer " + std::to_string(i) + " has a null weight");
+            if (reinterpret_cast<uintptr_t>(weight) & 15) return fail(HC_INVALID_ARGUMENT, "hc_attention_stack_host: weights must be 16-byte aligned");
+        }
+        if ((w.params.q_heads * w.params.head_dim) % 64 != 0) {
+            return fail(HC_DIM_MISMATCH, "hc_attention_stack_host: q_heads * head_dim must be a multiple of 64");
+        }
     }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const StackSpace space = stack_space(layers, n_layers, tokens, width);
@@ -1431,8 +1446,12 @@ hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_
         if (st == HC_OK) st = hc_linear(ctx, base + space.attended, w.wo, w.bo, hidden, hidden, tokens, o_width, width, HC_F32, stream);
     }
     if (st == HC_OK) st = check_cuda(cudaMemcpyAsync(hidden_out, hidden, bytes, cudaMemcpyDeviceToHost, s), "hidden states out");
-    if (st != HC_OK) return st;
-    return hc_context_check(ctx, stream);
+    if (st == HC_OK) return hc_context_check(ctx, stream);
+    // (Pages that ran out, or a launch that failed.)  The caller has its buffers back: nothing of the call is still on its way.
+    const std::string message = g_last_error;
+    cudaStreamSynchronize(s);
+    g_last_error = message;
+    return st;
 }
 
 // Where a call's next piece ends.  Each copy from the host costs some 15 us beside the traffic the other way, so

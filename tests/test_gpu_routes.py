@@ -399,3 +399,41 @@ def test_prompt_partials_of_ranks_without_a_key(hb, ctx, d, qh, kvh, window):
     want = ho.attention_rows(q, np.arange(tokens), k, v, 1 / np.sqrt(d), window, sinks=sinks)
     assert tl.within_tolerance(tl.to_host(out), want)
     layer.close()
+
+
+def test_a_stack_call_that_cannot_run_queues_nothing(hb, ctx):
+    """hc_attention_stack_host looks at every layer's positions before its first copy: a ring takes them, the full
+    layer behind it does not."""
+    import ctypes
+    import torch
+    capi, width, qh, kvh, d = hb.capi, 64, 2, 1, 64
+    cache = hb.KVCache(ctx, [dict(q_heads=qh, kv_heads=kvh, head_dim=d, window=128, storage=capi.HC_STORAGE_RING),
+                             dict(q_heads=qh, kv_heads=kvh, head_dim=d, window=0)], 256, prefill_chunk=128)
+    shapes = dict(input_norm=(width,), wq=(qh * d, width), wk=(kvh * d, width), wv=(kvh * d, width), wo=(width, qh * d))
+    weights = [{name: torch.ones(shape, device="cuda", dtype=torch.bfloat16) for name, shape in shapes.items()} for _ in range(2)]
+    blocks = (capi.BlockWeightsStruct * 2)()
+    for block, tensors, window in zip(blocks, weights, (128, 0)):
+        for name, tensor in tensors.items():
+            setattr(block, name, tensor.data_ptr())
+        block.params = hb.AttnParams(q_heads=qh, kv_heads=kvh, head_dim=d, window=window, sm_scale=0.125,
+                                     io_dtype=capi.HC_BF16).struct()
+    lib = capi.load()
+    tokens = 4
+    workspace = torch.empty(lib.hc_attention_stack_bytes(blocks, 2, tokens, width), dtype=torch.uint8, device="cuda")
+    host = np.ones((tokens, width), np.float32)
+
+    def call(first_position, space=workspace.data_ptr(), wide=width):
+        before = ctx.launch_count
+        status = lib.hc_attention_stack_host(ctx.handle, cache.handle, blocks, 2, 0, host.ctypes.data, host.ctypes.data, tokens,
+                                             wide, first_position, ctypes.c_float(1e-5), space, None)
+        return status, ctx.launch_count - before
+
+    assert call(254) == (capi.HC_KV_OVERFLOW, 0)
+    assert call(-1) == (capi.HC_INVALID_ARGUMENT, 0)
+    assert np.array_equal(host, np.ones_like(host))
+    blocks[1].wo = None
+    assert call(0) == (capi.HC_INVALID_ARGUMENT, 0)
+    blocks[1].wo = weights[1]["wo"].data_ptr()
+    status, launches = call(0)
+    assert status == 0 and launches > 0
+    cache.close()
