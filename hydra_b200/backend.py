@@ -12,7 +12,7 @@ libhydra_cuda.so.
 from __future__ import annotations
 
 import ctypes
-from dataclasses import dataclass, field
+from dataclasses import dataclass, field, fields
 from typing import Optional, Sequence
 
 from . import capi
@@ -70,7 +70,8 @@ def _ptr(buffer) -> Optional[int]:
         return None
     if isinstance(buffer, int):
         return buffer
-    return buffer.data_ptr()
+    address = buffer.data_ptr()
+    return address if type(address) is int else int(address)
 
 
 def _stream(stream) -> Optional[int]:
@@ -192,6 +193,14 @@ class AttnParams:
     def __setattr__(self, name, value) -> None:
         object.__setattr__(self, name, value)
         object.__setattr__(self, "_struct", None)
+
+    def __getstate__(self):
+        """What a copy (copy, deepcopy, pickle) takes along: the attributes, not the C struct."""
+        return {f.name: getattr(self, f.name) for f in fields(self)}
+
+    def __setstate__(self, state) -> None:
+        for name, value in state.items():
+            setattr(self, name, value)
 
     def struct(self) -> capi.AttnParamsStruct:
         """The C struct, filled once and again after any attribute changes (filling it takes as long as the library
