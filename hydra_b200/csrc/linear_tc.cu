@@ -115,17 +115,28 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, u
 // compiler may not move a load across a store, and a block's eight loads one after the other cost more
 // than its MMAs (o_proj of 4096 tokens: 141 us).
 constexpr int kLinStageBytes = 32 * 128;
-__device__ __forceinline__ float4 load_bias(const LinJob& job, int col0) {
-    const int col = col0 + (threadIdx.x & 7) * 4;
-    float b[4];
+// A tile's bias, eight columns a lane in one load while the tile is computed, and the four of them that a lane adds in a block
+// of 32 columns.  (Loaded block by block, one ahead, they were 1.4 us of a 256-column tile.)
+__device__ __forceinline__ uint4 load_bias(const LinJob& job, int col0) {
+    const int col = col0 + (threadIdx.x & 31) * 8;
+    if (job.bias == nullptr || col >= job.out_features) return make_uint4(0, 0, 0, 0);
+    if (col + 8 <= job.out_features && (reinterpret_cast<uintptr_t>(job.bias) & 15) == 0) return __ldg(reinterpret_cast<const uint4*>(job.bias + col));
+    uint32_t b[8];
     #pragma unroll
-    for (int i = 0; i < 4; ++i) b[i] = job.bias != nullptr && col + i < job.out_features ? bf16_bits_to_float(__ldg(job.bias + col + i)) : 0.0f;
-    return make_float4(b[0], b[1], b[2], b[3]);
+    for (int i = 0; i < 8; ++i) b[i] = col + i < job.out_features ? __ldg(job.bias + col + i) : 0u;
+    return make_uint4(b[0] | b[1] << 16, b[2] | b[3] << 16, b[4] | b[5] << 16, b[6] | b[7] << 16);
+}
+__device__ __forceinline__ float4 block_bias(const uint4& tile, int block) {
+    const int lane = threadIdx.x & 31, from = block * 4 + ((lane & 7) >> 1);
+    const uint32_t x = __shfl_sync(0xffffffffu, tile.x, from), y = __shfl_sync(0xffffffffu, tile.y, from);
+    const uint32_t z = __shfl_sync(0xffffffffu, tile.z, from), w = __shfl_sync(0xffffffffu, tile.w, from);
+    const uint32_t lo = (lane & 1) ? z : x, hi = (lane & 1) ? w : y;
+    return make_float4(__uint_as_float(lo << 16), __uint_as_float(lo & 0xffff0000u), __uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
 }
 __device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob& job, int row0, int col0, float4 (&z)[8]) {
+    if (job.residual == nullptr) return;                                        // z is not looked at
     #pragma unroll
     for (int k = 0; k < 8; ++k) z[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    if (job.residual == nullptr) return;
     const int lane = threadIdx.x & 31;
     const int col = col0 + (lane & 7) * 4;
     if (col + 4 > job.out_features || (job.out_features & 3) != 0) return;      // read element by element when it is added
@@ -139,9 +150,61 @@ __device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob&
         else z[k] = make_float4(src[0], src[1], src[2], src[3]);
     }
 }
+__device__ __forceinline__ float2 add2(float x0, float x1, float y0, float y1) {
+    uint64_t x = uint64_t(__float_as_uint(x0)) | (uint64_t(__float_as_uint(x1)) << 32);
+    const uint64_t y = uint64_t(__float_as_uint(y0)) | (uint64_t(__float_as_uint(y1)) << 32);
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(y));
+    return make_float2(__uint_as_float(uint32_t(x)), __uint_as_float(uint32_t(x >> 32)));
+}
+// A block of a job whose rows start on 8- or 16-byte boundaries.  One warp a scheduler walks the epilogue, so what it costs is
+// its instructions one after the other (five to seven clocks each): with a branch and an address for every row they were 420 a
+// block, 1500 ns, and a launch of one round of tiles took longer than without the pairs (400 tokens to 9216 columns 21.2
+// us before the pairs, 24.6 with them, 16.7 now; 64 -> 2560 features of 4096 tokens 27.5, 37.4 and 15.5).
+template <bool kFp32, bool kResidual>
+__device__ __forceinline__ void store_rows(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4& bias, const float4 (&z)[8],
+                                           int row0, int col0, unsigned char* stage, int width) {
+    const int lane = threadIdx.x & 31;
+    #pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        *reinterpret_cast<uint4*>(stage + lane * 128 + ((c ^ (lane & 7)) << 4)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+    }
+    __syncwarp();
+    const int chunk = lane & 7, r0 = lane >> 3;
+    float4 x[8];
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) x[k] = *reinterpret_cast<const float4*>(stage + (k * 4 + r0) * 128 + ((chunk ^ ((k & 1) * 4 + r0)) << 4));
+    const size_t at = size_t(row0 + r0) * job.out_features + col0 + chunk * 4;
+    unsigned char* dst = static_cast<unsigned char*>(job.y) + at * (kFp32 ? 4 : 2);
+    const size_t step = size_t(job.out_features) * (kFp32 ? 16 : 8);
+    const int rows = chunk * 4 < width && col0 + chunk * 4 < job.out_features ? args.tokens - row0 - r0 : 0;      // k * 4 of them
+    #pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        float2 lo = add2(x[k].x, x[k].y, bias.x, bias.y), hi = add2(x[k].z, x[k].w, bias.z, bias.w);
+        if (kResidual) {
+            lo = add2(lo.x, lo.y, z[k].x, z[k].y);
+            hi = add2(hi.x, hi.y, z[k].z, z[k].w);
+        }
+        if (kFp32) {
+            if (k * 4 < rows) *reinterpret_cast<float4*>(dst) = make_float4(lo.x, lo.y, hi.x, hi.y);
+        } else {
+            uint2 packed;
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed.x) : "f"(lo.y), "f"(lo.x));
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(packed.y) : "f"(hi.y), "f"(hi.x));
+            if (k * 4 < rows) *reinterpret_cast<uint2*>(dst) = packed;
+        }
+        dst += step;
+    }
+    __syncwarp();
+}
 __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4& bias, const float4 (&z)[8], int row0,
                                             int col0, unsigned char* stage, int width = 32) {
-    if (col0 >= job.out_features || row0 >= args.tokens) return;          // warp-uniform
+    if (col0 >= job.out_features || row0 >= args.tokens) return;          // warp-uniform, as the next
+    if ((job.out_features & 3) == 0) {
+        if (args.y_dtype != HC_F32) store_rows<false, false>(args, job, v, bias, z, row0, col0, stage, width);
+        else if (job.residual != nullptr) store_rows<true, true>(args, job, v, bias, z, row0, col0, stage, width);
+        else store_rows<true, false>(args, job, v, bias, z, row0, col0, stage, width);
+        return;
+    }
     const int lane = threadIdx.x & 31;
     #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -149,34 +212,17 @@ __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& j
     }
     __syncwarp();
     const int chunk = lane & 7, col = col0 + chunk * 4;
-    const bool mine = chunk * 4 < width;
-    const bool vectors = col + 4 <= job.out_features && (job.out_features & 3) == 0;
-    #pragma unroll
+    #pragma unroll 1
     for (int k = 0; k < 8; ++k) {
         const int r = k * 4 + (lane >> 3);
-        if (row0 + r >= args.tokens || !mine) continue;
+        if (row0 + r >= args.tokens || chunk * 4 >= width) continue;
         const float4 x = *reinterpret_cast<const float4*>(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
-        float y[4] = {__fadd_rn(x.x, bias.x), __fadd_rn(x.y, bias.y), __fadd_rn(x.z, bias.z), __fadd_rn(x.w, bias.w)};
+        const float y[4] = {__fadd_rn(x.x, bias.x), __fadd_rn(x.y, bias.y), __fadd_rn(x.z, bias.z), __fadd_rn(x.w, bias.w)};
         const size_t at = size_t(row0 + r) * job.out_features + col;
-        if (vectors) {
-            if (job.residual != nullptr) {
-                y[0] = __fadd_rn(y[0], z[k].x); y[1] = __fadd_rn(y[1], z[k].y); y[2] = __fadd_rn(y[2], z[k].z); y[3] = __fadd_rn(y[3], z[k].w);
-            }
-            if (args.y_dtype == HC_F32) {
-                *reinterpret_cast<float4*>(reinterpret_cast<float*>(job.y) + at) = make_float4(y[0], y[1], y[2], y[3]);
-            } else {
-                uint2 packed;
-                packed.x = uint32_t(float_to_bf16_bits(y[0])) | (uint32_t(float_to_bf16_bits(y[1])) << 16);
-                packed.y = uint32_t(float_to_bf16_bits(y[2])) | (uint32_t(float_to_bf16_bits(y[3])) << 16);
-                *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(job.y) + at) = packed;
-            }
-        } else {
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (col + i >= job.out_features) continue;
-                if (job.residual != nullptr) y[i] = __fadd_rn(y[i], job.residual[at + i]);
-                store_io(job.y, at + i, args.y_dtype, y[i]);
-            }
+        #pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (col + i >= job.out_features) continue;
+            store_io(job.y, at + i, args.y_dtype, job.residual != nullptr ? __fadd_rn(y[i], job.residual[at + i]) : y[i]);
         }
     }
     __syncwarp();
@@ -312,7 +358,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             const bool rows = quad * 32 < args.tokens;              // warp-uniform
             float4 z[8];
             if (rows) load_residual(args, job, quad * 32, where.tn * BN, z);
-            float4 bias = load_bias(job, where.tn * BN);
+            const uint4 bias = load_bias(job, where.tn * BN);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
             #pragma unroll 1
@@ -320,11 +366,8 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 uint32_t v[32];
                 HC_TMEM_LD32(tmem + lane_base + acc * 64 + col, v);
                 tc_wait_ld();
-                if (col > 0) {
-                    load_residual(args, job, quad * 32, where.tn * BN + col, z);
-                    bias = load_bias(job, where.tn * BN + col);
-                }
-                store_block(args, job, v, bias, z, quad * 32, where.tn * BN + col, stage, BN - col);
+                if (col > 0) load_residual(args, job, quad * 32, where.tn * BN + col, z);
+                store_block(args, job, v, block_bias(bias, col >> 5), z, quad * 32, where.tn * BN + col, stage, BN - col);
                 __syncwarp();          // the next tcgen05.ld is warp-wide
             }
             tc_fence_before();
@@ -451,6 +494,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             const int acc = int(count & 1);
             float4 z[8], z_next[8];
             load_residual(args, job, row0, where.tn * BN, z);
+            const uint4 bias = load_bias(job, where.tn * BN);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
             #pragma unroll 1
@@ -459,9 +503,11 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 HC_TMEM_LD32(tmem + lane_base + acc * BN + chunk * 32, v);
                 if (chunk + 1 < BN / 32) load_residual(args, job, row0, where.tn * BN + (chunk + 1) * 32, z_next);
                 tc_wait_ld();
-                store_block(args, job, v, load_bias(job, where.tn * BN + chunk * 32), z, row0, where.tn * BN + chunk * 32, stage);
-                #pragma unroll
-                for (int k = 0; k < 8; ++k) z[k] = z_next[k];
+                store_block(args, job, v, block_bias(bias, chunk), z, row0, where.tn * BN + chunk * 32, stage);
+                if (job.residual != nullptr) {
+                    #pragma unroll
+                    for (int k = 0; k < 8; ++k) z[k] = z_next[k];
+                }
                 __syncwarp();          // the next tcgen05.ld is warp-wide
             }
             tc_fence_before();
