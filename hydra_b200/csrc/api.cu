@@ -258,12 +258,13 @@ void release_pages(hc_kv_cache* cache, int seq, int first_tile) {
 
 // The body shared by hc_attention_prefill and hc_attention_prefill_partial.  With k_fused / v_fused set
 // (hc_layer_step, tokens <= the prologue workspace) the K/V append of the same tokens rides in the Q
-// prologue's launch, pass by pass: one pass, but with bidirectional blocks, which go chunk by chunk.
-// `most_in_ring`: how many tokens a ring layer may take at once (its margin by default).
+// prologue's launch, pass by pass.
+// `most_in_ring`: how many tokens a ring layer may take at once (its margin by default).  `block_chunk`: the chunks that
+// bidirectional blocks end with (the cache's prefill_chunk by default).
 hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, const void* q,
                        void* out, int tokens, int first_position, const hc_attn_params* p,
                        bool partial_mode, cudaStream_t stream, const void* k_fused = nullptr,
-                       const void* v_fused = nullptr, int most_in_ring = -1) {
+                       const void* v_fused = nullptr, int most_in_ring = -1, int block_chunk = 0) {
     if (!ctx || !q || !out) return fail(HC_INVALID_ARGUMENT, "null context or buffer");
     hc_status st = validate_params(cache, layer, p);
     if (st != HC_OK) return st;
@@ -283,9 +284,14 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
     const int mult = p->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
     const bool prep = needs_q_prepare(p, q, tensor);
     int step = prep ? cache->ws.qprep_capacity : tokens;
-    // Bidirectional blocks: chunk by chunk (a block ends with its token's chunk).
-    const int* blocks = p->block_ends;
-    if (blocks) step = std::min(step, cache->prefill_chunk);
+    // Bidirectional blocks: whole chunks of them, their keys appended before any of their queries attends.
+    if (block_chunk <= 0) block_chunk = cache->prefill_chunk;
+    Blocks blocks{block_chunk > 1 ? p->block_ends : nullptr, first_position, block_chunk, 0, 0};     // (a chunk of one token has no block)
+    if (blocks.ends) {
+        blocks.magic = uint32_t((kBlocksProduct + block_chunk - 1) / block_chunk);
+        step = int(std::min<long long>(step, kBlocksProduct / block_chunk - 1));
+        if (step < tokens) step = std::max(step / block_chunk, 1) * block_chunk;
+    }
 
     for (int start = 0; start < tokens; start += step) {
         const int count = std::min(step, tokens - start);
@@ -331,13 +337,12 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
         } else if (ep.gate_layout == HC_GATE_INTERLEAVED) {
             ep.gate = q_rows;
         }
-        if (tensor) {
-            st = tc_prefill(ctx, shape, L, view, seq, q_bf16, count, first_position + start, cache->ws, ep, stream,
-                            blocks ? blocks + start : nullptr);
-        } else {
-            st = simt_prefill(ctx, shape, view, seq, q_bf16, count, first_position + start, ep, stream,
-                              blocks ? blocks + start : nullptr);
-        }
+        Blocks pass = blocks;
+        if (blocks.ends) pass.ends += start;
+        pass.origin = first_position + start;
+        pass.appended = first_position + start + count;
+        if (tensor) st = tc_prefill(ctx, shape, L, view, seq, q_bf16, count, first_position + start, cache->ws, ep, stream, pass);
+        else st = simt_prefill(ctx, shape, view, seq, q_bf16, count, first_position + start, ep, stream, pass);
         if (st != HC_OK) return st;
     }
     return HC_OK;
@@ -1333,21 +1338,25 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
     if (tokens <= 0 || chunk <= 0) return fail(HC_INVALID_ARGUMENT, "tokens and chunk must be positive");
     const int d = params->head_dim;
     const int mult = params->gate_layout == HC_GATE_INTERLEAVED ? 2 : 1;
-    // What a chunk is makes no difference to a bit of the results (but for blocks, which end with their token's chunk),
-    // so the library takes as many tokens at a time as it can: all of the keys are appended, then all of the
-    // queries attend, in one launch each, whose row tiles fill the SMs evenly.  (Chunk by chunk, even with two
+    // What a chunk is makes no difference to a bit of the results (but for blocks, which end with their token's chunk, as the
+    // kernels are told), so the library takes as many tokens at a time as it can: all of the keys are appended, then all
+    // of the queries attend, in one launch each, whose row tiles fill the SMs evenly.  (Chunk by chunk, even with two
     // chunks in flight, every launch had its own ramp and ragged last wave.)  A ring takes what fits beside
     // the window of its first token.
     const hc_layer_store& L = cache->layers[size_t(layer)];
     if (L.ring > 0 && std::min(chunk, tokens) > L.ring_margin) {
         return check_positions(cache, L, first_position, std::min(chunk, tokens), params);
     }
+    // The chunks that blocks end with: the caller's, cut again at the cache's prefill_chunk.  (Where that does not give chunks
+    // of one size the caller's go one by one.)
+    const int block_chunk = std::min(chunk, cache->prefill_chunk);
     int step = chunk;
-    if (!params->block_ends) {
+    if (!params->block_ends || chunk % block_chunk == 0) {
         int most = L.ring > 0 ? L.ring - L.desc.window : tokens;
         most = std::max(std::min(most, cache->ws.qprep_capacity), std::min(chunk, tokens));
         const int parts = (tokens + most - 1) / most;
         step = std::min(most, ((tokens + parts - 1) / parts + kTileKeys - 1) / kTileKeys * kTileKeys);
+        if (params->block_ends && step < tokens) step = std::max(step / block_chunk, 1) * block_chunk;
     }
     for (int start = 0; start < tokens; start += step) {
         const int count = std::min(step, tokens - start);
@@ -1362,7 +1371,7 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
         void* out_rows = const_cast<unsigned char*>(offset_rows(out, size_t(start), size_t(params->q_heads) * d, params->io_dtype));
         if (count > 1 && count <= cache->ws.qprep_capacity) {
             st = prefill_impl(ctx, cache, layer, seq, q_rows, out_rows, count, first_position + start, &local, false,
-                              static_cast<cudaStream_t>(stream), k_rows, v_rows, step);
+                              static_cast<cudaStream_t>(stream), k_rows, v_rows, step, block_chunk);
         } else {
             st = hc_layer_step(ctx, cache, layer, seq, q_rows, k_rows, v_rows, out_rows, count, first_position + start, &local, stream);
         }

@@ -454,7 +454,7 @@ struct MergeRows {
     int first_position;      // prefill
     int tokens;              // query tokens, or batch entries
     int tokens_per_tile;     // prefill: tokens of a row tile, which share their slots
-    int last_of_all;         // prefill: the key that all of them reach to with bidirectional blocks, else -1
+    Blocks blocks;           // prefill
     BatchMeta meta;
 };
 
@@ -481,7 +481,8 @@ merge_rows_kernel(const AttnShape shape, const RowMap map, const MergeRows rows,
     } else {
         const int tile_row0 = (r / rows.tokens_per_tile) * rows.tokens_per_tile;
         first_pos = rows.first_position + tile_row0;
-        last_pos = rows.last_of_all >= 0 ? rows.last_of_all : rows.first_position + min(tile_row0 + rows.tokens_per_tile, rows.tokens) - 1;
+        last_pos = rows.first_position + min(tile_row0 + rows.tokens_per_tile, rows.tokens) - 1;
+        if (rows.blocks.ends != nullptr) last_pos = rows.blocks.reach(last_pos) - 1;
     }
     const int n_parts = min(visible_groups(first_pos, last_pos, shape.window, map.log_segment), slots);
 
@@ -557,7 +558,7 @@ merge_rows_kernel(const AttnShape shape, const RowMap map, const MergeRows rows,
 __global__ void __launch_bounds__(kThreads)
 prefill_rows_kernel(const AttnShape shape, const CacheView cache, int seq,
                     const uint16_t* __restrict__ q, int first_position, const EpilogueArgs ep,
-                    const int* __restrict__ block_ends, int appended) {
+                    const Blocks blocks) {
     extern __shared__ __align__(16) unsigned char raw[];
     const int G = shape.group, d = shape.head_dim;
     const int kv_head = blockIdx.x;
@@ -565,9 +566,9 @@ prefill_rows_kernel(const AttnShape shape, const CacheView cache, int seq,
     const int position = first_position + token;
     const int lo = shape.window > 0 ? max(0, position - shape.window + 1) : 0;
     // A token of a bidirectional block sees on to the block's end (batch.metal:351-352), as far as
-    // keys have been appended.
+    // the token's chunk goes.
     int hi = position;
-    if (block_ends != nullptr) hi = max(position, min(__ldg(block_ends + token), appended) - 1);
+    if (blocks.ends != nullptr) hi = max(position, min(__ldg(blocks.ends + token), blocks.reach(position)) - 1);
 
     FoldState st[2];                              // st[0]: the current segment; st[1]: the row
     SimtSmem sm = carve(raw, G, d, 2, st);
@@ -643,7 +644,7 @@ __global__ void combine_ranks_kernel(const float* __restrict__ gathered, int wor
 
 hc_status simt_prefill(hc_context* ctx, const AttnShape& shape, const CacheView& cache, int seq,
                        const uint16_t* q, int tokens, int first_position, const EpilogueArgs& ep,
-                       cudaStream_t stream, const int* block_ends) {
+                       cudaStream_t stream, const Blocks& blocks) {
     if (tokens <= 0) return HC_OK;
     const size_t smem = simt_smem_bytes(shape.group, shape.head_dim, 2);
     cudaError_t err = cudaFuncSetAttribute(prefill_rows_kernel,
@@ -652,6 +653,8 @@ hc_status simt_prefill(hc_context* ctx, const AttnShape& shape, const CacheView&
     for (int start = 0; start < tokens; start += 32768) {
         const int count = tokens - start < 32768 ? tokens - start : 32768;
         EpilogueArgs sub = ep;
+        Blocks sub_blocks = blocks;
+        if (blocks.ends) sub_blocks.ends += start;
         if (start > 0) {
             // Offsets are in rows; the epilogue indexes rows from its base pointer.
             const size_t out_row = ep.write_partial ? size_t(shape.q_heads) * (shape.head_dim + 2) * 4
@@ -667,7 +670,7 @@ hc_status simt_prefill(hc_context* ctx, const AttnShape& shape, const CacheView&
         dim3 grid(shape.kv_heads, count);
         prefill_rows_kernel<<<grid, kThreads, smem, stream>>>(
             shape, cache, seq, q + size_t(start) * shape.q_heads * shape.head_dim,
-            first_position + start, sub, block_ends ? block_ends + start : nullptr, first_position + tokens);
+            first_position + start, sub, sub_blocks);
         ctx->launches += 1;
         err = cudaGetLastError();
         if (err != cudaSuccess) return check_cuda(err, "prefill_rows_kernel launch");
@@ -790,13 +793,13 @@ hc_status launch_merge_decode(hc_context* ctx, const AttnShape& shape, const Row
 }
 
 hc_status launch_merge_prefill(hc_context* ctx, const AttnShape& shape, const RowMap& map, int tokens, int first_position,
-                               int tokens_per_tile, int last_of_all, const Workspace& ws, int slots, const EpilogueArgs& ep,
+                               int tokens_per_tile, const Blocks& blocks, const Workspace& ws, int slots, const EpilogueArgs& ep,
                                cudaStream_t stream) {
     MergeRows rows{};
     rows.first_position = first_position;
     rows.tokens = tokens;
     rows.tokens_per_tile = tokens_per_tile;
-    rows.last_of_all = last_of_all;
+    rows.blocks = blocks;
     return launch_merge_rows(ctx, shape, map, rows, ws, slots, ep, stream);
 }
 

@@ -404,9 +404,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
             int pos = valid ? w.first_pos + t_local : -1;
             const int lo = args.window > 0 ? max(0, pos - args.window + 1) : 0;
             // From here on `pos` is the last key the row sees: its own, or the end of its bidirectional
-            // block (Sources/HydraMetal/Shaders/batch.metal:351-352) as far as keys have been appended.
-            if (args.block_ends != nullptr && valid) {
-                pos = max(pos, min(__ldg(args.block_ends + (w.first_pos - args.first_position) + t_local), args.appended) - 1);
+            // block (Sources/HydraMetal/Shaders/batch.metal:351-352) as far as the token's chunk goes.
+            if (args.blocks.ends != nullptr && valid) {
+                pos = max(pos, min(__ldg(args.blocks.ends + (w.first_pos - args.first_position) + t_local), args.blocks.reach(pos)) - 1);
             }
             for (int j = 0; j < w.n_tiles; ++j, ++t) {
                 if (int(t & 1) != parity) continue;
@@ -1047,12 +1047,11 @@ static hc_status launch_any(hc_context* ctx, const AttnShape& shape, const TcArg
     return launch_attention_pair(ctx, layer, &args, shape.head_dim, stream);
 }
 
-// Segments and key tiles that a row tile of the pass spans, at most.  `last_of_all`: where every item reaches with
-// bidirectional blocks (else -1).
+// Segments and key tiles that a row tile of the pass spans, at most.
 struct PrefillSpan {
     int tokens_per_tile, mtiles, slots, tiles;
 };
-static PrefillSpan prefill_span(const AttnShape& shape, const RowMap& map, int tokens, int first_position, int last_of_all) {
+static PrefillSpan prefill_span(const AttnShape& shape, const RowMap& map, int tokens, int first_position, const Blocks& blocks) {
     PrefillSpan s;
     // Head_dim 256 and 512: row tiles of 256 rows on pairs of SMs.
     s.tokens_per_tile = (shape.head_dim >= 256 ? 2 : 1) * kRows / shape.group;
@@ -1060,26 +1059,25 @@ static PrefillSpan prefill_span(const AttnShape& shape, const RowMap& map, int t
     s.slots = s.tiles = 1;
     for (int mtile = 0; mtile < s.mtiles; ++mtile) {
         const int first = first_position + mtile * s.tokens_per_tile;
-        const int last = last_of_all >= 0 ? last_of_all : first_position + std::min((mtile + 1) * s.tokens_per_tile, tokens) - 1;
+        int last = first_position + std::min((mtile + 1) * s.tokens_per_tile, tokens) - 1;
+        if (blocks.ends) last = blocks.reach(last) - 1;
         s.slots = std::max(s.slots, visible_groups(first, last, shape.window, map.log_segment));
         s.tiles = std::max(s.tiles, row_tiles(map, first, last, shape.window).count);
     }
     return s;
 }
 
-// One attention launch (and its merge) for `tokens` tokens, with keys appended up to position appended - 1.
-// `merged`: the rows have to leave through the merge kernel.
+// One attention launch (and its merge) for `tokens` tokens.  `merged`: the rows have to leave through the merge kernel.
 static hc_status prefill_pass(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
-                              int seq, const uint16_t* q, int tokens, int first_position, int appended, const Workspace& ws,
-                              const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends, bool merged) {
+                              int seq, const uint16_t* q, int tokens, int first_position, const Workspace& ws,
+                              const EpilogueArgs& ep, cudaStream_t stream, const Blocks& blocks, bool merged) {
     TcArgs args{};
     fill_common_args(args, ctx, shape, cache, q, ws, ep);
     args.tokens = tokens;
     args.first_position = first_position;
     args.seq = seq;
     const bool pairs = shape.head_dim >= 256;
-    const int last_of_all = block_ends ? appended - 1 : -1;
-    const PrefillSpan span = prefill_span(shape, cache.map, tokens, first_position, last_of_all);
+    const PrefillSpan span = prefill_span(shape, cache.map, tokens, first_position, blocks);
     args.mtiles = span.mtiles;
     int slots = span.slots;
     // Whole rows per item, or one item per (row tile, kv head, segment) merged afterwards: whichever
@@ -1095,12 +1093,10 @@ static hc_status prefill_pass(hc_context* ctx, const AttnShape& shape, const hc_
     const int whole_time = ((whole_items + workers - 1) / workers) * (span.tiles + item_cost);
     const int split_time = ((whole_items * slots + workers - 1) / workers) * (std::min(span.tiles, 1 << cache.map.log_segment) + item_cost) +
                            (pairs ? 5 : 10);
-    // With bidirectional blocks every row tile reaches to the last key: whole rows per item (or the general kernel, if the
-    // row state does not fit).
-    if (block_ends && !merged && !can_finish) return simt_prefill(ctx, shape, cache, seq, q, tokens, first_position, ep, stream, block_ends);
-    args.block_ends = block_ends;
-    args.appended = appended;
-    const bool whole = !merged && (block_ends != nullptr || !can_split || (can_finish && whole_time <= split_time));
+    // With bidirectional blocks whole rows per item (or the general kernel, if the row state does not fit).
+    if (blocks.ends && !merged && !can_finish) return simt_prefill(ctx, shape, cache, seq, q, tokens, first_position, ep, stream, blocks);
+    args.blocks = blocks;
+    const bool whole = !merged && (blocks.ends != nullptr || !can_split || (can_finish && whole_time <= split_time));
     if (whole ? !can_finish : !can_split) {
         return fail(HC_KV_OVERFLOW, "prefill: the attention workspace is too small for this chunk (" + std::to_string(tokens) +
                                         " tokens over " + std::to_string(slots) + " segments)");
@@ -1113,15 +1109,14 @@ static hc_status prefill_pass(hc_context* ctx, const AttnShape& shape, const hc_
     args.magic_kv_heads = division_magic(uint32_t(shape.kv_heads), uint32_t(args.n_items));
     const hc_status st = launch_any(ctx, shape, args, layer, stream);
     if (st != HC_OK || args.finish) return st;
-    return launch_merge_prefill(ctx, shape, cache.map, tokens, first_position, span.tokens_per_tile, last_of_all, ws, slots, ep, stream);
+    return launch_merge_prefill(ctx, shape, cache.map, tokens, first_position, span.tokens_per_tile, blocks, ws, slots, ep, stream);
 }
 
 hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer, const CacheView& cache,
                      int seq, const uint16_t* q, int tokens, int first_position, const Workspace& ws,
-                     const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends) {
+                     const EpilogueArgs& ep, cudaStream_t stream, const Blocks& blocks) {
     if (!layer.tmap_k || !layer.tmap_v) return fail(HC_UNSUPPORTED, "this layer has no tensor maps");
     if (tokens <= 0) return HC_OK;
-    const int appended = first_position + tokens;
     const int tokens_per_tile = (shape.head_dim >= 256 ? 2 : 1) * kRows / shape.group;
     // The first `merged` tokens leave through the merge kernel, as many at a time as the workspace has partials for.
     int merged = 0;
@@ -1132,7 +1127,8 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
         // A row tile that sees no key tile of this rank is nobody's item: its rows' partials are the empty fold, which the
         // merge kernel writes.
         for (int start = 0; start < tokens; start += tokens_per_tile) {
-            const int last = block_ends ? appended - 1 : first_position + std::min(start + tokens_per_tile, tokens) - 1;
+            int last = first_position + std::min(start + tokens_per_tile, tokens) - 1;
+            if (blocks.ends) last = blocks.reach(last) - 1;
             if (row_tiles(cache.map, first_position + start, last, shape.window).count <= 0) merged = std::min(start + tokens_per_tile, tokens);
         }
     }
@@ -1143,15 +1139,17 @@ hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_sto
         const bool merge = start < merged;
         count = (merge ? merged : tokens) - start;
         for (; merge && count > 1; count = (count + 1) / 2) {
-            const PrefillSpan span = prefill_span(shape, cache.map, count, first_position + start, block_ends ? appended - 1 : -1);
+            const PrefillSpan span = prefill_span(shape, cache.map, count, first_position + start, blocks);
             const size_t parts = size_t(count) * shape.q_heads * span.slots;
             if (parts * shape.head_dim <= ws.part_o_floats && parts * 2 <= ws.part_ml_floats) break;
         }
         EpilogueArgs part = ep;
         part.out = static_cast<unsigned char*>(ep.out) + size_t(start) * out_row;
         if (ep.gate) part.gate = static_cast<const unsigned char*>(ep.gate) + size_t(start) * gate_row;
-        const hc_status st = prefill_pass(ctx, shape, layer, cache, seq, q + size_t(start) * q_row, count, first_position + start, appended,
-                                          ws, part, stream, block_ends ? block_ends + start : nullptr, merge);
+        Blocks part_blocks = blocks;
+        if (blocks.ends) part_blocks.ends += start;
+        const hc_status st = prefill_pass(ctx, shape, layer, cache, seq, q + size_t(start) * q_row, count, first_position + start, ws, part,
+                                          stream, part_blocks, merge);
         if (st != HC_OK) return st;
     }
     return HC_OK;

@@ -191,6 +191,23 @@ __host__ __device__ __forceinline__ TileRange row_tiles(const RowMap& map, int f
     return owned_tiles(map, first_visible_tile(first_pos, window), last_pos / kTileKeys);
 }
 
+// Bidirectional blocks of a call's tokens: `ends` holds one entry per token of the launch (one past the end of its block, 0 =
+// none; null: no blocks).  A block reaches no further than its token's chunk: chunks of `chunk` tokens from position `origin`
+// on, the last of them up to the last appended key, at appended - 1.
+struct Blocks {
+    const int* ends;
+    int origin, chunk, appended;
+    uint32_t magic;        // ceil(2^32 / chunk): the high word of n * magic is n / chunk while n * chunk < 2^32, chunk > 1
+    // One past the last key that a block may show a token at `position`.
+    __host__ __device__ __forceinline__ int reach(int position) const {
+        const uint32_t n = uint32_t(position - origin);
+        const int end = origin + int(uint32_t((uint64_t(n) * magic) >> 32) + 1) * chunk;
+        return end < appended ? end : appended;
+    }
+};
+// A call of more tokens than this times the chunk goes in parts (see magic).
+constexpr long long kBlocksProduct = 1LL << 32;
+
 // Where sequence `seq`, kv head `kv_head` keeps position `pos`: the plane of the cache (rows of one
 // head) and the row inside it.  Contiguous storage gives every (sequence, head) a plane of its own;
 // paged storage one plane per head, shared by the sequences through the page table.

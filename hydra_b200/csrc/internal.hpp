@@ -210,7 +210,7 @@ hc_status launch_output_gate(hc_context* ctx, void* output, const void* gate, si
 // attn_simt.cu
 hc_status simt_prefill(hc_context* ctx, const AttnShape& shape, const CacheView& cache, int seq,
                        const uint16_t* q, int tokens, int first_position, const EpilogueArgs& ep,
-                       cudaStream_t stream, const int* block_ends = nullptr);
+                       cudaStream_t stream, const Blocks& blocks);
 hc_status simt_decode(hc_context* ctx, const AttnShape& shape, const CacheView& cache,
                       const BatchMeta& meta, int n_seq, const uint16_t* q, const Workspace& ws,
                       const EpilogueArgs& ep, cudaStream_t stream);
@@ -234,7 +234,7 @@ hc_status launch_merge_decode(hc_context* ctx, const AttnShape& shape, const Row
                               int n_seq, const Workspace& ws, const DecodePlan& plan, const EpilogueArgs& ep,
                               cudaStream_t stream);
 hc_status launch_merge_prefill(hc_context* ctx, const AttnShape& shape, const RowMap& map, int tokens,
-                               int first_position, int tokens_per_tile, int last_of_all, const Workspace& ws, int slots,
+                               int first_position, int tokens_per_tile, const Blocks& blocks, const Workspace& ws, int slots,
                                const EpilogueArgs& ep, cudaStream_t stream);
 hc_status launch_combine(hc_context* ctx, const float* gathered, int world, int rows, int q_heads,
                          int d, const EpilogueArgs& ep, cudaStream_t stream);
@@ -250,7 +250,7 @@ hc_status tc_encode_3d(void* map, const void* base, uint64_t cols, uint64_t rows
 bool tc_supported(const AttnShape& shape);
 hc_status tc_prefill(hc_context* ctx, const AttnShape& shape, const hc_layer_store& layer,
                      const CacheView& cache, int seq, const uint16_t* q, int tokens,
-                     int first_position, const Workspace& ws, const EpilogueArgs& ep, cudaStream_t stream, const int* block_ends = nullptr);
+                     int first_position, const Workspace& ws, const EpilogueArgs& ep, cudaStream_t stream, const Blocks& blocks);
 // attn_decode.cu
 // How a tcgen05 decode launch cuts its rows' keys, and the workspace that takes.
 struct TcDecodePlan {

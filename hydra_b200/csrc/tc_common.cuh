@@ -38,11 +38,9 @@ struct TcArgs {
     float* row_state;         // fp32 [thread blocks][d][128], finish only
     // Multipliers for the divisions of tc_item (see fast_div); 0 = divide the ordinary way.
     uint32_t magic_slots, magic_kv_heads;
-    // Bidirectional blocks: per token of the call, one past the end of its block (0 =
-    // none), and the position one past the last key appended.  Every item then reaches to the last
-    // appended key's tile; rows that see nothing of a tile fold its empty partial, a no-op.
-    const int* block_ends;
-    int appended;
+    // With bidirectional blocks an item reaches to the end of its last token's chunk; rows that see nothing of a tile fold
+    // its empty partial, a no-op.
+    Blocks blocks;
 };
 
 // n / d for the small operands of the item list: with magic = ceil(2^32 / d) the high word of
@@ -79,7 +77,8 @@ __device__ __forceinline__ TcItem tc_item(const TcArgs& args, int index) {
     w.row0 = mtile * tokens_per_tile;
     w.valid_tokens = min(tokens_per_tile, args.tokens - w.row0);
     w.first_pos = args.first_position + w.row0;
-    const int last_pos = args.block_ends != nullptr ? args.appended - 1 : w.first_pos + w.valid_tokens - 1;
+    int last_pos = w.first_pos + w.valid_tokens - 1;
+    if (args.blocks.ends != nullptr) last_pos = args.blocks.reach(last_pos) - 1;
     const TileRange tiles = args.finish ? row_tiles(args.map, w.first_pos, last_pos, args.window)
                                         : group_tiles(args.map, w.first_pos, last_pos, args.window, slot, args.map.log_segment);
     w.tile_first = tiles.first;

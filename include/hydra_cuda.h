@@ -143,8 +143,8 @@ typedef struct hc_attn_params {
      * The call is worked in chunks of at most the cache's prefill_chunk tokens and a block reaches no
      * further than the end of its token's chunk, the last key appended by then (the reference reads
      * on, into rows not yet written, when a chunk boundary cuts an image).  The tensor-core kernels
-     * take the buffer (head_dim 64, 128, 256, 512: whole rows per item, every item reaching to the chunk's
-     * last key tile), the general kernel the rest.  Rows outside the blocks keep, bit for bit, the
+     * take the buffer (head_dim 64, 128, 256, 512: whole rows per item, every item reaching to its
+     * last token's chunk's last key tile), the general kernel the rest.  Rows outside the blocks keep, bit for bit, the
      * results of the call without the buffer, and so still equal their decode steps. */
     const int* block_ends;
 } hc_attn_params;
@@ -486,8 +486,8 @@ HC_API hc_status hc_layer_step(hc_context* ctx, hc_kv_cache* cache, int layer, i
 /* hc_layer_step for a whole prompt: `tokens` tokens in chunks of `chunk` (the reference's
  * PrefillRunner loop, Sources/HydraMetal/PrefillRunner.swift:128-184, one call per prompt instead of
  * one per chunk).  The results are bit for bit those of the chunk-by-chunk calls.  Chunks do not
- * matter to the results, except that a bidirectional block ends with its token's chunk, so without
- * block_ends the library takes as many tokens at a time as its workspace holds (64 MB of prepared
+ * matter to the results, except that a bidirectional block ends with its token's chunk, which the kernels
+ * are told: the library takes as many tokens at a time as its workspace holds (64 MB of prepared
  * queries), or on a ring as fit beside the window: usually one prologue and one attention launch. */
 HC_API hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int seq,
                                    const void* q, const void* k, const void* v, void* out,

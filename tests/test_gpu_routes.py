@@ -437,3 +437,49 @@ def test_a_stack_call_that_cannot_run_queues_nothing(hb, ctx):
     status, launches = call(0)
     assert status == 0 and launches > 0
     cache.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, chunk, cache_chunk, ring, io", [
+    (64, 16, 2, 0, 128, 512, False, "bf16"), (64, 16, 2, 200, 96, 96, False, "f32"), (64, 8, 8, 128, 128, 64, True, "bf16"),
+    (128, 8, 2, 0, 100, 512, False, "bf16"), (256, 16, 8, 300, 128, 128, True, "bf16"), (512, 8, 1, 0, 77, 200, False, "f32"),
+    (256, 4, 4, 0, 300, 128, False, "bf16"), (96, 4, 2, 0, 60, 512, False, "bf16"),
+])
+def test_blocks_of_a_prompt_end_with_their_chunks(hb, ctx, d, qh, kvh, window, chunk, cache_chunk, ring, io):
+    """A prompt with bidirectional blocks in one call: the bits of the chunk-by-chunk calls, whichever chunk boundaries cut
+    a block and however many chunks go in a launch (chunks that the cache's own do not divide included)."""
+    import torch
+    tokens, first = 1100, 0 if ring else 131
+    rng = np.random.default_rng(d + chunk)
+    q, k, v = (tl.normal_bf16(rng, (tokens, h, d)) for h in (qh, kvh, kvh))
+    old = [tl.normal_bf16(rng, (max(first, 1), kvh, d)) for _ in range(2)]
+    ends = np.zeros(tokens, np.int32)
+    for at, n in ((3, 40), (90, 120), (250, 300), (600, 1), (700, 390)):
+        ends[at:at + n] = first + at + n
+    device_ends = torch.from_numpy(ends).cuda()
+    storage = hb.capi.HC_STORAGE_RING if ring else hb.capi.HC_STORAGE_LINEAR
+    outs, rows = [], []
+    for at_once in (False, True):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 1536, window=window, io=io, prefill_chunk=cache_chunk, storage=storage)
+        if first:
+            layer.append(old[0], old[1], 0)
+        qd, kd, vd, out = tl.to_device(q, io), tl.to_device(k, io), tl.to_device(v, io), tl.device_empty((tokens, qh, d), io)
+        be, cache = layer.backend, layer.cache
+        if at_once:
+            be.prefill_chunks(cache, 0, qd, kd, vd, out, tokens, first, chunk, dataclasses.replace(layer.params, block_ends=device_ends))
+        else:
+            part = min(chunk, cache_chunk)
+            edges = sorted({a for c in range(0, tokens, chunk) for a in range(c, min(c + chunk, tokens), part)})
+            for a, b in zip(edges, edges[1:] + [tokens]):
+                params = dataclasses.replace(layer.params, block_ends=device_ends[a:])
+                be.write_key_value(cache, 0, kd[a:], vd[a:], b - a, first + a, params)
+                be.attention_prefill(cache, 0, qd[a:], out[a:], b - a, first + a, params)
+        ctx.check()
+        outs.append(tl.to_host(out))
+        layer.close()
+    assert np.array_equal(outs[0], outs[1])
+    edges = [a for c in range(0, tokens, chunk) for a in range(c, min(c + chunk, tokens), min(chunk, cache_chunk))] + [tokens]
+    clamped = np.array([min(e, first + next(x for x in edges if x > t)) if e else 0 for t, e in enumerate(ends)])
+    keys, values = (np.concatenate([o[:first], x]) for o, x in zip(old, (k, v)))
+    some = np.arange(0, tokens, 7)
+    want = ho.attention_rows(q[some], first + some, keys, values, 1 / np.sqrt(d), window, block_ends=clamped[some])
+    assert tl.within_tolerance(outs[1][some], want, bf16_output=io == "bf16")
