@@ -225,14 +225,19 @@ bool use_tensor_path(const hc_attn_params* p, const AttnShape& shape, hc_status*
 hc_status ensure_pages(hc_kv_cache* cache, const hc_layer_store& L, int seq, int first, int tokens, cudaStream_t stream) {
     if (!cache->pages_dev || L.ring != 0 || tokens <= 0) return HC_OK;
     int* table = cache->pages_host + size_t(seq) * cache->pages_per_seq;
-    int lo = -1, hi = -1;
-    for (int tile = first / kTileKeys; tile <= (first + tokens - 1) / kTileKeys; ++tile) {
-        if (table[tile] >= 0) continue;
-        if (cache->free_pages.empty()) {
+    const int first_tile = first / kTileKeys, last_tile = (first + tokens - 1) / kTileKeys;
+    // All or none: a page taken by an append that fails would stay in the host's table and never reach the device's.
+    size_t needed = 0;
+    for (int tile = first_tile; tile <= last_tile; ++tile) {
+        if (table[tile] < 0 && ++needed > cache->free_pages.size()) {
             return fail(HC_KV_OVERFLOW, "the paged cache is out of pages (" + std::to_string(cache->total_pages) +
                                             " of 128 rows): sequence " + std::to_string(seq) + " needs one for position " +
                                             std::to_string(tile * kTileKeys));
         }
+    }
+    int lo = -1, hi = -1;
+    for (int tile = first_tile; tile <= last_tile; ++tile) {
+        if (table[tile] >= 0) continue;
         table[tile] = cache->free_pages.back();
         cache->free_pages.pop_back();
         if (lo < 0) lo = tile;

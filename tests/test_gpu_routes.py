@@ -483,3 +483,27 @@ def test_blocks_of_a_prompt_end_with_their_chunks(hb, ctx, d, qh, kvh, window, c
     some = np.arange(0, tokens, 7)
     want = ho.attention_rows(q[some], first + some, keys, values, 1 / np.sqrt(d), window, block_ends=clamped[some])
     assert tl.within_tolerance(outs[1][some], want, bf16_output=io == "bf16")
+
+
+def test_pages_of_an_append_that_ran_out_are_not_lost(hb, ctx):
+    """An append that finds too few free pages takes none: the pages it could have had serve the next one."""
+    qh, kvh, d = 4, 2, 64
+    q, k, v = _inputs(5, 400, qh, kvh, d)
+    outs = []
+    for pages in (0, 4):
+        cache = hb.KVCache(ctx, [dict(q_heads=qh, kv_heads=kvh, head_dim=d, window=0)], 512, max_seqs=2, total_pages=pages)
+        be = hb.AttentionBackend(ctx)
+        params = hb.AttnParams(q_heads=qh, kv_heads=kvh, head_dim=d, sm_scale=0.125, io_dtype=hb.capi.HC_BF16)
+        qd, kd, vd = tl.to_device(q), tl.to_device(k), tl.to_device(v)
+        be.write_key_value(cache, 0, kd, vd, 200, 0, params, seq=0)              # two pages
+        if pages:
+            with pytest.raises(hb.HydraCudaError):
+                be.write_key_value(cache, 0, kd, vd, 400, 0, params, seq=1)      # needs four
+            assert cache.free_pages == 2
+        out = tl.device_empty((256, qh, d))
+        be.write_key_value(cache, 0, kd, vd, 256, 0, params, seq=1)
+        be.attention_prefill(cache, 0, qd, out, 256, 0, params, seq=1)
+        ctx.check()
+        outs.append(tl.to_host(out))
+        cache.close()
+    assert np.array_equal(outs[0], outs[1])
