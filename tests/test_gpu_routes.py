@@ -507,3 +507,34 @@ def test_pages_of_an_append_that_ran_out_are_not_lost(hb, ctx):
         outs.append(tl.to_host(out))
         cache.close()
     assert np.array_equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("qh, kvh, tokens, first, io, gated", [
+    (16, 2, 2300, 0, "bf16", False),      # Gemma's wide layer: the prompt crosses a segment of 2048 keys
+    (16, 1, 500, 3900, "f32", True),      # three segments, 16 heads a group, the gated epilogue
+    (4, 4, 300, 2000, "bf16", True),
+    (8, 1, 40, 4200, "f32", False),       # few rows: segments as items, merged
+])
+def test_head_dim_512_beyond_a_segment(hb, ctx, qh, kvh, tokens, first, io, gated):
+    """Whole rows that carry their second fold from segment to segment in two halves of 256 columns, and segments merged
+    afterwards: against the oracle, against the rows decoded one by one, and cut at another place."""
+    d, total = 512, first + tokens
+    rng = np.random.default_rng(total)
+    q = tl.normal_bf16(rng, (tokens, qh, d))
+    k, v = (tl.normal_bf16(rng, (total, kvh, d)) for _ in range(2))
+    gate = tl.normal_bf16(rng, (tokens, qh, d)) if gated else None
+    sinks = tl.normal_bf16(rng, (qh,))
+    layer = tl.Layer(hb, ctx, qh, kvh, d, 4608, sinks=sinks, io=io, prefill_chunk=512)
+    layer.append(k, v, 0)
+    prompt = layer.prefill(q, first, gate=gate)
+    some = sorted({0, 1, 15, 16, 17, tokens // 2, tokens - 1} | {t for t in (2047 - first, 2048 - first, 2049 - first) if 0 <= t < tokens})
+    for t in some:
+        one = layer.decode(q[t:t + 1], [first + t], gate=None if gate is None else gate[t:t + 1])
+        assert np.array_equal(one[0], prompt[t]), t
+    cut = tokens // 3
+    parts = [layer.prefill(q[a:b], first + a, gate=None if gate is None else gate[a:b]) for a, b in ((0, cut), (cut, tokens))]
+    assert np.array_equal(np.concatenate(parts), prompt)
+    want = ho.attention_rows(q[some], first + np.asarray(some), k, v, 1 / np.sqrt(d), 0, sinks=sinks,
+                             gate=None if gate is None else gate[some])
+    assert tl.within_tolerance(prompt[some], want, bf16_output=io == "bf16")
+    layer.close()
