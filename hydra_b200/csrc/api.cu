@@ -1472,15 +1472,23 @@ hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_
 // pieces are large; the first is short because nothing runs until it is there, and the last ones are, because their
 // kernel and their way back have nothing left to hide behind: 1, 2, 4, 4, 3 and 2 sixteenths of the call, in
 // steps of `quantum` tokens (about 2 MB of queries).  (4096 GPT-OSS tokens as eight pieces of 512 with a copy each
-// for q, k and v: 1410 us, now 1222; the two directions' bytes at the rate of both together take 810.)
-static int host_piece_end(int start, int tokens, int quantum, int most) {
+// for q, k and v: 1410 us, now 1212; the two directions' bytes at the rate of both together take 810.)
+// A call of at most two quanta goes as two halves once half of its queries take longer than a copy's 15 us, else at once
+// (GPT-OSS tokens in bf16, at once or as a quantum and the rest: 200 113 us, 300 152, 400 182; as halves 107, 135 and 170).
+constexpr size_t kHostHalves = size_t(3) << 19;      // bytes of queries
+static int host_piece_end(int start, int tokens, int quantum, int most, size_t q_row) {
     static const int kEnds[6] = {1, 3, 7, 11, 14, 16};
     int end = tokens;
-    for (int i = 5; i >= 0; --i) {
-        const long long at = ((long long)tokens * kEnds[i] / 16 + quantum - 1) / quantum * quantum;
-        if (at > start) end = int(std::min<long long>(at, tokens));
+    if (tokens <= 2 * quantum) {
+        const int half = ((tokens + 1) / 2 + 15) / 16 * 16;
+        if (start < half && q_row * tokens > kHostHalves) end = half;
+    } else {
+        for (int i = 5; i >= 0; --i) {
+            const long long at = ((long long)tokens * kEnds[i] / 16 + quantum - 1) / quantum * quantum;
+            if (at > start) end = int(std::min<long long>(at, tokens));
+        }
     }
-    return std::min(end, start + most);
+    return std::min(std::min(end, tokens), start + most);
 }
 
 // The body of the host-buffer entry points.  A piece's inputs are copied in on one stream while the pieces before it
@@ -1501,7 +1509,12 @@ static hc_status host_pieces(hc_context* ctx, hc_kv_cache* cache, int layer, int
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t kv_all = align(kv_row * tokens);
     const size_t least = kStageSlack + (q_row + g_row + o_row) * std::min(chunk, tokens);
-    const bool kv_ahead = kv_all <= cache->stage_bytes / 2 && cache->stage_bytes - kv_all >= least + 256;
+    const int quantum = int(((size_t(2) << 20) / q_row / kTileKeys + 1) * kTileKeys);
+    // The schedule's largest piece has to fit a slot, or chunks with their own K and V go (4096 fp32 tokens of 64 heads of
+    // 64, in pieces cut to the slots: 2437 us, chunk by chunk 2264).
+    const int largest = tokens <= 2 * quantum ? (tokens + 31) / 2 : (tokens / 4 + quantum - 1) / quantum * quantum;
+    const bool scheduled = kv_all + kStageSlack + (q_row + g_row + o_row) * std::min(largest, tokens) <= cache->stage_bytes;
+    const bool kv_ahead = scheduled && kv_all <= cache->stage_bytes / 2 && cache->stage_bytes - kv_all >= least + 256;
     const size_t slots_at = kv_ahead ? 2 * kv_all : 0;
     const size_t slot_bytes = (cache->stage_bytes - slots_at / 2) & ~size_t(255);
     const size_t piece_row = q_row + g_row + o_row + (kv_ahead ? 0 : 2 * kv_row);
@@ -1513,11 +1526,9 @@ static hc_status host_pieces(hc_context* ctx, hc_kv_cache* cache, int layer, int
     int most = int(std::min<size_t>((slot_bytes - kStageSlack) / piece_row, size_t(tokens)));
     // (A piece beyond the prepared-query buffer is appended by a call of its own, which takes the ring's margin at most.)
     if (L.ring > 0) most = std::min(most, std::max(std::min(L.ring - L.desc.window, cache->ws.qprep_capacity), std::min(chunk, tokens)));
-    if (params->block_ends) most = chunk;
-    const int quantum = int(((size_t(2) << 20) / q_row / kTileKeys + 1) * kTileKeys);
-    auto end_of = [&](int start) {
-        return params->block_ends ? std::min(start + chunk, tokens) : host_piece_end(start, tokens, quantum, most);
-    };
+    const bool by_chunk = params->block_ends || !scheduled;
+    if (by_chunk) most = chunk;
+    auto end_of = [&](int start) { return by_chunk ? std::min(start + chunk, tokens) : host_piece_end(start, tokens, quantum, most, q_row); };
     // One piece has nothing to overlap with: everything in the caller's stream, no events.
     const bool one = end_of(0) == tokens;
     cudaStream_t in = one ? s : cache->copy_in, back = one ? s : cache->copy_out;
@@ -1537,10 +1548,13 @@ static hc_status host_pieces(hc_context* ctx, hc_kv_cache* cache, int layer, int
     // The copies may start once the work already in the caller's stream has been reached.
     record(cache->entry, s);
     wait(in, cache->entry);
-    if (kv_ahead) {
+    // (Copies of up to 64 KB: a large one behind them starts 8 us late, they behind it do not: 64 GPT-OSS tokens 73 us, 64.5.)
+    const bool kv_last = kv_ahead && one && kv_row * tokens <= (size_t(64) << 10);
+    auto copy_kv = [&] {
         copy(stage, hk, kv_row * tokens, cudaMemcpyHostToDevice, in);
         copy(stage + kv_all, hv, kv_row * tokens, cudaMemcpyHostToDevice, in);
-    }
+    };
+    if (kv_ahead && !kv_last) copy_kv();
     int index = 0;
     for (int start = 0, end = 0; start < tokens && st == HC_OK && err == cudaSuccess; start = end, ++index) {
         end = end_of(start);
@@ -1557,6 +1571,7 @@ static hc_status host_pieces(hc_context* ctx, hc_kv_cache* cache, int layer, int
             copy(dev_k, hk + size_t(start) * kv_row, kv_row * count, cudaMemcpyHostToDevice, in);
             copy(dev_v, hv + size_t(start) * kv_row, kv_row * count, cudaMemcpyHostToDevice, in);
         }
+        if (kv_last) copy_kv();
         if (sep_gate) copy(dev_g, hg + size_t(start) * o_row, o_row * count, cudaMemcpyHostToDevice, in);
         record(cache->in_done[slot], in);
         wait(s, cache->in_done[slot]);

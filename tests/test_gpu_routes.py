@@ -538,3 +538,33 @@ def test_head_dim_512_beyond_a_segment(hb, ctx, qh, kvh, tokens, first, io, gate
                              gate=None if gate is None else gate[some])
     assert tl.within_tolerance(prompt[some], want, bf16_output=io == "bf16")
     layer.close()
+
+
+@pytest.mark.parametrize("qh, kvh, d, tokens, chunk, io", [
+    (64, 8, 64, 33, 512, "bf16"),       # at once, K and V behind the queries
+    (64, 8, 64, 150, 128, "bf16"),      # at once, K and V ahead
+    (64, 8, 64, 201, 128, "bf16"),      # two halves
+    (64, 8, 64, 767, 256, "bf16"),
+    (64, 8, 64, 769, 256, "bf16"),      # the schedule of six
+    (64, 8, 64, 1100, 128, "f32"),      # chunk by chunk: the slots are too small for it
+    (16, 2, 256, 257, 64, "f32"),
+])
+def test_host_prompt_schedules(hb, ctx, qh, kvh, d, tokens, chunk, io):
+    """A host prompt on both sides of every line its pieces are drawn by."""
+    import torch
+    dtype = torch.bfloat16 if io == "bf16" else torch.float32
+    host = [torch.from_numpy(a).to(dtype).pin_memory() for a in _inputs(tokens, tokens, qh, kvh, d)]
+    outs, rows = [], []
+    for on_host in (False, True):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 1280, io=io, prefill_chunk=chunk, rope_inv_freq=ho.inverse_frequencies(d, 10000.0))
+        q, k, v = host if on_host else [t.cuda() for t in host]
+        out = torch.zeros((tokens, qh, d), dtype=dtype)
+        out = out.pin_memory() if on_host else out.cuda()
+        call = layer.backend.prefill_host if on_host else layer.backend.prefill_chunks
+        call(layer.cache, 0, q, k, v, out, tokens, 0, chunk, layer.params)
+        ctx.check()
+        outs.append(tl.to_host(out))
+        rows.append(tl.read_cache(layer.cache, 0, tokens, kvh, d))
+        layer.close()
+    assert np.array_equal(outs[0], outs[1])
+    assert np.array_equal(rows[0][0], rows[1][0]) and np.array_equal(rows[0][1], rows[1][1])
