@@ -513,7 +513,7 @@ def run_cuda(args):
     events = []
 
     def one_step(index: int):
-        """The headline step: the prompt through hc_prefill_chunks (per chunk one prologue launch for
+        """The headline step: the prompt through hc_prefill_chunks (one prologue launch for
         k, v and q + the attention kernel), then one decode step (hc_layer_step with one token)."""
         s = index % n_sets
         backend.prefill_chunks(cache, 0, q_sets[s], k_sets[s], v_sets[s], o_sets[s], cfg.prompt, 0, cfg.chunk, params,
@@ -671,7 +671,7 @@ def run_cuda(args):
             "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "bf16",
             "data": "synthetic",
             "config": {"workload": "C2: 64q/8kv d64 full causal, 4096-token prompt in 512-token chunks "
-                                   "(hc_prefill_chunks: KV append + attention per chunk), then one decode step at context 4096",
+                                   "(hc_prefill_chunks: KV append + attention), then one decode step at context 4096",
                        "kv_heads_per_gpu": per, "parallelism": f"kv-head shard x{world}",
                        "l2": f"{n_sets} rotating copies of the prompt's buffers (> 2x L2); decode flushes L2"},
             "roofline": roofline, "decode": decode,

@@ -385,9 +385,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
         }
     }
     } else if (wg == 1 || wg == 2) {
-        // ===== softmax: warpgroup 1 takes the even tiles of the stream (S buffer 0), warpgroup 2 the
-        // odd ones (S buffer 1), so one group's exp2 phase overlaps the other's wait, load and
-        // maximum.  Thread = row; the row is read twice (maximum, then weights) to stay in registers. =====
+        // ===== softmax: warpgroup 1 takes the even tiles of the stream, warpgroup 2 the odd ones, so one
+        // group's exp2 phase overlaps the other's wait, load and maximum.  Thread = row: at d = 64 held
+        // in registers whole, at d = 128 read twice (maximum, then weights). =====
         if constexpr (LT::kRegsSoftmax > 128) reg_alloc<LT::kRegsSoftmax>(); else reg_dealloc<LT::kRegsSoftmax>();
         const int parity = wg - 1;
         const int quad = warp & 3;                           // the TMEM lane quadrant this warp may touch

@@ -221,9 +221,4 @@ __device__ __forceinline__ int cache_row(const RowMap& map, int seq, int pos) {
     return row_of_position(map, pos);
 }
 
-// First physical row of absolute tile j (callers only ask for tiles they own).
-__host__ __device__ __forceinline__ int row_of_tile(const RowMap& map, int tile) {
-    return row_of_position(map, tile * kTileKeys);
-}
-
 }  // namespace hc

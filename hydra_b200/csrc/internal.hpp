@@ -41,7 +41,6 @@ struct AttnShape {
     int count_sink;     // 0 on ranks > 0 of a sequence-sharded cache
 };
 
-// What the prologue does to one of q, k, v.
 // Launch with programmatic stream serialisation allowed (see pdl_wait in common.cuh).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
@@ -59,6 +58,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     return cudaLaunchKernelEx(&config, kernel, static_cast<KArgs>(args)...);
 }
 
+// What the prologue does to one of q, k, v.
 struct PrepJob {
     const void* src;
     int src_dtype;

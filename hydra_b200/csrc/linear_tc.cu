@@ -7,8 +7,7 @@
 // (Sources/HydraReference/ReferenceLayer.swift:104-113).  The weight keeps the reference's layout:
 // row-major [out_features][in_features] bf16, so both operands are K-major and no transpose is
 // needed.  Where the reference gives every output row its own threadgroup that streams that row
-// of the weight once per token, this kernel computes a 128 x 256 tile of y per step, so a weight
-// tile fetched by TMA serves 128 tokens.
+// of the weight once per token, a weight tile fetched by TMA serves up to 256 tokens here.
 //
 // Two kernels.  A call of up to 128 tokens reads the weights once and little else: linear_few_kernel, one CTA
 // per SM, narrow output tiles, up to nine 16 to 40 KB stages in flight.  Prompts are bound by the tensor pipe:

@@ -326,8 +326,8 @@ HC_API hc_status hc_kv_append_batch(hc_context* ctx, hc_kv_cache* cache, int lay
  * ForwardEncoder.attentionPrefill (Sources/HydraMetal/ForwardEncoder.swift:590-631): causal
  * attention of `tokens` queries at positions first_position .. first_position + tokens - 1 over
  * the cache (the chunk's own keys must have been appended first).  The q norm and rotation asked
- * for in params are applied to q first; the sigmoid gate is applied last.  Image blocks
- * (blockEnds) are not supported: text only. */
+ * for in params are applied to q first; the sigmoid gate is applied last.  With params->block_ends the
+ * call is worked in chunks of the cache's prefill_chunk, with which blocks end. */
 HC_API hc_status hc_attention_prefill(hc_context* ctx, hc_kv_cache* cache, int layer, int seq,
                                       const void* q, void* out, int tokens, int first_position,
                                       const hc_attn_params* params, void* stream);

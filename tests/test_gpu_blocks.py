@@ -2,7 +2,7 @@
 (Sources/HydraMetal/BatchEncoder.swift:210-217), the `blocks` buffer of attention_prefill
 (Sources/HydraMetal/Shaders/batch.metal:322-324, 340-352).  A token inside a block (an image's
 tokens) sees the whole block, forward as well as back; the window still bounds where its range
-starts.  The tensor-core kernels take the buffer for head_dim 64, 128 and 256, the general kernel for
+starts.  The tensor-core kernels take the buffer for head_dim 64, 128, 256 and 512, the general kernel for
 the rest.  The oracle applies the shader's loop bound to the reference's double-precision attention.
 """
 import dataclasses
@@ -73,7 +73,7 @@ def test_blocks_match_the_oracle(q_heads, kv_heads, d, window, prefix):
     causal = ho.attention_rows(q[prefix:], positions, k, v, layer.params.sm_scale, window)
     assert tl.max_abs(want[10], causal[10]) > 1e-3
     # Tokens outside the blocks are untouched by it: bit for bit the rows of the call without the
-    # buffer, on the tensor-core kernels (head_dim 64, 128, 256) and on the general ones (512, or forced).
+    # buffer, on the tensor-core kernels and on the general ones (forced).
     outside = ends == 0
     plain = layer.prefill(q[prefix:], prefix)
     assert np.array_equal(have[outside], plain[outside])
