@@ -264,8 +264,9 @@ void release_pages(hc_kv_cache* cache, int seq, int first_tile) {
 // The body shared by hc_attention_prefill and hc_attention_prefill_partial.  With k_fused / v_fused set
 // (hc_layer_step, tokens <= the prologue workspace) the K/V append of the same tokens rides in the Q
 // prologue's launch, pass by pass.
-// `most_in_ring`: how many tokens a ring layer may take at once (its margin by default).  `block_chunk`: the chunks that
-// bidirectional blocks end with (the cache's prefill_chunk by default).
+// `most_in_ring`: how many tokens a ring layer may take at once (its margin by default); more than fit beside the window of
+// the first attend in the layer's prompt store, and the ring gets the last rows of them (k_fused set).  `block_chunk`: the
+// chunks that bidirectional blocks end with (the cache's prefill_chunk by default).
 hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, const void* q,
                        void* out, int tokens, int first_position, const hc_attn_params* p,
                        bool partial_mode, cudaStream_t stream, const void* k_fused = nullptr,
@@ -282,7 +283,10 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
     st = check_shard_mode(cache, partial_mode);
     if (st != HC_OK) return st;
     const AttnShape shape = shape_of(cache, p, partial_mode);
-    const CacheView view = view_of(cache, L);
+    const bool beside = L.prompt && k_fused && tokens > L.ring - L.desc.window;
+    const hc_layer_store& S = beside ? *L.prompt : L;
+    const int store_seq = beside ? 0 : seq;
+    const CacheView view = view_of(cache, S);
     const bool tensor = use_tensor_path(p, shape, &st);
     if (st != HC_OK) return st;
     const int d = p->head_dim;
@@ -322,8 +326,16 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
             args.tokens = count;
             args.first_position = first_position + start;
             args.batched = 0;
-            args.seq = seq;
+            args.seq = store_seq;
             args.cache = view;
+            if (beside) {
+                const int at = first_position + start;
+                args.also = view_of(cache, L);
+                args.also_seq = seq;
+                args.also_from = std::max(at, at + count - L.ring);
+                st = launch_copy_rows(ctx, args.also, seq, view, first_visible_tile(at, p->window) * kTileKeys, at, d, stream);
+                if (st != HC_OK) return st;
+            }
             st = launch_prepare(ctx, args, stream);
             if (st != HC_OK) return st;
             if (prep) q_bf16 = prepared;
@@ -346,8 +358,8 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
         if (blocks.ends) pass.ends += start;
         pass.origin = first_position + start;
         pass.appended = first_position + start + count;
-        if (tensor) st = tc_prefill(ctx, shape, L, view, seq, q_bf16, count, first_position + start, cache->ws, ep, stream, pass);
-        else st = simt_prefill(ctx, shape, view, seq, q_bf16, count, first_position + start, ep, stream, pass);
+        if (tensor) st = tc_prefill(ctx, shape, S, view, store_seq, q_bf16, count, first_position + start, cache->ws, ep, stream, pass);
+        else st = simt_prefill(ctx, shape, view, store_seq, q_bf16, count, first_position + start, ep, stream, pass);
         if (st != HC_OK) return st;
     }
     return HC_OK;
@@ -814,7 +826,7 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         if (d == 64 || d == 128 || d == 256 || d == 512) {
             prefill_o_floats = std::max(prefill_o_floats, size_t(std::max(ctx->sm_count, 1)) * std::min(d, 256) * 128);
         }
-        st = tc_make_tensor_maps(cache, L);
+        st = tc_make_tensor_maps(L, size_t(paged ? 1 : max_seqs) * L.desc.kv_heads);
     }
     if (st == HC_OK && max_q_elems == 0) st = fail(HC_UNSUPPORTED, "no layer keeps a key/value history");
     if (st == HC_OK) {
@@ -838,7 +850,15 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         const size_t part_ml_at = part_o_at + align(part_o_floats * sizeof(float));
         const size_t tickets_at = part_ml_at + align(part_ml_floats * sizeof(float));
         const size_t stage_at = tickets_at + align(n_tickets * sizeof(unsigned));
-        err = cudaMalloc(&cache->workspace_dev, stage_at + 2 * cache->stage_bytes);
+        // Where prompts longer than a ring's margin attend: the window of the first token and a call's tokens, whole key tiles
+        // at both ends.  All ring layers share it.
+        const size_t prompt_at = stage_at + align(2 * cache->stage_bytes);
+        auto prompt_rows = [&](const hc_layer_store& L) { return round_up(L.desc.window + ws.qprep_capacity + 2 * kTileKeys, kTileKeys); };
+        size_t prompt_bytes = 0;
+        for (const hc_layer_store& L : cache->layers) {
+            if (L.ring > 0) prompt_bytes = std::max(prompt_bytes, 4 * size_t(L.desc.kv_heads) * prompt_rows(L) * L.desc.head_dim);
+        }
+        err = cudaMalloc(&cache->workspace_dev, prompt_at + prompt_bytes);
         if (err == cudaSuccess) {
             unsigned char* base = static_cast<unsigned char*>(cache->workspace_dev);
             ws.qprep = reinterpret_cast<uint16_t*>(base);
@@ -847,6 +867,21 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
             ws.tickets = reinterpret_cast<unsigned*>(base + tickets_at);
             cache->stage_dev = base + stage_at;
             err = cudaMemset(ws.tickets, 0, n_tickets * sizeof(unsigned));
+            // Zeros, as the caches: a row no key was written to yet has weight 0 and must not be a NaN.
+            if (err == cudaSuccess && prompt_bytes > 0) err = cudaMemset(base + prompt_at, 0, prompt_bytes);
+            for (size_t i = 0; i < cache->layers.size() && st == HC_OK; ++i) {
+                hc_layer_store& L = cache->layers[i];
+                if (L.ring == 0) continue;
+                L.prompt = std::make_unique<hc_layer_store>();
+                hc_layer_store& P = *L.prompt;
+                P.desc = L.desc;
+                P.ring = P.capacity = prompt_rows(L);
+                P.log_segment = L.log_segment;
+                P.keeps_history = true;
+                P.k = reinterpret_cast<uint16_t*>(base + prompt_at);
+                P.v = P.k + size_t(L.desc.kv_heads) * P.capacity * L.desc.head_dim;
+                st = tc_make_tensor_maps(P, size_t(L.desc.kv_heads));
+            }
         }
         if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&cache->copy_in, cudaStreamNonBlocking);
         if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&cache->copy_out, cudaStreamNonBlocking);
@@ -876,6 +911,7 @@ void hc_kv_cache_destroy(hc_kv_cache* cache) {
     for (hc_layer_store& L : cache->layers) {
         if (L.k) cudaFree(L.k);
         tc_free_tensor_maps(L);
+        if (L.prompt) tc_free_tensor_maps(*L.prompt);
     }
     if (cache->workspace_dev) cudaFree(cache->workspace_dev);
     if (cache->pages_dev) cudaFree(cache->pages_dev);
@@ -1347,7 +1383,7 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
     // kernels are told), so the library takes as many tokens at a time as it can: all of the keys are appended, then all
     // of the queries attend, in one launch each, whose row tiles fill the SMs evenly.  (Chunk by chunk, even with two
     // chunks in flight, every launch had its own ramp and ragged last wave.)  A ring takes what fits beside
-    // the window of its first token.
+    // the window of its first token; a longer prompt attends beside it.
     const hc_layer_store& L = cache->layers[size_t(layer)];
     if (L.ring > 0 && std::min(chunk, tokens) > L.ring_margin) {
         return check_positions(cache, L, first_position, std::min(chunk, tokens), params);
@@ -1357,7 +1393,7 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
     const int block_chunk = std::min(chunk, cache->prefill_chunk);
     int step = chunk;
     if (!params->block_ends || chunk % block_chunk == 0) {
-        int most = L.ring > 0 ? L.ring - L.desc.window : tokens;
+        int most = L.ring > 0 && !L.prompt ? L.ring - L.desc.window : tokens;
         most = std::max(std::min(most, cache->ws.qprep_capacity), std::min(chunk, tokens));
         const int parts = (tokens + most - 1) / most;
         step = std::min(most, ((tokens + parts - 1) / parts + kTileKeys - 1) / kTileKeys * kTileKeys);

@@ -955,7 +955,7 @@ hc_status tc_encode_3d(void* map, const void* base, uint64_t cols, uint64_t rows
 
 bool tc_supported(const AttnShape& shape) { return dim_ok(shape.head_dim) && shape.group <= 16; }
 
-hc_status tc_make_tensor_maps(hc_kv_cache* cache, hc_layer_store& layer) {
+hc_status tc_make_tensor_maps(hc_layer_store& layer, size_t planes) {
     if (!dim_ok(layer.desc.head_dim)) return HC_OK;
     EncodeTiledFn encode = encode_tiled();
     if (!encode) return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from this driver");
@@ -963,9 +963,7 @@ hc_status tc_make_tensor_maps(hc_kv_cache* cache, hc_layer_store& layer) {
     void** maps[3] = {&layer.tmap_k, &layer.tmap_v, &layer.tmap_k64};
     for (int which = 0; which < (d >= 256 ? 3 : 2); ++which) {
         CUtensorMap* map = new CUtensorMap;
-        const bool paged = cache->pages_dev != nullptr && layer.ring == 0;       // one plane per head, shared
-        const cuuint64_t dims[3] = {cuuint64_t(d), cuuint64_t(layer.capacity),
-                                    cuuint64_t(paged ? 1 : cache->max_seqs) * layer.desc.kv_heads};
+        const cuuint64_t dims[3] = {cuuint64_t(d), cuuint64_t(layer.capacity), cuuint64_t(planes)};
         const cuuint64_t strides[2] = {cuuint64_t(d) * 2, cuuint64_t(layer.capacity) * d * 2};
         const cuuint32_t box[3] = {64, cuuint32_t(which < 2 ? kTileKeys : 64), 1};
         const cuuint32_t elem[3] = {1, 1, 1};

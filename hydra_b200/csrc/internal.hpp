@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -84,6 +85,10 @@ struct PrepArgs {
     int batched;             // 1: token t is sequence meta.seq[t] at position meta.pos[t]
     int seq;                 // sequence when batched == 0
     CacheView cache;         // for kinds 1 and 2
+    // Rows at positions from also_from on go here too (a prompt whose keys attend outside its ring); 0 rows: nowhere.
+    CacheView also;
+    int also_from;
+    int also_seq;
     BatchMeta meta;
 };
 
@@ -160,6 +165,9 @@ struct hc_layer_store {
     void* tmap_k = nullptr;       // tensor maps of the tcgen05 path (host copies), or null
     void* tmap_v = nullptr;
     void* tmap_k64 = nullptr;     // keys in boxes of 64 rows: what a CTA of a pair loads (head_dim 256, 512)
+    // A ring holds too little of a prompt beside its window, so a longer one attends in the workspace: a ring of one sequence
+    // with room for the window and a whole call's tokens, used by one call at a time like the rest of the workspace.
+    std::unique_ptr<hc_layer_store> prompt;
 };
 
 struct hc_kv_cache {
@@ -200,6 +208,9 @@ hc_status check_cuda(cudaError_t err, const char* what);
 
 // prologue.cu
 hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t stream);
+// The rows of positions [first, end) of `from_seq` in `from`, keys and values, into sequence 0 of `to`.
+hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq, const CacheView& to, int first, int end, int d,
+                           cudaStream_t stream);
 hc_status launch_rms_norm_rows(hc_context* ctx, const void* x, const uint16_t* scale, void* out, int tokens, int width,
                                float eps, int x_dtype, int out_dtype, cudaStream_t stream);
 hc_status launch_split_query_gate(hc_context* ctx, const void* combined, void* query, void* gate,
@@ -274,7 +285,7 @@ hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* cons
 // attn_pair.cu (args_ptr: the TcArgs of tc_common.cuh)
 int pair_items_per_row_tile(int head_dim);
 hc_status launch_attention_pair(hc_context* ctx, const hc_layer_store& layer, const void* args_ptr, int head_dim, cudaStream_t stream);
-hc_status tc_make_tensor_maps(hc_kv_cache* cache, hc_layer_store& layer);
+hc_status tc_make_tensor_maps(hc_layer_store& layer, size_t planes);
 void tc_free_tensor_maps(hc_layer_store& layer);
 
 }  // namespace hc

@@ -31,6 +31,13 @@ __device__ __forceinline__ void store_io4(void* base, size_t index, int dtype, c
     }
 }
 
+// A key or value row's second place (PrepArgs::also).
+__device__ __forceinline__ uint16_t* also_row(const PrepArgs& args, int kind, int head, int position, int d) {
+    return (kind == 1 ? args.also.k : args.also.v) +
+           (size_t(cache_plane(args.also.map, args.also_seq, args.also.kv_heads, head)) * args.also.capacity +
+            cache_row(args.also.map, args.also_seq, position)) * d;
+}
+
 // The kernel for head_dim 64, 128, 256 and 512 (see HeadLanes: a warp holds 4, 2 or 1 vectors at a time and
 // every access is an 8- or 16-byte one).  A warp stays with its heads and walks over tokens, so what to do, where
 // from and where to, and the norm weights are worked out once: with every warp finding its next (token, head) by
@@ -81,6 +88,7 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
         }
         size_t base = src_base;
         bool active = in_range;
+        uint16_t* also = nullptr;
         if (kind == 0) {
             base = (size_t(token) * heads + head) * D;
         } else if (kind != 3) {
@@ -89,6 +97,7 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
             if (active) {
                 base = (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity +
                         cache_row(args.cache.map, seq, position)) * D;
+                if (args.also.capacity > 0 && position >= args.also_from) also = also_row(args, kind, head, position, D);
             }
         }
         prepare_head<D>(lo, hi, norm, wl, wh, args.eps, rope, c, s, any_norm);
@@ -102,8 +111,13 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
                 store_io4(dst, at, dtype, a);
                 store_io4(dst, at + D / 2, dtype, b);
             } else {
-                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at) = pack_bf16x4(a);
-                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at + D / 2) = pack_bf16x4(b);
+                const uint2 pa = pack_bf16x4(a), pb = pack_bf16x4(b);
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at) = pa;
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at + D / 2) = pb;
+                if (also != nullptr) {
+                    *reinterpret_cast<uint2*>(also + (at - base)) = pa;
+                    *reinterpret_cast<uint2*>(also + (at - base) + D / 2) = pb;
+                }
             }
         }
     }
@@ -147,13 +161,14 @@ prepare_heads_kernel(const PrepArgs args) {
     const bool rotate = job.rope != 0;
     const int table_row = position < args.table_positions ? position : args.table_positions - 1;
     // Destination of this head vector.
-    uint16_t* dst16 = nullptr;
+    uint16_t *dst16 = nullptr, *also = nullptr;
     if (job.kind == 0) {
         dst16 = reinterpret_cast<uint16_t*>(job.dst) + (size_t(token) * job.heads + head) * d;
     } else if (job.kind == 1 || job.kind == 2) {
         const int row = cache_row(args.cache.map, seq, position);
         uint16_t* base = job.kind == 1 ? args.cache.k : args.cache.v;
         dst16 = base + (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity + row) * d;
+        if (args.also.capacity > 0 && position >= args.also_from) also = also_row(args, job.kind, head, position, d);
     }
 
     // Stage the vector in shared memory.
@@ -194,8 +209,30 @@ prepare_heads_kernel(const PrepArgs args) {
         } else {
             dst16[i] = float_to_bf16_bits(x1);
             dst16[half + i] = float_to_bf16_bits(x2);
+            if (also != nullptr) {
+                also[i] = dst16[i];
+                also[half + i] = dst16[half + i];
+            }
         }
     }
+    }
+}
+
+// Rows of one sequence from one storage to another, a thread per 16 bytes (a row is 2 head_dim bytes, a multiple of 16).
+__global__ void __launch_bounds__(256)
+copy_rows_kernel(const CacheView from, int from_seq, const CacheView to, int first, int end, int pieces) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int heads = from.kv_heads;
+    const unsigned total = unsigned(end - first) * unsigned(heads) * unsigned(pieces);
+    for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+        const unsigned row = i / unsigned(pieces), piece = i - row * unsigned(pieces);
+        const int position = first + int(row / unsigned(heads)), head = int(row % unsigned(heads));
+        const size_t src = (size_t(cache_plane(from.map, from_seq, heads, head)) * from.capacity + cache_row(from.map, from_seq, position)) * pieces + piece;
+        const size_t dst = (size_t(cache_plane(to.map, 0, heads, head)) * to.capacity + cache_row(to.map, 0, position)) * pieces + piece;
+        const uint4 k = reinterpret_cast<const uint4*>(from.k)[src], v = reinterpret_cast<const uint4*>(from.v)[src];
+        reinterpret_cast<uint4*>(to.k)[dst] = k;
+        reinterpret_cast<uint4*>(to.v)[dst] = v;
     }
 }
 
@@ -341,6 +378,16 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
     }
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "prepare_heads_kernel launch");
+}
+
+hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq, const CacheView& to, int first, int end, int d,
+                           cudaStream_t stream) {
+    if (first >= end) return HC_OK;
+    const long long total = (long long)(end - first) * from.kv_heads * (d / 8);
+    const int grid = int(std::min<long long>((total + 255) / 256, (long long)std::max(ctx->sm_count, 1) * 8));
+    launch_pdl(copy_rows_kernel, grid, 256, 0, stream, from, from_seq, to, first, end, d / 8);
+    ctx->launches += 1;
+    return check_cuda(cudaGetLastError(), "copy_rows_kernel launch");
 }
 
 hc_status launch_rms_norm_rows(hc_context* ctx, const void* x, const uint16_t* scale, void* out, int tokens, int width,

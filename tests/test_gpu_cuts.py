@@ -179,3 +179,43 @@ def test_stack_call_equals_its_parts(hb, ctx, tokens):
     assert np.array_equal(host, want.cpu().numpy())
     for cache in caches:
         cache.close()
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, first, tokens, io, gated", [
+    (64, 16, 4, 128, 0, 256, "bf16", False),     # as many tokens as fit beside the ring's window
+    (64, 16, 4, 128, 0, 257, "bf16", False),     # one more: the prompt attends outside the ring
+    (64, 16, 4, 128, 131, 700, "f32", False),    # behind an odd history, which comes along
+    (96, 8, 4, 130, 259, 600, "bf16", False),    # the CUDA-core kernels, the general prologue
+    (128, 16, 2, 300, 640, 1290, "bf16", True),
+    (256, 16, 8, 256, 77, 1500, "bf16", False),
+    (256, 64, 4, 384, 515, 2300, "f32", False),  # more than the prepared queries have room for: two parts
+])
+def test_prompts_longer_than_a_ring_equal_linear_storage(hb, ctx, d, qh, kvh, window, first, tokens, io, gated):
+    """Outputs, the ring's rows and a decoded token behind them: the same bits as with linear storage, twice in a row."""
+    rng = np.random.default_rng(d + window + tokens)
+    end, width = first + tokens, d * (2 if gated else 1)
+    k, v = tl.normal_bf16(rng, (end + 1, kvh, d)), tl.normal_bf16(rng, (end + 1, kvh, d))
+    q = tl.normal_bf16(rng, (tokens + 1, qh, width))
+    sinks = tl.normal_bf16(rng, (qh,))
+    inv = ho.inverse_frequencies(d, 10000.0, d // 2)
+    got = []
+    for storage in (hb.capi.HC_STORAGE_RING, hb.capi.HC_STORAGE_LINEAR):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 4096, window=window, sinks=sinks, rope_inv_freq=inv, io=io, prefill_chunk=128,
+                         storage=storage, gate_layout=hb.capi.HC_GATE_INTERLEAVED if gated else 0, max_seqs=2)
+        dev = [tl.to_device(x, io) for x in (q, k, v)]
+        out = tl.device_empty((tokens + 1, qh, d), io)
+        for seq in (1, 1, 0):
+            for at in range(0, first, 128):
+                layer.append(k[at:min(at + 128, first)], v[at:min(at + 128, first)], at, seq=seq)
+            out.fill_(7.0)
+            layer.backend.prefill_chunks(layer.cache, 0, dev[0], dev[1][first:], dev[2][first:], out, tokens, first, 128,
+                                         layer.params, seq=seq)
+            layer.backend.layer_step(layer.cache, 0, dev[0][tokens:], dev[1][end:], dev[2][end:], out[tokens:], 1, end, layer.params,
+                                     seq=seq)
+        ctx.check()
+        held = min(end + 1, window + 128)
+        rows = tl.read_cache(layer.cache, 0, held, kvh, d, seq=0, position=end + 1 - held)
+        got.append([tl.to_host(out), *rows])
+        layer.close()
+    for ring, linear in zip(*got):
+        assert np.array_equal(ring, linear)
