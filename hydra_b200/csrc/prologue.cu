@@ -23,14 +23,6 @@ namespace {
 constexpr int kPrepWarps = 8;
 constexpr int kMaxHeadDim = 512;
 
-__device__ __forceinline__ void store_io4(void* base, size_t index, int dtype, const float (&v)[4]) {
-    if (dtype == 0) {
-        *reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + index) = make_float4(v[0], v[1], v[2], v[3]);
-    } else {
-        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(base) + index) = pack_bf16x4(v);
-    }
-}
-
 // A key or value row's second place (PrepArgs::also).
 __device__ __forceinline__ uint16_t* also_row(const PrepArgs& args, int kind, int head, int position, int d) {
     return (kind == 1 ? args.also.k : args.also.v) +
@@ -38,26 +30,88 @@ __device__ __forceinline__ uint16_t* also_row(const PrepArgs& args, int kind, in
             cache_row(args.also.map, args.also_seq, position)) * d;
 }
 
-// The kernel for head_dim 64, 128, 256 and 512 (see HeadLanes: a warp holds 4, 2 or 1 vectors at a time and
-// every access is an 8- or 16-byte one).  A warp stays with its heads and walks over tokens, so what to do, where
-// from and where to, and the norm weights are worked out once: with every warp finding its next (token, head) by
-// division the kernel was bound by instructions, 300 of them for 256 elements (8192 tokens of 16 x 256: 35 us).
+// The kernel for head_dim 64, 128, 256 and 512.  A warp stays with its heads and walks over tokens, so what to do, where
+// from and where to, and the norm weights are worked out once; the next token's vectors are on their way while this one's
+// are worked on.  What bounds it is its instructions, so a lane owns sixteen elements (8 m .. 8 m + 7 of each half, 16-byte
+// accesses; head_dim 512 as in HeadLanes): a warp has two vectors of 256 at a time, and reduces, and takes the root and the
+// addresses, once for both (8192 tokens of 32 x 256 with norms and rotation: 90 us with a vector a warp, a division by
+// head_dim and a remainder per cached row, now 64).  The bits are HeadLanes' and prepare_head's: a lane keeps the sums of two of
+// their lanes apart until the last step of the butterfly.
 // The launcher checks the alignment this needs and otherwise uses the general kernel below.
 template <int D>
-__global__ void __launch_bounds__(kPrepWarps * 32)
+struct WideLanes {
+    static constexpr bool kContiguous = D <= 256;
+    static constexpr int kLanes = D / 16;
+    static constexpr int kPerWarp = 32 / kLanes;
+    // Where elements 4 u .. 4 u + 3 of a lane's half lie in it.
+    __device__ static constexpr int at(int m, int u) { return kContiguous ? 8 * m + 4 * u : 4 * (m + u * kLanes); }
+};
+// A lane's elements as they come: [half][4 u ..].
+template <int D, bool F32>
+struct RawHead {
+    uint4 x[2][F32 ? 2 : 1];
+    __device__ __forceinline__ void load(const unsigned char* src, int m) {
+        using WL = WideLanes<D>;
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if constexpr (F32) {
+                #pragma unroll
+                for (int u = 0; u < 2; ++u) x[h][u] = *reinterpret_cast<const uint4*>(src + (h * (D / 2) + WL::at(m, u)) * 4);
+            } else if constexpr (WL::kContiguous) {
+                x[h][0] = *reinterpret_cast<const uint4*>(src + (h * (D / 2) + WL::at(m, 0)) * 2);
+            } else {
+                const uint2 a = *reinterpret_cast<const uint2*>(src + (h * (D / 2) + WL::at(m, 0)) * 2);
+                const uint2 b = *reinterpret_cast<const uint2*>(src + (h * (D / 2) + WL::at(m, 1)) * 2);
+                x[h][0] = make_uint4(a.x, a.y, b.x, b.y);
+            }
+        }
+    }
+    __device__ __forceinline__ void unpack(int h, float (&v)[8]) const {
+        const uint32_t w[4] = {x[h][0].x, x[h][0].y, x[h][0].z, x[h][0].w};
+        if constexpr (F32) {
+            const uint32_t w2[4] = {x[h][1].x, x[h][1].y, x[h][1].z, x[h][1].w};
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) { v[i] = __uint_as_float(w[i]); v[4 + i] = __uint_as_float(w2[i]); }
+        } else {
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+        }
+    }
+};
+// Eight values of a half to a row of bf16.
+template <int D>
+__device__ __forceinline__ void store_half(uint16_t* row, int h, int m, const float (&v)[8]) {
+    using WL = WideLanes<D>;
+    const float a[4] = {v[0], v[1], v[2], v[3]}, b[4] = {v[4], v[5], v[6], v[7]};
+    const uint2 pa = pack_bf16x4(a), pb = pack_bf16x4(b);
+    uint16_t* at = row + h * (D / 2);
+    if constexpr (WL::kContiguous) {
+        *reinterpret_cast<uint4*>(at + WL::at(m, 0)) = make_uint4(pa.x, pa.y, pb.x, pb.y);
+    } else {
+        *reinterpret_cast<uint2*>(at + WL::at(m, 0)) = pa;
+        *reinterpret_cast<uint2*>(at + WL::at(m, 1)) = pb;
+    }
+}
+
+// Thread blocks an SM holds.
+constexpr int prep_blocks(bool fp32) { return fp32 ? 2 : 3; }
+
+template <int D, bool F32>
+__global__ void __launch_bounds__(kPrepWarps * 32, prep_blocks(F32))
 prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
-    using HL = HeadLanes<D>;
+    using WL = WideLanes<D>;
+    constexpr int kBytes = F32 ? 4 : 2;
     pdl_launch_dependents();
     const unsigned warp = blockIdx.x * kPrepWarps + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    const int sub = lane / HL::kLanes;
-    const int m = lane % HL::kLanes;
+    const int sub = lane / WL::kLanes;
+    const int m = lane % WL::kLanes;
     const bool any_norm = (args.job[0].norm | (args.n_jobs > 1 ? args.job[1].norm : 0) | (args.n_jobs > 2 ? args.job[2].norm : 0)) != 0;
     // Warps side by side take the heads of a token.
-    const unsigned head_groups = unsigned(total_heads + HL::kPerWarp - 1) / HL::kPerWarp;
+    const unsigned head_groups = unsigned(total_heads + WL::kPerWarp - 1) / WL::kPerWarp;
     const unsigned step = gridDim.x * kPrepWarps / head_groups;
-    const unsigned first_token = warp / head_groups;
-    int head = int(warp - first_token * head_groups) * HL::kPerWarp + sub;
+    unsigned token = warp / head_groups;
+    int head = int(warp - token * head_groups) * WL::kPerWarp + sub;
     const bool in_range = head < total_heads;
     if (!in_range) head = total_heads - 1;               // keeps the lane's loads legal; nothing is stored
     int job_index = 0;
@@ -66,60 +120,133 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
         ++job_index;
     }
     const PrepJob& job = args.job[job_index];
-    const int norm = job.norm, kind = job.kind, dtype = job.src_dtype, heads = job.heads;
-    const bool rope = job.rope != 0;
-    const void* src = job.src;
-    const long long token_stride = job.token_stride;
-    const size_t head_offset = size_t(head) * job.head_stride;
-    void* dst = kind == 1 ? args.cache.k : kind == 2 ? args.cache.v : job.dst;
-    const uint16_t* weight = job.weight;
+    const int norm = job.norm, kind = job.kind;
+    const bool rope = job.rope != 0, cached = kind == 1 || kind == 2;
+    const RowMap& map = args.cache.map;
     pdl_wait();
-    float wl[HL::kElems], wh[HL::kElems];
-    if (norm == 1) load_head<D>(weight, 0, 1, m, wl, wh);
-    if (first_token >= step) return;
-    for (unsigned token = first_token; token < unsigned(args.tokens); token += step) {
-        const int position = args.batched ? args.meta.pos[token] : args.first_position + int(token);
-        const size_t src_base = size_t(token) * size_t(token_stride) + head_offset;
-        float lo[HL::kElems], hi[HL::kElems], c[HL::kElems], s[HL::kElems];
-        load_head<D>(src, src_base, dtype, m, lo, hi);
-        if (rope) {
-            const int table_row = min(position, args.table_positions - 1);
-            load_rotation<D>(args.cos + size_t(table_row) * (D / 2), args.sin + size_t(table_row) * (D / 2), m, c, s);
-        }
-        size_t base = src_base;
-        bool active = in_range;
-        uint16_t* also = nullptr;
-        if (kind == 0) {
-            base = (size_t(token) * heads + head) * D;
-        } else if (kind != 3) {
-            active = active && row_is_local(args.cache.map, position);           // else another rank's tile
-            const int seq = args.batched ? args.meta.seq[token] : args.seq;
-            if (active) {
-                base = (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity +
-                        cache_row(args.cache.map, seq, position)) * D;
-                if (args.also.capacity > 0 && position >= args.also_from) also = also_row(args, kind, head, position, D);
+    if (token >= step || token >= unsigned(args.tokens)) return;
+    float wl[8], wh[8];
+    if (norm == 1) {
+        RawHead<D, false> w;
+        w.load(reinterpret_cast<const unsigned char*>(job.weight), m);
+        w.unpack(0, wl);
+        w.unpack(1, wh);
+    }
+    const size_t src_step = size_t(step) * size_t(job.token_stride) * kBytes;
+    unsigned char* src = const_cast<unsigned char*>(static_cast<const unsigned char*>(job.src)) +
+                         (size_t(token) * size_t(job.token_stride) + size_t(head) * job.head_stride) * kBytes;
+    // Rows of a ring or of linear storage are counted along; other storage is asked for every row.
+    const bool counted = cached && args.batched == 0 && map.pages == nullptr && map.world <= 1;
+    uint16_t* dst = nullptr;
+    size_t dst_step = 0;
+    int row = 0, row_step = int(step);
+    if (kind == 0) {
+        dst = static_cast<uint16_t*>(job.dst) + (size_t(token) * job.heads + head) * D;
+        dst_step = size_t(step) * job.heads * D;
+    } else if (cached) {
+        dst = kind == 1 ? args.cache.k : args.cache.v;
+        if (counted) {
+            dst += size_t(cache_plane(map, args.seq, args.cache.kv_heads, head)) * args.cache.capacity * D;
+            row = args.first_position + int(token);
+            if (map.ring > 0) {
+                row %= map.ring;
+                row_step %= map.ring;
             }
         }
-        prepare_head<D>(lo, hi, norm, wl, wh, args.eps, rope, c, s, any_norm);
-        if (!active) continue;
-        #pragma unroll
-        for (int u = 0; u < HL::kVecs; ++u) {
-            const float a[4] = {lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]};
-            const float b[4] = {hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]};
-            const size_t at = base + 4 * (m + u * HL::kLanes);
-            if (kind == 3) {
-                store_io4(dst, at, dtype, a);
-                store_io4(dst, at + D / 2, dtype, b);
-            } else {
-                const uint2 pa = pack_bf16x4(a), pb = pack_bf16x4(b);
-                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at) = pa;
-                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at + D / 2) = pb;
-                if (also != nullptr) {
-                    *reinterpret_cast<uint2*>(also + (at - base)) = pa;
-                    *reinterpret_cast<uint2*>(also + (at - base) + D / 2) = pb;
+    }
+    RawHead<D, F32> now, ahead;
+    now.load(src, m);
+    for (;;) {
+        const bool more = token + step < unsigned(args.tokens);
+        if (more) ahead.load(src + src_step, m);
+        const int position = args.batched ? args.meta.pos[token] : args.first_position + int(token);
+        float c[8], s[8];
+        if (rope) {
+            const size_t table = size_t(min(position, args.table_positions - 1)) * (D / 2);
+            #pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const float4 cv = *reinterpret_cast<const float4*>(args.cos + table + WL::at(m, u));
+                const float4 sv = *reinterpret_cast<const float4*>(args.sin + table + WL::at(m, u));
+                c[4 * u] = cv.x; c[4 * u + 1] = cv.y; c[4 * u + 2] = cv.z; c[4 * u + 3] = cv.w;
+                s[4 * u] = sv.x; s[4 * u + 1] = sv.y; s[4 * u + 2] = sv.z; s[4 * u + 3] = sv.w;
+            }
+        }
+        float lo[8], hi[8];
+        now.unpack(0, lo);
+        now.unpack(1, hi);
+        if (any_norm) {                                  // warp-uniform
+            float part[2] = {0.0f, 0.0f};
+            constexpr int kParts = WL::kContiguous ? 2 : 1, kEach = 8 / kParts;
+            #pragma unroll
+            for (int p = 0; p < kParts; ++p) {
+                #pragma unroll
+                for (int i = 0; i < kEach; ++i) part[p] = __fmaf_rn(lo[kEach * p + i], lo[kEach * p + i], part[p]);
+                #pragma unroll
+                for (int i = 0; i < kEach; ++i) part[p] = __fmaf_rn(hi[kEach * p + i], hi[kEach * p + i], part[p]);
+            }
+            #pragma unroll
+            for (int offset = WL::kLanes / 2; offset > 0; offset >>= 1) {
+                #pragma unroll
+                for (int p = 0; p < kParts; ++p) part[p] = __fadd_rn(part[p], __shfl_xor_sync(0xffffffffu, part[p], offset));
+            }
+            if (norm != 0) {
+                const float inverse = head_norm<D>(kParts == 2 ? __fadd_rn(part[0], part[1]) : part[0], args.eps);
+                #pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    lo[i] = __fmul_rn(lo[i], inverse);
+                    hi[i] = __fmul_rn(hi[i], inverse);
+                }
+                if (norm == 1) {
+                    #pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        lo[i] = __fmul_rn(lo[i], wl[i]);
+                        hi[i] = __fmul_rn(hi[i], wh[i]);
+                    }
                 }
             }
         }
+        if (rope) {
+            #pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float a = lo[i], b = hi[i];
+                lo[i] = __fmaf_rn(a, c[i], -__fmul_rn(b, s[i]));
+                hi[i] = __fmaf_rn(b, c[i], __fmul_rn(a, s[i]));
+            }
+        }
+        uint16_t* to = dst;
+        bool active = in_range;
+        if (counted) {
+            to = dst + size_t(row) * D;
+            row += row_step;
+            if (map.ring > 0 && row >= map.ring) row -= map.ring;
+        } else if (cached) {
+            active = active && row_is_local(map, position);           // else another rank's tile
+            const int seq = args.batched ? args.meta.seq[token] : args.seq;
+            if (active) to = dst + (size_t(cache_plane(map, seq, args.cache.kv_heads, head)) * args.cache.capacity + cache_row(map, seq, position)) * D;
+        }
+        if (active) {
+            if (kind == 3 && F32) {
+                #pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    *reinterpret_cast<float4*>(src + WL::at(m, u) * 4) = make_float4(lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]);
+                    *reinterpret_cast<float4*>(src + (D / 2 + WL::at(m, u)) * 4) = make_float4(hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]);
+                }
+            } else {
+                if (kind == 3) to = reinterpret_cast<uint16_t*>(src);
+                store_half<D>(to, 0, m, lo);
+                store_half<D>(to, 1, m, hi);
+                if (cached && args.also.capacity > 0 && position >= args.also_from) {
+                    uint16_t* also = also_row(args, kind, head, position, D);
+                    store_half<D>(also, 0, m, lo);
+                    store_half<D>(also, 1, m, hi);
+                }
+            }
+        }
+        if (!more) break;
+        now = ahead;
+        token += step;
+        src += src_step;
+        if (kind == 0) dst += dst_step;
     }
 }
 
@@ -360,16 +487,20 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
         const PrepJob& job = args.job[j];
         if (job.heads == 0) continue;
         vector_ok = aligned16(job.src) && job.token_stride % 8 == 0 && job.head_stride % 8 == 0 &&
-                    (job.norm != 1 || aligned16(job.weight)) &&
+                    (job.norm != 1 || aligned16(job.weight)) && job.src_dtype == args.job[0].src_dtype &&
                     ((job.kind != 0 && job.kind != 3) || aligned16(job.dst));
     }
     if (vector_ok) {
-        const int per_warp = d >= 256 ? 1 : 256 / d;
+        const int per_warp = 512 / d;
         const long long head_groups = (total_heads + per_warp - 1) / per_warp, groups = args.tokens * head_groups;
         // (A warp stays with its heads, so there are never fewer warps than a token has groups of them.)
-        const int grid = int((std::max(std::min(groups, cap * kPrepWarps), head_groups) + kPrepWarps - 1) / kPrepWarps);
-        auto kernel = d == 64 ? prepare_heads_vec_kernel<64> : d == 128 ? prepare_heads_vec_kernel<128>
-                    : d == 256 ? prepare_heads_vec_kernel<256> : prepare_heads_vec_kernel<512>;
+        const bool fp32 = args.job[0].src_dtype == HC_F32;
+        const long long most = (long long)std::max(ctx->sm_count, 1) * prep_blocks(fp32) * kPrepWarps;
+        const int grid = int((std::max(std::min(groups, most), head_groups) + kPrepWarps - 1) / kPrepWarps);
+        auto kernel = d == 64 ? (fp32 ? prepare_heads_vec_kernel<64, true> : prepare_heads_vec_kernel<64, false>)
+                    : d == 128 ? (fp32 ? prepare_heads_vec_kernel<128, true> : prepare_heads_vec_kernel<128, false>)
+                    : d == 256 ? (fp32 ? prepare_heads_vec_kernel<256, true> : prepare_heads_vec_kernel<256, false>)
+                               : (fp32 ? prepare_heads_vec_kernel<512, true> : prepare_heads_vec_kernel<512, false>);
         launch_pdl(kernel, grid, kPrepWarps * 32, 0, stream, args, total_heads);
     } else {
         const long long wanted = (vectors + kPrepWarps - 1) / kPrepWarps;
