@@ -13,7 +13,8 @@
 // Shared memory holds one Q tile (64 or 128 KB) and a ring of 16 KB stages through which K and V tiles
 // pass in the order the MMAs take them: K0 K1 V0 K2 V1 .., across item boundaries.
 //
-//   warpgroup 0    warp 0 loads K and V, warp 1 of the leading CTA issues the MMAs, warp 2 loads Q (all TMA)
+//   warpgroup 0    warp 0 loads K and V, warp 1 of the leading CTA issues the MMAs, warp 2 works the items out and
+//                  loads Q (all TMA)
 //   warpgroups 1-2 softmax, thread = row; each group takes 64 of a tile's 128 columns.  With two S buffers the loop
 //                  S -> softmax -> P V -> next S of the buffer sets the pace, so what counts is the softmax's
 //                  latency (whole tiles in turn: 3100 clocks of it, 3250 a tile)
@@ -50,18 +51,6 @@ struct PairLayout {
     static constexpr int kSmemBytes = 1024 + kQBytes + kStages * kPairStageBytes + 8 * kPairStoreBytes;
 };
 
-struct PairBarriers {
-    uint64_t q_full, q_empty;
-    uint64_t full[9], empty[9];
-    uint64_t s_full[2], p_full[2], m_full[4], o_full[2], o_free[2];
-    uint32_t tmem_base;
-    int abort_flag;
-    float red[2][2][kRows];             // alternate tiles: the two halves' row maxima
-    float mm[4][kRows];                 // scaled maxima, softmax -> fold (ring of 4 tiles, like m_full and l)
-    float l[4][3][kRows];               // row sums: columns 0-63, 64-95, 96-127
-    float m2[2][kRows], l2[2][kRows];   // the rows' second fold between segments, per half
-};
-
 struct PairItem {
     int kv_head;
     int half;          // 256-column half of O (head_dim 512)
@@ -71,8 +60,7 @@ struct PairItem {
     int tile_first, n_tiles;
     int slot;          // ordinal of the item's segment among those the rows see (segment partials)
 };
-// BLOCKS: the launch has bidirectional blocks.  A template argument of everything that walks the items: six roles work out
-// each its own, and with the test and the chunk's end in all of them launches without blocks took 0.5 to 1.5 % longer.
+// BLOCKS: the launch has bidirectional blocks.
 template <int D, bool BLOCKS>
 __device__ __forceinline__ PairItem pair_item(const TcArgs& args, int index) {
     PairItem w;
@@ -96,45 +84,25 @@ __device__ __forceinline__ PairItem pair_item(const TcArgs& args, int index) {
     w.n_tiles = tiles.count;
     return w;
 }
-struct PairIter {
-    Snake at;
-    int item;
-    PairItem w;
-};
-template <int D, bool BLOCKS>
-__device__ __forceinline__ void pair_seek(const TcArgs& args, PairIter& it) {
-    for (; it.at.item < args.n_items; it.at.next()) {
-        it.item = it.at.item;
-        it.w = pair_item<D, BLOCKS>(args, it.item);
-        if (it.w.n_tiles > 0) return;
-    }
-    it.item = args.n_items;
-}
-template <int D, bool BLOCKS>
-__device__ __forceinline__ PairIter pair_begin(const TcArgs& args) {
-    PairIter it{Snake(int(blockIdx.x) >> 1, int(gridDim.x) >> 1), 0, PairItem{}};
-    pair_seek<D, BLOCKS>(args, it);
-    return it;
-}
-template <int D, bool BLOCKS>
-__device__ __forceinline__ void pair_next(const TcArgs& args, PairIter& it) {
-    it.at.next();
-    pair_seek<D, BLOCKS>(args, it);
-}
 
-// The walk tile by tile.
-template <int D, bool BLOCKS>
-struct PairCursor {
-    PairIter walk;
-    int j;
-    __device__ __forceinline__ explicit PairCursor(const TcArgs& args) : walk(pair_begin<D, BLOCKS>(args)), j(0) {}
-    __device__ __forceinline__ bool more(const TcArgs& args) const { return walk.item < args.n_items; }
-    __device__ __forceinline__ void next(const TcArgs& args) {
-        if (++j == walk.w.n_tiles) {
-            j = 0;
-            pair_next<D, BLOCKS>(args, walk);
-        }
-    }
+// A pair's items, worked out by the warp that loads Q and read by every other role (as in attn_tc.cu: the divisions, in each
+// role's own path, stood between two items).  The readers are never 16 items apart: what lies between the Q loader and
+// the fold is one item's Q and fewer than ten tiles.
+constexpr int kPairItems = 16;
+
+struct PairBarriers {
+    uint64_t q_full, q_empty;
+    uint64_t full[9], empty[9];
+    uint64_t s_full[2], p_full[2], m_full[4], o_full[2], o_free[2];
+    uint64_t item_full[kPairItems];
+    PairItem item[kPairItems];
+    uint32_t tmem_base;
+    int abort_flag;
+    int more[2][4];                     // alternate items, per quadrant: whether there is one (softmax)
+    float red[2][2][kRows];             // alternate tiles: the two halves' row maxima
+    float mm[4][kRows];                 // scaled maxima, softmax -> fold (ring of 4 tiles, like m_full and l)
+    float l[4][3][kRows];               // row sums: columns 0-63, 64-95, 96-127
+    float m2[2][kRows], l2[2][kRows];   // the rows' second fold between segments, per half
 };
 
 // (x0 + y0, x1 + y1) of two bf16 pairs, as one packed addition.
@@ -146,8 +114,7 @@ __device__ __forceinline__ uint64_t add2(uint64_t x, uint64_t y) {
 }
 
 // MODE: what becomes of an item's rows, a template argument so that a launch carries the code (and the registers) of its
-// own way only: bf16 rows (or, sequence-sharded, row partials; head_dim 512: all finished rows); rows with a gate or
-// in fp32; segment partials.
+// own way only: bf16 rows (or, sequence-sharded, row partials); rows with a gate or in fp32; segment partials.
 constexpr int kPairRowsOut = 0, kPairGatedOut = 1, kPairSegments = 2;
 template <int D, int MODE, bool BLOCKS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
@@ -169,6 +136,30 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
     const int rank = int(cluster_rank());
     const int token0 = rank * (kRows >> args.log_group);     // the first token of this CTA's half of a row tile
     volatile int* abort_flag = &bars->abort_flag;
+    // Item `it` of this pair into w; false behind the last one, or on abort.
+    auto read_item = [&](uint32_t it, PairItem& w) -> bool {
+        if (!mbar_wait(&bars->item_full[it % kPairItems], (it / kPairItems) & 1, abort_flag, args.status, 13)) return false;
+        w = bars->item[it % kPairItems];
+        return w.n_tiles > 0;
+    };
+    // The walk tile by tile.
+    struct Cursor {
+        PairItem w;
+        uint32_t it;
+        int j;
+        bool more;
+    };
+    auto begin = [&](Cursor& c) {
+        c.it = 0;
+        c.j = 0;
+        c.more = read_item(0, c.w);
+    };
+    auto next = [&](Cursor& c) {
+        if (++c.j == c.w.n_tiles) {
+            c.j = 0;
+            c.more = read_item(++c.it, c.w);
+        }
+    };
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
@@ -185,6 +176,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
             mbar_init(&bars->o_free[i], 8);                  // a half's fold warps of both CTAs
         }
         for (int i = 0; i < 4; ++i) mbar_init(&bars->m_full[i], 8);      // those of this one
+        for (int i = 0; i < kPairItems; ++i) mbar_init(&bars->item_full[i], 1);
         bars->abort_flag = 0;
         fence_barrier_init();
     }
@@ -222,22 +214,24 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                 if (two_boxes) tma_load_3d_pair(dst + kPairBoxBytes, map, full, col0 + 64, row, plane);
             };
             // K one tile ahead of V.
-            PairCursor<D, BLOCKS> keys(args), values(args);
+            Cursor keys, values;
+            begin(keys);
+            begin(values);
             auto load_keys = [&]() {                         // this CTA's 64 keys of the tile
-                const PairItem& w = keys.walk.w;
+                const PairItem& w = keys.w;
                 const int plane = cache_plane(args.map, args.seq, args.kv_heads, w.kv_head);
                 const int row = cache_row(args.map, args.seq, (w.tile_first + keys.j * world) * kTileKeys) + rank * 64;
                 for (int c = 0; ok && c < PL::kKChunks; ++c) load(&tmap_k, c * 128, row, plane, true);
-                keys.next(args);
+                next(keys);
             };
-            if (keys.more(args)) load_keys();
-            while (ok && values.more(args)) {
-                if (keys.more(args)) load_keys();
-                const PairItem& w = values.walk.w;           // this CTA's 64 columns of each half of O
+            if (keys.more) load_keys();
+            while (ok && values.more) {
+                if (keys.more) load_keys();
+                const PairItem& w = values.w;                // this CTA's 64 columns of each half of O
                 const int plane = cache_plane(args.map, args.seq, args.kv_heads, w.kv_head);
                 const int row = cache_row(args.map, args.seq, (w.tile_first + values.j * world) * kTileKeys);
                 for (int h = 0; ok && h < 2; ++h) load(&tmap_v, w.half * kPairO + h * 128 + rank * 64, row, plane, false);
-                values.next(args);
+                next(values);
             }
         }
     } else if (warp == 1) {
@@ -251,12 +245,13 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
             const uint64_t k_desc0 = smem_desc(smem_u32(ring), 16);
             const uint64_t v_desc0 = smem_desc(smem_u32(ring), 16);
             uint32_t n = 0;
-            PairCursor<D, BLOCKS> ahead(args);
-            uint32_t ta = 0, it = 0;                         // tile and item of S
+            Cursor ahead;
+            begin(ahead);
+            uint32_t ta = 0;                                 // tile of S
             auto issue_qk = [&]() -> bool {
                 const uint32_t t = ta;
-                const bool last = ahead.j + 1 == ahead.walk.w.n_tiles;
-                if (ahead.j == 0 && !mbar_wait(&bars->q_full, it & 1, abort_flag, args.status, 4)) return false;
+                const bool last = ahead.j + 1 == ahead.w.n_tiles;
+                if (ahead.j == 0 && !mbar_wait(&bars->q_full, ahead.it & 1, abort_flag, args.status, 4)) return false;
                 const uint32_t s_tmem = tmem + (t & 1) * kTileKeys;
                 #pragma unroll 1
                 for (int c = 0; c < PL::kKChunks; ++c, ++n) {
@@ -285,13 +280,12 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     __syncwarp();
                 }
                 ++ta;
-                if (last) ++it;
-                ahead.next(args);
+                next(ahead);
                 return true;
             };
-            bool ok = !ahead.more(args) || issue_qk();
+            bool ok = !ahead.more || issue_qk();
             for (uint32_t t = 0; ok && t < ta; ++t) {
-                if (ahead.more(args) && !issue_qk()) break;
+                if (ahead.more && !issue_qk()) break;
                 if (!mbar_wait(&bars->p_full[t & 1], (t >> 1) & 1, abort_flag, args.status, 5)) break;
                 const uint32_t p_tmem = tmem + (t & 1) * kTileKeys;
                 // The two halves of O one after the other: one is folded while the other is computed.
@@ -321,13 +315,20 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         if (lane == 0) {
             uint32_t it = 0;
             const uint32_t q_full = cluster_addr(&bars->q_full, 0);
-            for (PairIter walk = pair_begin<D, BLOCKS>(args); walk.item < args.n_items; pair_next<D, BLOCKS>(args, walk), ++it) {
-                const PairItem& w = walk.w;
+            for (Snake at(int(blockIdx.x) >> 1, int(gridDim.x) >> 1);; at.next()) {
+                const bool more = at.item < args.n_items;
+                PairItem& entry = bars->item[it % kPairItems];
+                entry.n_tiles = 0;
+                if (more) entry = pair_item<D, BLOCKS>(args, at.item);
+                if (more && entry.n_tiles <= 0) continue;
+                mbar_arrive(&bars->item_full[it % kPairItems]);
+                if (!more) break;
                 if (it > 0 && !mbar_wait(&bars->q_empty, (it - 1) & 1, abort_flag, args.status, 10)) break;
                 if (rank == 0) mbar_expect_tx(&bars->q_full, 2 * PL::kQBytes);
                 for (int b = 0; b < D / 64; ++b) {
-                    tma_load_3d_pair(q_smem + b * (kRows * 128), &tmap_q, q_full, b * 64, w.kv_head * G, w.row0 + token0);
+                    tma_load_3d_pair(q_smem + b * (kRows * 128), &tmap_q, q_full, b * 64, entry.kv_head * G, entry.row0 + token0);
                 }
+                ++it;
             }
         }
     }
@@ -343,8 +344,17 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         const uint32_t p_full[2] = {cluster_addr(&bars->p_full[0], 0), cluster_addr(&bars->p_full[1], 0)};
         const float neg_inf = __int_as_float(0xff800000);
         uint32_t t = 0;
-        for (PairIter walk = pair_begin<D, BLOCKS>(args); walk.item < args.n_items; pair_next<D, BLOCKS>(args, walk)) {
-            const PairItem& w = walk.w;
+        for (uint32_t it = 0;; ++it) {
+            // Both warps of a row go by what the first of them reads.
+            PairItem w;
+            int* more = &bars->more[it & 1][quad];
+            if (cols == 0) {
+                const bool there = read_item(it, w);
+                if (lane == 0) *more = there ? 1 : 0;
+            }
+            named_barrier(1 + quad, 64);
+            if (*more == 0) break;
+            if (cols != 0) w = bars->item[it % kPairItems];
             const bool valid = t_local < w.valid_tokens;
             const bool warp_has_rows = quad * 32 < ((w.valid_tokens - token0) << args.log_group);
             int pos = valid ? w.first_pos + t_local : -1;
@@ -363,11 +373,13 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     const int c_lo = lo - key0;
                     const int c_hi = pos - key0;
                     const bool full = c_lo <= 0 && c_hi >= 63;
+                    // By bits of a word for each 32 columns (two comparisons a column were twice the code, fetched cold).
                     auto mask = [&](uint32_t (&s)[32], int base_col) {
-                        const int a = c_lo - base_col, b = c_hi - base_col;
+                        const int from = min(max(c_lo - base_col, 0), 32), to = min(max(c_hi + 1 - base_col, 0), 32);
+                        const uint32_t visible = uint32_t((1ull << to) - 1) & ~uint32_t((1ull << from) - 1);
                         #pragma unroll
                         for (int i = 0; i < 32; ++i) {
-                            if (i < a || i > b) s[i] = __float_as_uint(neg_inf);
+                            if (((visible >> i) & 1u) == 0) s[i] = __float_as_uint(neg_inf);
                         }
                     };
                     // Pass 1: the row maximum (exact under any association).
@@ -441,28 +453,42 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
         // This thread's values between segments: 32 groups of four, a row's group beside the next row's.
         float4* const state = reinterpret_cast<float4*>(args.row_state + size_t(blockIdx.x) * (kPairO * kRows)) + half * 32 * kRows + row;
         // (M, L) the second fold stands at: what the last segment end left, or the seed.
-        auto second_fold_state = [&](bool state_holds, int head, float& M2, float& L2) {
+        auto second_fold_state = [&](bool state_holds, uint16_t sink, float& M2, float& L2) {
             if (state_holds) {
                 M2 = bars->m2[half][row];
                 L2 = bars->l2[half][row];
             } else if (args.count_sink) {
-                M2 = __fmul_rn(bf16_bits_to_float(args.sinks != nullptr ? __ldg(args.sinks + head) : kNoSinkBits), kLog2e);
+                M2 = __fmul_rn(bf16_bits_to_float(sink), kLog2e);
                 L2 = 1.0f;
             } else {
                 M2 = kEmptyMax;
                 L2 = 0.0f;
             }
         };
-        // The gated epilogue uses an item's last O buffer and frees it.
-        constexpr bool keep_o = MODE == kPairGatedOut;
-        uint32_t t = 0;
+        auto free_o = [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster_relaxed(o_free);      // nothing but tensor memory was read
+        };
+        // Four values of the row's state, zeros before its first segment is complete.
+        auto state4 = [&](bool holds, int i) -> float4 { return holds ? state[(i >> 2) * kRows] : make_float4(0.0f, 0.0f, 0.0f, 0.0f); };
+        // x[0..3] <- before * a + x * b
+        auto join = [&](uint32_t* x, const float4& before, float a, float b) {
+            float y[4] = {before.x, before.y, before.z, before.w};
+            fold_value2(y[0], y[1], a, x[0], x[1], b);
+            fold_value2(y[2], y[3], a, x[2], x[3], b);
+            #pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = __float_as_uint(y[u]);
+        };
+        uint32_t t = 0, it = 0;
         bool ok = true;
-        for (PairIter walk = pair_begin<D, BLOCKS>(args); ok && walk.item < args.n_items; pair_next<D, BLOCKS>(args, walk)) {
-            const PairItem& w = walk.w;
-            const int head = w.kv_head * G + g;
+        PairItem w;
+        for (; ok && read_item(it, w); ++it) {
+            // The head's sink, in time for the item's (or a segment's) end.
+            uint16_t sink = kNoSinkBits;
+            if (MODE != kPairSegments && args.count_sink && args.sinks != nullptr) sink = __ldg(args.sinks + w.kv_head * G + g);
             const bool valid = t_local < w.valid_tokens;
             const bool warp_has_rows = quad * 32 < ((w.valid_tokens - token0) << args.log_group);
-            const size_t vec = size_t(w.row0 + t_local) * args.q_heads + head;
             // The running segment's partial: a fold over its tiles from the empty state (both halves of
             // the row carry M and L, the same chain, the same bits).
             float M = kEmptyMax, L = 0.0f;
@@ -471,6 +497,9 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
             for (int i = 0; i < 128; ++i) A[i] = 0.0f;
             bool state_holds = false;
             for (int j = 0; j < w.n_tiles; ++j, ++t) {
+                const int tile = w.tile_first + j * world;
+                const bool last = j + 1 == w.n_tiles;
+                const bool ends = last || (MODE != kPairSegments && (tile >> args.map.log_segment) != ((tile + world) >> args.map.log_segment));
                 // The coefficients while O is on its way.
                 if (!mbar_wait(&bars->m_full[t & 3], (t >> 2) & 1, abort_flag, args.status, 11)) { ok = false; break; }
                 float Mn, a, b;
@@ -479,138 +508,102 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                 M = Mn;
                 if (!mbar_wait(&bars->o_full[half], t & 1, abort_flag, args.status, 9)) { ok = false; break; }
                 tc_fence_after();
-                if (warp_has_rows) {
-                    #pragma unroll
-                    for (int chunk = 0; chunk < 8; ++chunk) {
-                        uint32_t o[16];
-                        HC_TMEM_LD16(o_tmem + chunk * 16, o);
-                        tc_wait_ld();
-                        if (chunk == 7 && !(keep_o && j + 1 == w.n_tiles)) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive_cluster_relaxed(o_free);      // nothing but tensor memory was read
-                        }
-                        #pragma unroll
-                        for (int i = 0; i < 16; i += 2) fold_value2(A[chunk * 16 + i], A[chunk * 16 + i + 1], a, o[i], o[i + 1], b);
-                    }
-                } else {
+                if (!warp_has_rows) {
                     if (lane == 0) mbar_arrive_cluster_relaxed(o_free);
+                    continue;
                 }
-                const int tile = w.tile_first + j * world;
-                if (MODE == kPairSegments || j + 1 == w.n_tiles || (tile >> args.map.log_segment) == ((tile + world) >> args.map.log_segment)) continue;
-                // A segment is complete and another follows: fold it into the row's state, which is kept out of the
-                // registers ((M2, L2) in shared memory, the values in global memory), and start over.
-                if (!warp_has_rows) continue;
-                float M2, L2;
-                second_fold_state(state_holds, head, M2, L2);
-                float Mn2, a2, b2;
-                fold_coefficients(M2, M, Mn2, a2, b2);
-                bars->m2[half][row] = Mn2;
-                bars->l2[half][row] = __fmaf_rn(L2, a2, __fmul_rn(L, b2));
                 #pragma unroll
-                for (int i0 = 0; i0 < 128; i0 += 16) {
-                    float4 before[4];
+                for (int chunk = 0; chunk < 8; ++chunk) {
+                    uint32_t o[16];
+                    HC_TMEM_LD16(o_tmem + chunk * 16, o);
+                    tc_wait_ld();
+                    if (chunk == 7 && !ends) free_o();
                     #pragma unroll
-                    for (int i = 0; i < 4; ++i) before[i] = state_holds ? state[(i0 / 4 + i) * kRows] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        float* v = &A[i0 + 4 * i];
-                        state[(i0 / 4 + i) * kRows] = make_float4(fold_value(before[i].x, a2, v[0], b2), fold_value(before[i].y, a2, v[1], b2),
-                                                                 fold_value(before[i].z, a2, v[2], b2), fold_value(before[i].w, a2, v[3], b2));
-                        v[0] = v[1] = v[2] = v[3] = 0.0f;
-                    }
-                    asm volatile("" ::: "memory");      // sixteen values in flight, not all of them
+                    for (int i = 0; i < 16; i += 2) fold_value2(A[chunk * 16 + i], A[chunk * 16 + i + 1], a, o[i], o[i + 1], b);
                 }
+                if (!ends) continue;
+                // A segment or the item ends.  Its values go back to tensor memory, in place of the O that was folded last, so
+                // that what is done with them can be a rolled loop over the columns, short code with few registers (straight-line
+                // over the 128 registers an item's end took 10800 clocks and spilled, now 6300; 777 gated fp32 tokens behind
+                // 1291, 16 heads of 256: 76 us, now 58; 8192 tokens with a window of 1024: 160, now 147).
+                #pragma unroll
+                for (int i = 0; i < 128; i += 16) {
+                    uint32_t v[16];
+                    #pragma unroll
+                    for (int u = 0; u < 16; ++u) v[u] = __float_as_uint(A[i + u]);
+                    HC_TMEM_ST16(o_tmem + i, v);
+                }
+                tc_wait_st();
+                if (last) {
+                    ++t;
+                    break;
+                }
+                // Another segment follows: this one joins the row's state, which is kept out of the registers ((M2, L2) in
+                // shared memory, the values in global memory).
+                float M2, L2;
+                second_fold_state(state_holds, sink, M2, L2);
+                fold_coefficients(M2, M, Mn, a, b);
+                bars->m2[half][row] = Mn;
+                bars->l2[half][row] = __fmaf_rn(L2, a, __fmul_rn(L, b));
+                float4 before[8];
+                #pragma unroll
+                for (int u = 0; u < 8; ++u) before[u] = state4(state_holds, 4 * u);
+                #pragma unroll 1
+                for (int i = 0; i < 128; i += 32) {
+                    uint32_t v[32];
+                    HC_TMEM_LD32(o_tmem + i, v);
+                    float4 after[8];
+                    #pragma unroll
+                    for (int u = 0; u < 8; ++u) after[u] = state4(state_holds && i < 96, i + 32 + 4 * u);
+                    tc_wait_ld();
+                    #pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        join(v + 4 * u, before[u], a, b);
+                        state[(i / 4 + u) * kRows] = make_float4(__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1]), __uint_as_float(v[4 * u + 2]),
+                                                                 __uint_as_float(v[4 * u + 3]));
+                        before[u] = after[u];
+                    }
+                }
+                free_o();
+                #pragma unroll
+                for (int i = 0; i < 128; ++i) A[i] = 0.0f;
                 M = kEmptyMax;
                 L = 0.0f;
                 state_holds = true;
             }
             if (!ok) break;
+            if (!warp_has_rows) continue;
+            const size_t vec = size_t(w.row0 + t_local) * args.q_heads + w.kv_head * G + g;
             const int col0 = w.half * kPairO + half * 128;
             if constexpr (MODE == kPairSegments) {
                 // The segment's partial goes to the workspace (a merge kernel runs the second fold).
-                if (valid) {
-                    const size_t prow = vec * args.slots + w.slot;
-                    float* dst = args.part_o + prow * D + col0;
+                const size_t prow = vec * args.slots + w.slot;
+                float* dst = args.part_o + prow * D + col0;
+                #pragma unroll 1
+                for (int i = 0; i < 128; i += 32) {
+                    uint32_t v[32];
+                    HC_TMEM_LD32(o_tmem + i, v);
+                    tc_wait_ld();
                     #pragma unroll
-                    for (int i = 0; i < 128; i += 4) {
-                        *reinterpret_cast<float4*>(dst + i) = make_float4(A[i], A[i + 1], A[i + 2], A[i + 3]);
-                    }
-                    if (half == 0 && w.half == 0) *reinterpret_cast<float2*>(args.part_ml + prow * 2) = make_float2(M, L);
+                    for (int u = 0; valid && u < 32; u += 4) *reinterpret_cast<uint4*>(dst + i + u) = make_uint4(v[u], v[u + 1], v[u + 2], v[u + 3]);
                 }
+                free_o();
+                if (valid && half == 0 && w.half == 0) *reinterpret_cast<float2*>(args.part_ml + prow * 2) = make_float2(M, L);
                 continue;
             }
             // The row's last segment: the last step of the second fold, which started from the sink (or
             // from the empty state).
+            float a, b;
             {
-                float M2, L2;
-                second_fold_state(state_holds, valid ? head : 0, M2, L2);
-                float Mn, a, b;
+                float M2, L2, Mn;
+                second_fold_state(state_holds, sink, M2, L2);
                 fold_coefficients(M2, M, Mn, a, b);
                 L = __fmaf_rn(L2, a, __fmul_rn(L, b));
                 M = Mn;
-                if (state_holds) {
-                    #pragma unroll
-                    for (int i0 = 0; i0 < 128; i0 += 16) {
-                        float4 before[4];
-                        #pragma unroll
-                        for (int i = 0; i < 4; ++i) before[i] = state[(i0 / 4 + i) * kRows];
-                        #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            float* v = &A[i0 + 4 * i];
-                            v[0] = fold_value(before[i].x, a, v[0], b);
-                            v[1] = fold_value(before[i].y, a, v[1], b);
-                            v[2] = fold_value(before[i].z, a, v[2], b);
-                            v[3] = fold_value(before[i].w, a, v[3], b);
-                        }
-                        asm volatile("" ::: "memory");
-                    }
-                } else {
-                    // fold_value(0, a, A, b) = 0 * a + A * b = A * b exactly: one multiply.
-                    #pragma unroll
-                    for (int i = 0; i < 128; ++i) A[i] = __fmul_rn(A[i], b);
-                }
             }
-            if (MODE == kPairRowsOut && args.ep.write_partial) {
-                if (!valid) continue;
-                float* dst = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2) + col0;
-                #pragma unroll
-                for (int i = 0; i < 128; i += 2) *reinterpret_cast<float2*>(dst + i) = make_float2(A[i], A[i + 1]);
-                if (half == 0 && w.half == 0) {
-                    float* tail = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2) + D;
-                    tail[0] = M;
-                    tail[1] = L;
-                }
-                continue;
-            }
-            // Rows leave through shared memory, 64 bytes of each at a time, so that a store instruction touches 8
-            // lines and not 32 (a thread storing its own row took 4300 clocks an item).  Lane l moves piece l % 4 of
-            // rows l / 4, l / 4 + 8, ..
-            if (!warp_has_rows) continue;
             const float inverse = __frcp_rn(L);
-            unsigned char* stage = store_smem + (warp - 12) * kPairStoreBytes;
-            auto piece = [&](int r, int c) -> uint4* { return reinterpret_cast<uint4*>(stage + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); };
-            const int c = lane & 3;
-            auto row_of = [&](int k, size_t& out_row) -> bool {
-                const int r = quad * 32 + k * 8 + (lane >> 2);
-                const int token = token0 + (r >> args.log_group);
-                out_row = size_t(w.row0 + token) * args.q_heads + size_t(w.kv_head) * G + (r & (G - 1));
-                return token < w.valid_tokens;
-            };
             if constexpr (MODE == kPairGatedOut) {
-                // With a gate, or fp32 rows.  The values go back to tensor memory, in place of the last O, so that the
-                // rest can be a rolled loop, thread = row, with registers to spare for the next 16 columns' gates: eight
-                // copies of it, fetched cold, and gate loads that waited for one another were 17 us of a launch
-                // (777 tokens behind 1291, 16 gated heads of 256: 97 us, now 83).
-                #pragma unroll
-                for (int i = 0; i < 128; i += 16) {
-                    uint32_t v[16];
-                    #pragma unroll
-                    for (int u = 0; u < 16; ++u) v[u] = __float_as_uint(__fmul_rn(A[i + u], inverse));
-                    HC_TMEM_ST16(o_tmem + i, v);
-                }
-                tc_wait_st();
-                asm volatile("" ::: "memory");
+                // With a gate, or fp32 rows: thread = row, with registers to spare for the next 16 columns' gates.
                 const bool gated = args.ep.gate_layout != HC_GATE_NONE, fp32 = args.ep.io_dtype == HC_F32;
                 const int bytes = fp32 ? 4 : 2;
                 const size_t gate_at = args.ep.gate_layout == HC_GATE_INTERLEAVED ? vec * size_t(2 * D) + D : vec * size_t(D);
@@ -630,19 +623,29 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     return make_float4(__uint_as_float(two.x << 16), __uint_as_float(two.x & 0xffff0000u),
                                        __uint_as_float(two.y << 16), __uint_as_float(two.y & 0xffff0000u));
                 };
-                float4 now[4], next[4];
+                float4 now[4], next[4], before[4], after[4];
                 #pragma unroll
-                for (int u = 0; u < 4; ++u) now[u] = gate4(4 * u);
+                for (int u = 0; u < 4; ++u) {
+                    now[u] = gate4(4 * u);
+                    before[u] = state4(state_holds, 4 * u);
+                }
                 #pragma unroll 1
                 for (int i = 0; i < 128; i += 16) {
                     uint32_t v[16];
                     HC_TMEM_LD16(o_tmem + i, v);
                     #pragma unroll
-                    for (int u = 0; u < 4; ++u) next[u] = gate4(i < 112 ? i + 16 + 4 * u : 0);
+                    for (int u = 0; u < 4; ++u) {
+                        next[u] = gate4(i < 112 ? i + 16 + 4 * u : 0);
+                        after[u] = state4(state_holds && i < 112, i + 16 + 4 * u);
+                    }
                     tc_wait_ld();
+                    if (i == 112) free_o();
                     #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        float r[4] = {__uint_as_float(v[4 * u]), __uint_as_float(v[4 * u + 1]), __uint_as_float(v[4 * u + 2]), __uint_as_float(v[4 * u + 3])};
+                        join(v + 4 * u, before[u], a, b);
+                        float r[4];
+                        #pragma unroll
+                        for (int x = 0; x < 4; ++x) r[x] = __fmul_rn(__uint_as_float(v[4 * u + x]), inverse);
                         if (gated) {
                             r[0] = __fmul_rn(r[0], sigmoid_gate(now[u].x));
                             r[1] = __fmul_rn(r[1], sigmoid_gate(now[u].y));
@@ -650,6 +653,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                             r[3] = __fmul_rn(r[3], sigmoid_gate(now[u].w));
                         }
                         now[u] = next[u];
+                        before[u] = after[u];
                         if (!valid) continue;
                         if (fp32) {
                             *reinterpret_cast<float4*>(out + (i + 4 * u) * 4) = make_float4(r[0], r[1], r[2], r[3]);
@@ -658,66 +662,63 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                         }
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster_relaxed(o_free);
                 continue;
             }
-            if (D == 256 || (args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32)) {
-                uint16_t* out = reinterpret_cast<uint16_t*>(args.ep.out) + col0 + c * 8;
-                #pragma unroll
-                for (int i = 0; i < 128; i += 32) {
-                    #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float* v = &A[i + u * 8];
-                        *piece(lane, u) = make_uint4(pack_bf16x2(__fmul_rn(v[0], inverse), __fmul_rn(v[1], inverse)),
-                                                     pack_bf16x2(__fmul_rn(v[2], inverse), __fmul_rn(v[3], inverse)),
-                                                     pack_bf16x2(__fmul_rn(v[4], inverse), __fmul_rn(v[5], inverse)),
-                                                     pack_bf16x2(__fmul_rn(v[6], inverse), __fmul_rn(v[7], inverse)));
-                    }
-                    __syncwarp();
-                    #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        size_t out_row;
-                        if (row_of(k, out_row)) *reinterpret_cast<uint4*>(out + out_row * D + i) = *piece(k * 8 + (lane >> 2), c);
-                    }
-                    __syncwarp();
-                }
-            } else if constexpr (D == 512) {
-                const int gate_layout = args.ep.gate_layout;
-                const size_t gate_stride = gate_layout == HC_GATE_INTERLEAVED ? size_t(2 * D) : size_t(D);
-                const size_t gate_first = (gate_layout == HC_GATE_INTERLEAVED ? D : 0) + col0 + c * 4;
-                #pragma unroll
-                for (int i = 0; i < 128; i += 16) {
-                    #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float* v = &A[i + u * 4];
-                        *piece(lane, u) = make_uint4(__float_as_uint(__fmul_rn(v[0], inverse)), __float_as_uint(__fmul_rn(v[1], inverse)),
-                                                     __float_as_uint(__fmul_rn(v[2], inverse)), __float_as_uint(__fmul_rn(v[3], inverse)));
-                    }
-                    __syncwarp();
-                    #pragma unroll 1
-                    for (int k = 0; k < 4; ++k) {
-                        size_t out_row;
-                        if (!row_of(k, out_row)) continue;
-                        const uint4 x = *piece(k * 8 + (lane >> 2), c);
-                        float r[4] = {__uint_as_float(x.x), __uint_as_float(x.y), __uint_as_float(x.z), __uint_as_float(x.w)};
-                        if (gate_layout != HC_GATE_NONE) {
-                            const size_t at = out_row * gate_stride + gate_first + i;
-                            #pragma unroll
-                            for (int u = 0; u < 4; ++u) r[u] = __fmul_rn(r[u], sigmoid_gate(load_io(args.ep.gate, at + u, args.ep.io_dtype)));
-                        }
-                        const size_t at = out_row * D + col0 + i + c * 4;
-                        if (args.ep.io_dtype == HC_F32) {
-                            *reinterpret_cast<float4*>(reinterpret_cast<float*>(args.ep.out) + at) = make_float4(r[0], r[1], r[2], r[3]);
-                        } else {
-                            *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(args.ep.out) + at) =
-                                make_uint2(pack_bf16x2(r[0], r[1]), pack_bf16x2(r[2], r[3]));
-                        }
-                    }
-                    __syncwarp();
-                }
+            // bf16 rows leave through shared memory, 64 bytes of each at a time, so that a store instruction touches 8
+            // lines and not 32 (a thread storing its own row took 4300 clocks an item).  Lane l moves piece l % 4 of
+            // rows l / 4, l / 4 + 8, ..  Row partials (a sequence-sharded cache) are stored by their own threads.
+            unsigned char* stage = store_smem + (warp - 12) * kPairStoreBytes;
+            auto piece = [&](int r, int c) -> uint4* { return reinterpret_cast<uint4*>(stage + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); };
+            const int c = lane & 3;
+            uint16_t* rows_out[4];
+            #pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = quad * 32 + k * 8 + (lane >> 2);
+                const int token = token0 + (r >> args.log_group);
+                const size_t out_row = size_t(w.row0 + token) * args.q_heads + size_t(w.kv_head) * G + (r & (G - 1));
+                rows_out[k] = token < w.valid_tokens ? reinterpret_cast<uint16_t*>(args.ep.out) + out_row * D + col0 + c * 8 : nullptr;
             }
+            float* partial = reinterpret_cast<float*>(args.ep.out) + vec * size_t(D + 2) + col0;
+            const bool partials = args.ep.write_partial != 0;
+            float4 before[8];
+            #pragma unroll
+            for (int u = 0; u < 8; ++u) before[u] = state4(state_holds, 4 * u);
+            #pragma unroll 1
+            for (int i = 0; i < 128; i += 32) {
+                uint32_t v[32];
+                HC_TMEM_LD32(o_tmem + i, v);
+                float4 after[8];
+                #pragma unroll
+                for (int u = 0; u < 8; ++u) after[u] = state4(state_holds && i < 96, i + 32 + 4 * u);
+                tc_wait_ld();
+                if (i == 96) free_o();
+                #pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    join(v + 4 * u, before[u], a, b);
+                    before[u] = after[u];
+                }
+                if (partials) {
+                    #pragma unroll
+                    for (int u = 0; valid && u < 32; u += 2) *reinterpret_cast<uint2*>(partial + i + u) = make_uint2(v[u], v[u + 1]);
+                    continue;
+                }
+                #pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    uint32_t p[4];
+                    #pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        p[x] = pack_bf16x2(__fmul_rn(__uint_as_float(v[8 * u + 2 * x]), inverse), __fmul_rn(__uint_as_float(v[8 * u + 2 * x + 1]), inverse));
+                    }
+                    *piece(lane, u) = make_uint4(p[0], p[1], p[2], p[3]);
+                }
+                __syncwarp();
+                #pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (rows_out[k] != nullptr) *reinterpret_cast<uint4*>(rows_out[k] + i) = *piece(k * 8 + (lane >> 2), c);
+                }
+                __syncwarp();
+            }
+            if (partials && valid && half == 0 && w.half == 0) *reinterpret_cast<float2*>(partial + D) = make_float2(M, L);
         }
     }
 
@@ -754,9 +755,10 @@ hc_status launch_pair_kernel(hc_context* ctx, const hc_layer_store& layer, const
 template <bool BLOCKS>
 hc_status launch_pair(hc_context* ctx, const hc_layer_store& layer, const CUtensorMap& tmap_q, const TcArgs& args, int head_dim, bool gated,
                       cudaStream_t stream) {
-    auto launch = head_dim == 512 ? (args.finish ? launch_pair_kernel<512, kPairRowsOut, BLOCKS> : launch_pair_kernel<512, kPairSegments, BLOCKS>)
-                : !args.finish    ? launch_pair_kernel<256, kPairSegments, BLOCKS>
-                : gated           ? launch_pair_kernel<256, kPairGatedOut, BLOCKS> : launch_pair_kernel<256, kPairRowsOut, BLOCKS>;
+    const bool wide = head_dim == 512;
+    auto launch = !args.finish ? (wide ? launch_pair_kernel<512, kPairSegments, BLOCKS> : launch_pair_kernel<256, kPairSegments, BLOCKS>)
+                : gated        ? (wide ? launch_pair_kernel<512, kPairGatedOut, BLOCKS> : launch_pair_kernel<256, kPairGatedOut, BLOCKS>)
+                               : (wide ? launch_pair_kernel<512, kPairRowsOut, BLOCKS> : launch_pair_kernel<256, kPairRowsOut, BLOCKS>);
     return launch(ctx, layer, tmap_q, args, stream);
 }
 
@@ -772,7 +774,6 @@ hc_status launch_attention_pair(hc_context* ctx, const hc_layer_store& layer, co
     const hc_status st = tc_encode_3d(&tmap_q, args.q, uint64_t(head_dim), uint64_t(args.q_heads), uint64_t(args.tokens), uint32_t(group),
                                       uint32_t(kRows / group));
     if (st != HC_OK) return st;
-    // (Head_dim 512 has one epilogue for all: apart, its kernel for bf16 rows came out 6 % slower.)
     const bool gated = !args.ep.write_partial && (args.ep.gate_layout != HC_GATE_NONE || args.ep.io_dtype == HC_F32);
     return args.blocks.ends ? launch_pair<true>(ctx, layer, tmap_q, args, head_dim, gated, stream)
                             : launch_pair<false>(ctx, layer, tmap_q, args, head_dim, gated, stream);
