@@ -141,6 +141,15 @@ __device__ __forceinline__ void fma2_inplace(uint32_t& x0, uint32_t& x1, float c
     x1 = uint32_t(x >> 32);
 }
 
+// (x0, x1) <- (x0 * c, x1 * c).
+__device__ __forceinline__ void mul2_inplace(float& x0, float& x1, float c) {
+    uint64_t x = uint64_t(__float_as_uint(x0)) | (uint64_t(__float_as_uint(x1)) << 32);
+    const uint64_t cc = uint64_t(__float_as_uint(c)) | (uint64_t(__float_as_uint(c)) << 32);
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(cc));
+    x0 = __uint_as_float(uint32_t(x));
+    x1 = __uint_as_float(uint32_t(x >> 32));
+}
+
 // Two steps of the fold at once: (A0, A1) <- (A0 * a + (o0 * b), A1 * a + (o1 * b)), every product
 // and sum rounded exactly as fold_value does, in two packed instructions instead of four.
 __device__ __forceinline__ void fold_value2(float& A0, float& A1, float a, uint32_t o0, uint32_t o1, float b) {
