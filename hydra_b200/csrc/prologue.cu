@@ -35,7 +35,7 @@ __device__ __forceinline__ uint16_t* also_row(const PrepArgs& args, int kind, in
 // are worked on.  What bounds it is its instructions, so a lane owns sixteen elements (8 m .. 8 m + 7 of each half, 16-byte
 // accesses; head_dim 512 as in HeadLanes): a warp has two vectors of 256 at a time, and reduces, and takes the root and the
 // addresses, once for both (8192 tokens of 32 x 256 with norms and rotation: 90 us with a vector a warp, a division by
-// head_dim and a remainder per cached row, now 64).  The bits are HeadLanes' and prepare_head's: a lane keeps the sums of two of
+// head_dim and a remainder per cached row, 64 without the prefetch into L2, now 55).  The bits are HeadLanes' and prepare_head's: a lane keeps the sums of two of
 // their lanes apart until the last step of the butterfly.
 // The launcher checks the alignment this needs and otherwise uses the general kernel below.
 template <int D>
@@ -159,6 +159,12 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
     for (;;) {
         const bool more = token + step < unsigned(args.tokens);
         if (more) ahead.load(src + src_step, m);
+        if (token + 3 * step < unsigned(args.tokens)) {              // two further on their way into L2
+            #pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(src + 3 * src_step + (h * (D / 2) + WL::at(m, 0)) * kBytes));
+            }
+        }
         const int position = args.batched ? args.meta.pos[token] : args.first_position + int(token);
         float c[8], s[8];
         if (rope) {
