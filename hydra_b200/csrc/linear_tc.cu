@@ -80,10 +80,63 @@ struct LinArgs {
     int y_dtype;              // HC_F32 or HC_BF16
     int tokens;
     int tiles_m, n_tiles, k_steps;   // tiles of 128 rows (few tokens) or 256 (pairs)
+    int n_wide;               // pairs, 256 columns: the first n_wide tiles are that wide, the others half of it
     int a_bytes;              // few tokens: of one x box, as many rows of 128 bytes as there are tokens (rounded up to 8)
     int stages;               // few tokens
     int* status;
 };
+
+// Tiles of two widths.  A job's columns are cut in wide tiles, and what is left of an odd number of halves is a half tile.
+// The list has n_wide of the wide tiles, then the halves of the others and the odd halves, so that a launch's last
+// round of pairs can be one of half tiles.
+struct LinWide {
+    int job, col, tm, width;
+};
+template <int BN>
+__host__ __device__ __forceinline__ LinWide decode_wide(const LinArgs& args, int tile) {
+    LinWide t{0, 0, 0, BN};
+    int all = 0;                                             // wide tiles of all jobs
+    #pragma unroll
+    for (int j = 0; j < kLinJobs; ++j) {
+        if (j < args.n_jobs) all += args.job[j].out_features / BN * args.tiles_m;
+    }
+    int wide = tile, half = 0;
+    if (tile >= args.n_wide) {
+        t.width = BN / 2;
+        wide = args.n_wide + ((tile - args.n_wide) >> 1);
+        half = (tile - args.n_wide) & 1;
+    }
+    if (wide < all) {
+        int left = wide;
+        #pragma unroll
+        for (int j = 0; j < kLinJobs; ++j) {
+            const int tiles = j < args.n_jobs ? args.job[j].out_features / BN * args.tiles_m : 0;
+            if (j < args.n_jobs && left >= 0 && left < tiles) {
+                t.job = j;
+                t.col = left / args.tiles_m;
+                t.tm = left - t.col * args.tiles_m;
+                t.col = t.col * BN + half * (BN / 2);
+            }
+            left -= tiles;
+        }
+        return t;
+    }
+    // Behind them a job's last columns: one or two half tiles a row tile.
+    int left = tile - args.n_wide - 2 * (all - args.n_wide);
+    #pragma unroll
+    for (int j = 0; j < kLinJobs; ++j) {
+        const int first = j < args.n_jobs ? args.job[j].out_features / BN * BN : 0;
+        const int tiles = j < args.n_jobs ? (args.job[j].out_features - first + BN / 2 - 1) / (BN / 2) * args.tiles_m : 0;
+        if (left >= 0 && left < tiles) {
+            t.job = j;
+            t.col = left / args.tiles_m;
+            t.tm = left - t.col * args.tiles_m;
+            t.col = first + t.col * (BN / 2);
+        }
+        left -= tiles;
+    }
+    return t;
+}
 
 struct LinTile {
     int job, tn, tm;
@@ -385,7 +438,8 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
     if (warp == 1) tmem_dealloc(tmem, kFewTmemCols);
 }
 
-// Two SMs per 256 x BN tile; see the head of the file.  The leading CTA's barriers count both CTAs' loads.
+// Two SMs per 256 x BN tile (BN 256: of tiles of 128 columns too, see decode_wide); see the head of the file.  The leading
+// CTA's barriers count both CTAs' loads.
 template <int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLinThreads, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
@@ -430,29 +484,37 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     pdl_wait();
 
     const int n_tiles = args.n_tiles;
+    constexpr bool kTwoWidths = BN == 256;
+    auto tile_at = [&](int tile) -> LinWide {
+        if constexpr (kTwoWidths) return decode_wide<BN>(args, tile);
+        const LinTile where = decode_tile(args, tile);
+        return LinWide{where.job, where.tn * BN, where.tm, BN};
+    };
     if (warp == 0) {
         // ===== producer: this CTA's rows of x and its half of the weight tile, counted by the leader =====
         if (lane == 0) {
             uint32_t step = 0;
             bool ok = true;
             for (int tile = pair; ok && tile < n_tiles; tile += pairs) {
-                const LinTile where = decode_tile(args, tile);
-                const int tn = where.tn, tm = where.tm;
+                const LinWide where = tile_at(tile);
+                const int tm = where.tm, w_row = where.col + rank * (where.width / 2);
                 const CUtensorMap* tmap_w = where.job == 0 ? &tmap_w0 : where.job == 1 ? &tmap_w1 : where.job == 2 ? &tmap_w2 : &tmap_w3;
                 for (int k = 0; k < args.k_steps; ++k, ++step) {
                     const int slot = int(step % PS::kStages);
                     const uint32_t round = step / PS::kStages;
                     if (round > 0 && !mbar_wait(&bars->empty[slot], (round - 1) & 1, abort_flag, args.status, 21)) { ok = false; break; }
                     const uint32_t full = cluster_addr(&bars->full[slot], 0);
-                    if (rank == 0) mbar_expect_tx(&bars->full[slot], 2 * (kLinABytes + PS::kBBytes));
+                    if (rank == 0) mbar_expect_tx(&bars->full[slot], 2 * (kLinABytes + where.width / 2 * kLinK * 2));
                     tma_load_2d_pair(a_smem + slot * kLinABytes, &tmap_x, full, k * kLinK, tm * (2 * kLinM) + rank * kLinM);
-                    tma_load_2d_pair(b_smem + slot * PS::kBBytes, tmap_w, full, k * kLinK, tn * BN + rank * (BN / 2));
+                    tma_load_2d_pair(b_smem + slot * PS::kBBytes, tmap_w, full, k * kLinK, w_row);
+                    if (kTwoWidths && where.width == BN) {       // (boxes of 64 rows)
+                        tma_load_2d_pair(b_smem + slot * PS::kBBytes + PS::kBBytes / 2, tmap_w, full, k * kLinK, w_row + BN / 4);
+                    }
                 }
             }
         }
     } else if (warp == 1 && rank == 0) {
         // ===== MMA issuer (the warp walks the loop converged; one elected lane issues) =====
-        constexpr uint32_t idesc = instr_desc_pair(BN, false);
         const uint64_t a_desc0 = smem_desc(smem_u32(a_smem), 16);
         const uint64_t b_desc0 = smem_desc(smem_u32(b_smem), 16);
         uint32_t step = 0, count = 0;
@@ -462,6 +524,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             // The epilogues must have taken this accumulator's previous tile out.
             if (count >= 2 && !mbar_wait(&bars->acc_empty[acc], ((count >> 1) - 1) & 1, abort_flag, args.status, 22)) break;
             tc_fence_after();
+            const uint32_t idesc = kTwoWidths && tile >= args.n_wide ? instr_desc_pair(BN / 2, false) : instr_desc_pair(BN, false);
             for (int k = 0; k < args.k_steps; ++k, ++step) {
                 const int slot = int(step % PS::kStages);
                 if (!mbar_wait(&bars->full[slot], (step / PS::kStages) & 1, abort_flag, args.status, 23)) { ok = false; break; }
@@ -487,22 +550,22 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         const uint32_t lane_base = uint32_t(quad * 32) << 16;
         uint32_t count = 0;
         for (int tile = pair; tile < n_tiles; tile += pairs, ++count) {
-            const LinTile where = decode_tile(args, tile);
+            const LinWide where = tile_at(tile);
             const LinJob& job = args.job[where.job];
             const int row0 = where.tm * (2 * kLinM) + rank * kLinM + quad * 32;
             const int acc = int(count & 1);
             float4 z[8], z_next[8];
-            load_residual(args, job, row0, where.tn * BN, z);
-            const uint4 bias = load_bias(job, where.tn * BN);
+            load_residual(args, job, row0, where.col, z);
+            const uint4 bias = load_bias(job, where.col);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
             #pragma unroll 1
-            for (int chunk = 0; chunk < BN / 32; ++chunk) {
+            for (int chunk = 0; chunk < where.width / 32; ++chunk) {
                 uint32_t v[32];
                 HC_TMEM_LD32(tmem + lane_base + acc * BN + chunk * 32, v);
-                if (chunk + 1 < BN / 32) load_residual(args, job, row0, where.tn * BN + (chunk + 1) * 32, z_next);
+                if (chunk + 1 < where.width / 32) load_residual(args, job, row0, where.col + (chunk + 1) * 32, z_next);
                 tc_wait_ld();
-                store_block(args, job, v, block_bias(bias, chunk), z, row0, where.tn * BN + chunk * 32, stage);
+                store_block(args, job, v, block_bias(bias, chunk), z, row0, where.col + chunk * 32, stage);
                 if (job.residual != nullptr) {
                     #pragma unroll
                     for (int k = 0; k < 8; ++k) z[k] = z_next[k];
@@ -627,10 +690,15 @@ static hc_status launch_few(hc_context* ctx, const void* x, const void* const* w
 }
 
 template <int BN>
-static hc_status launch_pair(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features, cudaStream_t stream) {
+static hc_status launch_pair(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features, cudaStream_t stream,
+                             int n_wide = 0, int n_tiles = 0) {
     LinMaps maps;
-    const hc_status st = prepare_linear(maps, x, w, args, in_features, 2 * kLinM, BN, kLinM, BN / 2);
+    const hc_status st = prepare_linear(maps, x, w, args, in_features, 2 * kLinM, BN, kLinM, BN == 256 ? BN / 4 : BN / 2);
     if (st != HC_OK) return st;
+    if (BN == 256) {
+        args.n_wide = n_wide;
+        args.n_tiles = n_tiles;
+    }
     static bool configured[64] = {};
     constexpr int smem = PairShape<BN>::kSmemBytes + int(sizeof(LinBarriers)) + 4 * kLinStageBytes;
     static_assert(smem <= 227 * 1024, "shared memory of one CTA");
@@ -672,19 +740,40 @@ hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* cons
     const int pairs = std::max(ctx->sm_count / 2, 1);
     const int widths[4] = {256, 192, 160, 128};
     const double step[4] = {546.0, 478.0, 443.0, 410.0};
+    const int tiles_m = (tokens + 2 * kLinM - 1) / (2 * kLinM);
     int best = 0;
     double least = 0.0;
     for (int i = 0; i < 4; ++i) {
         long long tiles = 0;
-        for (int j = 0; j < n_jobs; ++j) tiles += (long long)((tokens + 2 * kLinM - 1) / (2 * kLinM)) * ((out_features[j] + widths[i] - 1) / widths[i]);
+        for (int j = 0; j < n_jobs; ++j) tiles += (long long)tiles_m * ((out_features[j] + widths[i] - 1) / widths[i]);
         const double t = double((tiles + pairs - 1) / pairs) * step[i];
         if (i == 0 || t < least) {
             least = t;
             best = i;
         }
     }
+    // Or wide tiles in whole rounds and half tiles for the rest, in the last round or two: 4096 tokens to 2880 columns are two
+    // rounds of 256 and one of 128 instead of three of 256 (81.2 us, now 77.8; 2048 tokens to q, k and v of 4096 and 512 columns
+    // 48.7, now 46.0).  Where another choice is predicted as fast it is faster: its K steps are of one size, its ring deeper
+    // (600 tokens of 2816 to 8192 columns 28.7 against 31.6).
+    long long wide = 0, odd = 0;
+    for (int j = 0; j < n_jobs; ++j) {
+        wide += (long long)tiles_m * (out_features[j] / 256);
+        odd += (long long)tiles_m * ((out_features[j] % 256 + 127) / 128);
+    }
+    long long n_wide = wide;                                 // 256 columns throughout: the last of a job's in half tiles
+    for (long long rounds = 1; rounds * pairs <= wide; ++rounds) {
+        const long long n = rounds * pairs, total = (n + 2 * (wide - n) + odd + pairs - 1) / pairs;
+        const double t = double(rounds) * step[0] + double(total - rounds) * step[3];
+        if (t < least) {
+            least = t;
+            best = 0;
+            n_wide = n;
+        }
+    }
+    const long long n_tiles = n_wide + 2 * (wide - n_wide) + odd;
     switch (widths[best]) {
-        case 256: return launch_pair<256>(ctx, x, w, args, in_features, stream);
+        case 256: return launch_pair<256>(ctx, x, w, args, in_features, stream, int(n_wide), int(n_tiles));
         case 192: return launch_pair<192>(ctx, x, w, args, in_features, stream);
         case 160: return launch_pair<160>(ctx, x, w, args, in_features, stream);
         default: return launch_pair<128>(ctx, x, w, args, in_features, stream);

@@ -109,3 +109,27 @@ def test_linear_refuses_what_it_cannot_tile():
     with pytest.raises(hb.DimensionMismatch):
         backend.linear(x, w, None, y, 4, 72, 16)
     ctx.close()
+
+
+@pytest.mark.parametrize("tokens, width, outs", [
+    (4096, 64, (2880,)),               # two rounds of wide tiles and one of halves, an odd half of 64 columns
+    (3900, 128, (2880,)),              # a ragged last row tile
+    (2048, 64, (4096, 512, 512)),      # three jobs; the cut lies in the first
+    (4096, 64, (1000, 2880, 130)),     # last columns of one and two halves
+    (4096, 64, (4096, 513)),           # a last half of one column
+    (9000, 64, (100, 90)),             # no wide tile at all
+])
+def test_linear_tiles_of_two_widths(tokens, width, outs):
+    """Sums of 64 or 128 products in fp32 against float64: 128 roundings of 2^-24 of sums below 40 stay under 4e-4."""
+    import torch
+    import hydra_b200 as hb
+    ctx = hb.Context(0)
+    gen = torch.Generator(device="cuda").manual_seed(tokens + width)
+    x = torch.randn(tokens, width, device="cuda", generator=gen).to(torch.bfloat16)
+    w = [torch.randn(n, width, device="cuda", generator=gen).to(torch.bfloat16) for n in outs]
+    y = [torch.full((tokens, n), 7.0, device="cuda") for n in outs]
+    hb.AttentionBackend(ctx).linear_group(x, w, [None] * len(outs), y, tokens, width, y_dtype=hb.capi.HC_F32)
+    ctx.check()
+    for got, weight in zip(y, w):
+        assert float((got.double() - x.double() @ weight.double().T).abs().max()) < 4e-4
+    ctx.close()
