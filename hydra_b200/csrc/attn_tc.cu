@@ -749,9 +749,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 M = Mn;
                 float* const state = state_of_row();
                 if (LT::kStateInSmem && args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32 && !args.ep.write_partial) {
-                    // bf16 rows: scaled, rounded and packed in their threads, then through shared memory so that a store
-                    // writes whole lines (a row is one, the G heads of a token lie side by side).  (By the loop below an item's
-                    // end took 6500 clocks, now 4000: 4096 tokens with a window of 128 73 us, now 62.)
+                    // bf16 rows: scaled, rounded, packed and stored by their threads, a row's line in 32-byte stores.  (By the
+                    // loop below an item's end took 6500 clocks; packed here and through shared memory, eight lanes a
+                    // row, 4000: 4096 tokens with a window of 128 73 and 62 us, now 58.)
                     if (!warp_has_rows) continue;
                     if (state_holds) {
                         #pragma unroll
@@ -762,29 +762,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         for (int i = 0; i < D; i += 2) mul2_inplace(A[i], A[i + 1], b);
                     }
                     const float inverse = __frcp_rn(L);
-                    unsigned char* const stage = reinterpret_cast<unsigned char*>(warp_state);
-                    __syncwarp();                            // every lane has read its state, and stored the item before
+                    uint16_t* const out = reinterpret_cast<uint16_t*>(args.ep.out) + (out_row * args.q_heads + head) * D;
                     #pragma unroll
-                    for (int ch = 0; ch < 8; ++ch) {
-                        uint32_t packed[4];
+                    for (int i = 0; i < D; i += 16) {
+                        uint32_t packed[8];
                         #pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            float &x = A[ch * 8 + 2 * u], &y = A[ch * 8 + 2 * u + 1];
-                            mul2_inplace(x, y, inverse);
-                            packed[u] = pack_bf16x2(x, y);
+                        for (int u = 0; u < 8; ++u) {
+                            mul2_inplace(A[i + 2 * u], A[i + 2 * u + 1], inverse);
+                            packed[u] = pack_bf16x2(A[i + 2 * u], A[i + 2 * u + 1]);
                         }
-                        *reinterpret_cast<uint4*>(stage + lane * 128 + ((ch ^ (lane & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                    }
-                    __syncwarp();
-                    const int ch = lane & 7, first = quad * 32 + (lane >> 3);
-                    uint16_t* const out = reinterpret_cast<uint16_t*>(args.ep.out) +
-                                          (size_t(w.row0) * args.q_heads + size_t(w.kv_head) * G) * D + ch * 8;
-                    const unsigned token_stride = unsigned(args.q_heads) * D;
-                    #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const int r = first + k * 4, token = r >> args.log_group;
-                        const uint4 value = *reinterpret_cast<const uint4*>(stage + (k * 4 + (lane >> 3)) * 128 + ((ch ^ ((k * 4 + (lane >> 3)) & 7)) << 4));
-                        if (token < w.valid_tokens) *reinterpret_cast<uint4*>(out + size_t(token) * token_stride + (r & (G - 1)) * D) = value;
+                        if (valid) store_32bytes(out + i, packed);
                     }
                     continue;
                 }

@@ -141,6 +141,17 @@ __device__ __forceinline__ void fma2_inplace(uint32_t& x0, uint32_t& x1, float c
     x1 = uint32_t(x >> 32);
 }
 
+// Eight words to a 16-byte boundary, in one store where it is a 32-byte one (all of a launch's rows lie alike).
+__device__ __forceinline__ void store_32bytes(void* dst, const uint32_t (&v)[8]) {
+    if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                     ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+    } else {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+        *(reinterpret_cast<uint4*>(dst) + 1) = make_uint4(v[4], v[5], v[6], v[7]);
+    }
+}
+
 // (x0, x1) <- (x0 * c, x1 * c).
 __device__ __forceinline__ void mul2_inplace(float& x0, float& x1, float c) {
     uint64_t x = uint64_t(__float_as_uint(x0)) | (uint64_t(__float_as_uint(x1)) << 32);

@@ -219,3 +219,17 @@ def test_prompts_longer_than_a_ring_equal_linear_storage(hb, ctx, d, qh, kvh, wi
         layer.close()
     for ring, linear in zip(*got):
         assert np.array_equal(ring, linear)
+
+
+@pytest.mark.parametrize("d, qh, kvh, tokens, window", [(64, 16, 2, 77, 0), (64, 64, 8, 300, 128), (256, 16, 8, 140, 0), (256, 8, 8, 515, 256),
+                                                       (512, 8, 1, 65, 0)])
+def test_outputs_on_16_byte_boundaries_that_are_no_32_byte_ones(hb, ctx, d, qh, kvh, tokens, window):
+    import torch
+    layer, q, k, v, sinks, _ = _filled(hb, ctx, d, qh, kvh, window, tokens)
+    want = layer.prefill(q, 0)
+    flat = torch.full((tokens * qh * d + 16,), 7.0, device="cuda", dtype=torch.bfloat16)
+    layer.backend.attention_prefill(layer.cache, 0, tl.to_device(q), flat[8:-8].view(tokens, qh, d), tokens, 0, layer.params)
+    ctx.check()
+    assert np.array_equal(tl.to_host(flat[8:-8]).reshape(want.shape), want)
+    assert bool((flat[:8] == 7).all()) and bool((flat[-8:] == 7).all())
+    layer.close()
