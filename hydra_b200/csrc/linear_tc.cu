@@ -185,7 +185,7 @@ __device__ __forceinline__ float4 block_bias(const uint4& tile, int block) {
     const uint32_t lo = (lane & 1) ? z : x, hi = (lane & 1) ? w : y;
     return make_float4(__uint_as_float(lo << 16), __uint_as_float(lo & 0xffff0000u), __uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
 }
-__device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob& job, int row0, int col0, float4 (&z)[8]) {
+__device__ __forceinline__ void load_residual(const LinJob& job, int row0, int row_end, int col0, float4 (&z)[8]) {
     if (job.residual == nullptr) return;                                        // z is not looked at
     #pragma unroll
     for (int k = 0; k < 8; ++k) z[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -196,7 +196,7 @@ __device__ __forceinline__ void load_residual(const LinArgs& args, const LinJob&
     #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const int row = row0 + k * 4 + (lane >> 3);
-        if (row >= args.tokens) continue;
+        if (row >= row_end) continue;
         const float* src = job.residual + size_t(row) * job.out_features + col;
         if (aligned) z[k] = *reinterpret_cast<const float4*>(src);
         else z[k] = make_float4(src[0], src[1], src[2], src[3]);
@@ -213,8 +213,8 @@ __device__ __forceinline__ float2 add2(float x0, float x1, float y0, float y1) {
 // block, 1500 ns, and a launch of one round of tiles took longer than without the pairs (400 tokens to 9216 columns 21.2
 // us before the pairs, 24.6 with them, 16.7 now; 64 -> 2560 features of 4096 tokens 27.5, 37.4 and 15.5).
 template <bool kFp32, bool kResidual>
-__device__ __forceinline__ void store_rows(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4& bias, const float4 (&z)[8],
-                                           int row0, int col0, unsigned char* stage, int width) {
+__device__ __forceinline__ void store_rows(const LinJob& job, const uint32_t (&v)[32], const float4& bias, const float4 (&z)[8],
+                                           int row0, int row_end, int col0, unsigned char* stage, int width) {
     const int lane = threadIdx.x & 31;
     #pragma unroll
     for (int c = 0; c < 8; ++c) {
@@ -228,7 +228,7 @@ __device__ __forceinline__ void store_rows(const LinArgs& args, const LinJob& jo
     const size_t at = size_t(row0 + r0) * job.out_features + col0 + chunk * 4;
     unsigned char* dst = static_cast<unsigned char*>(job.y) + at * (kFp32 ? 4 : 2);
     const size_t step = size_t(job.out_features) * (kFp32 ? 16 : 8);
-    const int rows = chunk * 4 < width && col0 + chunk * 4 < job.out_features ? args.tokens - row0 - r0 : 0;      // k * 4 of them
+    const int rows = chunk * 4 < width && col0 + chunk * 4 < job.out_features ? row_end - row0 - r0 : 0;      // k * 4 of them
     #pragma unroll
     for (int k = 0; k < 8; ++k) {
         float2 lo = add2(x[k].x, x[k].y, bias.x, bias.y), hi = add2(x[k].z, x[k].w, bias.z, bias.w);
@@ -248,13 +248,14 @@ __device__ __forceinline__ void store_rows(const LinArgs& args, const LinJob& jo
     }
     __syncwarp();
 }
+// (Rows up to row_end.)
 __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& job, const uint32_t (&v)[32], const float4& bias, const float4 (&z)[8], int row0,
-                                            int col0, unsigned char* stage, int width = 32) {
-    if (col0 >= job.out_features || row0 >= args.tokens) return;          // warp-uniform, as the next
+                                            int row_end, int col0, unsigned char* stage, int width = 32) {
+    if (col0 >= job.out_features || row0 >= row_end) return;              // warp-uniform, as the next
     if ((job.out_features & 3) == 0) {
-        if (args.y_dtype != HC_F32) store_rows<false, false>(args, job, v, bias, z, row0, col0, stage, width);
-        else if (job.residual != nullptr) store_rows<true, true>(args, job, v, bias, z, row0, col0, stage, width);
-        else store_rows<true, false>(args, job, v, bias, z, row0, col0, stage, width);
+        if (args.y_dtype != HC_F32) store_rows<false, false>(job, v, bias, z, row0, row_end, col0, stage, width);
+        else if (job.residual != nullptr) store_rows<true, true>(job, v, bias, z, row0, row_end, col0, stage, width);
+        else store_rows<true, false>(job, v, bias, z, row0, row_end, col0, stage, width);
         return;
     }
     const int lane = threadIdx.x & 31;
@@ -267,7 +268,7 @@ __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& j
     #pragma unroll 1
     for (int k = 0; k < 8; ++k) {
         const int r = k * 4 + (lane >> 3);
-        if (row0 + r >= args.tokens || chunk * 4 >= width) continue;
+        if (row0 + r >= row_end || chunk * 4 >= width) continue;
         const float4 x = *reinterpret_cast<const float4*>(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
         const float y[4] = {__fadd_rn(x.x, bias.x), __fadd_rn(x.y, bias.y), __fadd_rn(x.z, bias.z), __fadd_rn(x.w, bias.w)};
         const size_t at = size_t(row0 + r) * job.out_features + col;
@@ -285,7 +286,10 @@ __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, 
                  ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1) : "memory");
 }
 
-template <int BN, int SUBS>
+// ROWS: of the MMA, 128 or 64.  An MMA of so few columns takes as long as its operands take out of shared memory, 32 clocks for
+// 128 rows of x and BN / 4 for the weights, and the chain of K steps is what a launch of one token lasts (256 MMAs at o_proj): up to
+// 64 tokens go as 64 rows.  Their accumulators lie in the first 16 lanes of each warp's quarter of tensor memory.
+template <int BN, int SUBS, int ROWS>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w0,
                   const __grid_constant__ CUtensorMap tmap_w1, const __grid_constant__ CUtensorMap tmap_w2,
@@ -358,7 +362,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         }
     } else if (warp == 1) {
         // ===== MMA issuer (the warp walks the loop converged; one elected lane issues) =====
-        constexpr uint32_t idesc = instr_desc(BN, false);
+        constexpr uint32_t idesc = (instr_desc(BN, false) & ~(0x1fu << 24)) | (uint32_t(ROWS >> 4) << 24);
         const uint64_t a_desc0 = smem_desc(smem_u32(a_smem), 16);
         const uint64_t w_desc0 = smem_desc(smem_u32(w_smem), 16);
         int slot = 0;
@@ -398,7 +402,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             }
         }
     } else if (warp >= 4) {
-        // ===== epilogue: thread = token =====
+        // ===== epilogue: thread = token (of 64 rows: every other 16 threads) =====
         const int quad = warp & 3;
         unsigned char* stage = reinterpret_cast<unsigned char*>(bars + 1) + quad * kLinStageBytes;
         const uint32_t lane_base = uint32_t(quad * 32) << 16;
@@ -407,9 +411,11 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
             const LinTile where = decode_tile(args, tile);
             const LinJob& job = args.job[where.job];
             const int acc = int(count & 1);
-            const bool rows = quad * 32 < args.tokens;              // warp-uniform
+            constexpr int kQuadRows = ROWS / 4;
+            const int row0 = quad * kQuadRows, row_end = min(args.tokens, row0 + kQuadRows);
+            const bool rows = row0 < row_end;                       // warp-uniform
             float4 z[8];
-            if (rows) load_residual(args, job, quad * 32, where.tn * BN, z);
+            if (rows) load_residual(job, row0, row_end, where.tn * BN, z);
             const uint4 bias = load_bias(job, where.tn * BN);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
@@ -418,8 +424,8 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 uint32_t v[32];
                 HC_TMEM_LD32(tmem + lane_base + acc * 64 + col, v);
                 tc_wait_ld();
-                if (col > 0) load_residual(args, job, quad * 32, where.tn * BN + col, z);
-                store_block(args, job, v, block_bias(bias, col >> 5), z, quad * 32, where.tn * BN + col, stage, BN - col);
+                if (col > 0) load_residual(job, row0, row_end, where.tn * BN + col, z);
+                store_block(args, job, v, block_bias(bias, col >> 5), z, row0, row_end, where.tn * BN + col, stage, BN - col);
                 __syncwarp();          // the next tcgen05.ld is warp-wide
             }
             tc_fence_before();
@@ -555,7 +561,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             const int row0 = where.tm * (2 * kLinM) + rank * kLinM + quad * 32;
             const int acc = int(count & 1);
             float4 z[8], z_next[8];
-            load_residual(args, job, row0, where.col, z);
+            load_residual(job, row0, args.tokens, where.col, z);
             const uint4 bias = load_bias(job, where.col);
             if (!mbar_wait(&bars->acc_full[acc], (count >> 1) & 1, abort_flag, args.status, 24)) break;
             tc_fence_after();
@@ -563,9 +569,9 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             for (int chunk = 0; chunk < where.width / 32; ++chunk) {
                 uint32_t v[32];
                 HC_TMEM_LD32(tmem + lane_base + acc * BN + chunk * 32, v);
-                if (chunk + 1 < where.width / 32) load_residual(args, job, row0, where.col + (chunk + 1) * 32, z_next);
+                if (chunk + 1 < where.width / 32) load_residual(job, row0, args.tokens, where.col + (chunk + 1) * 32, z_next);
                 tc_wait_ld();
-                store_block(args, job, v, block_bias(bias, chunk), z, row0, where.col + chunk * 32, stage);
+                store_block(args, job, v, block_bias(bias, chunk), z, row0, args.tokens, where.col + chunk * 32, stage);
                 if (job.residual != nullptr) {
                     #pragma unroll
                     for (int k = 0; k < 8; ++k) z[k] = z_next[k];
@@ -664,7 +670,7 @@ static hc_status launch_linear_kernel(hc_context* ctx, Kernel kernel, bool (&con
     return check_cuda(launched, "linear kernel launch");
 }
 
-template <int BN>
+template <int BN, int ROWS>
 static hc_status launch_few(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features, cudaStream_t stream) {
     LinMaps maps;
     // A box that reaches past the last token is filled with zeros, and that fill measured slower than
@@ -685,8 +691,8 @@ static hc_status launch_few(hc_context* ctx, const void* x, const void* const* w
     const int grid = std::max(1, std::min(args.n_tiles, std::max(ctx->sm_count, 1)));
     constexpr int smem = 1024 + kFewSmemBytes + int(sizeof(LinBarriers)) + 4 * kLinStageBytes;
     static_assert(smem <= 227 * 1024, "shared memory of one CTA");
-    return subs == 4 ? launch_linear_kernel(ctx, linear_few_kernel<BN, 4>, configured4, grid, smem, maps, args, stream)
-                     : launch_linear_kernel(ctx, linear_few_kernel<BN, 2>, configured2, grid, smem, maps, args, stream);
+    return subs == 4 ? launch_linear_kernel(ctx, linear_few_kernel<BN, 4, ROWS>, configured4, grid, smem, maps, args, stream)
+                     : launch_linear_kernel(ctx, linear_few_kernel<BN, 2, ROWS>, configured2, grid, smem, maps, args, stream);
 }
 
 template <int BN>
@@ -728,10 +734,18 @@ hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* cons
             for (int j = 0; j < n_jobs; ++j) n += (out_features[j] + bn - 1) / bn;
             return n;
         };
-        if (tiles(16) <= sms) return launch_few<16>(ctx, x, w, args, in_features, stream);
-        if (tiles(32) <= sms) return launch_few<32>(ctx, x, w, args, in_features, stream);
-        if (tiles(48) <= sms) return launch_few<48>(ctx, x, w, args, in_features, stream);
-        return launch_few<64>(ctx, x, w, args, in_features, stream);
+        if (tokens <= 64) {                                  // (64 rows take columns in eights)
+            if (tiles(16) <= sms) return launch_few<16, 64>(ctx, x, w, args, in_features, stream);
+            if (tiles(24) <= sms) return launch_few<24, 64>(ctx, x, w, args, in_features, stream);
+            if (tiles(32) <= sms) return launch_few<32, 64>(ctx, x, w, args, in_features, stream);
+            if (tiles(40) <= sms) return launch_few<40, 64>(ctx, x, w, args, in_features, stream);
+            if (tiles(48) <= sms) return launch_few<48, 64>(ctx, x, w, args, in_features, stream);
+            return launch_few<64, 64>(ctx, x, w, args, in_features, stream);
+        }
+        if (tiles(16) <= sms) return launch_few<16, 128>(ctx, x, w, args, in_features, stream);
+        if (tiles(32) <= sms) return launch_few<32, 128>(ctx, x, w, args, in_features, stream);
+        if (tiles(48) <= sms) return launch_few<48, 128>(ctx, x, w, args, in_features, stream);
+        return launch_few<64, 128>(ctx, x, w, args, in_features, stream);
     }
     // The column tile whose rounds of pairs take least.  A K step costs an SM the larger of its MMAs (2 clocks a column)
     // and of (128 + BN / 2) x 128 bytes out of L2, of which about 60 arrive per clock and SM with all of them

@@ -133,3 +133,39 @@ def test_linear_tiles_of_two_widths(tokens, width, outs):
     for got, weight in zip(y, w):
         assert float((got.double() - x.double() @ weight.double().T).abs().max()) < 4e-4
     ctx.close()
+
+
+@pytest.mark.parametrize("outs", [(2000,), (2880,), (4600,), (4096, 512, 512), (6000,), (9600,), (41, 2, 130)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_linear_of_few_tokens_at_the_edges_of_its_row_tiles(outs, residual):
+    """64 and 128 rows an MMA and every width of column tile: the bits of the same rows in a call of 140 tokens, which
+    the other kernel computes, and the fp32 sums of 192 products of float64's (192 roundings of 2^-24 of sums below 60)."""
+    import torch
+    import hydra_b200 as hb
+    ctx = hb.Context(0)
+    backend = hb.AttentionBackend(ctx)
+    gen = torch.Generator(device="cuda").manual_seed(sum(outs))
+    x = torch.randn(140, 192, device="cuda", generator=gen).to(torch.bfloat16)
+    w = [torch.randn(n, 192, device="cuda", generator=gen).to(torch.bfloat16) for n in outs]
+    b = [torch.randn(n, device="cuda", generator=gen).to(torch.bfloat16) for n in outs]
+    res = [torch.randn(140, n, device="cuda", generator=gen) for n in outs]
+
+    def call(tokens):
+        y = [torch.full((tokens + 1, n), 7.0, device="cuda") for n in outs]
+        if residual:
+            for weight, bias, r, out in zip(w, b, res, y):
+                backend.linear(x, weight, bias, out, tokens, 192, weight.shape[0], residual=r)
+        else:
+            backend.linear_group(x, w, b, y, tokens, 192, y_dtype=hb.capi.HC_F32)
+        ctx.check()
+        assert all(bool((out[tokens] == 7.0).all()) for out in y)
+        return [out[:tokens] for out in y]
+
+    whole = call(140)
+    for got, weight, bias, r in zip(whole, w, b, res):
+        want = x.double() @ weight.double().T + bias.double() + (r.double() if residual else 0.0)
+        assert float((got.double() - want).abs().max()) < 1e-3
+    for tokens in (1, 8, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 96, 127, 128, 129):
+        for got, want in zip(call(tokens), whole):
+            assert torch.equal(got, want[:tokens])
+    ctx.close()
