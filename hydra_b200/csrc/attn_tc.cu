@@ -966,6 +966,20 @@ hc_status tc_encode_2d(void* map, const void* base, uint64_t rows, uint64_t cols
     return HC_OK;
 }
 
+hc_status tc_encode_blocks(void* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks) {
+    EncodeTiledFn encode = encode_tiled();
+    if (!encode) return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from this driver");
+    const cuuint64_t dims[3] = {64, cuuint64_t(rows), cuuint64_t(cols / 64)};
+    const cuuint64_t strides[2] = {cuuint64_t(cols) * 2, 128};
+    const cuuint32_t box[3] = {64, cuuint32_t(box_rows), cuuint32_t(box_blocks)};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    const CUresult rc = encode(static_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+                               strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled failed with code " + std::to_string(int(rc)));
+    return HC_OK;
+}
+
 hc_status tc_encode_3d(void* map, const void* base, uint64_t cols, uint64_t rows, uint64_t planes, uint32_t box_rows, uint32_t box_planes) {
     EncodeTiledFn encode = encode_tiled();
     if (!encode) return fail(HC_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from this driver");

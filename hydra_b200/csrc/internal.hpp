@@ -211,6 +211,8 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
 // The rows of positions [first, end) of `from_seq` in `from`, keys and values, into sequence 0 of `to`.
 hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq, const CacheView& to, int first, int end, int d,
                            cudaStream_t stream);
+// `count` floats, a multiple of 4 on 16-byte boundaries, one side possibly in pinned host memory.
+hc_status launch_copy_floats(hc_context* ctx, float* dst, const float* src, size_t count, cudaStream_t stream);
 hc_status launch_rms_norm_rows(hc_context* ctx, const void* x, const uint16_t* scale, void* out, int tokens, int width,
                                float eps, int x_dtype, int out_dtype, cudaStream_t stream);
 hc_status launch_split_query_gate(hc_context* ctx, const void* combined, void* query, void* gate,
@@ -256,6 +258,8 @@ hc_status static_scratch_prepare(int device, float** address);
 // A tensor map (CUtensorMap behind `map`) over a row-major bf16 matrix: boxes of 64 columns x box_rows
 // rows, 128-byte swizzle, zeros beyond the edges.
 hc_status tc_encode_2d(void* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
+// The same with the 64-column blocks as a third dimension: boxes of box_blocks of them, [block][row][64 columns] in shared memory.
+hc_status tc_encode_blocks(void* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_blocks);
 // The same over [planes][rows][cols]: boxes of 64 columns x box_rows x box_planes.
 hc_status tc_encode_3d(void* map, const void* base, uint64_t cols, uint64_t rows, uint64_t planes, uint32_t box_rows, uint32_t box_planes);
 bool tc_supported(const AttnShape& shape);

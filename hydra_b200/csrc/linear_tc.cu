@@ -154,13 +154,6 @@ __device__ __forceinline__ LinTile decode_tile(const LinArgs& args, int tile) {
     return t;
 }
 
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-        : "memory");
-}
-
 // 32 accumulator columns of a warp's 32 rows (lane = row in `v`): + bias (+ residual), to y.  The block goes through
 // 4 KB of shared memory so that a store instruction writes four rows' whole 128-byte lines (64 for bf16)
 // instead of 16 bytes of 32 rows, and the residual is read the same way, a block ahead: it may be y itself, so the
@@ -281,9 +274,9 @@ __device__ __forceinline__ void store_block(const LinArgs& args, const LinJob& j
     __syncwarp();
 }
 
-__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int c0, int c1) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1) : "memory");
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
 
 // ROWS: of the MMA, 128 or 64.  An MMA of so few columns takes as long as its operands take out of shared memory, 32 clocks for
@@ -325,7 +318,7 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
         // While the kernel before this one finishes, the weights come into L2 (where it may still change them: nothing
         // is read into this CTA before the wait below).
         const LinTile where = decode_tile(args, blockIdx.x);
-        for (int k = lane; k < k_steps; k += 32) tma_prefetch_2d(weight_map(where.job), k * kLinK, where.tn * BN);
+        for (int k = lane * SUBS; k < k_steps; k += 32 * SUBS) tma_prefetch_3d(weight_map(where.job), 0, where.tn * BN, k);
     }
     if (warp == 0 && lane == 0) prefetch_tensormap(&tmap_x);
     tc_fence_before();
@@ -344,15 +337,12 @@ linear_few_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_const
                 const LinTile where = decode_tile(args, tile);
                 const CUtensorMap* tmap_w = weight_map(where.job);
                 for (int k = 0; k < k_steps; k += SUBS) {
-                    const int count = min(SUBS, k_steps - k);
                     if (round > 0 && !mbar_wait(&bars->empty[slot], (round - 1) & 1, abort_flag, args.status, 21)) { ok = false; break; }
-                    mbar_expect_tx(&bars->full[slot], uint32_t(count * (args.a_bytes + kWBytes)));
-                    for (int u = 0; u < count; ++u) {
-                        tma_load_2d(w_smem + slot * w_stage + u * kWBytes, tmap_w, &bars->full[slot], (k + u) * kLinK, where.tn * BN);
-                    }
-                    for (int u = 0; u < count; ++u) {
-                        tma_load_2d(a_smem + slot * a_stage + u * args.a_bytes, &tmap_x, &bars->full[slot], (k + u) * kLinK, 0);
-                    }
+                    // A stage's K steps in one copy each: the maps have them as a third dimension (zeros behind the last, which
+                    // count).  Step by step a launch of one token was 128 copies from one thread.
+                    mbar_expect_tx(&bars->full[slot], uint32_t(w_stage + a_stage));
+                    tma_load_3d(w_smem + slot * w_stage, tmap_w, &bars->full[slot], 0, where.tn * BN, k);
+                    tma_load_3d(a_smem + slot * a_stage, &tmap_x, &bars->full[slot], 0, 0, k);
                     if (++slot == args.stages) {
                         slot = 0;
                         ++round;
@@ -601,11 +591,12 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 // Encoding a tensor map costs a few microseconds of host time, as much as a decode-sized call's
 // kernel; weights and activation buffers recur from call to call, so the last maps are kept, keyed
 // by what determines them.  One caller thread per context: the cache is per thread.
-static hc_status cached_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+// k_blocks: 0, boxes of one K step; or so many of them in a box.
+static hc_status cached_map(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t k_blocks) {
     struct Entry {
         const void* base;
         uint64_t rows, cols;
-        uint32_t box_rows;
+        uint32_t box_rows, k_blocks;
         CUtensorMap map;
     };
     constexpr int kEntries = 32;
@@ -613,13 +604,13 @@ static hc_status cached_map(CUtensorMap* out, const void* base, uint64_t rows, u
     static thread_local int used = 0, next = 0;
     for (int i = 0; i < used; ++i) {
         const Entry& e = entries[i];
-        if (e.base == base && e.rows == rows && e.cols == cols && e.box_rows == box_rows) {
+        if (e.base == base && e.rows == rows && e.cols == cols && e.box_rows == box_rows && e.k_blocks == k_blocks) {
             *out = e.map;
             return HC_OK;
         }
     }
     Entry& e = entries[next];
-    const hc_status st = tc_encode_2d(&e.map, base, rows, cols, box_rows);
+    const hc_status st = k_blocks == 0 ? tc_encode_2d(&e.map, base, rows, cols, box_rows) : tc_encode_blocks(&e.map, base, rows, cols, box_rows, k_blocks);
     if (st != HC_OK) {
         e.base = nullptr;
         return st;
@@ -628,6 +619,7 @@ static hc_status cached_map(CUtensorMap* out, const void* base, uint64_t rows, u
     e.rows = rows;
     e.cols = cols;
     e.box_rows = box_rows;
+    e.k_blocks = k_blocks;
     *out = e.map;
     next = (next + 1) % kEntries;
     used = std::min(used + 1, kEntries);
@@ -635,18 +627,18 @@ static hc_status cached_map(CUtensorMap* out, const void* base, uint64_t rows, u
 }
 
 // Tensor maps and the tile list of a launch with column tiles of `bn` and row tiles of `bm` over boxes of x_rows and
-// w_rows rows.
+// w_rows rows (and k_blocks K steps).
 struct LinMaps {
     CUtensorMap x, w[kLinJobs];
 };
 static hc_status prepare_linear(LinMaps& maps, const void* x, const void* const* w, LinArgs& args, int in_features, int bm, int bn,
-                                int x_rows, int w_rows) {
-    hc_status st = cached_map(&maps.x, x, uint64_t(args.tokens), uint64_t(in_features), uint32_t(x_rows));
+                                int x_rows, int w_rows, int k_blocks) {
+    hc_status st = cached_map(&maps.x, x, uint64_t(args.tokens), uint64_t(in_features), uint32_t(x_rows), uint32_t(k_blocks));
     args.tiles_m = (args.tokens + bm - 1) / bm;
     int tiles = 0;
     for (int j = 0; j < kLinJobs && st == HC_OK; ++j) {
         const int source = j < args.n_jobs ? j : 0;            // unused maps repeat the first
-        st = cached_map(&maps.w[j], w[source], uint64_t(args.job[source].out_features), uint64_t(in_features), uint32_t(w_rows));
+        st = cached_map(&maps.w[j], w[source], uint64_t(args.job[source].out_features), uint64_t(in_features), uint32_t(w_rows), uint32_t(k_blocks));
         if (j < args.n_jobs) {
             args.job[j].first_tile = tiles;
             tiles += args.tiles_m * ((args.job[j].out_features + bn - 1) / bn);
@@ -685,7 +677,7 @@ static hc_status launch_few(hc_context* ctx, const void* x, const void* const* w
     const int room = kFewSmemBytes - kLinABytes;
     const int subs = 16 * step_bytes <= room ? 4 : 2;
     args.stages = std::max(1, std::min(kFewMaxStages, room / (subs * step_bytes)));
-    const hc_status st = prepare_linear(maps, x, w, args, in_features, kLinM, BN, x_rows, BN);
+    const hc_status st = prepare_linear(maps, x, w, args, in_features, kLinM, BN, x_rows, BN, subs);
     if (st != HC_OK) return st;
     static bool configured4[64] = {}, configured2[64] = {};
     const int grid = std::max(1, std::min(args.n_tiles, std::max(ctx->sm_count, 1)));
@@ -699,7 +691,7 @@ template <int BN>
 static hc_status launch_pair(hc_context* ctx, const void* x, const void* const* w, LinArgs args, int in_features, cudaStream_t stream,
                              int n_wide = 0, int n_tiles = 0) {
     LinMaps maps;
-    const hc_status st = prepare_linear(maps, x, w, args, in_features, 2 * kLinM, BN, kLinM, BN == 256 ? BN / 4 : BN / 2);
+    const hc_status st = prepare_linear(maps, x, w, args, in_features, 2 * kLinM, BN, kLinM, BN == 256 ? BN / 4 : BN / 2, 0);
     if (st != HC_OK) return st;
     if (BN == 256) {
         args.n_wide = n_wide;
