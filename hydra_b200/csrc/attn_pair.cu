@@ -37,6 +37,7 @@ constexpr int kPairThreads = 640;                    // five warpgroups
 constexpr int kPairRows = 2 * kRows;                 // query rows of a pair
 constexpr int kPairO = 256;                          // O columns of an item
 constexpr int kPairOCol = 2 * kTileKeys;             // their place in tensor memory
+constexpr int kPairPCol = 32;                        // P of keys 32 .. 63 (of 64) begins in the columns of their S
 constexpr int kPairStageBytes = 16 * 1024;           // K: 64 keys x 128 of head_dim; V: 128 keys x 64 columns; per CTA
 constexpr int kPairBoxBytes = 64 * 128;              // a box of 64 rows x 64 elements
 constexpr int kPairStoreBytes = 32 * 64;
@@ -300,7 +301,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                     if (elect_one()) {
                         #pragma unroll
                         for (int ks = 0; ks < kTileKeys / 16; ++ks) {
-                            mma_ts_pair(d_tmem, a_tmem + (ks & 3) * 8 + (ks >> 2) * 64, v_desc + uint64_t((ks * 2048) >> 4), idesc_pv,
+                            mma_ts_pair(d_tmem, a_tmem + (ks & 1) * 8 + ((ks >> 1) & 1) * kPairPCol + (ks >> 2) * 64, v_desc + uint64_t((ks * 2048) >> 4), idesc_pv,
                                         ks != 0 ? 1u : 0u);
                         }
                         tc_commit_pair(&bars->empty[slot]);
@@ -382,14 +383,7 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                             if (((visible >> i) & 1u) == 0) s[i] = __float_as_uint(neg_inf);
                         }
                     };
-                    // Pass 1: the row maximum (exact under any association).
-                    float m = neg_inf;
-                    #pragma unroll 1
-                    for (int g = 0; g < 2; ++g) {
-                        uint32_t s[32];
-                        HC_TMEM_LD32(s_tmem + g * 32, s);
-                        tc_wait_ld();
-                        if (!full) mask(s, g * 32);
+                    auto maximum = [&](const uint32_t (&s)[32]) -> float {
                         float mx[4];
                         #pragma unroll
                         for (int u = 0; u < 4; ++u) {
@@ -398,45 +392,67 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                             mx[u] = fmax3(mx[u], __uint_as_float(s[u + 20]), __uint_as_float(s[u + 24]));
                             mx[u] = fmaxf(mx[u], __uint_as_float(s[u + 28]));
                         }
-                        m = fmax3(m, fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
-                    }
+                        return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+                    };
+                    auto weights = [&](uint32_t (&s)[32], uint32_t (&packed)[16], float neg_mc) {
+                        #pragma unroll
+                        for (int i = 0; i < 16; ++i) fma2_inplace(s[2 * i], s[2 * i + 1], args.c, neg_mc);
+                        #pragma unroll
+                        for (int i = 0; i < 16; ++i) packed[i] = pack_bf16x2(ex2(__uint_as_float(s[2 * i])), ex2(__uint_as_float(s[2 * i + 1])));
+                    };
+                    // The row sum has a fixed shape: groups of 32 columns by the butterfly tree (i with i + 16, then + 8,
+                    // + 4, + 2, + 1; two columns an addition), the four groups in order (the last two are added by the fold).
+                    auto sum = [&](const uint32_t (&packed)[16]) -> float {
+                        uint64_t a[2];
+                        #pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            auto level = [&](int n) -> uint64_t { return add2(unpack_pair(packed[n]), unpack_pair(packed[n + 8])); };
+                            a[i] = add2(add2(level(i), level(i + 4)), add2(level(i + 2), level(i + 6)));
+                        }
+                        a[0] = add2(a[0], a[1]);
+                        return __fadd_rn(__uint_as_float(uint32_t(a[0])), __uint_as_float(uint32_t(a[0] >> 32)));
+                    };
+                    // A tile's time here is what one of prompts too short for the power limit takes (777 gated tokens behind 1291 59 us, now 55), so
+                    // as little as may be stands in a row: the second 32 columns stay in the registers between the
+                    // passes, the first ones come back behind the sums of the others, and their own sum follows P.
+                    uint32_t s[32], packed[16];
+                    HC_TMEM_LD32(s_tmem, s);
+                    tc_wait_ld();
+                    if (!full) mask(s, 0);
+                    float m = maximum(s);
+                    HC_TMEM_LD32(s_tmem + 32, s);
+                    tc_wait_ld();
+                    if (!full) mask(s, 32);
+                    m = fmaxf(m, maximum(s));
                     bars->red[sb][cols][row] = m;
                     named_barrier(1 + quad, 64);
                     m = fmaxf(m, bars->red[sb][cols ^ 1][row]);
                     const float neg_mc = -__fmul_rn((m == neg_inf) ? 0.0f : m, args.c);
-                    // Pass 2: weights; P overwrites the S columns already consumed.  The row sum has a
-                    // fixed shape: groups of 32 columns by the butterfly tree (i with i + 16, then + 8, + 4, + 2,
-                    // + 1; two columns an addition), the four groups in order (the last two are added by the fold).
-                    #pragma unroll 1
-                    for (int g = 0; g < 2; ++g) {
-                        uint32_t s[32];
-                        HC_TMEM_LD32(s_tmem + g * 32, s);
-                        tc_wait_ld();
-                        if (!full) mask(s, g * 32);
-                        #pragma unroll
-                        for (int i = 0; i < 16; ++i) fma2_inplace(s[2 * i], s[2 * i + 1], args.c, neg_mc);
-                        uint32_t packed[16];
-                        #pragma unroll
-                        for (int i = 0; i < 16; ++i) packed[i] = pack_bf16x2(ex2(__uint_as_float(s[2 * i])), ex2(__uint_as_float(s[2 * i + 1])));
-                        HC_TMEM_ST16(s_tmem + g * 16, packed);
-                        uint64_t a[8];
-                        #pragma unroll
-                        for (int i = 0; i < 8; ++i) a[i] = add2(unpack_pair(packed[i]), unpack_pair(packed[i + 8]));
-                        #pragma unroll
-                        for (int i = 0; i < 4; ++i) a[i] = add2(a[i], a[i + 4]);
-                        a[0] = add2(add2(a[0], a[2]), add2(a[1], a[3]));
-                        float group = __fadd_rn(__uint_as_float(uint32_t(a[0])), __uint_as_float(uint32_t(a[0] >> 32)));
-                        if (cols == 0 && g == 1) group = __fadd_rn(bars->l[t & 3][0][row], group);
-                        bars->l[t & 3][cols == 0 ? 0 : 1 + g][row] = group;
-                    }
-                    if (cols == 0) bars->mm[t & 3][row] = __fmul_rn(m, args.c);
+                    weights(s, packed, neg_mc);
+                    HC_TMEM_ST16(s_tmem + kPairPCol, packed);            // P in place of S columns already consumed
+                    HC_TMEM_LD32(s_tmem, s);
+                    const float sum1 = sum(packed);
+                    tc_wait_ld();
+                    if (!full) mask(s, 0);
+                    weights(s, packed, neg_mc);
+                    HC_TMEM_ST16(s_tmem, packed);
                     tc_wait_st();
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&bars->m_full[t & 3]);       // the maxima and sums, to this CTA's fold
-                    mbar_arrive_cluster_relaxed(p_full[sb]); // (P itself is ordered by the fences around tensor memory)
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster_relaxed(p_full[sb]);  // (P itself is ordered by the fences around tensor memory)
+                    const float sum0 = sum(packed);
+                    if (cols == 0) {
+                        bars->mm[t & 3][row] = __fmul_rn(m, args.c);
+                        bars->l[t & 3][0][row] = __fadd_rn(sum0, sum1);
+                    } else {
+                        bars->l[t & 3][1][row] = sum0;
+                        bars->l[t & 3][2][row] = sum1;
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->m_full[t & 3]);        // the maxima and sums, to this CTA's fold
+                } else if (lane == 0) {
+                    mbar_arrive_cluster_relaxed(p_full[sb]);
+                    mbar_arrive(&bars->m_full[t & 3]);
                 }
             }
         }
