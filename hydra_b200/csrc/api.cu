@@ -1451,6 +1451,19 @@ size_t hc_attention_stack_bytes(const hc_block_weights* layers, int n_layers, in
     return stack_space(layers, n_layers, tokens, width).bytes;
 }
 
+// A few hidden states to or from pinned host memory, which a kernel reads and writes where it is: a copy engine's turn
+// between two kernels costs more than the bytes.  Larger copies are the engines'.
+constexpr size_t kHostDirect = size_t(64) << 10;
+static bool host_direct(const void* p, size_t bytes) {
+    if (bytes > kHostDirect || (reinterpret_cast<uintptr_t>(p) & 15) != 0) return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeHost && at.devicePointer == p;
+}
+
 hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_block_weights* layers, int n_layers, int seq,
                                   const float* hidden_in, float* hidden_out, int tokens, int width, int first_position, float eps,
                                   void* workspace, void* stream) {
@@ -1481,7 +1494,8 @@ hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_
     unsigned char* base = static_cast<unsigned char*>(workspace);
     float* hidden = reinterpret_cast<float*>(base);
     const size_t bytes = size_t(tokens) * width * sizeof(float);
-    hc_status st = check_cuda(cudaMemcpyAsync(hidden, hidden_in, bytes, cudaMemcpyHostToDevice, s), "hidden states in");
+    hc_status st = host_direct(hidden_in, bytes) ? launch_copy_floats(ctx, hidden, hidden_in, bytes / sizeof(float), s)
+                                                 : check_cuda(cudaMemcpyAsync(hidden, hidden_in, bytes, cudaMemcpyHostToDevice, s), "hidden states in");
     for (int i = 0; i < n_layers && st == HC_OK; ++i) {
         const hc_block_weights& w = layers[i];
         const hc_attn_params& p = w.params;
@@ -1495,7 +1509,10 @@ hc_status hc_attention_stack_host(hc_context* ctx, hc_kv_cache* cache, const hc_
         if (st == HC_OK) st = hc_layer_step(ctx, cache, i, seq, qkv[0], qkv[1], qkv[2], base + space.attended, tokens, first_position, &p, stream);
         if (st == HC_OK) st = hc_linear(ctx, base + space.attended, w.wo, w.bo, hidden, hidden, tokens, o_width, width, HC_F32, stream);
     }
-    if (st == HC_OK) st = check_cuda(cudaMemcpyAsync(hidden_out, hidden, bytes, cudaMemcpyDeviceToHost, s), "hidden states out");
+    if (st == HC_OK) {
+        st = host_direct(hidden_out, bytes) ? launch_copy_floats(ctx, hidden_out, hidden, bytes / sizeof(float), s)
+                                            : check_cuda(cudaMemcpyAsync(hidden_out, hidden, bytes, cudaMemcpyDeviceToHost, s), "hidden states out");
+    }
     if (st == HC_OK) return hc_context_check(ctx, stream);
     // (Pages that ran out, or a launch that failed.)  The caller has its buffers back: nothing of the call is still on its way.
     const std::string message = g_last_error;

@@ -369,6 +369,14 @@ copy_rows_kernel(const CacheView from, int from_seq, const CacheView to, int fir
     }
 }
 
+// A multiple of four floats, either side in pinned host memory.
+__global__ void __launch_bounds__(256) copy_floats_kernel(float4* dst, const float4* src, int count) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < count) dst[i] = src[i];
+}
+
 // RMSNorm of whole rows (the layer's input norm): out = x * rsqrt(mean(x^2) + eps) * scale.  One block
 // per token; replaces rms_norm and rms_norm_batch (Sources/HydraMetal/Shaders/attention.metal:9-43,
 // batch.metal:184-218).  The output may be bf16, ready to be the A operand of hc_linear.
@@ -525,6 +533,13 @@ hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq,
     launch_pdl(copy_rows_kernel, grid, 256, 0, stream, from, from_seq, to, first, end, d / 8);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "copy_rows_kernel launch");
+}
+
+hc_status launch_copy_floats(hc_context* ctx, float* dst, const float* src, size_t count, cudaStream_t stream) {
+    const int vectors = int(count / 4);
+    launch_pdl(copy_floats_kernel, (vectors + 255) / 256, 256, 0, stream, reinterpret_cast<float4*>(dst), reinterpret_cast<const float4*>(src), vectors);
+    ctx->launches += 1;
+    return check_cuda(cudaGetLastError(), "copy_floats_kernel launch");
 }
 
 hc_status launch_rms_norm_rows(hc_context* ctx, const void* x, const uint16_t* scale, void* out, int tokens, int width,

@@ -74,3 +74,29 @@ def test_runner_prefill_forward_verify_and_rewind():
                      want[prompt:])
     runner.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("tokens", [1, 5, 6, 40])
+def test_hidden_states_in_pinned_and_in_pageable_memory(tokens):
+    """Up to 64 KB of pinned hidden states (five of 2880) are read and written where they are, the rest is copied."""
+    import torch
+    import hydra_b200 as hb
+    from hydra_b200.runner import AttentionLayerWeights, AttentionStackRunner
+    ctx = hb.Context(0)
+    rng = np.random.default_rng(tokens)
+    size, qh, kvh, d = 2880, 8, 2, 64
+    w = AttentionLayerWeights(
+        input_norm=np.ones(size), wq=rng.normal(0, 0.02, (qh * d, size)), bq=np.zeros(qh * d), wk=rng.normal(0, 0.02, (kvh * d, size)),
+        bk=np.zeros(kvh * d), wv=rng.normal(0, 0.02, (kvh * d, size)), bv=np.zeros(kvh * d), wo=rng.normal(0, 0.02, (size, qh * d)),
+        bo=np.zeros(size), sinks=np.zeros(qh), window=0, inv_freq=ho.inverse_frequencies(d, 10000.0, d // 2))
+    states = rng.standard_normal((2, tokens, size)).astype(np.float32)
+    got = []
+    for pinned in (True, False):
+        runner = AttentionStackRunner(ctx, [w], size, qh, kvh, d, context_length=256, prefill_chunk_tokens=64)
+        if not pinned:
+            runner._pinned = [torch.empty((64, size)) for _ in range(2)]
+            runner._host = [p.numpy() for p in runner._pinned]
+        got.append([runner.verify(x) for x in states])
+        runner.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
+    ctx.close()
