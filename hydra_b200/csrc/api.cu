@@ -110,6 +110,10 @@ bool needs_q_prepare(const hc_attn_params* p, const void* q, bool tensor) {
            p->gate_layout == HC_GATE_INTERLEAVED || (tensor && (reinterpret_cast<uintptr_t>(q) & 15) != 0);
 }
 
+// Whether a prompt of the ring layer L may attend in the prompt store.  Only calls that use the workspace anyhow, for their
+// prepared queries, do: those that do not may overlap with others on the cache.
+bool attends_beside(const hc_layer_store& L, const hc_attn_params* p) { return L.prompt && needs_q_prepare(p, nullptr, false); }
+
 // What aligning the five parts of a staging slot to 256 bytes may cost.
 constexpr size_t kStageSlack = 5 * 256;
 
@@ -283,7 +287,7 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
     st = check_shard_mode(cache, partial_mode);
     if (st != HC_OK) return st;
     const AttnShape shape = shape_of(cache, p, partial_mode);
-    const bool beside = L.prompt && k_fused && tokens > L.ring - L.desc.window;
+    const bool beside = k_fused && attends_beside(L, p) && tokens > L.ring - L.desc.window;
     const hc_layer_store& S = beside ? *L.prompt : L;
     const int store_seq = beside ? 0 : seq;
     const CacheView view = view_of(cache, S);
@@ -1383,7 +1387,7 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
     // kernels are told), so the library takes as many tokens at a time as it can: all of the keys are appended, then all
     // of the queries attend, in one launch each, whose row tiles fill the SMs evenly.  (Chunk by chunk, even with two
     // chunks in flight, every launch had its own ramp and ragged last wave.)  A ring takes what fits beside
-    // the window of its first token; a longer prompt attends beside it.
+    // the window of its first token; a longer prompt attends beside it (attends_beside).
     const hc_layer_store& L = cache->layers[size_t(layer)];
     if (L.ring > 0 && std::min(chunk, tokens) > L.ring_margin) {
         return check_positions(cache, L, first_position, std::min(chunk, tokens), params);
@@ -1393,7 +1397,7 @@ hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int 
     const int block_chunk = std::min(chunk, cache->prefill_chunk);
     int step = chunk;
     if (!params->block_ends || chunk % block_chunk == 0) {
-        int most = L.ring > 0 && !L.prompt ? L.ring - L.desc.window : tokens;
+        int most = L.ring > 0 && !attends_beside(L, params) ? L.ring - L.desc.window : tokens;
         most = std::max(std::min(most, cache->ws.qprep_capacity), std::min(chunk, tokens));
         const int parts = (tokens + most - 1) / most;
         step = std::min(most, ((tokens + parts - 1) / parts + kTileKeys - 1) / kTileKeys * kTileKeys);

@@ -233,3 +233,34 @@ def test_outputs_on_16_byte_boundaries_that_are_no_32_byte_ones(hb, ctx, d, qh, 
     assert np.array_equal(tl.to_host(flat[8:-8]).reshape(want.shape), want)
     assert bool((flat[:8] == 7).all()) and bool((flat[-8:] == 7).all())
     layer.close()
+
+
+@pytest.mark.parametrize("d", [64, 128, 256, 512])
+def test_fp32_rows_on_16_byte_boundaries_that_are_no_32_byte_ones(hb, ctx, d):
+    """The prologue reads and writes fp32 vectors 32 bytes a lane where they lie so: appended rows and vectors normalised in
+    place are the same bits where they do not."""
+    import torch
+    tokens, heads = 700, 5
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    x = torch.randn(2, tokens, heads, d, device="cuda", generator=gen)
+    weight = (1 + 0.1 * torch.randn(d, device="cuda", generator=gen)).to(torch.bfloat16)
+    inv = ho.inverse_frequencies(d, 10000.0, d // 2)
+    layer = tl.Layer(hb, ctx, heads, heads, d, 1024, rope_inv_freq=inv, io="f32")
+    got = []
+    for offset in (0, 4):
+        flat = torch.full((2, tokens * heads * d + 8), 7.0, device="cuda")
+        k, v = (flat[i, offset:offset + tokens * heads * d].view(tokens, heads, d) for i in range(2))
+        k.copy_(x[0])
+        v.copy_(x[1])
+        layer.backend.write_key_value(layer.cache, 0, k, v, tokens, 0, layer.params)
+        ctx.check()
+        rows = tl.read_cache(layer.cache, 0, tokens, heads, d)
+        layer.backend.rms_norm_heads(k, weight, tokens, heads, d, 1e-6)
+        ctx.check()
+        got.append([*rows, k.cpu().numpy()])
+        assert float(flat[0, :offset].sub(7).abs().sum()) == 0.0 and bool((flat[0, offset + tokens * heads * d:] == 7).all())
+    layer.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
+    want = x[0].double()
+    want = want / torch.sqrt((want * want).mean(-1, keepdim=True) + 1e-6) * weight.double()
+    assert np.max(np.abs(got[0][2] - want.cpu().numpy())) < 1e-5
