@@ -93,6 +93,11 @@ __device__ __forceinline__ void store_half(uint16_t* row, int h, int m, const fl
     }
 }
 
+__device__ __forceinline__ void store8(void* dst, const float (&v)[8]) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+
 // Thread blocks an SM holds.
 constexpr int prep_blocks(bool fp32) { return fp32 ? 2 : 3; }
 
@@ -155,6 +160,7 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
         }
     }
     RawHead<D, F32> now, ahead;
+    const bool by32 = (reinterpret_cast<uintptr_t>(src) & 31) == 0;      // (of all vectors or none)
     now.load(src, m);
     for (;;) {
         const bool more = token + step < unsigned(args.tokens);
@@ -177,6 +183,18 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
                 s[4 * u] = sv.x; s[4 * u + 1] = sv.y; s[4 * u + 2] = sv.z; s[4 * u + 3] = sv.w;
             }
         }
+        // Where to, while the loads are on their way.
+        uint16_t* to = dst;
+        bool active = in_range;
+        if (counted) {
+            to = dst + size_t(row) * D;
+            row += row_step;
+            if (map.ring > 0 && row >= map.ring) row -= map.ring;
+        } else if (cached) {
+            active = active && row_is_local(map, position);           // else another rank's tile
+            const int seq = args.batched ? args.meta.seq[token] : args.seq;
+            if (active) to = dst + (size_t(cache_plane(map, seq, args.cache.kv_heads, head)) * args.cache.capacity + cache_row(map, seq, position)) * D;
+        }
         float lo[8], hi[8];
         now.unpack(0, lo);
         now.unpack(1, hi);
@@ -196,7 +214,9 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
                 for (int p = 0; p < kParts; ++p) part[p] = __fadd_rn(part[p], __shfl_xor_sync(0xffffffffu, part[p], offset));
             }
             if (norm != 0) {
-                const float inverse = head_norm<D>(kParts == 2 ? __fadd_rn(part[0], part[1]) : part[0], args.eps);
+                // (Dividing by a power of two and multiplying by its inverse round alike.)
+                const float mean = __fmul_rn(kParts == 2 ? __fadd_rn(part[0], part[1]) : part[0], 1.0f / float(D));
+                const float inverse = __frsqrt_rn(__fadd_rn(mean, args.eps));
                 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     lo[i] = __fmul_rn(lo[i], inverse);
@@ -219,23 +239,17 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
                 hi[i] = __fmaf_rn(b, c[i], __fmul_rn(a, s[i]));
             }
         }
-        uint16_t* to = dst;
-        bool active = in_range;
-        if (counted) {
-            to = dst + size_t(row) * D;
-            row += row_step;
-            if (map.ring > 0 && row >= map.ring) row -= map.ring;
-        } else if (cached) {
-            active = active && row_is_local(map, position);           // else another rank's tile
-            const int seq = args.batched ? args.meta.seq[token] : args.seq;
-            if (active) to = dst + (size_t(cache_plane(map, seq, args.cache.kv_heads, head)) * args.cache.capacity + cache_row(map, seq, position)) * D;
-        }
         if (active) {
             if (kind == 3 && F32) {
-                #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    *reinterpret_cast<float4*>(src + WL::at(m, u) * 4) = make_float4(lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]);
-                    *reinterpret_cast<float4*>(src + (D / 2 + WL::at(m, u)) * 4) = make_float4(hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]);
+                if (WL::kContiguous && by32) {               // (by halves of them 2000 x 16 x 256 take 12.5 us, so 8.4)
+                    store8(src + WL::at(m, 0) * 4, lo);
+                    store8(src + (D / 2 + WL::at(m, 0)) * 4, hi);
+                } else {
+                    #pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        *reinterpret_cast<float4*>(src + WL::at(m, u) * 4) = make_float4(lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]);
+                        *reinterpret_cast<float4*>(src + (D / 2 + WL::at(m, u)) * 4) = make_float4(hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]);
+                    }
                 }
             } else {
                 if (kind == 3) to = reinterpret_cast<uint16_t*>(src);

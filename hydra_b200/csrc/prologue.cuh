@@ -64,12 +64,6 @@ __device__ __forceinline__ void load_rotation(const float* cos_row, const float*
     }
 }
 
-// 1 / sqrt(mean + eps) of a vector's squares.  (Dividing by a power of two and multiplying by its inverse round alike.)
-template <int D>
-__device__ __forceinline__ float head_norm(float sum, float eps) {
-    return __frsqrt_rn(__fadd_rn(__fmul_rn(sum, 1.0f / float(D)), eps));
-}
-
 // In place: the norm (0 none, 1 with `weight`, 2 weightless), then the rotation when `rope`.  The lanes of
 // a warp may hold vectors with different settings: the shuffles are executed by all of them.
 // wl, wh: the weight's elements of this lane (norm 1).
@@ -91,7 +85,7 @@ __device__ __forceinline__ void prepare_head(float (&lo)[HeadLanes<D>::kElems], 
             sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, offset));
         }
         if (norm != 0) {
-            const float inverse = head_norm<D>(sum, eps);
+            const float inverse = __frsqrt_rn(__fadd_rn(__fdiv_rn(sum, float(D)), eps));
             #pragma unroll
             for (int j = 0; j < kElems; ++j) { lo[j] = __fmul_rn(lo[j], inverse); hi[j] = __fmul_rn(hi[j], inverse); }
             if (norm == 1) {
