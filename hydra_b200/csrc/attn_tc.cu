@@ -748,8 +748,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 L = __fmaf_rn(L2, a, __fmul_rn(L, b));
                 M = Mn;
                 float* const state = state_of_row();
-                if (LT::kStateInSmem && args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32 && !args.ep.write_partial) {
-                    // bf16 rows: scaled, rounded, packed and stored by their threads, a row's line in 32-byte stores.  (By the
+                if (LT::kStateInSmem && args.ep.gate_layout == HC_GATE_NONE && !args.ep.write_partial) {
+                    // Rows without a gate: scaled, rounded, packed and stored by their threads, 32 bytes a store, a bf16 row one line.  (By the
                     // loop below an item's end took 6500 clocks; packed here and through shared memory, eight lanes a
                     // row, 4000: 4096 tokens with a window of 128 73 and 62 us, now 58.)
                     if (!warp_has_rows) continue;
@@ -762,16 +762,28 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         for (int i = 0; i < D; i += 2) mul2_inplace(A[i], A[i + 1], b);
                     }
                     const float inverse = __frcp_rn(L);
-                    uint16_t* const out = reinterpret_cast<uint16_t*>(args.ep.out) + (out_row * args.q_heads + head) * D;
                     #pragma unroll
-                    for (int i = 0; i < D; i += 16) {
-                        uint32_t packed[8];
+                    for (int i = 0; i < D; i += 2) mul2_inplace(A[i], A[i + 1], inverse);
+                    if (!valid) continue;
+                    const size_t at = (out_row * args.q_heads + head) * D;
+                    if (args.ep.io_dtype == HC_F32) {
+                        float* const out = reinterpret_cast<float*>(args.ep.out) + at;
                         #pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            mul2_inplace(A[i + 2 * u], A[i + 2 * u + 1], inverse);
-                            packed[u] = pack_bf16x2(A[i + 2 * u], A[i + 2 * u + 1]);
+                        for (int i = 0; i < D; i += 8) {
+                            uint32_t v[8];
+                            #pragma unroll
+                            for (int u = 0; u < 8; ++u) v[u] = __float_as_uint(A[i + u]);
+                            store_32bytes(out + i, v);
                         }
-                        if (valid) store_32bytes(out + i, packed);
+                    } else {
+                        uint16_t* const out = reinterpret_cast<uint16_t*>(args.ep.out) + at;
+                        #pragma unroll
+                        for (int i = 0; i < D; i += 16) {
+                            uint32_t packed[8];
+                            #pragma unroll
+                            for (int u = 0; u < 8; ++u) packed[u] = pack_bf16x2(A[i + 2 * u], A[i + 2 * u + 1]);
+                            store_32bytes(out + i, packed);
+                        }
                     }
                     continue;
                 }
@@ -800,7 +812,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 }
             }
             if constexpr (LT::kStateInSmem) {
-                // With a gate, in fp32, or row partials.
+                // With a gate, or row partials.
                 __syncwarp();
                 if (warp_has_rows) {
                     const bool gated = args.ep.gate_layout != HC_GATE_NONE;

@@ -270,6 +270,71 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
     }
 }
 
+// The same for calls of few vectors, a token a warp (one thread block an SM at most): what counts there is the time of one
+// vector, so a lane has half as many elements (HeadLanes) and nothing is prepared for a walk.
+template <int D>
+__global__ void __launch_bounds__(kPrepWarps * 32)
+prepare_heads_few_kernel(const PrepArgs args, int total_heads) {
+    using HL = HeadLanes<D>;
+    pdl_launch_dependents();
+    const unsigned warp = blockIdx.x * kPrepWarps + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const int sub = lane / HL::kLanes;
+    const int m = lane % HL::kLanes;
+    const bool any_norm = (args.job[0].norm | (args.n_jobs > 1 ? args.job[1].norm : 0) | (args.n_jobs > 2 ? args.job[2].norm : 0)) != 0;
+    const unsigned head_groups = unsigned(total_heads + HL::kPerWarp - 1) / HL::kPerWarp;
+    const unsigned token = warp / head_groups;
+    int head = int(warp - token * head_groups) * HL::kPerWarp + sub;
+    bool active = head < total_heads;
+    if (!active) head = total_heads - 1;                 // keeps the lane's loads legal; nothing is stored
+    int job_index = 0;
+    while (head >= args.job[job_index].heads) {
+        head -= args.job[job_index].heads;
+        ++job_index;
+    }
+    const PrepJob& job = args.job[job_index];
+    const int norm = job.norm, kind = job.kind, dtype = job.src_dtype;
+    const bool rope = job.rope != 0;
+    pdl_wait();
+    if (token >= unsigned(args.tokens)) return;
+    float wl[HL::kElems], wh[HL::kElems], lo[HL::kElems], hi[HL::kElems], c[HL::kElems], s[HL::kElems];
+    if (norm == 1) load_head<D>(job.weight, 0, 1, m, wl, wh);
+    const int position = args.batched ? args.meta.pos[token] : args.first_position + int(token);
+    const size_t src_base = size_t(token) * size_t(job.token_stride) + size_t(head) * job.head_stride;
+    load_head<D>(job.src, src_base, dtype, m, lo, hi);
+    if (rope) {
+        const int table_row = min(position, args.table_positions - 1);
+        load_rotation<D>(args.cos + size_t(table_row) * (D / 2), args.sin + size_t(table_row) * (D / 2), m, c, s);
+    }
+    void* dst = kind == 1 ? args.cache.k : kind == 2 ? args.cache.v : job.dst;
+    size_t base = src_base;
+    if (kind == 0) {
+        base = (size_t(token) * job.heads + head) * D;
+    } else if (kind != 3) {
+        active = active && row_is_local(args.cache.map, position);           // else another rank's tile
+        const int seq = args.batched ? args.meta.seq[token] : args.seq;
+        if (active) {
+            base = (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity +
+                    cache_row(args.cache.map, seq, position)) * D;
+        }
+    }
+    prepare_head<D>(lo, hi, norm, wl, wh, args.eps, rope, c, s, any_norm);
+    if (!active) return;
+    #pragma unroll
+    for (int u = 0; u < HL::kVecs; ++u) {
+        const float a[4] = {lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]};
+        const float b[4] = {hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]};
+        const size_t at = base + 4 * (m + u * HL::kLanes);
+        if (kind == 3 && dtype == HC_F32) {
+            *reinterpret_cast<float4*>(static_cast<float*>(dst) + at) = make_float4(a[0], a[1], a[2], a[3]);
+            *reinterpret_cast<float4*>(static_cast<float*>(dst) + at + D / 2) = make_float4(b[0], b[1], b[2], b[3]);
+        } else {
+            *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at) = pack_bf16x4(a);
+            *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at + D / 2) = pack_bf16x4(b);
+        }
+    }
+}
+
 // The general kernel: any even head_dim up to 512, any alignment.  One warp per head vector, staged
 // in shared memory.
 __global__ void __launch_bounds__(kPrepWarps * 32)
@@ -518,7 +583,13 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
                     (job.norm != 1 || aligned16(job.weight)) && job.src_dtype == args.job[0].src_dtype &&
                     ((job.kind != 0 && job.kind != 3) || aligned16(job.dst));
     }
-    if (vector_ok) {
+    // One thread block an SM: a warp a group of vectors as the few kernel has them.
+    const long long few_groups = args.tokens * ((total_heads + (d < 256 ? 256 / d : 1) - 1) / (d < 256 ? 256 / d : 1));
+    if (vector_ok && args.also.capacity == 0 && few_groups <= (long long)std::max(ctx->sm_count, 1) * kPrepWarps) {
+        auto kernel = d == 64 ? prepare_heads_few_kernel<64> : d == 128 ? prepare_heads_few_kernel<128>
+                    : d == 256 ? prepare_heads_few_kernel<256> : prepare_heads_few_kernel<512>;
+        launch_pdl(kernel, int((few_groups + kPrepWarps - 1) / kPrepWarps), kPrepWarps * 32, 0, stream, args, total_heads);
+    } else if (vector_ok) {
         const int per_warp = 512 / d;
         const long long head_groups = (total_heads + per_warp - 1) / per_warp, groups = args.tokens * head_groups;
         // (A warp stays with its heads, so there are never fewer warps than a token has groups of them.)
