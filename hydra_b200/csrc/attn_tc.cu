@@ -110,14 +110,15 @@ struct TcBarriers {
 
 
 // MODE says what becomes of an item's rows (TcArgs: finish), so that a launch carries the code of its
-// own way only: 0 = the kernel finishes them, 1 = segment partials.
-constexpr int kModeFinish = 0, kModeSegments = 1;
+// own way only: 0 = the kernel finishes them, 1 = segment partials, 2 = d = 64, it finishes fp32 rows without a gate (with
+// their code in the kernel of the others 4096 bf16 tokens take 226 us instead of 220).
+constexpr int kModeFinish = 0, kModeSegments = 1, kModeFinishFp32 = 2;
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                     const TcArgs args) {
-    constexpr bool kFinish = MODE == kModeFinish;
+    constexpr bool kFinish = MODE != kModeSegments;
     using LT = TcLayout<D>;
     extern __shared__ unsigned char raw_smem[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(raw_smem) + 1023) & ~uintptr_t(1023));
@@ -748,10 +749,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 L = __fmaf_rn(L2, a, __fmul_rn(L, b));
                 M = Mn;
                 float* const state = state_of_row();
-                if (LT::kStateInSmem && args.ep.gate_layout == HC_GATE_NONE && !args.ep.write_partial) {
-                    // Rows without a gate: scaled, rounded, packed and stored by their threads, 32 bytes a store, a bf16 row one line.  (By the
-                    // loop below an item's end took 6500 clocks; packed here and through shared memory, eight lanes a
-                    // row, 4000: 4096 tokens with a window of 128 73 and 62 us, now 58.)
+                // Rows without a gate (d = 64) are scaled, rounded, packed and stored by their threads, 32 bytes a store, a bf16
+                // row one line.  (By the loop below an item's end took 6500 clocks; packed here and through shared memory, eight
+                // lanes a row, 4000: 4096 tokens with a window of 128 73 and 62 us, now 58.)
+                const bool own = MODE == kModeFinishFp32 ||
+                                 (args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32 && !args.ep.write_partial);
+                if (LT::kStateInSmem && own) {
                     if (!warp_has_rows) continue;
                     if (state_holds) {
                         #pragma unroll
@@ -762,28 +765,23 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         for (int i = 0; i < D; i += 2) mul2_inplace(A[i], A[i + 1], b);
                     }
                     const float inverse = __frcp_rn(L);
-                    #pragma unroll
-                    for (int i = 0; i < D; i += 2) mul2_inplace(A[i], A[i + 1], inverse);
-                    if (!valid) continue;
                     const size_t at = (out_row * args.q_heads + head) * D;
-                    if (args.ep.io_dtype == HC_F32) {
-                        float* const out = reinterpret_cast<float*>(args.ep.out) + at;
+                    constexpr int kStore = MODE == kModeFinishFp32 ? 8 : 16;      // elements of 32 bytes
+                    unsigned char* const out = static_cast<unsigned char*>(args.ep.out) + at * (32 / kStore);
+                    #pragma unroll
+                    for (int i = 0; i < D; i += kStore) {
+                        uint32_t v[8];
                         #pragma unroll
-                        for (int i = 0; i < D; i += 8) {
-                            uint32_t v[8];
-                            #pragma unroll
-                            for (int u = 0; u < 8; ++u) v[u] = __float_as_uint(A[i + u]);
-                            store_32bytes(out + i, v);
+                        for (int u = 0; u < kStore; u += 2) {
+                            mul2_inplace(A[i + u], A[i + u + 1], inverse);
+                            if constexpr (kStore == 16) {
+                                v[u / 2] = pack_bf16x2(A[i + u], A[i + u + 1]);
+                            } else {
+                                v[u] = __float_as_uint(A[i + u]);
+                                v[u + 1] = __float_as_uint(A[i + u + 1]);
+                            }
                         }
-                    } else {
-                        uint16_t* const out = reinterpret_cast<uint16_t*>(args.ep.out) + at;
-                        #pragma unroll
-                        for (int i = 0; i < D; i += 16) {
-                            uint32_t packed[8];
-                            #pragma unroll
-                            for (int u = 0; u < 8; ++u) packed[u] = pack_bf16x2(A[i + 2 * u], A[i + 2 * u + 1]);
-                            store_32bytes(out + i, packed);
-                        }
+                        if (valid) store_32bytes(out + i * (32 / kStore), v);
                     }
                     continue;
                 }
@@ -811,16 +809,18 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                     for (int i = 0; i < D; ++i) A[i] = __fmul_rn(A[i], b);
                 }
             }
+            if constexpr (MODE == kModeFinishFp32) continue;
             if constexpr (LT::kStateInSmem) {
                 // With a gate, or row partials.
                 __syncwarp();
                 if (warp_has_rows) {
                     const bool gated = args.ep.gate_layout != HC_GATE_NONE;
                     const int column = (lane & 7) * 8;
+                    const float inverse = __frcp_rn(L);
                     #pragma unroll 1
                     for (int k = 0; k < 8; ++k) {
                         const int rl = k * 4 + (lane >> 3);
-                        const float row_l = __shfl_sync(0xffffffffu, L, rl);
+                        const float row_l = __shfl_sync(0xffffffffu, args.ep.write_partial ? L : inverse, rl);
                         const float row_m = __shfl_sync(0xffffffffu, M, rl);
                         const int t2 = (quad * 32 + rl) >> args.log_group;
                         if (t2 >= w.valid_tokens) continue;
@@ -839,7 +839,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                         const size_t gate = (args.ep.gate_layout == HC_GATE_INTERLEAVED ? vec * size_t(2 * D) + D : vec * size_t(D)) + column;
                         #pragma unroll
                         for (int u = 0; u < 8; ++u) {
-                            r[u] = finish_value(r[u], row_l, gated, gated ? load_io(args.ep.gate, gate + u, args.ep.io_dtype) : 0.0f);
+                            r[u] = __fmul_rn(r[u], row_l);
+                            if (gated) r[u] = __fmul_rn(r[u], sigmoid_gate(load_io(args.ep.gate, gate + u, args.ep.io_dtype)));
                         }
                         if (args.ep.io_dtype == HC_F32) {
                             float* dst = reinterpret_cast<float*>(args.ep.out) + vec * D + column;
@@ -1061,6 +1062,10 @@ static hc_status launch_tc_mode(hc_context* ctx, const TcArgs& args, const hc_la
 
 template <int D>
 static hc_status launch_tc(hc_context* ctx, const TcArgs& args, const hc_layer_store& layer, cudaStream_t stream) {
+    if constexpr (TcLayout<D>::kStateInSmem) {
+        const bool fp32 = !args.ep.write_partial && args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype == HC_F32;
+        if (args.finish && fp32) return launch_tc_mode<D, kModeFinishFp32>(ctx, args, layer, stream);
+    }
     if (args.finish) return launch_tc_mode<D, kModeFinish>(ctx, args, layer, stream);
     return launch_tc_mode<D, kModeSegments>(ctx, args, layer, stream);
 }
