@@ -337,7 +337,10 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
                 args.also = view_of(cache, L);
                 args.also_seq = seq;
                 args.also_from = std::max(at, at + count - L.ring);
-                st = launch_copy_rows(ctx, args.also, seq, view, first_visible_tile(at, p->window) * kTileKeys, at, d, stream);
+                // (The keys of the last tile that nobody sees have weight 0, and their values lie where the prompt before this one
+                // left its own, of any sequence and layer: 0 x infinity would be a NaN.)
+                st = launch_copy_rows(ctx, args.also, seq, view, first_visible_tile(at, p->window) * kTileKeys, at, at + count, d,
+                                      stream);
                 if (st != HC_OK) return st;
             }
             st = launch_prepare(ctx, args, stream);

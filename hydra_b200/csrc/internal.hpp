@@ -208,9 +208,10 @@ hc_status check_cuda(cudaError_t err, const char* what);
 
 // prologue.cu
 hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t stream);
-// The rows of positions [first, end) of `from_seq` in `from`, keys and values, into sequence 0 of `to`.
-hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq, const CacheView& to, int first, int end, int d,
-                           cudaStream_t stream);
+// The rows of positions [first, end) of `from_seq` in `from`, keys and values, into sequence 0 of `to`, and zeros to the values
+// there from call_end to the end of its key tile.
+hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq, const CacheView& to, int first, int end, int call_end,
+                           int d, cudaStream_t stream);
 // `count` floats, a multiple of 4 on 16-byte boundaries, one side possibly in pinned host memory.
 hc_status launch_copy_floats(hc_context* ctx, float* dst, const float* src, size_t count, cudaStream_t stream);
 hc_status launch_rms_norm_rows(hc_context* ctx, const void* x, const uint16_t* scale, void* out, int tokens, int width,

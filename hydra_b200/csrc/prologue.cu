@@ -430,18 +430,24 @@ prepare_heads_kernel(const PrepArgs args) {
     }
 }
 
-// Rows of one sequence from one storage to another, a thread per 16 bytes (a row is 2 head_dim bytes, a multiple of 16).
+// Rows [first, end) of one sequence from one storage to another, and zeros to the values of [clear, clear_end) there, a thread
+// per 16 bytes (a row is 2 head_dim bytes, a multiple of 16).
 __global__ void __launch_bounds__(256)
-copy_rows_kernel(const CacheView from, int from_seq, const CacheView to, int first, int end, int pieces) {
+copy_rows_kernel(const CacheView from, int from_seq, const CacheView to, int first, int end, int clear, int clear_end, int pieces) {
     pdl_launch_dependents();
     pdl_wait();
-    const int heads = from.kv_heads;
-    const unsigned total = unsigned(end - first) * unsigned(heads) * unsigned(pieces);
+    const int heads = from.kv_heads, copied = end - first;
+    const unsigned total = unsigned(copied + clear_end - clear) * unsigned(heads) * unsigned(pieces);
     for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
         const unsigned row = i / unsigned(pieces), piece = i - row * unsigned(pieces);
-        const int position = first + int(row / unsigned(heads)), head = int(row % unsigned(heads));
-        const size_t src = (size_t(cache_plane(from.map, from_seq, heads, head)) * from.capacity + cache_row(from.map, from_seq, position)) * pieces + piece;
+        const int at = int(row / unsigned(heads)), head = int(row % unsigned(heads));
+        const int position = at < copied ? first + at : clear + (at - copied);
         const size_t dst = (size_t(cache_plane(to.map, 0, heads, head)) * to.capacity + cache_row(to.map, 0, position)) * pieces + piece;
+        if (at >= copied) {
+            reinterpret_cast<uint4*>(to.v)[dst] = make_uint4(0, 0, 0, 0);
+            continue;
+        }
+        const size_t src = (size_t(cache_plane(from.map, from_seq, heads, head)) * from.capacity + cache_row(from.map, from_seq, position)) * pieces + piece;
         const uint4 k = reinterpret_cast<const uint4*>(from.k)[src], v = reinterpret_cast<const uint4*>(from.v)[src];
         reinterpret_cast<uint4*>(to.k)[dst] = k;
         reinterpret_cast<uint4*>(to.v)[dst] = v;
@@ -610,12 +616,13 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
     return check_cuda(cudaGetLastError(), "prepare_heads_kernel launch");
 }
 
-hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq, const CacheView& to, int first, int end, int d,
-                           cudaStream_t stream) {
-    if (first >= end) return HC_OK;
-    const long long total = (long long)(end - first) * from.kv_heads * (d / 8);
+hc_status launch_copy_rows(hc_context* ctx, const CacheView& from, int from_seq, const CacheView& to, int first, int end, int call_end,
+                           int d, cudaStream_t stream) {
+    const int clear_end = (call_end + kTileKeys - 1) / kTileKeys * kTileKeys;
+    const long long total = (long long)(end - first + clear_end - call_end) * from.kv_heads * (d / 8);
+    if (total == 0) return HC_OK;
     const int grid = int(std::min<long long>((total + 255) / 256, (long long)std::max(ctx->sm_count, 1) * 8));
-    launch_pdl(copy_rows_kernel, grid, 256, 0, stream, from, from_seq, to, first, end, d / 8);
+    launch_pdl(copy_rows_kernel, grid, 256, 0, stream, from, from_seq, to, first, end, call_end, clear_end, d / 8);
     ctx->launches += 1;
     return check_cuda(cudaGetLastError(), "copy_rows_kernel launch");
 }

@@ -3,6 +3,7 @@ a segment and a row tile, ragged batches, column widths of the projections, piec
 reference is the oracle, plain PyTorch in fp32 for the projections, and the path's own invariant: a position's
 result is the same bits whether it came in a prompt or as a decoded token."""
 import ctypes
+import dataclasses
 
 import numpy as np
 import pytest
@@ -219,6 +220,58 @@ def test_prompts_longer_than_a_ring_equal_linear_storage(hb, ctx, d, qh, kvh, wi
         layer.close()
     for ring, linear in zip(*got):
         assert np.array_equal(ring, linear)
+
+
+@pytest.mark.parametrize("d, qh, kvh, window, first, tokens, blocks", [
+    (64, 16, 4, 128, 0, 645, False),      # no history: nothing is copied out of the ring
+    (64, 16, 4, 128, 259, 645, True),
+    (96, 8, 4, 130, 77, 600, False),      # the CUDA-core kernels
+    (96, 8, 4, 130, 0, 601, True),
+    (128, 16, 2, 300, 131, 1001, False),
+    (256, 16, 8, 256, 0, 1151, False),
+    (256, 16, 8, 256, 77, 1027, True),
+    (256, 64, 4, 384, 515, 2300, False),  # two parts, the first of which ends inside a key tile as well
+    (512, 8, 1, 200, 3, 900, False),
+])
+def test_prompts_beside_a_ring_see_no_other_prompt(hb, ctx, d, qh, kvh, window, first, tokens, blocks):
+    """Infinities and NaN in another sequence's prompt, of the same ring layer and of one of another geometry, right before
+    it: the bits of linear storage, in which sequences and layers lie apart."""
+    import torch
+    geometry = [(qh, kvh, d, window), (6, 3, 64, 200)]
+    rng = np.random.default_rng(d + first + tokens)
+    bad = [torch.full((1100, k, dim), float("nan"), device="cuda") for _, k, dim, _ in geometry]
+    for x in bad:
+        x[::2] = float("inf")
+    ends = np.zeros(tokens, np.int32)
+    for at, n in ((3, 40), (90, 120), (tokens - 60, 60)):
+        ends[at:at + n] = first + at + n
+    ends = torch.from_numpy(ends).cuda() if blocks else None
+    inputs = [[tl.to_device(tl.normal_bf16(rng, (n, heads, dim)), "f32") for n, heads in ((tokens, q), (first + tokens, k), (first + tokens, k))]
+              for q, k, dim, _ in geometry]
+    got = []
+    for storage in (hb.capi.HC_STORAGE_RING, hb.capi.HC_STORAGE_LINEAR):
+        cache = hb.KVCache(ctx, [dict(q_heads=q, kv_heads=k, head_dim=dim, window=w, storage=storage) for q, k, dim, w in geometry],
+                           4096, prefill_chunk=128, max_seqs=2)
+        be = hb.AttentionBackend(ctx)
+        params = [hb.AttnParams(q_heads=q, kv_heads=k, head_dim=dim, window=w, sm_scale=dim ** -0.5, io_dtype=hb.capi.HC_F32)
+                  for q, k, dim, w in geometry]
+        outs = []
+        for other in (0, 1):
+            for layer, ((q, k, dim, _), (xq, xk, xv)) in enumerate(zip(geometry, inputs)):
+                for at in range(0, first, 128):
+                    n = min(128, first - at)
+                    be.write_key_value(cache, layer, xk[at:], xv[at:], n, at, params[layer], seq=1)
+                wide = torch.ones(1100, geometry[other][0], geometry[other][2], device="cuda")
+                be.prefill_chunks(cache, other, wide, bad[other], bad[other], torch.empty_like(wide), 1100, 0, 128, params[other], seq=0)
+                out = torch.full((tokens, q, dim), 7.0, device="cuda")
+                be.prefill_chunks(cache, layer, xq, xk[first:], xv[first:], out, tokens, first, 128,
+                                  dataclasses.replace(params[layer], block_ends=ends), seq=1)
+                ctx.check()
+                outs.append(out.cpu().numpy())
+        got.append(outs)
+        cache.close()
+    for ring, linear in zip(*got):
+        assert np.all(np.isfinite(linear)) and np.array_equal(ring, linear)
 
 
 @pytest.mark.parametrize("d, qh, kvh, tokens, window", [(64, 16, 2, 77, 0), (64, 64, 8, 300, 128), (256, 16, 8, 140, 0), (256, 8, 8, 515, 256),
