@@ -110,9 +110,11 @@ struct TcBarriers {
 
 
 // MODE says what becomes of an item's rows (TcArgs: finish), so that a launch carries the code of its
-// own way only: 0 = the kernel finishes them, 1 = segment partials, 2 = d = 64, it finishes fp32 rows without a gate (with
-// their code in the kernel of the others 4096 bf16 tokens take 226 us instead of 220).
-constexpr int kModeFinish = 0, kModeSegments = 1, kModeFinishFp32 = 2;
+// own way only: 0 = the kernel finishes them, 1 = segment partials.  At d = 64 its code places the others': 0 finishes bf16 rows
+// without a gate and row partials, 2 fp32 rows without a gate (with their code in mode 0 4096 bf16 tokens of 64 heads take 226 us
+// instead of 220), 3 rows with a gate (2000 tokens with a window of 128 in mode 0 80 us, here 73; all the same mode 0 keeps the
+// loop that serves both: with less of it 4096 bf16 tokens take 219 us instead of 214).
+constexpr int kModeFinish = 0, kModeSegments = 1, kModeFinishFp32 = 2, kModeFinishGated = 3;
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(kTcThreads, 1)
@@ -753,7 +755,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_con
                 // row one line.  (By the loop below an item's end took 6500 clocks; packed here and through shared memory, eight
                 // lanes a row, 4000: 4096 tokens with a window of 128 73 and 62 us, now 58.)
                 const bool own = MODE == kModeFinishFp32 ||
-                                 (args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32 && !args.ep.write_partial);
+                                 (MODE == kModeFinish && args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype != HC_F32 && !args.ep.write_partial);
                 if (LT::kStateInSmem && own) {
                     if (!warp_has_rows) continue;
                     if (state_holds) {
@@ -1063,8 +1065,9 @@ static hc_status launch_tc_mode(hc_context* ctx, const TcArgs& args, const hc_la
 template <int D>
 static hc_status launch_tc(hc_context* ctx, const TcArgs& args, const hc_layer_store& layer, cudaStream_t stream) {
     if constexpr (TcLayout<D>::kStateInSmem) {
-        const bool fp32 = !args.ep.write_partial && args.ep.gate_layout == HC_GATE_NONE && args.ep.io_dtype == HC_F32;
-        if (args.finish && fp32) return launch_tc_mode<D, kModeFinishFp32>(ctx, args, layer, stream);
+        const bool gated = args.ep.gate_layout != HC_GATE_NONE;
+        if (args.finish && gated) return launch_tc_mode<D, kModeFinishGated>(ctx, args, layer, stream);
+        if (args.finish && !args.ep.write_partial && args.ep.io_dtype == HC_F32) return launch_tc_mode<D, kModeFinishFp32>(ctx, args, layer, stream);
     }
     if (args.finish) return launch_tc_mode<D, kModeFinish>(ctx, args, layer, stream);
     return launch_tc_mode<D, kModeSegments>(ctx, args, layer, stream);

@@ -45,6 +45,7 @@ def _filled(hb, ctx, d, qh, kvh, window, tokens, seqs=1, io="bf16", gated=False)
     (64, 64, 8, 0, 2203, "bf16", False),       # three segments of 1024, a last row tile of 11 tokens
     (64, 64, 8, 128, 1100, "f32", False),      # two tiles a row
     (64, 8, 8, 0, 1153, "bf16", True),         # one head a group: 128 tokens a row tile
+    (64, 16, 2, 200, 1301, "f32", True),       # gated fp32 rows, several segments
     (128, 16, 2, 0, 1290, "bf16", False),
     (256, 16, 8, 1024, 2180, "bf16", False),   # pairs of SMs; the window crosses a segment of 2048
     (256, 16, 2, 0, 2305, "bf16", True),       # the gated epilogue
