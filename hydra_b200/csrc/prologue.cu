@@ -103,7 +103,7 @@ constexpr int prep_blocks(bool fp32) { return fp32 ? 2 : 3; }
 
 template <int D, bool F32>
 __global__ void __launch_bounds__(kPrepWarps * 32, prep_blocks(F32))
-prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
+prepare_heads_vec_kernel(const PrepArgs args, int total_heads, int prefetch) {
     using WL = WideLanes<D>;
     constexpr int kBytes = F32 ? 4 : 2;
     pdl_launch_dependents();
@@ -165,7 +165,7 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
     for (;;) {
         const bool more = token + step < unsigned(args.tokens);
         if (more) ahead.load(src + src_step, m);
-        if (token + 3 * step < unsigned(args.tokens)) {              // two further on their way into L2
+        if (prefetch && token + 3 * step < unsigned(args.tokens)) {              // two further on their way into L2
             #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(src + 3 * src_step + (h * (D / 2) + WL::at(m, 0)) * kBytes));
@@ -270,8 +270,18 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads) {
     }
 }
 
-// The same for calls of few vectors, a token a warp (one thread block an SM at most): what counts there is the time of one
-// vector, so a lane has half as many elements (HeadLanes) and nothing is prepared for a walk.
+__device__ __forceinline__ void store_io4(void* base, size_t index, int dtype, const float (&v)[4]) {
+    if (dtype == 0) {
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + index) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+        *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(base) + index) = pack_bf16x4(v);
+    }
+}
+
+// The same where every warp has one token: what counts there is the time of one vector, so a lane has half as many elements
+// (HeadLanes; head_dim 512 as many) and nothing is prepared for a walk.  All of the job is read ahead of the wait, and the loop,
+// which goes round once, keeps the norm weights' load ahead of the sum that is worked out meanwhile (without it a row of 2 x 512
+// appended behind another took 1.8 us, now 1.55; 8 x 64 1.56 and 1.4; one wave of 64 x 256 3.0, by the kernel above, and 2.25).
 template <int D>
 __global__ void __launch_bounds__(kPrepWarps * 32)
 prepare_heads_few_kernel(const PrepArgs args, int total_heads) {
@@ -282,55 +292,65 @@ prepare_heads_few_kernel(const PrepArgs args, int total_heads) {
     const int sub = lane / HL::kLanes;
     const int m = lane % HL::kLanes;
     const bool any_norm = (args.job[0].norm | (args.n_jobs > 1 ? args.job[1].norm : 0) | (args.n_jobs > 2 ? args.job[2].norm : 0)) != 0;
+    // Warps side by side take the heads of a token.
     const unsigned head_groups = unsigned(total_heads + HL::kPerWarp - 1) / HL::kPerWarp;
-    const unsigned token = warp / head_groups;
-    int head = int(warp - token * head_groups) * HL::kPerWarp + sub;
-    bool active = head < total_heads;
-    if (!active) head = total_heads - 1;                 // keeps the lane's loads legal; nothing is stored
+    const unsigned step = gridDim.x * kPrepWarps / head_groups;
+    const unsigned first_token = warp / head_groups;
+    int head = int(warp - first_token * head_groups) * HL::kPerWarp + sub;
+    const bool in_range = head < total_heads;
+    if (!in_range) head = total_heads - 1;               // keeps the lane's loads legal; nothing is stored
     int job_index = 0;
     while (head >= args.job[job_index].heads) {
         head -= args.job[job_index].heads;
         ++job_index;
     }
     const PrepJob& job = args.job[job_index];
-    const int norm = job.norm, kind = job.kind, dtype = job.src_dtype;
+    const int norm = job.norm, kind = job.kind, dtype = job.src_dtype, heads = job.heads;
     const bool rope = job.rope != 0;
-    pdl_wait();
-    if (token >= unsigned(args.tokens)) return;
-    float wl[HL::kElems], wh[HL::kElems], lo[HL::kElems], hi[HL::kElems], c[HL::kElems], s[HL::kElems];
-    if (norm == 1) load_head<D>(job.weight, 0, 1, m, wl, wh);
-    const int position = args.batched ? args.meta.pos[token] : args.first_position + int(token);
-    const size_t src_base = size_t(token) * size_t(job.token_stride) + size_t(head) * job.head_stride;
-    load_head<D>(job.src, src_base, dtype, m, lo, hi);
-    if (rope) {
-        const int table_row = min(position, args.table_positions - 1);
-        load_rotation<D>(args.cos + size_t(table_row) * (D / 2), args.sin + size_t(table_row) * (D / 2), m, c, s);
-    }
+    const void* src = job.src;
+    const long long token_stride = job.token_stride;
+    const size_t head_offset = size_t(head) * job.head_stride;
     void* dst = kind == 1 ? args.cache.k : kind == 2 ? args.cache.v : job.dst;
-    size_t base = src_base;
-    if (kind == 0) {
-        base = (size_t(token) * job.heads + head) * D;
-    } else if (kind != 3) {
-        active = active && row_is_local(args.cache.map, position);           // else another rank's tile
-        const int seq = args.batched ? args.meta.seq[token] : args.seq;
-        if (active) {
-            base = (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity +
-                    cache_row(args.cache.map, seq, position)) * D;
+    const uint16_t* weight = job.weight;
+    pdl_wait();
+    float wl[HL::kElems], wh[HL::kElems];
+    if (first_token >= step || first_token >= unsigned(args.tokens)) return;
+    if (norm == 1) load_head<D>(weight, 0, 1, m, wl, wh);
+    for (unsigned token = first_token; token < unsigned(args.tokens); token += step) {
+        const int position = args.batched ? args.meta.pos[token] : args.first_position + int(token);
+        const size_t src_base = size_t(token) * size_t(token_stride) + head_offset;
+        float lo[HL::kElems], hi[HL::kElems], c[HL::kElems], s[HL::kElems];
+        load_head<D>(src, src_base, dtype, m, lo, hi);
+        if (rope) {
+            const int table_row = min(position, args.table_positions - 1);
+            load_rotation<D>(args.cos + size_t(table_row) * (D / 2), args.sin + size_t(table_row) * (D / 2), m, c, s);
         }
-    }
-    prepare_head<D>(lo, hi, norm, wl, wh, args.eps, rope, c, s, any_norm);
-    if (!active) return;
-    #pragma unroll
-    for (int u = 0; u < HL::kVecs; ++u) {
-        const float a[4] = {lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]};
-        const float b[4] = {hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]};
-        const size_t at = base + 4 * (m + u * HL::kLanes);
-        if (kind == 3 && dtype == HC_F32) {
-            *reinterpret_cast<float4*>(static_cast<float*>(dst) + at) = make_float4(a[0], a[1], a[2], a[3]);
-            *reinterpret_cast<float4*>(static_cast<float*>(dst) + at + D / 2) = make_float4(b[0], b[1], b[2], b[3]);
-        } else {
-            *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at) = pack_bf16x4(a);
-            *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at + D / 2) = pack_bf16x4(b);
+        size_t base = src_base;
+        bool active = in_range;
+        if (kind == 0) {
+            base = (size_t(token) * heads + head) * D;
+        } else if (kind != 3) {
+            active = active && row_is_local(args.cache.map, position);           // else another rank's tile
+            const int seq = args.batched ? args.meta.seq[token] : args.seq;
+            if (active) {
+                base = (size_t(cache_plane(args.cache.map, seq, args.cache.kv_heads, head)) * args.cache.capacity +
+                        cache_row(args.cache.map, seq, position)) * D;
+            }
+        }
+        prepare_head<D>(lo, hi, norm, wl, wh, args.eps, rope, c, s, any_norm);
+        if (!active) continue;
+        #pragma unroll
+        for (int u = 0; u < HL::kVecs; ++u) {
+            const float a[4] = {lo[4 * u], lo[4 * u + 1], lo[4 * u + 2], lo[4 * u + 3]};
+            const float b[4] = {hi[4 * u], hi[4 * u + 1], hi[4 * u + 2], hi[4 * u + 3]};
+            const size_t at = base + 4 * (m + u * HL::kLanes);
+            if (kind == 3 && (D == 512 || dtype == HC_F32)) {
+                store_io4(dst, at, dtype, a);
+                store_io4(dst, at + D / 2, dtype, b);
+            } else {
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at) = pack_bf16x4(a);
+                *reinterpret_cast<uint2*>(static_cast<uint16_t*>(dst) + at + D / 2) = pack_bf16x4(b);
+            }
         }
     }
 }
@@ -589,24 +609,31 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
                     (job.norm != 1 || aligned16(job.weight)) && job.src_dtype == args.job[0].src_dtype &&
                     ((job.kind != 0 && job.kind != 3) || aligned16(job.dst));
     }
-    // One thread block an SM: a warp a group of vectors as the few kernel has them.
-    const long long few_groups = args.tokens * ((total_heads + (d < 256 ? 256 / d : 1) - 1) / (d < 256 ? 256 / d : 1));
-    if (vector_ok && args.also.capacity == 0 && few_groups <= (long long)std::max(ctx->sm_count, 1) * kPrepWarps) {
+    const bool fp32 = args.job[0].src_dtype == HC_F32;
+    const bool large = size_t(vectors) * d * (fp32 ? 4 : 2) > (size_t(64) << 20);      // does not stay in L2
+    auto groups_of = [&](int per_warp) -> long long { return (total_heads + per_warp - 1) / per_warp; };     // of a token
+    const long long sms = std::max(ctx->sm_count, 1);
+    const int few_blocks = d == 512 ? 3 : 4;             // thread blocks of the few kernel an SM holds
+    const long long few = groups_of(std::max(256 / d, 1));
+    // What one wave holds goes a token a warp, at 16 x 64 up to 1184 tokens (1000 of them 2.4 us, by the other kernel 2.9; 2000 3.7
+    // and 3.4), and so do, in a walk, fp32 rows of 512 that come from and go to DRAM (8000 x 16 59 us, by the other 68).
+    if (vector_ok && args.also.capacity == 0 && (args.tokens * few <= sms * few_blocks * kPrepWarps || (fp32 && d == 512 && large))) {
+        const int grid = int((std::max(std::min(args.tokens * few, cap * kPrepWarps), few) + kPrepWarps - 1) / kPrepWarps);
         auto kernel = d == 64 ? prepare_heads_few_kernel<64> : d == 128 ? prepare_heads_few_kernel<128>
                     : d == 256 ? prepare_heads_few_kernel<256> : prepare_heads_few_kernel<512>;
-        launch_pdl(kernel, int((few_groups + kPrepWarps - 1) / kPrepWarps), kPrepWarps * 32, 0, stream, args, total_heads);
+        launch_pdl(kernel, grid, kPrepWarps * 32, 0, stream, args, total_heads);
     } else if (vector_ok) {
-        const int per_warp = 512 / d;
-        const long long head_groups = (total_heads + per_warp - 1) / per_warp, groups = args.tokens * head_groups;
+        const long long groups = groups_of(512 / d);
         // (A warp stays with its heads, so there are never fewer warps than a token has groups of them.)
-        const bool fp32 = args.job[0].src_dtype == HC_F32;
-        const long long most = (long long)std::max(ctx->sm_count, 1) * prep_blocks(fp32) * kPrepWarps;
-        const int grid = int((std::max(std::min(groups, most), head_groups) + kPrepWarps - 1) / kPrepWarps);
+        const int grid = int((std::max(std::min(args.tokens * groups, sms * prep_blocks(fp32) * kPrepWarps), groups) + kPrepWarps - 1) / kPrepWarps);
+        // Prefetched bf16 rows are 90 us -> 55 (above).  Of fp32 rows a warp has enough on its way without (8000 x 64 x 256 146 us
+        // with, 130 without; in place 47.5 and 43), but for those in place that L2 keeps (2000 x 16 x 256 12.4 with, 13.4 without).
+        const int prefetch = !fp32 || (args.job[0].kind == 3 && !large) ? 1 : 0;
         auto kernel = d == 64 ? (fp32 ? prepare_heads_vec_kernel<64, true> : prepare_heads_vec_kernel<64, false>)
                     : d == 128 ? (fp32 ? prepare_heads_vec_kernel<128, true> : prepare_heads_vec_kernel<128, false>)
                     : d == 256 ? (fp32 ? prepare_heads_vec_kernel<256, true> : prepare_heads_vec_kernel<256, false>)
                                : (fp32 ? prepare_heads_vec_kernel<512, true> : prepare_heads_vec_kernel<512, false>);
-        launch_pdl(kernel, grid, kPrepWarps * 32, 0, stream, args, total_heads);
+        launch_pdl(kernel, grid, kPrepWarps * 32, 0, stream, args, total_heads, prefetch);
     } else {
         const long long wanted = (vectors + kPrepWarps - 1) / kPrepWarps;
         const int grid = int(std::min<long long>(wanted, cap));

@@ -318,3 +318,54 @@ def test_fp32_rows_on_16_byte_boundaries_that_are_no_32_byte_ones(hb, ctx, d):
     want = x[0].double()
     want = want / torch.sqrt((want * want).mean(-1, keepdim=True) + 1e-6) * weight.double()
     assert np.max(np.abs(got[0][2] - want.cpu().numpy())) < 1e-5
+
+
+@pytest.mark.parametrize("io", ["bf16", "f32"])
+@pytest.mark.parametrize("d, heads", [(64, 5), (128, 6), (256, 16), (512, 3)])
+def test_prologue_of_a_wave_and_of_more(hb, ctx, d, heads, io):
+    """One token fewer and more than one wave of the kernel for few vectors holds: appended rows and vectors normed in place
+    are the bits of a call for each half, which that kernel takes; normed vectors are float64's (relative error of the sum
+    d 2^-24, of the root and two products 2^-22; bf16, which has 8 significant bits, half a step 2^-8 more)."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    per_warp, blocks = max(256 // d, 1), 3 if d == 512 else 4
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    weight = (1 + 0.1 * torch.randn(d, device="cuda", generator=gen)).to(torch.bfloat16)
+    dtype, code = (torch.bfloat16, hb.capi.HC_BF16) if io == "bf16" else (torch.float32, hb.capi.HC_F32)
+    most = sms * blocks * 8
+    layer = tl.Layer(hb, ctx, heads, heads, d, most, rope_inv_freq=ho.inverse_frequencies(d, 10000.0, d // 2), io=io)
+    be, bound = layer.backend, d * 2.0 ** -24 + 2.0 ** -22 + (2.0 ** -8 if io == "bf16" else 0)
+    for tokens in [n + e for n in {most // -(-heads // per_warp), most // -(-2 * heads // per_warp)} for e in (0, 1)]:
+        x = torch.randn(2, tokens, heads, d, device="cuda", generator=gen).to(dtype)
+        got = []
+        for cut in (tokens, tokens // 2):
+            y = x[0].clone()
+            for a, b in ((0, cut), (cut, tokens)):
+                if a == b:
+                    continue
+                be.write_key_value(layer.cache, 0, x[0, a:], x[1, a:], b - a, a, layer.params)
+                be.rms_norm_heads(y[a:], weight, b - a, heads, d, 1e-6, io_dtype=code)
+            ctx.check()
+            got.append([y.float().cpu().numpy(), *tl.read_cache(layer.cache, 0, tokens, heads, d)])
+        assert all(np.array_equal(a, b) for a, b in zip(*got))
+        want = x[0].double()
+        want = (want / torch.sqrt((want * want).mean(-1, keepdim=True) + 1e-6) * weight.double()).cpu().numpy()
+        assert np.max(np.abs(got[0][0] - want) / np.maximum(np.abs(want), 1e-30)) < bound
+    layer.close()
+
+
+def test_fp32_rows_of_512_that_exceed_l2(hb, ctx):
+    """More than 64 MB of them are appended by the kernel for few vectors, in a walk: the bits of a call for each third."""
+    import torch
+    tokens, heads, d = 2200, 8, 512                       # 72 MB of keys and values
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(2, tokens, heads, d, device="cuda", generator=gen)
+    layer = tl.Layer(hb, ctx, heads, heads, d, tokens, rope_inv_freq=ho.inverse_frequencies(d, 10000.0, d // 2), io="f32")
+    got = []
+    for step in (tokens, 734):
+        for a in range(0, tokens, step):
+            layer.backend.write_key_value(layer.cache, 0, x[0, a:], x[1, a:], min(step, tokens - a), a, layer.params)
+        ctx.check()
+        got.append(tl.read_cache(layer.cache, 0, tokens, heads, d))
+    layer.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
