@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "internal.hpp"
+#include "linear_plan.hpp"
 #include "tc_ptx.cuh"
 
 namespace hc {
@@ -62,8 +63,6 @@ struct LinBarriers {
 };
 static_assert(sizeof(LinBarriers) % 16 == 0, "the staging behind it is 16-byte aligned");
 
-constexpr int kLinJobs = 4;
-
 // One launch may carry several projections of the same x (q, k and v of a layer): their output tiles
 // form one list, job after job.
 struct LinJob {
@@ -85,58 +84,6 @@ struct LinArgs {
     int stages;               // few tokens
     int* status;
 };
-
-// Tiles of two widths.  A job's columns are cut in wide tiles, and what is left of an odd number of halves is a half tile.
-// The list has n_wide of the wide tiles, then the halves of the others and the odd halves, so that a launch's last
-// round of pairs can be one of half tiles.
-struct LinWide {
-    int job, col, tm, width;
-};
-template <int BN>
-__host__ __device__ __forceinline__ LinWide decode_wide(const LinArgs& args, int tile) {
-    LinWide t{0, 0, 0, BN};
-    int all = 0;                                             // wide tiles of all jobs
-    #pragma unroll
-    for (int j = 0; j < kLinJobs; ++j) {
-        if (j < args.n_jobs) all += args.job[j].out_features / BN * args.tiles_m;
-    }
-    int wide = tile, half = 0;
-    if (tile >= args.n_wide) {
-        t.width = BN / 2;
-        wide = args.n_wide + ((tile - args.n_wide) >> 1);
-        half = (tile - args.n_wide) & 1;
-    }
-    if (wide < all) {
-        int left = wide;
-        #pragma unroll
-        for (int j = 0; j < kLinJobs; ++j) {
-            const int tiles = j < args.n_jobs ? args.job[j].out_features / BN * args.tiles_m : 0;
-            if (j < args.n_jobs && left >= 0 && left < tiles) {
-                t.job = j;
-                t.col = left / args.tiles_m;
-                t.tm = left - t.col * args.tiles_m;
-                t.col = t.col * BN + half * (BN / 2);
-            }
-            left -= tiles;
-        }
-        return t;
-    }
-    // Behind them a job's last columns: one or two half tiles a row tile.
-    int left = tile - args.n_wide - 2 * (all - args.n_wide);
-    #pragma unroll
-    for (int j = 0; j < kLinJobs; ++j) {
-        const int first = j < args.n_jobs ? args.job[j].out_features / BN * BN : 0;
-        const int tiles = j < args.n_jobs ? (args.job[j].out_features - first + BN / 2 - 1) / (BN / 2) * args.tiles_m : 0;
-        if (left >= 0 && left < tiles) {
-            t.job = j;
-            t.col = left / args.tiles_m;
-            t.tm = left - t.col * args.tiles_m;
-            t.col = first + t.col * (BN / 2);
-        }
-        left -= tiles;
-    }
-    return t;
-}
 
 struct LinTile {
     int job, tn, tm;
@@ -739,47 +686,9 @@ hc_status linear_tc(hc_context* ctx, const void* x, int n_jobs, const void* cons
         if (tiles(48) <= sms) return launch_few<48, 128>(ctx, x, w, args, in_features, stream);
         return launch_few<64, 128>(ctx, x, w, args, in_features, stream);
     }
-    // The column tile whose rounds of pairs take least.  A K step costs an SM the larger of its MMAs (2 clocks a column)
-    // and of (128 + BN / 2) x 128 bytes out of L2, of which about 60 arrive per clock and SM with all of them
-    // loading: 546 clocks for 256 columns, 478, 443, 410.  Measured on 4096, 1024, 600 and 300 tokens of the three
-    // geometries: the choice is the fastest of the four or within a few percent of it.
-    const int pairs = std::max(ctx->sm_count / 2, 1);
-    const int widths[4] = {256, 192, 160, 128};
-    const double step[4] = {546.0, 478.0, 443.0, 410.0};
-    const int tiles_m = (tokens + 2 * kLinM - 1) / (2 * kLinM);
-    int best = 0;
-    double least = 0.0;
-    for (int i = 0; i < 4; ++i) {
-        long long tiles = 0;
-        for (int j = 0; j < n_jobs; ++j) tiles += (long long)tiles_m * ((out_features[j] + widths[i] - 1) / widths[i]);
-        const double t = double((tiles + pairs - 1) / pairs) * step[i];
-        if (i == 0 || t < least) {
-            least = t;
-            best = i;
-        }
-    }
-    // Or wide tiles in whole rounds and half tiles for the rest, in the last round or two: 4096 tokens to 2880 columns are two
-    // rounds of 256 and one of 128 instead of three of 256 (81.2 us, now 77.8; 2048 tokens to q, k and v of 4096 and 512 columns
-    // 48.7, now 46.0).  Where another choice is predicted as fast it is faster: its K steps are of one size, its ring deeper
-    // (600 tokens of 2816 to 8192 columns 28.7 against 31.6).
-    long long wide = 0, odd = 0;
-    for (int j = 0; j < n_jobs; ++j) {
-        wide += (long long)tiles_m * (out_features[j] / 256);
-        odd += (long long)tiles_m * ((out_features[j] % 256 + 127) / 128);
-    }
-    long long n_wide = wide;                                 // 256 columns throughout: the last of a job's in half tiles
-    for (long long rounds = 1; rounds * pairs <= wide; ++rounds) {
-        const long long n = rounds * pairs, total = (n + 2 * (wide - n) + odd + pairs - 1) / pairs;
-        const double t = double(rounds) * step[0] + double(total - rounds) * step[3];
-        if (t < least) {
-            least = t;
-            best = 0;
-            n_wide = n;
-        }
-    }
-    const long long n_tiles = n_wide + 2 * (wide - n_wide) + odd;
-    switch (widths[best]) {
-        case 256: return launch_pair<256>(ctx, x, w, args, in_features, stream, int(n_wide), int(n_tiles));
+    const LinPlan plan = plan_pairs(out_features, n_jobs, (tokens + 2 * kLinM - 1) / (2 * kLinM), std::max(ctx->sm_count / 2, 1));
+    switch (plan.width) {
+        case 256: return launch_pair<256>(ctx, x, w, args, in_features, stream, int(plan.n_wide), int(plan.n_tiles));
         case 192: return launch_pair<192>(ctx, x, w, args, in_features, stream);
         case 160: return launch_pair<160>(ctx, x, w, args, in_features, stream);
         default: return launch_pair<128>(ctx, x, w, args, in_features, stream);

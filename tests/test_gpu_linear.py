@@ -118,9 +118,14 @@ def test_linear_refuses_what_it_cannot_tile():
     (4096, 64, (1000, 2880, 130)),     # last columns of one and two halves
     (4096, 64, (4096, 513)),           # a last half of one column
     (9000, 64, (100, 90)),             # no wide tile at all
+    (4096, 64, (904,)),                # a last tile of 136 columns: wide, with zeros
+    (4096, 64, (2200, 385, 511)),      # the same behind others, 152, 129 and 255 columns
+    (4096, 64, (4680, 384)),           # a wide tile of 72 columns more than half among those cut in halves
 ])
 def test_linear_tiles_of_two_widths(tokens, width, outs):
-    """Sums of 64 or 128 products in fp32 against float64: 128 roundings of 2^-24 of sums below 40 stay under 4e-4."""
+    """Sums of 64 or 128 products in fp32 against float64: 128 roundings of 2^-24 of sums below 40 stay under 4e-4.  With
+    biases and residuals, which have a half tile's own columns: two roundings more of values below 50, 2^-24 each; in bf16
+    half a step of 8 significant bits."""
     import torch
     import hydra_b200 as hb
     ctx = hb.Context(0)
@@ -132,6 +137,19 @@ def test_linear_tiles_of_two_widths(tokens, width, outs):
     ctx.check()
     for got, weight in zip(y, w):
         assert float((got.double() - x.double() @ weight.double().T).abs().max()) < 4e-4
+    b = [torch.randn(n, device="cuda", generator=gen).to(torch.bfloat16) for n in outs]
+    half = [torch.full((tokens, n), 7.0, device="cuda", dtype=torch.bfloat16) for n in outs]
+    hb.AttentionBackend(ctx).linear_group(x, w, b, half, tokens, width, y_dtype=hb.capi.HC_BF16)
+    ctx.check()
+    for got, weight, bias in zip(half, w, b):
+        want = x.double() @ weight.double().T + bias.double()
+        assert bool(((got.double() - want).abs() <= 4.1e-4 + 2.0 ** -8 * want.abs()).all())
+    for weight, bias in zip(w, b):
+        residual = torch.randn(tokens, weight.shape[0], device="cuda", generator=gen)
+        got = torch.full_like(residual, 7.0)
+        hb.AttentionBackend(ctx).linear(x, weight, bias, got, tokens, width, weight.shape[0], residual=residual)
+        ctx.check()
+        assert float((got.double() - x.double() @ weight.double().T - bias.double() - residual.double()).abs().max()) < 4.1e-4
     ctx.close()
 
 
