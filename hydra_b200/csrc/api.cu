@@ -2,6 +2,7 @@
 // its bookkeeping, and the choice of kernels for each call.  All device work is in the other files.
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -337,8 +338,8 @@ hc_status prefill_impl(hc_context* ctx, hc_kv_cache* cache, int layer, int seq, 
                 args.also = view_of(cache, L);
                 args.also_seq = seq;
                 args.also_from = std::max(at, at + count - L.ring);
-                // (The keys of the last tile that nobody sees have weight 0, and their values lie where the prompt before this one
-                // left its own, of any sequence and layer: 0 x infinity would be a NaN.)
+                // (The keys of the last tile that nobody sees have weight 0, but their values lie where the prompt before this one
+                // left its own, of any sequence and layer, or nothing was written yet: 0 x infinity would be a NaN.)
                 st = launch_copy_rows(ctx, args.also, seq, view, first_visible_tile(at, p->window) * kTileKeys, at, at + count, d,
                                       stream);
                 if (st != HC_OK) return st;
@@ -858,14 +859,23 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
         const size_t tickets_at = part_ml_at + align(part_ml_floats * sizeof(float));
         const size_t stage_at = tickets_at + align(n_tickets * sizeof(unsigned));
         // Where prompts longer than a ring's margin attend: the window of the first token and a call's tokens, whole key tiles
-        // at both ends.  All ring layers share it.
+        // at both ends (0 rows: no call has more tokens than fit beside the window, or more rows than an int counts).  All ring
+        // layers share it.  A cache that fits without it is one without it: its prompts take the ring in pieces.
         const size_t prompt_at = stage_at + align(2 * cache->stage_bytes);
-        auto prompt_rows = [&](const hc_layer_store& L) { return round_up(L.desc.window + ws.qprep_capacity + 2 * kTileKeys, kTileKeys); };
+        auto prompt_rows = [&](const hc_layer_store& L) -> int {
+            const long long rows = (long long)L.desc.window + ws.qprep_capacity + 3 * kTileKeys - 1;
+            return L.ring == 0 || L.ring - L.desc.window >= ws.qprep_capacity || rows > INT_MAX ? 0 : int(rows) / kTileKeys * kTileKeys;
+        };
         size_t prompt_bytes = 0;
         for (const hc_layer_store& L : cache->layers) {
-            if (L.ring > 0) prompt_bytes = std::max(prompt_bytes, 4 * size_t(L.desc.kv_heads) * prompt_rows(L) * L.desc.head_dim);
+            prompt_bytes = std::max(prompt_bytes, 4 * size_t(L.desc.kv_heads) * prompt_rows(L) * L.desc.head_dim);
         }
         err = cudaMalloc(&cache->workspace_dev, prompt_at + prompt_bytes);
+        if (err != cudaSuccess && prompt_bytes > 0) {
+            cudaGetLastError();
+            prompt_bytes = 0;
+            err = cudaMalloc(&cache->workspace_dev, prompt_at);
+        }
         if (err == cudaSuccess) {
             unsigned char* base = static_cast<unsigned char*>(cache->workspace_dev);
             ws.qprep = reinterpret_cast<uint16_t*>(base);
@@ -874,12 +884,11 @@ hc_status hc_kv_cache_create_paged(hc_context* ctx, const hc_layer_desc* layers,
             ws.tickets = reinterpret_cast<unsigned*>(base + tickets_at);
             cache->stage_dev = base + stage_at;
             err = cudaMemset(ws.tickets, 0, n_tickets * sizeof(unsigned));
-            // Zeros, as the caches: a row no key was written to yet has weight 0 and must not be a NaN.
-            if (err == cudaSuccess && prompt_bytes > 0) err = cudaMemset(base + prompt_at, 0, prompt_bytes);
-            for (size_t i = 0; i < cache->layers.size() && st == HC_OK; ++i) {
+            for (size_t i = 0; prompt_bytes > 0 && i < cache->layers.size() && st == HC_OK; ++i) {
                 hc_layer_store& L = cache->layers[i];
-                if (L.ring == 0) continue;
-                L.prompt = std::make_unique<hc_layer_store>();
+                if (prompt_rows(L) == 0) continue;
+                L.prompt.reset(new (std::nothrow) hc_layer_store());
+                if (!L.prompt) continue;
                 hc_layer_store& P = *L.prompt;
                 P.desc = L.desc;
                 P.ring = P.capacity = prompt_rows(L);

@@ -166,7 +166,8 @@ struct hc_layer_store {
     void* tmap_v = nullptr;
     void* tmap_k64 = nullptr;     // keys in boxes of 64 rows: what a CTA of a pair loads (head_dim 256, 512)
     // A ring holds too little of a prompt beside its window, so a longer one attends in the workspace: a ring of one sequence
-    // with room for the window and a whole call's tokens, used by one call at a time like the rest of the workspace.
+    // with room for the window and a whole call's tokens, used by one call at a time like the rest of the workspace.  Null where
+    // no call is longer than that, or the store did not fit: the prompts take the ring in pieces.
     std::unique_ptr<hc_layer_store> prompt;
 };
 

@@ -275,6 +275,30 @@ def test_prompts_beside_a_ring_see_no_other_prompt(hb, ctx, d, qh, kvh, window, 
         assert np.all(np.isfinite(linear)) and np.array_equal(ring, linear)
 
 
+def test_a_ring_without_room_for_its_prompt_store(hb, ctx):
+    """The ring takes more than half of the free memory, so that the store, as large, does not fit: prompts take the ring in
+    pieces, with the bits of linear storage."""
+    import torch
+    torch.cuda.empty_cache()
+    qh, kvh, d, tokens = 8, 8, 512, 700
+    window = int(0.55 * torch.cuda.mem_get_info()[0]) // (4 * kvh * d) // 128 * 128
+    rng = np.random.default_rng(7)
+    q, k, v = (tl.normal_bf16(rng, (tokens, kvh, d)) for _ in range(3))
+    got, launches = [], []
+    for storage, w in ((hb.capi.HC_STORAGE_RING, window), (hb.capi.HC_STORAGE_RING, 1024), (hb.capi.HC_STORAGE_LINEAR, 1024)):
+        layer = tl.Layer(hb, ctx, qh, kvh, d, 4096, window=w, storage=storage, io="f32", prefill_chunk=128)
+        out = tl.device_empty((tokens, qh, d), "f32")
+        before = ctx.launch_count
+        layer.backend.prefill_chunks(layer.cache, 0, tl.to_device(q, "f32"), tl.to_device(k, "f32"), tl.to_device(v, "f32"), out, tokens,
+                                     0, 128, layer.params)
+        ctx.check()
+        launches.append(ctx.launch_count - before)
+        got.append(tl.to_host(out))
+        layer.close()
+    assert np.array_equal(got[0], got[2]) and np.array_equal(got[1], got[2])
+    assert launches[0] > launches[1]
+
+
 @pytest.mark.parametrize("d, qh, kvh, tokens, window", [(64, 16, 2, 77, 0), (64, 64, 8, 300, 128), (256, 16, 8, 140, 0), (256, 8, 8, 515, 256),
                                                        (512, 8, 1, 65, 0)])
 def test_outputs_on_16_byte_boundaries_that_are_no_32_byte_ones(hb, ctx, d, qh, kvh, tokens, window):
