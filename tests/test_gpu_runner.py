@@ -76,27 +76,36 @@ def test_runner_prefill_forward_verify_and_rewind():
     ctx.close()
 
 
-@pytest.mark.parametrize("tokens", [1, 5, 6, 40])
-def test_hidden_states_in_pinned_and_in_pageable_memory(tokens):
-    """Up to 64 KB of pinned hidden states (five of 2880) are read and written where they are, the rest is copied."""
+@pytest.mark.parametrize("tokens, width", [(1, 2880), (5, 2880), (6, 2880), (40, 2880), (256, 64), (257, 64)])
+def test_hidden_states_in_pinned_and_in_pageable_memory(tokens, width):
+    """Up to 64 KB of pinned hidden states (five of 2880; 256 of 64 to the byte) are read and written where they are, by a
+    launch each; the rest, pageable memory and buffers off a 16-byte boundary are copied."""
+    import ctypes
     import torch
     import hydra_b200 as hb
-    from hydra_b200.runner import AttentionLayerWeights, AttentionStackRunner
+    capi, qh, kvh, d = hb.capi, 8, 2, 64
     ctx = hb.Context(0)
-    rng = np.random.default_rng(tokens)
-    size, qh, kvh, d = 2880, 8, 2, 64
-    w = AttentionLayerWeights(
-        input_norm=np.ones(size), wq=rng.normal(0, 0.02, (qh * d, size)), bq=np.zeros(qh * d), wk=rng.normal(0, 0.02, (kvh * d, size)),
-        bk=np.zeros(kvh * d), wv=rng.normal(0, 0.02, (kvh * d, size)), bv=np.zeros(kvh * d), wo=rng.normal(0, 0.02, (size, qh * d)),
-        bo=np.zeros(size), sinks=np.zeros(qh), window=0, inv_freq=ho.inverse_frequencies(d, 10000.0, d // 2))
-    states = rng.standard_normal((2, tokens, size)).astype(np.float32)
-    got = []
-    for pinned in (True, False):
-        runner = AttentionStackRunner(ctx, [w], size, qh, kvh, d, context_length=256, prefill_chunk_tokens=64)
-        if not pinned:
-            runner._pinned = [torch.empty((64, size)) for _ in range(2)]
-            runner._host = [p.numpy() for p in runner._pinned]
-        got.append([runner.verify(x) for x in states])
-        runner.close()
-    assert all(np.array_equal(a, b) for a, b in zip(*got))
+    lib = capi.load()
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    shapes = dict(input_norm=(width,), wq=(qh * d, width), wk=(kvh * d, width), wv=(kvh * d, width), wo=(width, qh * d))
+    weights = {name: (0.02 * torch.randn(shape, device="cuda", generator=gen)).to(torch.bfloat16) for name, shape in shapes.items()}
+    block = (capi.BlockWeightsStruct * 1)()
+    for name, tensor in weights.items():
+        setattr(block[0], name, tensor.data_ptr())
+    block[0].params = hb.AttnParams(q_heads=qh, kv_heads=kvh, head_dim=d, sm_scale=0.125, io_dtype=capi.HC_BF16).struct()
+    workspace = torch.empty(lib.hc_attention_stack_bytes(block, 1, tokens, width), dtype=torch.uint8, device="cuda")
+    states = torch.from_numpy(np.random.default_rng(tokens).standard_normal((tokens, width)).astype(np.float32))
+    count, got, launches = tokens * width, [], []
+    for pinned, offset in ((False, 0), (True, 0), (True, 1)):
+        cache = hb.KVCache(ctx, [dict(q_heads=qh, kv_heads=kvh, head_dim=d, window=0)], 512, prefill_chunk=512)
+        source, result = (torch.empty(count + offset, pin_memory=pinned)[offset:] for _ in range(2))
+        source.copy_(states.reshape(-1))
+        before = ctx.launch_count
+        assert lib.hc_attention_stack_host(ctx.handle, cache.handle, block, 1, 0, source.data_ptr(), result.data_ptr(), tokens, width, 0,
+                                           ctypes.c_float(1e-5), workspace.data_ptr(), None) == capi.HC_OK
+        launches.append(ctx.launch_count - before)
+        got.append(result.numpy().copy())
+        cache.close()
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+    assert launches[1] - launches[0] == (2 if 4 * count <= 65536 else 0) and launches[2] == launches[0]
     ctx.close()
