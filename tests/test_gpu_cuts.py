@@ -191,11 +191,17 @@ def test_stack_call_equals_its_parts(hb, ctx, tokens):
     (128, 16, 2, 300, 640, 1290, "bf16", True),
     (256, 16, 8, 256, 77, 1500, "bf16", False),
     (256, 64, 4, 384, 515, 2300, "f32", False),  # more than the prepared queries have room for: two parts
+    (256, 64, 4, 384, 515, 2300, "bf16", "separate"),     # a gate of its own, which the parts are given their rows of
+    (64, 16, 4, 128, 131, 700, "f32", "separate"),
+    (256, 16, 8, 256, 77, 1500, "bf16", "norms"),         # queries, keys and values normed
+    (96, 8, 4, 130, 259, 600, "f32", "norms"),
 ])
 def test_prompts_longer_than_a_ring_equal_linear_storage(hb, ctx, d, qh, kvh, window, first, tokens, io, gated):
     """Outputs, the ring's rows and a decoded token behind them: the same bits as with linear storage, twice in a row."""
     rng = np.random.default_rng(d + window + tokens)
-    end, width = first + tokens, d * (2 if gated else 1)
+    end, width = first + tokens, d * (2 if gated is True else 1)
+    gate = tl.to_device(tl.normal_bf16(rng, (tokens + 1, qh, d)), io) if gated == "separate" else None
+    norms = dict(q_norm=1 + 0.1 * tl.normal_bf16(rng, (d,)), k_norm=1 + 0.1 * tl.normal_bf16(rng, (d,)), norm_v=True) if gated == "norms" else {}
     k, v = tl.normal_bf16(rng, (end + 1, kvh, d)), tl.normal_bf16(rng, (end + 1, kvh, d))
     q = tl.normal_bf16(rng, (tokens + 1, qh, width))
     sinks = tl.normal_bf16(rng, (qh,))
@@ -203,7 +209,10 @@ def test_prompts_longer_than_a_ring_equal_linear_storage(hb, ctx, d, qh, kvh, wi
     got = []
     for storage in (hb.capi.HC_STORAGE_RING, hb.capi.HC_STORAGE_LINEAR):
         layer = tl.Layer(hb, ctx, qh, kvh, d, 4096, window=window, sinks=sinks, rope_inv_freq=inv, io=io, prefill_chunk=128,
-                         storage=storage, gate_layout=hb.capi.HC_GATE_INTERLEAVED if gated else 0, max_seqs=2)
+                         storage=storage, gate_layout=hb.capi.HC_GATE_INTERLEAVED if gated is True else 0, max_seqs=2, **norms)
+        prompt_params = decode_params = layer.params
+        if gate is not None:
+            prompt_params, decode_params = layer._with_gate(gate), layer._with_gate(gate[tokens:])
         dev = [tl.to_device(x, io) for x in (q, k, v)]
         out = tl.device_empty((tokens + 1, qh, d), io)
         for seq in (1, 1, 0):
@@ -211,8 +220,8 @@ def test_prompts_longer_than_a_ring_equal_linear_storage(hb, ctx, d, qh, kvh, wi
                 layer.append(k[at:min(at + 128, first)], v[at:min(at + 128, first)], at, seq=seq)
             out.fill_(7.0)
             layer.backend.prefill_chunks(layer.cache, 0, dev[0], dev[1][first:], dev[2][first:], out, tokens, first, 128,
-                                         layer.params, seq=seq)
-            layer.backend.layer_step(layer.cache, 0, dev[0][tokens:], dev[1][end:], dev[2][end:], out[tokens:], 1, end, layer.params,
+                                         prompt_params, seq=seq)
+            layer.backend.layer_step(layer.cache, 0, dev[0][tokens:], dev[1][end:], dev[2][end:], out[tokens:], 1, end, decode_params,
                                      seq=seq)
         ctx.check()
         held = min(end + 1, window + 128)

@@ -443,6 +443,8 @@ def test_a_stack_call_that_cannot_run_queues_nothing(hb, ctx):
     (64, 16, 2, 0, 128, 512, False, "bf16"), (64, 16, 2, 200, 96, 96, False, "f32"), (64, 8, 8, 128, 128, 64, True, "bf16"),
     (128, 8, 2, 0, 100, 512, False, "bf16"), (256, 16, 8, 300, 128, 128, True, "bf16"), (512, 8, 1, 0, 77, 200, False, "f32"),
     (256, 4, 4, 0, 300, 128, False, "bf16"), (96, 4, 2, 0, 60, 512, False, "bf16"),
+    # (beside the ring, whose pieces bf16 queries as they come take)
+    (64, 8, 8, 128, 128, 64, True, "f32"), (256, 16, 8, 300, 128, 128, True, "f32"), (96, 4, 2, 130, 64, 64, True, "f32"),
 ])
 def test_blocks_of_a_prompt_end_with_their_chunks(hb, ctx, d, qh, kvh, window, chunk, cache_chunk, ring, io):
     """A prompt with bidirectional blocks in one call: the bits of the chunk-by-chunk calls, whichever chunk boundaries cut
