@@ -626,9 +626,10 @@ hc_status launch_prepare(hc_context* ctx, const PrepArgs& args, cudaStream_t str
         const long long groups = groups_of(512 / d);
         // (A warp stays with its heads, so there are never fewer warps than a token has groups of them.)
         const int grid = int((std::max(std::min(args.tokens * groups, sms * prep_blocks(fp32) * kPrepWarps), groups) + kPrepWarps - 1) / kPrepWarps);
-        // Prefetched bf16 rows are 90 us -> 55 (above).  Of fp32 rows a warp has enough on its way without (8000 x 64 x 256 146 us
-        // with, 130 without; in place 47.5 and 43), but for those in place that L2 keeps (2000 x 16 x 256 12.4 with, 13.4 without).
-        const int prefetch = !fp32 || (args.job[0].kind == 3 && !large) ? 1 : 0;
+        // Prefetched bf16 rows are 64 us -> 55 (above).  Of fp32 rows a warp has enough on its way without (appends of 8000 x 64 x 256
+        // 146 us with, 130 without, of 1000 x 64 x 256 15.7 and 14.7; in place 8000 x 16 x 256 47.5 and 43.2), but for queries and
+        // rows in place that L2 keeps (2000 x 16 x 256 in place 12.4 with, 13.4 without; a prompt of 777 gated tokens 58.7 and 59).
+        const int prefetch = !fp32 || (args.job[0].kind != 1 && !large) ? 1 : 0;
         auto kernel = d == 64 ? (fp32 ? prepare_heads_vec_kernel<64, true> : prepare_heads_vec_kernel<64, false>)
                     : d == 128 ? (fp32 ? prepare_heads_vec_kernel<128, true> : prepare_heads_vec_kernel<128, false>)
                     : d == 256 ? (fp32 ? prepare_heads_vec_kernel<256, true> : prepare_heads_vec_kernel<256, false>)
