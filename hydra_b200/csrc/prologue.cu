@@ -165,7 +165,7 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads, int prefetch) {
     for (;;) {
         const bool more = token + step < unsigned(args.tokens);
         if (more) ahead.load(src + src_step, m);
-        if (prefetch && token + 3 * step < unsigned(args.tokens)) {              // two further on their way into L2
+        if ((!F32 || prefetch) && token + 3 * step < unsigned(args.tokens)) {              // two further on their way into L2
             #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(src + 3 * src_step + (h * (D / 2) + WL::at(m, 0)) * kBytes));
@@ -183,18 +183,22 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads, int prefetch) {
                 s[4 * u] = sv.x; s[4 * u + 1] = sv.y; s[4 * u + 2] = sv.z; s[4 * u + 3] = sv.w;
             }
         }
-        // Where to, while the loads are on their way.
+        // Where to: of fp32 rows while the loads are on their way (1000 x 16 x 256 in place 6.1 us behind the sums, so 5.8), of bf16
+        // ones behind the sums (ahead of them they spill: 4000 x 64 x 256 56.3 us, so 53.4).
         uint16_t* to = dst;
         bool active = in_range;
-        if (counted) {
-            to = dst + size_t(row) * D;
-            row += row_step;
-            if (map.ring > 0 && row >= map.ring) row -= map.ring;
-        } else if (cached) {
-            active = active && row_is_local(map, position);           // else another rank's tile
-            const int seq = args.batched ? args.meta.seq[token] : args.seq;
-            if (active) to = dst + (size_t(cache_plane(map, seq, args.cache.kv_heads, head)) * args.cache.capacity + cache_row(map, seq, position)) * D;
-        }
+        auto where_to = [&]() {
+            if (counted) {
+                to = dst + size_t(row) * D;
+                row += row_step;
+                if (map.ring > 0 && row >= map.ring) row -= map.ring;
+            } else if (cached) {
+                active = active && row_is_local(map, position);           // else another rank's tile
+                const int seq = args.batched ? args.meta.seq[token] : args.seq;
+                if (active) to = dst + (size_t(cache_plane(map, seq, args.cache.kv_heads, head)) * args.cache.capacity + cache_row(map, seq, position)) * D;
+            }
+        };
+        if constexpr (F32) where_to();
         float lo[8], hi[8];
         now.unpack(0, lo);
         now.unpack(1, hi);
@@ -239,6 +243,7 @@ prepare_heads_vec_kernel(const PrepArgs args, int total_heads, int prefetch) {
                 hi[i] = __fmaf_rn(b, c[i], __fmul_rn(a, s[i]));
             }
         }
+        if constexpr (!F32) where_to();
         if (active) {
             if (kind == 3 && F32) {
                 if (WL::kContiguous && by32) {               // (by halves of them 2000 x 16 x 256 take 12.5 us, so 8.4)
