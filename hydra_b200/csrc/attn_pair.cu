@@ -412,9 +412,9 @@ attention_pair_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_c
                         a[0] = add2(a[0], a[1]);
                         return __fadd_rn(__uint_as_float(uint32_t(a[0])), __uint_as_float(uint32_t(a[0] >> 32)));
                     };
-                    // A tile's time here is what one of prompts too short for the power limit takes (777 gated tokens behind 1291 59 us, now 55), so
-                    // as little as may be stands in a row: the second 32 columns stay in the registers between the
-                    // passes, the first ones come back behind the sums of the others, and their own sum follows P.
+                    // A tile's time here is what one of prompts too short for the power limit takes, so as little as may be stands in a
+                    // row: the second 32 columns stay in the registers between the passes, the first ones come back behind the sums
+                    // of the others, and their own sum follows P (777 tokens behind 1291, 16 heads of 256: the launch 43.0 us, now 39.3).
                     uint32_t s[32], packed[16];
                     HC_TMEM_LD32(s_tmem, s);
                     tc_wait_ld();

@@ -35,8 +35,8 @@ __device__ __forceinline__ uint16_t* also_row(const PrepArgs& args, int kind, in
 // are worked on.  What bounds it is its instructions, so a lane owns sixteen elements (8 m .. 8 m + 7 of each half, 16-byte
 // accesses; head_dim 512 as in HeadLanes): a warp has two vectors of 256 at a time, and reduces, and takes the root and the
 // addresses, once for both (8192 tokens of 32 x 256 with norms and rotation: 90 us with a vector a warp, a division by
-// head_dim and a remainder per cached row, 64 without the prefetch into L2, now 55).  The bits are HeadLanes' and prepare_head's: a lane keeps the sums of two of
-// their lanes apart until the last step of the butterfly.
+// head_dim and a remainder per cached row, 64 without the prefetch into L2, now 55).  The bits are HeadLanes' and
+// prepare_head's: a lane keeps the sums of two of their lanes apart until the last step of the butterfly.
 // The launcher checks the alignment this needs and otherwise uses the general kernel below.
 template <int D>
 struct WideLanes {

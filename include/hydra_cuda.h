@@ -490,7 +490,8 @@ HC_API hc_status hc_layer_step(hc_context* ctx, hc_kv_cache* cache, int layer, i
  * are told: the library takes as many tokens at a time as its workspace holds (64 MB of prepared
  * queries): usually one prologue and one attention launch.  On a ring the keys and values of more tokens than
  * fit beside the window lie in the workspace meanwhile, and the ring gets the last of them (bf16 queries that are attended as
- * they come, without norm, rotation or an interleaved gate, take the ring in pieces). */
+ * they come, without norm, rotation or an interleaved gate, take the ring in pieces, and so do all where the device had no room
+ * for that part of the workspace when the cache was created). */
 HC_API hc_status hc_prefill_chunks(hc_context* ctx, hc_kv_cache* cache, int layer, int seq,
                                    const void* q, const void* k, const void* v, void* out,
                                    int tokens, int first_position, int chunk,
